@@ -7,9 +7,12 @@ Python or CPU fallback for any operator.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libsparsewave_b200.so"
+BINDING_PATH = LIB_PATH.with_name("swb_torch.so")
 
 SWB_OK = 0
 SWB_ERR_INVALID_OPTION = -1
@@ -124,6 +127,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_binding = None
 
 
 def load() -> C.CDLL:
@@ -142,3 +146,20 @@ def load() -> C.CDLL:
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+def binding(error_type):
+    """The extension module with the device-tensor operator calls (csrc/binding); `error_type` is what it raises for a
+    non-zero status."""
+    global _binding
+    if _binding is None:
+        load()
+        import torch  # noqa: F401  (its libraries must be in the process first)
+        if not BINDING_PATH.exists():
+            raise RuntimeError(f"{BINDING_PATH} is missing: build it with `python -m sparsewave_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("swb_torch", str(BINDING_PATH))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("swb_torch", loader))
+        loader.exec_module(module)
+        module.bind(error_type, SwbOptions)
+        _binding = module
+    return _binding

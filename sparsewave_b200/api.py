@@ -12,6 +12,7 @@ call goes to libsparsewave_b200.so.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from typing import Optional
 
 import numpy as np
@@ -45,6 +46,10 @@ def make_options(text: str = "", **fields) -> SwbOptions:
     return o
 
 
+# Parsed texts of the calls below, which only read the block (make_options returns a fresh one).
+_parsed_options = functools.lru_cache(maxsize=256)(make_options)
+
+
 def _dev_ptr(t: Optional[torch.Tensor], dtype: torch.dtype, name: str) -> Optional[int]:
     if t is None:
         return None
@@ -76,6 +81,7 @@ class Context:
 
     def __init__(self, device: int = 0):
         self._lib = _lib.load()
+        self._fast = _lib.binding(SparseWaveError)
         self._ctx = C.c_void_p()
         st = self._lib.swb_create(C.byref(self._ctx), int(device))
         if st != 0:
@@ -109,7 +115,7 @@ class Context:
     def _opts(options) -> SwbOptions:
         if isinstance(options, SwbOptions):
             return options
-        return make_options(options or "")
+        return _parsed_options(options or "")
 
     def _stream(self) -> int:
         return torch.cuda.current_stream(self.device).cuda_stream
@@ -212,17 +218,7 @@ class Context:
     # -- operators on device tensors ---------------------------------------------
     def spmv(self, options, row_ptr, col_idx, val, x, y=None, *, rows=None):
         """y = A @ x for CSR A; returns y (allocated when not given)."""
-        rows = int(row_ptr.numel() - 1 if rows is None else rows)
-        cols, nnz = int(x.numel()), int(val.numel())
-        if y is None:
-            y = torch.empty(rows, dtype=torch.float32, device=x.device)
-        o = self._opts(options)
-        self._check(self._lib.swb_spmv(
-            self._ctx, C.byref(o), rows, cols, nnz,
-            _dev_ptr(row_ptr, torch.int32, "row_ptr"), _dev_ptr(col_idx, torch.int32, "col_idx"),
-            _dev_ptr(val, torch.float32, "val"), _dev_ptr(x, torch.float32, "x"),
-            _dev_ptr(y, torch.float32, "y"), self._stream()))
-        return y
+        return self._fast.spmv(self._ctx.value, self.device, options, row_ptr, col_idx, val, x, y, rows)
 
     def spmv_sharded(self, options, row_ptr, col_idx, val, x_owned, cols: int, y=None, *, rows=None):
         """Row shard of y = A @ x: gathers every rank's chunk of x (this rank's is `x_owned`), then runs the
@@ -264,15 +260,7 @@ class Context:
 
     def coo_spmv(self, options, rows: int, row_idx, col_idx, val, x, y=None):
         """y = A @ x for COO A (entries in any order, duplicates accumulate)."""
-        cols, nnz = int(x.numel()), int(val.numel())
-        if y is None:
-            y = torch.empty(rows, dtype=torch.float32, device=x.device)
-        o = self._opts(options)
-        self._check(self._lib.swb_coo_spmv(
-            self._ctx, C.byref(o), int(rows), cols, nnz, _dev_ptr(row_idx, torch.int32, "row_idx"),
-            _dev_ptr(col_idx, torch.int32, "col_idx"), _dev_ptr(val, torch.float32, "val"),
-            _dev_ptr(x, torch.float32, "x"), _dev_ptr(y, torch.float32, "y"), self._stream()))
-        return y
+        return self._fast.coo_spmv(self._ctx.value, self.device, options, rows, row_idx, col_idx, val, x, y)
 
     def spmv_position_trace(self, options, row_ptr, col_idx, val, x):
         """Position-mapped SpMV that also returns (row, worker, segment_end) per position."""
@@ -290,40 +278,12 @@ class Context:
 
     def spmm(self, options, row_ptr, col_idx, val, B, C_out=None, *, rows=None):
         """C = A @ B for CSR A and row-major dense B (cols x N)."""
-        rows = int(row_ptr.numel() - 1 if rows is None else rows)
-        cols, n_rhs, nnz = int(B.shape[0]), int(B.shape[1]), int(val.numel())
-        if C_out is None:
-            C_out = torch.empty((rows, n_rhs), dtype=torch.float32, device=B.device)
-        o = self._opts(options)
-        self._check(self._lib.swb_spmm(
-            self._ctx, C.byref(o), rows, cols, nnz, n_rhs,
-            _dev_ptr(row_ptr, torch.int32, "row_ptr"), _dev_ptr(col_idx, torch.int32, "col_idx"),
-            _dev_ptr(val, torch.float32, "val"), _dev_ptr(B, torch.float32, "B"),
-            _dev_ptr(C_out, torch.float32, "C"), self._stream()))
-        return C_out
+        return self._fast.spmm(self._ctx.value, self.device, options, row_ptr, col_idx, val, B, C_out, rows)
 
     def bsr_spmm(self, options, block_row_ptr, block_col_idx, block_values, B, block_size: int, C_out=None):
         """C = A @ B for BSR A; f32 or bf16 chosen by the dtype of block_values."""
-        brows = int(block_row_ptr.numel() - 1)
-        rows, cols, n_rhs = brows * block_size, int(B.shape[0]), int(B.shape[1])
-        nnzb = int(block_col_idx.numel())
-        dt = block_values.dtype
-        if dt not in (torch.float32, torch.bfloat16):
-            raise TypeError("block_values must be float32 or bfloat16")
-        if int(block_values.numel()) != nnzb * block_size * block_size:
-            raise SparseWaveError(_lib.SWB_ERR_INVALID_SHAPE,
-                                  "block values size must equal the number of blocks times block_size squared, "
-                                  f"but got {int(block_values.numel())} and {nnzb} blocks")
-        if C_out is None:
-            C_out = torch.empty((rows, n_rhs), dtype=dt, device=B.device)
-        fn = self._lib.swb_bsr_spmm_f32 if dt == torch.float32 else self._lib.swb_bsr_spmm_bf16
-        o = self._opts(options)
-        self._check(fn(self._ctx, C.byref(o), rows, cols, nnzb, block_size, n_rhs,
-                       _dev_ptr(block_row_ptr, torch.int32, "block_row_ptr"),
-                       _dev_ptr(block_col_idx, torch.int32, "block_col_idx"),
-                       _dev_ptr(block_values, dt, "block_values"), _dev_ptr(B, dt, "B"),
-                       _dev_ptr(C_out, dt, "C"), self._stream()))
-        return C_out
+        return self._fast.bsr_spmm(self._ctx.value, self.device, options, block_row_ptr, block_col_idx, block_values, B,
+                                   block_size, C_out)
 
     def bundle_launch(self, operation: str, n: int, args) -> None:
         """lrrt-style launch: five device pointers (rowOffsets, columnIndices, values, rhs, output)."""

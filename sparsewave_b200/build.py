@@ -11,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -79,6 +80,7 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> Path:
         os.replace(fresh, LIB)
     build_runner(verbose)
     build_loaders(verbose)
+    build_binding(verbose)
     return LIB
 
 
@@ -114,6 +116,31 @@ def build_loaders(verbose: bool = False) -> Path:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
     return LOADERS
+
+
+BINDING_SRC = CSRC / "binding" / "swb_torch_binding.cpp"
+BINDING = LIBDIR / "swb_torch.so"
+
+
+def build_binding(verbose: bool = False) -> Path:
+    """CPython extension over torch tensors and the C ABI (g++; host code only): the operator calls of api.Context."""
+    if _stale(BINDING, [BINDING_SRC, ROOT / "include" / "sparsewave_b200.h", Path(__file__)]):
+        import torch
+        torch_dir = Path(torch.__file__).resolve().parent
+        cuda = Path(_nvcc()).resolve().parent.parent
+        fresh = BINDING.with_suffix(".so.new")
+        cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               "-isystem", str(torch_dir / "include"), "-isystem", str(torch_dir / "include/torch/csrc/api/include"),
+               "-isystem", str(cuda / "include"), "-isystem", sysconfig.get_paths()["include"],
+               str(BINDING_SRC), "-o", str(fresh), "-L", str(LIBDIR), "-lsparsewave_b200",
+               "-L", str(torch_dir / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10",
+               "-Wl,-rpath,$ORIGIN"]  # torch's libraries are loaded by `import torch` before the module is
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        subprocess.run(cmd, check=True)
+        os.replace(fresh, BINDING)
+    return BINDING
 
 
 if __name__ == "__main__":
