@@ -86,36 +86,10 @@ __global__ void fill_zero_kernel(float *__restrict__ y, int64_t n) {
 }
 
 // ---------------------------------------------------------------------------
-// thread-per-row (ThreadPerRowSpMVPattern, SparseWaveToGPU.cpp:216-274)
-// row = blockIdx * blockDim + threadIdx; sequential sum from 0.0f in position
-// order; plain store.
+// thread-per-row (ThreadPerRowSpMVPattern, SparseWaveToGPU.cpp:216-274): sequential sum from 0.0f in position order;
+// plain store.
 // ---------------------------------------------------------------------------
-__global__ void spmv_thread_per_row_kernel(int64_t rows,
-                                           const int32_t *__restrict__ row_ptr,
-                                           const int32_t *__restrict__ col,
-                                           const float *__restrict__ val,
-                                           const float *__restrict__ x,
-                                           float *__restrict__ y) {
-  int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= rows) return;
-  int p = row_ptr[row];
-  const int end = row_ptr[row + 1];
-  float sum = 0.0f;
-  // Four independent (col, val, x) loads in flight, summed in position order.
-  for (; p + 4 <= end; p += 4) {
-    int c0 = ld_stream(col + p), c1 = ld_stream(col + p + 1);
-    int c2 = ld_stream(col + p + 2), c3 = ld_stream(col + p + 3);
-    float v0 = ld_stream(val + p), v1 = ld_stream(val + p + 1);
-    float v2 = ld_stream(val + p + 2), v3 = ld_stream(val + p + 3);
-    float x0 = __ldg(x + c0), x1 = __ldg(x + c1), x2 = __ldg(x + c2), x3 = __ldg(x + c3);
-    sum = add(sum, mul(v0, x0));
-    sum = add(sum, mul(v1, x1));
-    sum = add(sum, mul(v2, x2));
-    sum = add(sum, mul(v3, x3));
-  }
-  for (; p < end; ++p) sum = add(sum, mul(ld_stream(val + p), __ldg(x + ld_stream(col + p))));
-  y[row] = sum;
-}
+#include "row_products.cuh"
 
 // Partial sum of positions [start, end) taken by participant `who` of `count`
 // participants with stride `count`.  Rows of at least VEC_MIN positions use
@@ -712,12 +686,24 @@ cudaError_t launch_coo_spmv_thread_per_nonzero(int64_t rows, int64_t nnz, const 
   return cudaGetLastError();
 }
 
-cudaError_t launch_spmv_thread_per_row(const CsrSpmvArgs &a, int block, cudaStream_t s,
-                                       int64_t *launches) {
-  spmv_thread_per_row_kernel<<<grid_of(ceil_div(a.rows, block)), block, 0, s>>>(
-      a.rows, a.row_ptr, a.col_idx, a.val, a.x, a.y);
+cudaError_t launch_row_products(const CsrSpmmArgs &a, cudaStream_t s) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(a.B);
+  switch (a.n_rhs) {
+    case 1: return launch_row_products_of<1, true>(a, s);
+    case 2: return at % 8 == 0 ? launch_row_products_of<2, true>(a, s) : launch_row_products_of<2, false>(a, s);
+    case 3: return launch_row_products_of<3, false>(a, s);
+    case 4: return at % 16 == 0 ? launch_row_products_of<4, true>(a, s) : launch_row_products_of<4, false>(a, s);
+  }
+  return cudaErrorInvalidValue;
+}
+
+int64_t row_products_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs) {
+  return max1(ceil_div(rows, product_rows_per_block(rows, nnz, n_rhs)));
+}
+
+cudaError_t launch_spmv_thread_per_row(const CsrSpmvArgs &a, cudaStream_t s, int64_t *launches) {
   ++*launches;
-  return cudaGetLastError();
+  return launch_row_products({a.rows, a.cols, a.nnz, 1, a.row_ptr, a.col_idx, a.val, a.x, a.y}, s);
 }
 
 cudaError_t launch_spmv_wave_per_row(const CsrSpmvArgs &a, int block, cudaStream_t s,

@@ -488,7 +488,7 @@ int swb_launch_shape_query(swb_context *ctx, const swb_options *o, int64_t rows,
       case SWB_THREAD_PER_ROW:
         r.work_units = rows;
         r.logical_grid = max1(ceil_div(rows, B));
-        r.physical_grid = r.logical_grid;
+        r.physical_grid = swb::row_products_physical_grid(rows, nnz, 1);
         break;
       case SWB_WAVE_PER_ROW:
         r.work_units = rows;
@@ -574,7 +574,7 @@ static int spmv_impl(swb_context *ctx, const swb_options *o, int64_t rows, int64
   const int B = (int)o->block_size;
   cudaError_t e = cudaSuccess;
   switch (o->mapping) {
-    case SWB_THREAD_PER_ROW: e = swb::launch_spmv_thread_per_row(a, B, stream, &ctx->launches); break;
+    case SWB_THREAD_PER_ROW: e = swb::launch_spmv_thread_per_row(a, stream, &ctx->launches); break;
     case SWB_WAVE_PER_ROW: e = swb::launch_spmv_wave_per_row(a, B, stream, &ctx->launches); break;
     case SWB_BLOCK_PER_ROW: e = swb::launch_spmv_block_per_row(a, B, stream, &ctx->launches); break;
     case SWB_THREAD_PER_POSITION:

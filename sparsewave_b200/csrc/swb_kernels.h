@@ -69,8 +69,10 @@ cudaError_t launch_coo_spmv_thread_per_nonzero(int64_t rows, int64_t nnz, const 
                                                cudaStream_t s, int64_t *launches);
 
 // --- SpMV row mappings
-cudaError_t launch_spmv_thread_per_row(const CsrSpmvArgs &a, int block,
-                                       cudaStream_t s, int64_t *launches);
+cudaError_t launch_spmv_thread_per_row(const CsrSpmvArgs &a, cudaStream_t s, int64_t *launches);
+// Sequential row sums for n_rhs = 1 to 4 (row_products.cuh); also SpMM.
+cudaError_t launch_row_products(const CsrSpmmArgs &a, cudaStream_t s);
+int64_t row_products_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs);
 cudaError_t launch_spmv_wave_per_row(const CsrSpmvArgs &a, int block,
                                      cudaStream_t s, int64_t *launches);
 cudaError_t launch_spmv_block_per_row(const CsrSpmvArgs &a, int block,
