@@ -10,23 +10,36 @@
 // gather of x on large ones: 206,501 rows of 6 on average 13.0 -> 9.6 us, 1 M rows of 32 289 -> 139 us (32 M gathers
 // at 230 G/s), 50,000 power-law rows of up to 25,000 positions 1163 -> 140 us.
 //
-// The tile is padded by one word in 32, so that rows of 32 or 64 positions do not start in one bank.
+// N = 1, 2, 4, 8 on aligned rows of B: a thread forms the products of a position, with one or two vector loads.  Other N
+// up to 8: a thread forms one product, so that neighbouring lanes read a row of B together.
+//
+// The tile is padded by one element (of 4, 8 or 16 bytes) in 32, so that rows of 32 or 64 positions do not start in one
+// bank.
 #pragma once
 
 constexpr int PRODUCT_THREADS = 256;
 constexpr int PRODUCT_WORDS = 4096;  // products of a tile, before padding
 
-__device__ __forceinline__ int padded(int i) { return i + (i >> 5); }
+template <int W> struct Words;  // what one load brings
+template <> struct Words<1> { using T = float; };
+template <> struct Words<2> { using T = float2; };
+template <> struct Words<4> { using T = float4; };
 
-// N right-hand sides; VEC: a row of B is aligned to its size and is read with one load (N = 1, 2, 4).
-template <int N, bool VEC>
+// N right-hand sides; W words per load: N (8 takes two loads of 4), or 1 for the thread-per-product form.
+template <int N, int W>
 __global__ void __launch_bounds__(PRODUCT_THREADS)
     row_products_kernel(int64_t rows, int rows_per_block, const int32_t *__restrict__ row_ptr,
                         const int32_t *__restrict__ col, const float *__restrict__ val, const float *__restrict__ B,
                         float *__restrict__ C, bool accumulate) {
-  constexpr int TILE = PRODUCT_WORDS / N;  // positions
-  constexpr int PER = N <= 2 ? 4 : 2;      // positions in flight per thread
-  __shared__ float products[PRODUCT_WORDS + PRODUCT_WORDS / 32];
+  using T = typename Words<W>::T;
+  constexpr int TILE = PRODUCT_WORDS / N;     // positions
+  constexpr bool BY_PRODUCT = W == 1;         // items are products, else positions
+  constexpr int ITEMS = BY_PRODUCT ? N : 1;   // items per position
+  constexpr int LOADS = BY_PRODUCT ? 1 : N / W;
+  constexpr int PER = LOADS * W >= 8 ? 2 : 4; // items in flight per thread
+  constexpr int UNITS = PRODUCT_WORDS / W;    // the tile in units of one load
+  __shared__ T tile_mem[UNITS + UNITS / 32];
+  const float *products = reinterpret_cast<const float *>(tile_mem);
   __shared__ int offsets[PRODUCT_THREADS + 1];
   const int tid = threadIdx.x;
   const int64_t r0 = (int64_t)blockIdx.x * rows_per_block;
@@ -35,48 +48,48 @@ __global__ void __launch_bounds__(PRODUCT_THREADS)
   for (int i = tid; i <= count; i += PRODUCT_THREADS) offsets[i] = row_ptr[r0 + i];
   __syncthreads();
   const int first = offsets[0], last = offsets[count];
-  // outputs of this thread: (row, column) pairs tid, tid + PRODUCT_THREADS, ... (rows_per_block <= PRODUCT_THREADS)
-  float sum[N];
+  float sum[N];  // of outputs tid, tid + PRODUCT_THREADS, ... (rows_per_block <= PRODUCT_THREADS)
 #pragma unroll
   for (int k = 0; k < N; ++k) sum[k] = 0.0f;
   for (int tile = first; tile < last; tile += TILE) {
-    const int stop = last - tile < TILE ? last : tile + TILE;
-    for (int p0 = tile + tid; p0 < stop; p0 += PER * PRODUCT_THREADS) {
+    const int items = (last - tile < TILE ? last - tile : TILE) * ITEMS;
+    for (int i0 = tid; i0 < items; i0 += PER * PRODUCT_THREADS) {
       int c[PER];
       float v[PER];
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
-        const int p = p0 + k * PRODUCT_THREADS;
-        c[k] = p < stop ? ld_stream(col + p) : 0;
-        v[k] = p < stop ? ld_stream(val + p) : 0.0f;
+        const int i = i0 + k * PRODUCT_THREADS, p = tile + i / ITEMS;
+        c[k] = i < items ? ld_stream(col + p) : 0;
+        v[k] = i < items ? ld_stream(val + p) : 0.0f;
       }
-      float b[PER][N];
+      T b[PER][LOADS];
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
-        if (p0 + k * PRODUCT_THREADS < stop) {
-          const float *src = B + (int64_t)c[k] * N;
-          if constexpr (N == 4 && VEC) {
-            const float4 t = __ldg(reinterpret_cast<const float4 *>(src));
-            b[k][0] = t.x; b[k][1] = t.y; b[k][2] = t.z; b[k][3] = t.w;
-          } else if constexpr (N == 2 && VEC) {
-            const float2 t = __ldg(reinterpret_cast<const float2 *>(src));
-            b[k][0] = t.x; b[k][1] = t.y;
-          } else {
+        const int i = i0 + k * PRODUCT_THREADS;
+        if (i < items) {
+          const T *src = reinterpret_cast<const T *>(B + (int64_t)c[k] * N + (BY_PRODUCT ? i % ITEMS : 0));
 #pragma unroll
-            for (int j = 0; j < N; ++j) b[k][j] = __ldg(src + j);
-          }
+          for (int j = 0; j < LOADS; ++j) b[k][j] = __ldg(src + j);
         }
       }
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
-        const int p = p0 + k * PRODUCT_THREADS;
-        if (p < stop) {
+        const int i = i0 + k * PRODUCT_THREADS;
+        if (i < items) {
 #pragma unroll
-          for (int j = 0; j < N; ++j) products[padded((p - tile) * N + j)] = mul(v[k], b[k][j]);
+          for (int j = 0; j < LOADS; ++j) {
+            T w = b[k][j];
+            float *f = reinterpret_cast<float *>(&w);
+#pragma unroll
+            for (int e = 0; e < W; ++e) f[e] = mul(v[k], f[e]);
+            const int unit = i * LOADS + j;
+            tile_mem[unit + (unit >> 5)] = w;
+          }
         }
       }
     }
     __syncthreads();
+    auto product = [&](int word) { return products[word + (word / (32 * W)) * W]; };
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       const int o = tid + k * PRODUCT_THREADS;
@@ -87,11 +100,11 @@ __global__ void __launch_bounds__(PRODUCT_THREADS)
         if (end > TILE) end = TILE;
         float s = sum[k];
         for (; p + 4 <= end; p += 4) {
-          const float a0 = products[padded(p * N + j)], a1 = products[padded((p + 1) * N + j)];
-          const float a2 = products[padded((p + 2) * N + j)], a3 = products[padded((p + 3) * N + j)];
+          const float a0 = product(p * N + j), a1 = product((p + 1) * N + j);
+          const float a2 = product((p + 2) * N + j), a3 = product((p + 3) * N + j);
           s = add(add(add(add(s, a0), a1), a2), a3);
         }
-        for (; p < end; ++p) s = add(s, products[padded(p * N + j)]);
+        for (; p < end; ++p) s = add(s, product(p * N + j));
         sum[k] = s;
       }
     }
@@ -107,23 +120,23 @@ __global__ void __launch_bounds__(PRODUCT_THREADS)
   }
 }
 
-// Rows per block: as many as fill a tile, but no fewer blocks than four per SM while a block keeps a row for every lane
-// of a warp (below that the sums, one thread per row, run on part of a warp).
+// Rows per block: as many as fill a tile, but no fewer blocks than four per SM while a block keeps 16 rows (the sums
+// take one thread per row and column).
 inline int64_t product_rows_per_block(int64_t rows, int64_t nnz, int64_t n_rhs) {
   const int64_t mean = rows > 0 ? nnz / rows : 0;
   int64_t per = PRODUCT_WORDS / n_rhs * 7 / 8 / (mean > 0 ? mean : 1);
   const int64_t spread = ceil_div(rows, 148 * 4);
   if (per > spread) per = spread;
-  if (per < 32) per = 32;
+  if (per < 16) per = 16;
   return per > PRODUCT_THREADS ? PRODUCT_THREADS : per;
 }
 
-template <int N, bool VEC>
+template <int N, int W>
 cudaError_t launch_row_products_of(const CsrSpmmArgs &a, cudaStream_t s) {
   const int64_t per = product_rows_per_block(a.rows, a.nnz, N);
   unsigned grid = 0;
   if (!grid_dim(ceil_div(a.rows, per), &grid)) return cudaErrorInvalidConfiguration;
-  row_products_kernel<N, VEC><<<grid, PRODUCT_THREADS, 0, s>>>(a.rows, (int)per, a.row_ptr, a.col_idx, a.val, a.B, a.C,
+  row_products_kernel<N, W><<<grid, PRODUCT_THREADS, 0, s>>>(a.rows, (int)per, a.row_ptr, a.col_idx, a.val, a.B, a.C,
                                                               a.accumulate);
   return cudaGetLastError();
 }

@@ -12,74 +12,10 @@ constexpr unsigned FULL = 0xffffffffu;
 __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
 
-// ---------------------------------------------------------------------------
-// thread-per-output (ThreadPerOutputSpMMPattern, SparseWaveToGPU.cpp:489-558)
-// element = blockIdx * blockDim + threadIdx; row = element / N; column =
-// element % N; sequential sum in position order (bit-identical to the CPU
-// CSR loop).
-// ---------------------------------------------------------------------------
-__global__ void spmm_thread_per_output_kernel(int64_t rows, int64_t N,
-                                              const int32_t *__restrict__ row_ptr,
-                                              const int32_t *__restrict__ col,
-                                              const float *__restrict__ val,
-                                              const float *__restrict__ B, float *__restrict__ C) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= rows * N) return;
-  const int64_t row = e / N, j = e % N;
-  int p = row_ptr[row];
-  const int end = row_ptr[row + 1];
-  const float *Bj = B + j;
-  float sum = 0.0f;
-  for (; p + 4 <= end; p += 4) {
-    int c0 = __ldg(col + p), c1 = __ldg(col + p + 1), c2 = __ldg(col + p + 2), c3 = __ldg(col + p + 3);
-    float v0 = __ldg(val + p), v1 = __ldg(val + p + 1), v2 = __ldg(val + p + 2), v3 = __ldg(val + p + 3);
-    float b0 = __ldg(Bj + (int64_t)c0 * N), b1 = __ldg(Bj + (int64_t)c1 * N);
-    float b2 = __ldg(Bj + (int64_t)c2 * N), b3 = __ldg(Bj + (int64_t)c3 * N);
-    sum = add(sum, mul(v0, b0));
-    sum = add(sum, mul(v1, b1));
-    sum = add(sum, mul(v2, b2));
-    sum = add(sum, mul(v3, b3));
-  }
-  for (; p < end; ++p) sum = add(sum, mul(__ldg(val + p), __ldg(Bj + (int64_t)__ldg(col + p) * N)));
-  C[e] = sum;
-}
-
-// The same mapping where N and the block size are multiples of 32: the 32 outputs of a warp lie in one
-// matrix row, so the warp reads 32 positions of col and val with one coalesced load each and passes them
-// around by shuffles instead of every lane loading every position (three L1 requests per position become
-// one).  Each thread still adds its products in position order: bit-identical to the kernel above.
-__global__ void spmm_thread_per_output_warp_row_kernel(int64_t rows, int64_t N,
-                                                       const int32_t *__restrict__ row_ptr,
-                                                       const int32_t *__restrict__ col,
-                                                       const float *__restrict__ val,
-                                                       const float *__restrict__ B, float *__restrict__ C) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= rows * N) return;  // rows * N is a multiple of 32: whole warps leave
-  const int lane = threadIdx.x & 31;
-  const int64_t row = e / N, j = e % N;
-  const int start = row_ptr[row], end = row_ptr[row + 1];
-  const float *Bj = B + j;
-  float sum = 0.0f;
-  for (int base = start; base < end; base += 32) {
-    const int left = end - base < 32 ? end - base : 32;
-    const int cl = lane < left ? __ldg(col + base + lane) : 0;
-    const float vl = lane < left ? __ldg(val + base + lane) : 0.0f;
-    int k = 0;
-    for (; k + 4 <= left; k += 4) {
-      const int c0 = __shfl_sync(FULL, cl, k), c1 = __shfl_sync(FULL, cl, k + 1);
-      const int c2 = __shfl_sync(FULL, cl, k + 2), c3 = __shfl_sync(FULL, cl, k + 3);
-      const float b0 = __ldg(Bj + (int64_t)c0 * N), b1 = __ldg(Bj + (int64_t)c1 * N);
-      const float b2 = __ldg(Bj + (int64_t)c2 * N), b3 = __ldg(Bj + (int64_t)c3 * N);
-      sum = add(sum, mul(__shfl_sync(FULL, vl, k), b0));
-      sum = add(sum, mul(__shfl_sync(FULL, vl, k + 1), b1));
-      sum = add(sum, mul(__shfl_sync(FULL, vl, k + 2), b2));
-      sum = add(sum, mul(__shfl_sync(FULL, vl, k + 3), b3));
-    }
-    for (; k < left; ++k)
-      sum = add(sum, mul(__shfl_sync(FULL, vl, k), __ldg(Bj + (int64_t)__shfl_sync(FULL, cl, k) * N)));
-  }
-  C[e] = sum;
-}
+// thread-per-output (ThreadPerOutputSpMMPattern, SparseWaveToGPU.cpp:489-558): sequential sums in position order,
+// bit-identical to the CPU CSR loop.
+#include "spmm_columns.cuh"
+#include "spmm_staged_rows.cuh"
 
 // ---------------------------------------------------------------------------
 // wave-per-row-tile (WavePerRowTileSpMMPattern, SparseWaveToGPU.cpp:1057-1256)
@@ -639,15 +575,6 @@ cudaError_t launch_tile(const CsrSpmmArgs &a, int block, int T, cudaStream_t s) 
   return cudaGetLastError();
 }
 
-template <int G, int L>
-cudaError_t launch_subwarp(const CsrSpmmArgs &a, int block, cudaStream_t s) {
-  const int64_t warps = ceil_div(a.rows, 32 / L);
-  SWB_GRID(grid, ceil_div(warps, block / 32));
-  spmm_subwarp_row_kernel<G, L><<<grid, block, 0, s>>>(
-      a.rows, a.n_rhs, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
-  return cudaGetLastError();
-}
-
 // Lanes per matrix row for rows of B of 4*G floats: at least 4 lanes (and at least G), at most the warp,
 // doubled while a lane group would get more than positions_per_lane_group(G) of the mean row's positions.
 // The figures are measured (1 M and 2 M rows, uniform columns, 2 to 64 positions per row): few lanes per row
@@ -656,6 +583,136 @@ cudaError_t launch_subwarp(const CsrSpmmArgs &a, int block, cudaStream_t s) {
 // N = 16, 24 per row 0.492 -> 0.205 ms; N = 32, 10 per row 0.514 -> 0.246 ms; N = 64, 5 per row (half a warp
 // instead of a warp) 1.02 -> 0.53 ms.
 constexpr int64_t positions_per_lane_group(int G) { return G == 1 ? 6 : G == 2 ? 12 : G <= 8 ? 16 : 12; }
+
+// ---- launches of the staged-rows kernel -------------------------------------------------------
+
+// Lanes per row and rows per block for M runs of columns, R of them per lane.
+struct RowsShape {
+  int64_t tiles, per;
+  int G;
+};
+
+// A block takes about 640 positions, which fit its shared memory with room for uneven rows, but no more rows than leave
+// 8 blocks for every SM (one wave of them), and at least one row for every group of lanes.
+inline RowsShape rows_shape(int64_t rows, int64_t nnz, int64_t M, int R) {
+  RowsShape h;
+  h.tiles = ceil_div(M, 32 * R);
+  h.G = (int)(M < 32 ? M : ceil_div(ceil_div(M, h.tiles), R));
+  const int64_t mean = rows > 0 ? nnz / rows : 0, in_hand = 32 / h.G * (STAGE_THREADS / 32);
+  const int64_t spread = ceil_div(rows * h.tiles, 148 * 8);
+  h.per = 640 / (mean > 0 ? mean : 1);
+  if (h.per > spread) h.per = spread;
+  if (h.per < in_hand) h.per = in_hand;
+  if (h.per > STAGE_ROWS) h.per = STAGE_ROWS;
+  return h;
+}
+
+// `per` > 0: rows per block, instead of the rule above.
+template <int V, int R, int Q, typename Pitch = uint32_t>
+cudaError_t launch_rows_as(const CsrSpmmArgs &a, cudaStream_t s, int64_t per = 0) {
+  RowsShape h = rows_shape(a.rows, a.nnz, a.n_rhs / V, R);
+  if (per > 0) h.per = per;
+  SWB_GRID(grid, ceil_div(a.rows, h.per) * h.tiles);
+  spmm_staged_rows_kernel<V, R, Q, Pitch><<<grid, STAGE_THREADS, 0, s>>>(
+      a.rows, a.n_rhs, (Pitch)(a.n_rhs * 4), h.G, (int)h.per, h.tiles, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
+  return cudaGetLastError();
+}
+
+// Runs of columns per lane: enough that 32 lanes hold the row of C, else column tiles (the widest odd row without
+// tiles, 224 columns, takes seven single columns per lane).
+inline int runs_per_lane(int64_t M, int V) {
+  if (M <= 96) return (int)(M > 0 ? ceil_div(M, 32) : 1);
+  return V > 1 || M <= 128 ? 4 : M <= 160 ? 5 : 7;
+}
+
+template <int V>
+cudaError_t launch_rows_columns(const CsrSpmmArgs &a, cudaStream_t s) {
+  switch (runs_per_lane(a.n_rhs / V, V)) {
+    case 1: return launch_rows_as<V, 1, V <= 2 ? 8 : 4>(a, s);
+    case 2: return launch_rows_as<V, 2, 4>(a, s);
+    case 3: return launch_rows_as<V, 3, 4>(a, s);
+    case 4: return launch_rows_as<V, 4, 4>(a, s);
+  }
+  if constexpr (V == 1) return a.n_rhs <= 160 ? launch_rows_as<V, 5, 4>(a, s) : launch_rows_as<V, 7, 4>(a, s);
+  return cudaErrorInvalidValue;
+}
+
+// Up to four columns, and up to eight on few rows, the sums run over products staged by the whole block (row_products.cuh):
+// 300,000 ragged rows of 20, N = 4: 55 us against 77 here; 3,000 rows of 40, N = 8: 12.6 against 16.7.
+inline bool takes_row_products(int64_t rows, int64_t n_rhs) { return n_rhs <= 4 || (n_rhs <= 8 && rows <= 8192); }
+
+// Columns per lane: the widest run that divides N and that the rows of B and C are aligned to, for the fewest
+// instructions per position.  With few rows lanes would idle, and what counts is how many rows of B a row of A has in
+// flight: narrower runs then, and column tiles rather than several runs per lane.  Measured (us with 1 / 2 / 4 columns):
+// 3,000 rows of 40: N = 64 18.5 / 22 / 29, N = 256 29 / 26 / 31; 18,772 rows of 21: N = 16 16.5 / 16.6 / 22,
+// N = 32 18.7 / 19.9 / 21.6, N = 64 27 / 22 / 25, N = 128 41 / 33 / 30; 60,000 rows of 10: N = 8 9.1 / 8.9 / 5.9,
+// N = 32 20 / 16 / 13.
+// A narrow C has many rows in hand per block; narrower runs keep their positions within the staged ones.
+inline int columns_per_lane(int64_t rows, int64_t nnz, int64_t n_rhs, uintptr_t alignment_bits) {
+  int V = n_rhs % 4 == 0 && alignment_bits % 16 == 0 ? 4 : n_rhs % 2 == 0 && alignment_bits % 8 == 0 ? 2 : 1;
+  const int most = rows <= 8192 ? (n_rhs <= 128 ? 1 : 2) : rows <= 32768 ? (n_rhs <= 32 ? 1 : n_rhs <= 64 ? 2 : 4) : 4;
+  if (V > most) V = most;
+  while (V > 1 && n_rhs / V < 32 && 32 / (n_rhs / V) * (STAGE_THREADS / 32) * (nnz / (rows > 0 ? rows : 1)) > 1300) V /= 2;
+  return V;
+}
+// ... and whether each lane keeps to one run, with more positions a step.
+inline bool few_rows(int64_t rows, int64_t n_rhs) { return rows <= 8192 || (rows <= 32768 && n_rhs <= 32); }
+
+cudaError_t launch_rows(const CsrSpmmArgs &a, cudaStream_t s) {
+  if (takes_row_products(a.rows, a.n_rhs)) return launch_row_products(a, s);
+  if (a.n_rhs > 0x3fffffffLL) return launch_rows_as<1, 7, 4, uint64_t>(a, s);
+  const int V = columns_per_lane(a.rows, a.nnz, a.n_rhs, reinterpret_cast<uintptr_t>(a.B) | reinterpret_cast<uintptr_t>(a.C));
+  if (few_rows(a.rows, a.n_rhs)) return V == 2 ? launch_rows_as<2, 1, 8>(a, s) : launch_rows_as<1, 1, 16>(a, s);
+  if (V == 4) return launch_rows_columns<4>(a, s);
+  return V == 2 ? launch_rows_columns<2>(a, s) : launch_rows_columns<1>(a, s);
+}
+
+int64_t rows_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs) {  // 16-byte aligned operands
+  if (takes_row_products(rows, n_rhs)) return row_products_physical_grid(rows, nnz, n_rhs);
+  const bool wide = n_rhs > 0x3fffffffLL;
+  const int V = wide ? 1 : columns_per_lane(rows, nnz, n_rhs, 0);
+  const RowsShape h = rows_shape(rows, nnz, n_rhs / V, !wide && few_rows(rows, n_rhs) ? 1 : runs_per_lane(n_rhs / V, V));
+  return max1(ceil_div(rows, h.per) * h.tiles);
+}
+
+// Whether wave-per-row-tile takes the staged-rows kernel.  It wins where there are rows enough to balance the blocks;
+// rows many times longer than usual in a small matrix are one lane group's chain there, while a warp per row splits
+// them.  Measured against the kernels with a warp or part of one per row:
+//   N = 16, 32, 64, 128 (300,000 ragged rows of 5: 41 -> 29, 69 -> 45, 110 -> 89, 184 -> 141 us), with the sizes and mean
+//   lengths up to which each wins; N = 8 and rows of 50 and more do not gain;
+//   other multiples of 4 from 12 to 124 (150,000 rows of 20, N = 100: 182 -> 126 us; 15,000 rows of 20, N = 24: a draw);
+//   the rest up to 512 columns, which else read B by single columns (250,001 rows of 20, N = 50: 664 -> 128 us;
+//   102,040 rows of 20, N = 147: 742 -> 145 us; 15,000 rows of 20, N = 7: 10 us there against 13 here).
+inline bool tile_takes_staged_rows(int64_t rows, int64_t nnz, int64_t N) {
+  const int64_t outputs = rows * N, mean = rows > 0 ? nnz / rows : 0;
+  switch (N) {
+    case 1: return true;
+    case 2: case 3: return rows > 8192;  // products summed per row: 300,000 rows of 20, N = 1: 113 -> 37 us
+    case 4: case 8: case 256: case 384: case 512: return false;
+    case 16: return outputs >= 2500000 && mean <= 14;
+    case 32: return outputs >= 4000000 && mean <= 48;
+    case 64: return outputs >= 6000000 && mean <= 48;
+    case 128: return outputs >= 8000000;
+  }
+  if (N > 512 || rows < 100 * mean) return false;
+  if (N % 4 == 0 && N >= 12 && N < 128 && mean >= 8) return outputs >= 512000 && (N >= 32 || mean <= 32);
+  return outputs >= 256000;
+}
+
+// Rows per block of that kernel for N = 64 and short rows: those of a block of the (row, tile) units, with half a warp or
+// a warp per row; 0: the kernel's own rule.
+inline int64_t tile_rows_per_block(int64_t N, int64_t mean, int block) {
+  return N == 64 && mean <= 13 && block >= 128 ? (mean <= 12 ? 2 : 1) * (block / 32) : 0;
+}
+
+template <int G, int L>
+cudaError_t launch_subwarp(const CsrSpmmArgs &a, int block, cudaStream_t s) {
+  const int64_t warps = ceil_div(a.rows, 32 / L);
+  SWB_GRID(grid, ceil_div(warps, block / 32));
+  spmm_subwarp_row_kernel<G, L><<<grid, block, 0, s>>>(
+      a.rows, a.n_rhs, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
+  return cudaGetLastError();
+}
 
 template <int G>
 cudaError_t launch_row_of_tiles(const CsrSpmmArgs &a, int block, cudaStream_t s) {
@@ -678,16 +735,9 @@ cudaError_t launch_row_of_tiles(const CsrSpmmArgs &a, int block, cudaStream_t s)
 
 }  // namespace
 
-cudaError_t launch_spmm_thread_per_output(const CsrSpmmArgs &a, int block, cudaStream_t s,
-                                          int64_t *launches) {
-  SWB_GRID(grid, ceil_div(a.rows * a.n_rhs, block));
-  if (a.n_rhs % 32 == 0 && block % 32 == 0)
-    spmm_thread_per_output_warp_row_kernel<<<grid, block, 0, s>>>(a.rows, a.n_rhs, a.row_ptr, a.col_idx, a.val, a.B,
-                                                                  a.C);
-  else
-    spmm_thread_per_output_kernel<<<grid, block, 0, s>>>(a.rows, a.n_rhs, a.row_ptr, a.col_idx, a.val, a.B, a.C);
+cudaError_t launch_spmm_thread_per_output(const CsrSpmmArgs &a, cudaStream_t s, int64_t *launches) {
   ++*launches;
-  return cudaGetLastError();
+  return launch_rows(a, s);
 }
 
 cudaError_t launch_spmm_wave_per_row_tile(const CsrSpmmArgs &a, int block, int tile,
@@ -698,6 +748,11 @@ cudaError_t launch_spmm_wave_per_row_tile(const CsrSpmmArgs &a, int block, int t
   // warp, or by part of a warp where the rows are short.
   const int64_t N = a.n_rhs;
   const bool pow2_row = N >= 4 && N <= 128 && (N & (N - 1)) == 0;
+  const bool aligned = aligned16(a.B) && aligned16(a.C);
+  if (tile_takes_staged_rows(a.rows, a.nnz, N) && (aligned || N % 4 != 0)) {
+    const int64_t per = tile_rows_per_block(N, a.nnz / a.rows, block);
+    return per > 0 ? launch_rows_as<4, 1, 4>(a, s, per) : launch_rows(a, s);
+  }
   if ((N == 256 || N == 384 || N == 512) && aligned16(a.B) && aligned16(a.C)) {
     SWB_GRID(grid, ceil_div(a.rows, block / 32));
     if (N == 256)
@@ -736,9 +791,17 @@ cudaError_t launch_spmm_wave_per_row_tile(const CsrSpmmArgs &a, int block, int t
   return launch_tile<32>(a, block, tile, s);
 }
 
+int64_t thread_per_output_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs) {
+  return rows_physical_grid(rows, nnz, n_rhs);
+}
+
 int64_t wave_per_row_tile_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs, int block, int tile) {
   // Mirrors launch_spmm_wave_per_row_tile and launch_row_of_tiles for 16-byte aligned operands.
   const int64_t wpb = block / 32;
+  if (tile_takes_staged_rows(rows, nnz, n_rhs)) {
+    const int64_t per = tile_rows_per_block(n_rhs, nnz / rows, block);
+    return per > 0 ? max1(ceil_div(rows, per)) : rows_physical_grid(rows, nnz, n_rhs);
+  }
   const bool pow2_row = n_rhs >= 4 && n_rhs <= 128 && (n_rhs & (n_rhs - 1)) == 0;
   if (n_rhs == 256 || n_rhs == 384 || n_rhs == 512) return max1(ceil_div(rows, wpb));
   if (n_rhs >= 12 && n_rhs < 128 && n_rhs % 4 == 0 && !pow2_row && rows > 0 && nnz / rows >= 8)
@@ -747,7 +810,7 @@ int64_t wave_per_row_tile_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs
   if (n_rhs > 64) return max1(ceil_div(rows, wpb));
   const int64_t G = n_rhs / 4, mean = rows > 0 ? nnz / rows : 0;
   int64_t lanes = G > 4 ? G : 4;
-  while (lanes < 32 && (lanes / G) * positions_per_lane_group((int)G) < mean) lanes *= 2;
+  while (lanes < 32 && G<=16 && (lanes / G) * positions_per_lane_group((int)G) < mean) lanes *= 2;
   return max1(ceil_div(ceil_div(rows, 32 / lanes), wpb));
 }
 

@@ -689,10 +689,14 @@ cudaError_t launch_coo_spmv_thread_per_nonzero(int64_t rows, int64_t nnz, const 
 cudaError_t launch_row_products(const CsrSpmmArgs &a, cudaStream_t s) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(a.B);
   switch (a.n_rhs) {
-    case 1: return launch_row_products_of<1, true>(a, s);
-    case 2: return at % 8 == 0 ? launch_row_products_of<2, true>(a, s) : launch_row_products_of<2, false>(a, s);
-    case 3: return launch_row_products_of<3, false>(a, s);
-    case 4: return at % 16 == 0 ? launch_row_products_of<4, true>(a, s) : launch_row_products_of<4, false>(a, s);
+    case 1: return launch_row_products_of<1, 1>(a, s);
+    case 2: return at % 8 == 0 ? launch_row_products_of<2, 2>(a, s) : launch_row_products_of<2, 1>(a, s);
+    case 3: return launch_row_products_of<3, 1>(a, s);
+    case 4: return at % 16 == 0 ? launch_row_products_of<4, 4>(a, s) : launch_row_products_of<4, 1>(a, s);
+    case 5: return launch_row_products_of<5, 1>(a, s);
+    case 6: return launch_row_products_of<6, 1>(a, s);
+    case 7: return launch_row_products_of<7, 1>(a, s);
+    case 8: return at % 16 == 0 ? launch_row_products_of<8, 4>(a, s) : launch_row_products_of<8, 1>(a, s);
   }
   return cudaErrorInvalidValue;
 }

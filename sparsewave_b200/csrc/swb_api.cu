@@ -538,10 +538,15 @@ int swb_launch_shape_query(swb_context *ctx, const swb_options *o, int64_t rows,
     if (o->spmm_mapping == SWB_WAVE_PER_ROW_TILE)  // rows of B of 4 ... 128 floats: the tiles of a row are fused
       r.physical_grid = swb::wave_per_row_tile_physical_grid(rows, nnz, n_rhs, (int)B, (int)o->spmm_tile_size);
   }
-  if (r.physical_grid > swb::kMaxGridX)
+  int64_t blocks = r.physical_grid;
+  if (n_rhs != 0 && o->spmm_mapping == SWB_THREAD_PER_OUTPUT) {  // fewer blocks; refused by the reference's grid all the same
+    blocks = r.logical_grid;
+    r.physical_grid = swb::thread_per_output_physical_grid(rows, nnz, n_rhs);
+  }
+  if (blocks > swb::kMaxGridX)
     return fail(ctx, SWB_ERR_UNSUPPORTED,
                 "the launch needs %lld blocks, more than a CUDA grid holds (%lld); use a larger block or tile size",
-                (long long)r.physical_grid, (long long)swb::kMaxGridX);
+                (long long)blocks, (long long)swb::kMaxGridX);
   *out = r;
   return SWB_OK;
 }
@@ -703,7 +708,7 @@ int swb_spmm(swb_context *ctx, const swb_options *o, int64_t rows, int64_t cols,
   const int Bs = (int)o->spmm_block_size;
   cudaError_t e = cudaSuccess;
   switch (o->spmm_mapping) {
-    case SWB_THREAD_PER_OUTPUT: e = swb::launch_spmm_thread_per_output(a, Bs, s, &ctx->launches); break;
+    case SWB_THREAD_PER_OUTPUT: e = swb::launch_spmm_thread_per_output(a, s, &ctx->launches); break;
     case SWB_WAVE_PER_ROW_TILE:
       // Opt-in (SWB_SPMM_STAGED=1): the rows of B around the diagonal staged in shared memory by TMA, for
       // banded matrices.  Measured on a banded-plus-random matrix it does not beat the fused-row kernel (the

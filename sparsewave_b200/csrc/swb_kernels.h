@@ -104,8 +104,8 @@ int64_t wave_per_position_auto_batch(int64_t nnz, int block,
 int64_t wave_per_position_physical_grid(int64_t nnz, int block, int64_t batch);
 
 // --- SpMM
-cudaError_t launch_spmm_thread_per_output(const CsrSpmmArgs &a, int block,
-                                          cudaStream_t s, int64_t *launches);
+cudaError_t launch_spmm_thread_per_output(const CsrSpmmArgs &a, cudaStream_t s, int64_t *launches);
+int64_t thread_per_output_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs);
 cudaError_t launch_spmm_wave_per_row_tile(const CsrSpmmArgs &a, int block,
                                           int tile, cudaStream_t s,
                                           int64_t *launches);

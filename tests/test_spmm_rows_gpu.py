@@ -1,0 +1,61 @@
+"""SpMM by groups of lanes that take whole rows in turn, and by staged products for up to four columns: thread-per-output
+for every N, wave-per-row-tile from the sizes where it takes these kernels."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from tests.helpers import assert_within_bound, dev, random_csr
+
+pytestmark = pytest.mark.gpu
+
+# one, two and four columns per lane; 1 to 7 runs of them; the last width without column tiles and the first with
+WIDTHS = [1, 2, 3, 4, 5, 8, 31, 32, 33, 64, 66, 96, 97, 100, 128, 129, 161, 224, 225, 256, 260, 512, 516]
+
+
+def _spmm(ctx, opts, rp, ci, v, B, C=None):
+    return ctx.spmm(opts, dev(rp), dev(ci), dev(v), B, C)
+
+
+@pytest.mark.parametrize("n", WIDTHS)
+@pytest.mark.parametrize("rows,mean", [(1, 70), (300, 9), (20000, 3)])
+def test_thread_per_output_widths(ctx, n, rows, mean):
+    rp, ci, v = random_csr(rows, 433, mean, seed=n + rows)
+    B = np.random.default_rng(n).uniform(-1, 1, (433, n)).astype(np.float32)
+    want = oracle.csr_spmm(rp, ci, v, B, parallel=True)
+    assert np.array_equal(_spmm(ctx, "", rp, ci, v, dev(B)).cpu().numpy(), want)
+    # B and C that start four bytes past a 16-byte boundary: single columns
+    Bu = torch.empty(B.size + 1, device="cuda")[1:].view(B.shape).copy_(torch.from_numpy(B))
+    Cu = torch.empty(rows * n + 1, device="cuda")[1:].view(rows, n)
+    assert np.array_equal(_spmm(ctx, "", rp, ci, v, Bu, Cu).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n", [4, 32, 50, 147])
+def test_rows_beyond_the_staged_positions(ctx, n):
+    rng = np.random.default_rng(n)
+    lens = rng.integers(0, 30, 3000)
+    lens[[0, 777, 2999]] = 5000, 1537, 4096
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = rng.integers(0, 6000, rp[-1]).astype(np.int32)
+    v = rng.uniform(-1, 1, rp[-1]).astype(np.float32)
+    B = rng.uniform(-1, 1, (6000, n)).astype(np.float32)
+    assert np.array_equal(_spmm(ctx, "", rp, ci, v, dev(B)).cpu().numpy(), oracle.csr_spmm(rp, ci, v, B, parallel=True))
+
+
+@pytest.mark.parametrize("rows,mean,n", [(50000, 6, 1), (50000, 6, 3), (60000, 5, 7), (200000, 5, 16), (150000, 9, 32),
+                                         (40000, 12, 50), (100000, 4, 64), (110000, 16, 64), (70000, 7, 128), (20000, 8, 84),
+                                         (9000, 6, 147), (3000, 5, 500)])
+def test_wave_per_row_tile_takes_the_rows_kernel(ctx, rows, mean, n):
+    opts = "spmm-mapping=wave-per-row-tile spmm-tile-size=8 spmm-block-size=256"
+    rng = np.random.default_rng(n)
+    lens = rng.integers(0, 2 * mean + 1, rows)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = rng.integers(0, 2000, rp[-1]).astype(np.int32)
+    v = rng.uniform(-1, 1, rp[-1]).astype(np.float32)
+    B = rng.uniform(-1, 1, (2000, n)).astype(np.float32)
+    want, bound = oracle.csr_spmm(rp, ci, v, B, parallel=True), oracle.csr_abs_bound(rp, ci, v, B)
+    assert ctx.launch_shape(opts, rows, int(rp[-1]), n).physical_grid < rows
+    assert np.array_equal(_spmm(ctx, opts, rp, ci, v, dev(B)).cpu().numpy(), want)
+    C = torch.ones((rows, n), device="cuda")
+    _spmm(ctx, opts + " accumulate=1", rp, ci, v, dev(B), C)
+    assert_within_bound(C.cpu().numpy(), want + 1.0, bound + 1.0)
