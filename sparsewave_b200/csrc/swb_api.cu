@@ -753,8 +753,7 @@ int swb_bsr_spmm_f32(swb_context *ctx, const swb_options *o, int64_t rows, int64
   if (!brp || (nnzb > 0 && (!bci || !bv)) || (cols > 0 && !B) || (rows > 0 && !C))
     return fail(ctx, SWB_ERR_INVALID_ARGUMENT, "bsr_spmm: NULL operand pointer");
   swb::BsrSpmmArgs a{rows, cols, nnzb, bs, n_rhs, brp, bci, bv, B, C};
-  cudaError_t e = swb::launch_bsr_spmm_thread_per_output_f32(a, (int)o->spmm_block_size,
-                                                             static_cast<cudaStream_t>(stream), &ctx->launches);
+  cudaError_t e = swb::launch_bsr_spmm_thread_per_output_f32(a, static_cast<cudaStream_t>(stream), &ctx->launches);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "bsr_spmm launch");
   return SWB_OK;
 }
@@ -776,7 +775,7 @@ int swb_bsr_spmm_bf16(swb_context *ctx, const swb_options *o, int64_t rows, int6
   if (swb::bsr16_tcgen05_supported(a))
     e = swb::launch_bsr16_spmm_tcgen05(a, ctx->status_flag, ctx->dev, s, &ctx->launches);
   else
-    e = swb::launch_bsr_spmm_thread_per_output_bf16(a, (int)o->spmm_block_size, s, &ctx->launches);
+    e = swb::launch_bsr_spmm_thread_per_output_bf16(a, s, &ctx->launches);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "bsr_spmm launch");
   return SWB_OK;
 }

@@ -121,12 +121,8 @@ cudaError_t launch_spmm_thread_per_position(const CsrSpmmArgs &a, int block,
                                             int64_t *launches);
 
 // --- BSR SpMM
-cudaError_t launch_bsr_spmm_thread_per_output_f32(const BsrSpmmArgs &a,
-                                                  int block, cudaStream_t s,
-                                                  int64_t *launches);
-cudaError_t launch_bsr_spmm_thread_per_output_bf16(const BsrSpmmArgs &a,
-                                                   int block, cudaStream_t s,
-                                                   int64_t *launches);
+cudaError_t launch_bsr_spmm_thread_per_output_f32(const BsrSpmmArgs &a, cudaStream_t s, int64_t *launches);
+cudaError_t launch_bsr_spmm_thread_per_output_bf16(const BsrSpmmArgs &a, cudaStream_t s, int64_t *launches);
 // 16x16 bf16 blocks on the tcgen05 tensor cores.  `status_flag` is a device
 // int the kernel sets non-zero when one of its bounded waits gives up.
 bool bsr16_tcgen05_supported(const BsrSpmmArgs &a);
