@@ -11,6 +11,7 @@
 // pipe, 18 us of L2); 8 x 8, 8,192 block rows of 12, N = 64: 304 -> 70 us; 32 x 32 bf16, N = 64: 740 -> 245 us.
 #include <cuda_bf16.h>
 
+#include "swb_chain.cuh"
 #include "swb_index.h"
 #include "swb_kernels.h"
 
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(TILE_THREADS, BS == 4 ? 7 : 1) bsr_spmm_row_ti
                                                                 const int32_t *__restrict__ bci,
                                                                 const T *__restrict__ bv, const T *__restrict__ B,
                                                                 T *__restrict__ C) {
+  after_previous_kernel();
   constexpr int TR = BS ? BS : 8;
   constexpr int K = BS ? (BS % 4 == 0 ? 4 : BS) : 4;
   constexpr bool AHEAD = BS == 3 || BS == 4 || BS == 8;  // rows of B requested a step ahead of their sums
@@ -180,7 +182,7 @@ cudaError_t launch_tiles(const BsrSpmmArgs &a, cudaStream_t s) {
   // loads of K values start at multiples of K from an aligned base (K divides bs where BS is constant)
   const bool wide = reinterpret_cast<uintptr_t>(a.block_values) % (4 * sizeof(T)) == 0 && (BS == 2 || bs % 4 == 0);
 #define SWB_BSR(WIDE)                                                                                             \
-  bsr_spmm_row_tile_kernel<T, BS, V, WIDE><<<grid, TILE_THREADS, 0, s>>>(                                                   \
+  launch_chained(bsr_spmm_row_tile_kernel<T, BS, V, WIDE>, grid, TILE_THREADS, 0, s,                                                    \
       brows, a.n_rhs, bs, (int)tiles, a.block_row_ptr, a.block_col_idx, static_cast<const T *>(a.block_values), \
       static_cast<const T *>(a.B), static_cast<T *>(a.C))
   if (wide) SWB_BSR(true); else SWB_BSR(false);

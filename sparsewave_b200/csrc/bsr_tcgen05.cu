@@ -46,6 +46,7 @@
 #include <atomic>
 #include <cstdio>
 
+#include "swb_chain.cuh"
 #include "swb_index.h"
 #include "swb_kernels.h"
 
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(THREADS) bsr16_spmm_tcgen05_kernel(
   const int n0 = (int)((blockIdx.x % n_tiles) * TILE_N);
   const int halves = ((int64_t)n0 + HALF_N < N) ? 2 : 1;  // the second 128 columns may lie wholly past N
   const uint32_t stage0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  after_previous_kernel();
   const int start = brp[br], end = brp[br + 1];
   const int nblk = end - start;
 
@@ -336,7 +338,7 @@ cudaError_t launch_bsr16_spmm_tcgen05(const BsrSpmmArgs &a, int *status_flag, co
   // Block values as (nnzb*16) x 16 bf16, one 16 x 16 box per block, 32-byte swizzle.
   if (!make_map_2d(&map_A, a.block_values, 16, (uint64_t)a.nnzb * 16, 16, 16, CU_TENSOR_MAP_SWIZZLE_32B))
     return cudaErrorInvalidValue;
-  bsr16_spmm_tcgen05_kernel<false><<<(unsigned)grid, THREADS, SMEM_BYTES, s>>>(
+  launch_chained(bsr16_spmm_tcgen05_kernel<false>, (unsigned)grid, THREADS, SMEM_BYTES, s,
       map_B, map_A, n_tiles, a.n_rhs, a.block_row_ptr, a.block_col_idx, static_cast<__nv_bfloat16 *>(a.C),
       status_flag);
   ++*launches;
@@ -475,7 +477,7 @@ extern "C" __attribute__((visibility("default"))) int swb_bsr16_spmm_bf16_static
   // The words keep the previous call's outcome: clear the ones this call uses.
   e = cudaMemsetAsync(status, 0, (size_t)grid * sizeof(int), s);
   if (e != cudaSuccess) return static_fail(kCuda, cudaGetErrorString(e));
-  bsr16_spmm_tcgen05_kernel<true><<<(unsigned)grid, THREADS, SMEM_BYTES, s>>>(
+  launch_chained(bsr16_spmm_tcgen05_kernel<true>, (unsigned)grid, THREADS, SMEM_BYTES, s,
       map_B, map_A, n_tiles, n_rhs, block_row_ptr, block_col_idx, reinterpret_cast<__nv_bfloat16 *>(C), status);
   e = cudaGetLastError();
   if (e != cudaSuccess) return static_fail(kCuda, cudaGetErrorString(e));

@@ -31,6 +31,7 @@ __global__ void __launch_bounds__(PRODUCT_THREADS)
     row_products_kernel(int64_t rows, int rows_per_block, const int32_t *__restrict__ row_ptr,
                         const int32_t *__restrict__ col, const float *__restrict__ val, const float *__restrict__ B,
                         float *__restrict__ C, bool accumulate) {
+  after_previous_kernel();
   using T = typename Words<W>::T;
   constexpr int TILE = PRODUCT_WORDS / N;     // positions
   constexpr bool BY_PRODUCT = W == 1;         // items are products, else positions
@@ -136,7 +137,7 @@ cudaError_t launch_row_products_of(const CsrSpmmArgs &a, cudaStream_t s) {
   const int64_t per = product_rows_per_block(a.rows, a.nnz, N);
   unsigned grid = 0;
   if (!grid_dim(ceil_div(a.rows, per), &grid)) return cudaErrorInvalidConfiguration;
-  row_products_kernel<N, W><<<grid, PRODUCT_THREADS, 0, s>>>(a.rows, (int)per, a.row_ptr, a.col_idx, a.val, a.B, a.C,
+  launch_chained(row_products_kernel<N, W>, grid, PRODUCT_THREADS, 0, s, a.rows, (int)per, a.row_ptr, a.col_idx, a.val, a.B, a.C,
                                                               a.accumulate);
   return cudaGetLastError();
 }

@@ -1,6 +1,7 @@
 // CSR SpMM kernels for sm_100a: thread-per-output, wave-per-row-tile and
 // thread-per-position mappings of sparsewave.spmm.  B is cols x N and C is
 // rows x N, row-major.  Products and sums are separate f32 operations.
+#include "swb_chain.cuh"
 #include "swb_index.h"
 #include "swb_kernels.h"
 
@@ -95,6 +96,7 @@ __global__ void spmm_wave_per_row_tile_kernel(int64_t rows, int64_t N, int T, in
                                               const float *__restrict__ val,
                                               const float *__restrict__ B, float *__restrict__ C,
                                               bool accumulate) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int64_t unit = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (unit >= rows * tiles) return;
@@ -150,6 +152,7 @@ __global__ void spmm_wave_per_row_tile_vec_kernel(int64_t rows, int64_t N, int64
                                                   const float *__restrict__ val,
                                                   const float *__restrict__ B, float *__restrict__ C,
                                                   bool accumulate) {
+  after_previous_kernel();
   constexpr int T = 4 * G, PG = 32 / G;
   const int lane = threadIdx.x & 31;
   const int64_t unit = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -252,6 +255,7 @@ __global__ void spmm_wave_per_row_fused_kernel(int64_t rows, int64_t N, const in
                                                const int32_t *__restrict__ col, const float *__restrict__ val,
                                                const float *__restrict__ B, float *__restrict__ C,
                                                bool accumulate) {
+  after_previous_kernel();
   constexpr int PG = 32 / G;
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -328,6 +332,7 @@ __global__ void spmm_wave_per_row_any_kernel(int64_t rows, int64_t N, int G, con
                                              const int32_t *__restrict__ col, const float *__restrict__ val,
                                              const float *__restrict__ B, float *__restrict__ C,
                                              bool accumulate) {
+  after_previous_kernel();
   const int PG = 32 / G;
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -397,6 +402,7 @@ __global__ void spmm_wave_per_row_wide_kernel(int64_t rows, int64_t N, const int
                                               const int32_t *__restrict__ col, const float *__restrict__ val,
                                               const float *__restrict__ B, float *__restrict__ C,
                                               bool accumulate) {
+  after_previous_kernel();
   constexpr int U = R == 2 ? 2 : 1;  // positions in flight
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -464,6 +470,7 @@ template <int G, int L>
 __global__ void spmm_subwarp_row_kernel(int64_t rows, int64_t N, const int32_t *__restrict__ row_ptr,
                                         const int32_t *__restrict__ col, const float *__restrict__ val,
                                         const float *__restrict__ B, float *__restrict__ C, bool accumulate) {
+  after_previous_kernel();
   constexpr int PG = L / G, RW = 32 / L;
   static_assert(L >= G && L < 32 && PG >= 1, "lanes per row");
   const int lane = threadIdx.x & 31;
@@ -524,6 +531,7 @@ __global__ void spmm_thread_per_position_kernel(int64_t rows, int64_t nnz, int64
                                                 const int32_t *__restrict__ col,
                                                 const float *__restrict__ val,
                                                 const float *__restrict__ B, float *__restrict__ C) {
+  after_previous_kernel();
   const int64_t worker = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t begin, end;
   chunk_bounds(0, nnz * N, worker, chunk, begin, end);
@@ -566,10 +574,10 @@ cudaError_t launch_tile(const CsrSpmmArgs &a, int block, int T, cudaStream_t s) 
                    aligned16(a.B) && aligned16(a.C);
   if (vec) {
     if constexpr (TCAP >= 4)
-      spmm_wave_per_row_tile_vec_kernel<TCAP / 4><<<grid, block, 0, s>>>(a.rows, a.n_rhs, tiles, a.row_ptr,
+      launch_chained(spmm_wave_per_row_tile_vec_kernel<TCAP / 4>, grid, block, 0, s, a.rows, a.n_rhs, tiles, a.row_ptr,
                                                                           a.col_idx, a.val, a.B, a.C, a.accumulate);
   } else {
-    spmm_wave_per_row_tile_kernel<TCAP><<<grid, block, 0, s>>>(
+    launch_chained(spmm_wave_per_row_tile_kernel<TCAP>, grid, block, 0, s,
         a.rows, a.n_rhs, T, tiles, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
   }
   return cudaGetLastError();
@@ -613,7 +621,7 @@ cudaError_t launch_rows_as(const CsrSpmmArgs &a, cudaStream_t s, int64_t per = 0
   RowsShape h = rows_shape(a.rows, a.nnz, a.n_rhs / V, R);
   if (per > 0) h.per = per;
   SWB_GRID(grid, ceil_div(a.rows, h.per) * h.tiles);
-  spmm_staged_rows_kernel<V, R, Q, Pitch><<<grid, STAGE_THREADS, 0, s>>>(
+  launch_chained(spmm_staged_rows_kernel<V, R, Q, Pitch>, grid, STAGE_THREADS, 0, s,
       a.rows, a.n_rhs, (Pitch)(a.n_rhs * 4), h.G, (int)h.per, h.tiles, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
   return cudaGetLastError();
 }
@@ -709,7 +717,7 @@ template <int G, int L>
 cudaError_t launch_subwarp(const CsrSpmmArgs &a, int block, cudaStream_t s) {
   const int64_t warps = ceil_div(a.rows, 32 / L);
   SWB_GRID(grid, ceil_div(warps, block / 32));
-  spmm_subwarp_row_kernel<G, L><<<grid, block, 0, s>>>(
+  launch_chained(spmm_subwarp_row_kernel<G, L>, grid, block, 0, s,
       a.rows, a.n_rhs, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
   return cudaGetLastError();
 }
@@ -725,7 +733,7 @@ cudaError_t launch_row_of_tiles(const CsrSpmmArgs &a, int block, cudaStream_t s)
   if (lanes == 16) return launch_subwarp<G, 16>(a, block, s);
   if constexpr (G >= 4) {  // a warp per row, col/val handed to the lane groups by shuffles
     SWB_GRID(grid, ceil_div(a.rows, block / 32));
-    spmm_wave_per_row_fused_kernel<G><<<grid, block, 0, s>>>(a.rows, a.n_rhs, a.row_ptr, a.col_idx, a.val, a.B, a.C,
+    launch_chained(spmm_wave_per_row_fused_kernel<G>, grid, block, 0, s, a.rows, a.n_rhs, a.row_ptr, a.col_idx, a.val, a.B, a.C,
                                                              a.accumulate);
     return cudaGetLastError();
   } else {
@@ -756,11 +764,11 @@ cudaError_t launch_spmm_wave_per_row_tile(const CsrSpmmArgs &a, int block, int t
   if ((N == 256 || N == 384 || N == 512) && aligned16(a.B) && aligned16(a.C)) {
     SWB_GRID(grid, ceil_div(a.rows, block / 32));
     if (N == 256)
-      spmm_wave_per_row_wide_kernel<2><<<grid, block, 0, s>>>(a.rows, N, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
+      launch_chained(spmm_wave_per_row_wide_kernel<2>, grid, block, 0, s, a.rows, N, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
     else if (N == 384)
-      spmm_wave_per_row_wide_kernel<3><<<grid, block, 0, s>>>(a.rows, N, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
+      launch_chained(spmm_wave_per_row_wide_kernel<3>, grid, block, 0, s, a.rows, N, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
     else
-      spmm_wave_per_row_wide_kernel<4><<<grid, block, 0, s>>>(a.rows, N, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
+      launch_chained(spmm_wave_per_row_wide_kernel<4>, grid, block, 0, s, a.rows, N, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
     return cudaGetLastError();
   }
   // other multiples of 4 up to 124 (rows of B of 12, 20, 24 ... floats) where a matrix row has enough positions
@@ -768,7 +776,7 @@ cudaError_t launch_spmm_wave_per_row_tile(const CsrSpmmArgs &a, int block, int t
   if (N >= 12 && N < 128 && N % 4 == 0 && !pow2_row && a.rows > 0 && a.nnz / a.rows >= 8 && aligned16(a.B) &&
       aligned16(a.C)) {
     SWB_GRID(grid, ceil_div(a.rows, block / 32));
-    spmm_wave_per_row_any_kernel<<<grid, block, 0, s>>>(a.rows, N, (int)(N / 4), a.row_ptr, a.col_idx, a.val, a.B,
+    launch_chained(spmm_wave_per_row_any_kernel, grid, block, 0, s, a.rows, N, (int)(N / 4), a.row_ptr, a.col_idx, a.val, a.B,
                                                        a.C, a.accumulate);
     return cudaGetLastError();
   }
@@ -779,7 +787,7 @@ cudaError_t launch_spmm_wave_per_row_tile(const CsrSpmmArgs &a, int block, int t
     if (N == 32) return launch_row_of_tiles<8>(a, block, s);
     if (N == 64) return launch_row_of_tiles<16>(a, block, s);  // half a warp per row where rows are short
     SWB_GRID(grid, ceil_div(a.rows, block / 32));
-    spmm_wave_per_row_fused_kernel<32><<<grid, block, 0, s>>>(a.rows, N, a.row_ptr, a.col_idx, a.val, a.B, a.C,
+    launch_chained(spmm_wave_per_row_fused_kernel<32>, grid, block, 0, s, a.rows, N, a.row_ptr, a.col_idx, a.val, a.B, a.C,
                                                                a.accumulate);
     return cudaGetLastError();
   }
@@ -823,7 +831,7 @@ cudaError_t launch_spmm_thread_per_position(const CsrSpmmArgs &a, int block, int
     cudaError_t e = launch_fill_zero(a.C, a.rows * a.n_rhs, block, s, launches);
     if (e != cudaSuccess) return e;
   }
-  spmm_thread_per_position_kernel<<<grid, block, 0, s>>>(a.rows, a.nnz, a.n_rhs, chunk, a.row_ptr,
+  launch_chained(spmm_thread_per_position_kernel, grid, block, 0, s, a.rows, a.nnz, a.n_rhs, chunk, a.row_ptr,
                                                          a.col_idx, a.val, a.B, a.C);
   ++*launches;
   return cudaGetLastError();

@@ -23,6 +23,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, V * R > 4 || Q > 8 ? 8 : 10)
                             const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col,
                             const float *__restrict__ val, const float *__restrict__ B, float *__restrict__ C,
                             bool accumulate) {
+  after_previous_kernel();
   constexpr int U = V * R >= 16 ? 1 : V * R >= 8 ? 2 : Q;  // rows of B in flight: at most 16 registers of them, or Q
   __shared__ __align__(16) int2 s_pos[STAGE_POSITIONS + 16];  // (column, value bits)
   __shared__ int s_off[STAGE_ROWS + 1];

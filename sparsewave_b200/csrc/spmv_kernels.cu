@@ -8,6 +8,7 @@
 // cooperative mappings add the same products in a tree order.
 #include <atomic>
 
+#include "swb_chain.cuh"
 #include "swb_index.h"
 #include "swb_kernels.h"
 
@@ -77,9 +78,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // zero fill (buildOutputInitialization, SparsePositionScheduling.cpp:31-47)
 // ---------------------------------------------------------------------------
 __global__ void fill_zero_kernel(float *__restrict__ y, int64_t n) {
-  // A kernel launched behind this one with programmatic stream serialisation may start its prologue now
-  // (it waits with griddepcontrol.wait before it touches y).
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  after_previous_kernel();  // the kernel behind this one may start its prologue now: it reads the matrix before it waits
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (; i < n; i += stride) y[i] = 0.0f;
@@ -156,6 +155,7 @@ __global__ void spmv_wave_per_row_kernel(int64_t rows, const int32_t *__restrict
                                          const float *__restrict__ val,
                                          const float *__restrict__ x, float *__restrict__ y,
                                          bool vec_ok) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -288,6 +288,7 @@ __global__ void spmv_thread_per_position_kernel(int64_t rows, int64_t nnz, int64
                                                 const float *__restrict__ val,
                                                 const float *__restrict__ x,
                                                 float *__restrict__ y, PositionTrace trace) {
+  after_previous_kernel();
   const int64_t worker = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t begin, end;
   chunk_bounds(0, nnz, worker, chunk, begin, end);
@@ -386,6 +387,7 @@ __global__ void coo_spmv_thread_per_nonzero_kernel(int64_t nnz, const int32_t *_
                                                    const int32_t *__restrict__ col,
                                                    const float *__restrict__ val,
                                                    const float *__restrict__ x, float *__restrict__ y) {
+  after_previous_kernel();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (WHOLE_WARPS) {
     // Entries of one row that sit in adjacent lanes (row-sorted files) share one atomicAdd.
@@ -460,6 +462,7 @@ __global__ void __launch_bounds__(MAX_BLOCK) spmv_wave_per_position_kernel(int64
                                               const float *__restrict__ val,
                                               const float *__restrict__ x, float *__restrict__ y,
                                               PositionTrace trace) {
+  after_previous_kernel();
   extern __shared__ int smem_rows[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -668,7 +671,7 @@ cudaError_t launch_fill_zero(float *y, int64_t n, int block, cudaStream_t s, int
   // is capped and threads stride, which stores the same zeros.
   int64_t blocks = max1(ceil_div(n, block));
   if (blocks > 148 * 32) blocks = 148 * 32;
-  fill_zero_kernel<<<(unsigned)blocks, block, 0, s>>>(y, n);
+  launch_chained(fill_zero_kernel, (unsigned)blocks, block, 0, s, y, n);
   ++*launches;
   return cudaGetLastError();
 }
@@ -679,9 +682,9 @@ cudaError_t launch_coo_spmv_thread_per_nonzero(int64_t rows, int64_t nnz, const 
   cudaError_t e = launch_fill_zero(y, rows, block, s, launches);
   if (e != cudaSuccess) return e;
   if (block % 32 == 0)
-    coo_spmv_thread_per_nonzero_kernel<true><<<grid_of(ceil_div(nnz, block)), block, 0, s>>>(nnz, row, col, val, x, y);
+    launch_chained(coo_spmv_thread_per_nonzero_kernel<true>, grid_of(ceil_div(nnz, block)), block, 0, s, nnz, row, col, val, x, y);
   else
-    coo_spmv_thread_per_nonzero_kernel<false><<<grid_of(ceil_div(nnz, block)), block, 0, s>>>(nnz, row, col, val, x, y);
+    launch_chained(coo_spmv_thread_per_nonzero_kernel<false>, grid_of(ceil_div(nnz, block)), block, 0, s, nnz, row, col, val, x, y);
   ++*launches;
   return cudaGetLastError();
 }
@@ -713,7 +716,7 @@ cudaError_t launch_spmv_thread_per_row(const CsrSpmvArgs &a, cudaStream_t s, int
 cudaError_t launch_spmv_wave_per_row(const CsrSpmvArgs &a, int block, cudaStream_t s,
                                      int64_t *launches) {
   const bool vec_ok = aligned16(a.col_idx) && aligned16(a.val);
-  spmv_wave_per_row_kernel<<<grid_of(ceil_div(a.rows, block / 32)), block, 0, s>>>(
+  launch_chained(spmv_wave_per_row_kernel, grid_of(ceil_div(a.rows, block / 32)), block, 0, s,
       a.rows, a.row_ptr, a.col_idx, a.val, a.x, a.y, vec_ok);
   ++*launches;
   return cudaGetLastError();
@@ -742,10 +745,10 @@ cudaError_t launch_spmv_thread_per_position(const CsrSpmvArgs &a, int block, int
 #define SWB_TPP(SEG, TR)                                                                         \
   do {                                                                                           \
     if (coop)                                                                                    \
-      spmv_thread_per_position_kernel<SEG, TR, true><<<grid, block, 0, s>>>(                      \
+      launch_chained(spmv_thread_per_position_kernel<SEG, TR, true>, grid, block, 0, s,                       \
           a.rows, a.nnz, chunk, a.row_ptr, a.col_idx, a.val, a.x, a.y, trace);                    \
     else                                                                                         \
-      spmv_thread_per_position_kernel<SEG, TR, false><<<grid, block, 0, s>>>(                     \
+      launch_chained(spmv_thread_per_position_kernel<SEG, TR, false>, grid, block, 0, s,                      \
           a.rows, a.nnz, chunk, a.row_ptr, a.col_idx, a.val, a.x, a.y, trace);                    \
   } while (0)
   if (trace.enabled()) {
@@ -871,7 +874,7 @@ cudaError_t launch_spmv_wave_per_position(const CsrSpmvArgs &a, int block, int64
       cudaLaunchKernelEx(&cfg, spmv_wave_span_kernel<TR, MB>, a.rows, a.nnz, waves, batch, a.row_ptr, a.col_idx, \
                          a.val, a.x, a.y, trace, long_min, shift);                         \
     else                                                                                  \
-      spmv_wave_per_position_kernel<TR, MB><<<(unsigned)grid, block, smem, s>>>(           \
+      launch_chained(spmv_wave_per_position_kernel<TR, MB>, (unsigned)grid, block, smem, s,            \
           a.rows, a.nnz, waves, batch, a.row_ptr, a.col_idx, a.val, a.x, a.y, trace);      \
   } while (0)
   if (trace.enabled()) {
