@@ -155,7 +155,6 @@ __global__ void spmv_wave_per_row_kernel(int64_t rows, const int32_t *__restrict
                                          const float *__restrict__ val,
                                          const float *__restrict__ x, float *__restrict__ y,
                                          bool vec_ok) {
-  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -192,6 +191,8 @@ __global__ void spmv_block_per_row_kernel(int64_t rows, const int32_t *__restric
     if (lane == 0) y[row] = v;
   }
 }
+
+#include "spmv_rows.cuh"
 
 // ---------------------------------------------------------------------------
 // thread-per-position (ThreadPositionReducePattern and
@@ -713,21 +714,99 @@ cudaError_t launch_spmv_thread_per_row(const CsrSpmvArgs &a, cudaStream_t s, int
   return launch_row_products({a.rows, a.cols, a.nnz, 1, a.row_ptr, a.col_idx, a.val, a.x, a.y}, s);
 }
 
-cudaError_t launch_spmv_wave_per_row(const CsrSpmvArgs &a, int block, cudaStream_t s,
+namespace {
+
+// x reaches beyond L1, a good part of it can be staged, and the gathers saved cost more than staging it (4 us).
+inline bool stages_x(const CsrSpmvArgs &a) {
+  return a.cols > SHARED_X_FLOATS && a.cols <= 4 * SHARED_X_FLOATS && aligned16(a.x) &&
+         a.nnz / a.cols * SHARED_X_FLOATS >= 4000000;
+}
+
+template <int L>
+cudaError_t launch_rows_of(const CsrSpmvArgs &a, const DeviceInfo &dev, cudaStream_t s) {
+  int64_t blocks = ceil_div(a.rows, ROWS_THREADS / L);
+  if (blocks > (int64_t)dev.sm_count * 8) blocks = (int64_t)dev.sm_count * 8;
+  return launch_chained(spmv_rows_kernel<L>, grid_of(blocks), ROWS_THREADS, 0, s, a.rows, a.nnz, a.row_ptr, a.col_idx,
+                        a.val, a.x, a.y);
+}
+
+// Lanes per row so that a row of mean length is in flight at once.
+int lanes_per_short_row(int64_t mean) { return mean <= 24 ? 4 : mean <= 50 ? 8 : 16; }
+
+cudaError_t launch_short_rows(const CsrSpmvArgs &a, const DeviceInfo &dev, cudaStream_t s) {
+  switch (lanes_per_short_row(a.nnz / a.rows)) {
+    case 4: return launch_rows_of<4>(a, dev, s);
+    case 8: return launch_rows_of<8>(a, dev, s);
+  }
+  return launch_rows_of<16>(a, dev, s);
+}
+
+cudaError_t launch_row_stream(const CsrSpmvArgs &a, const DeviceInfo &dev, cudaStream_t s) {
+  static std::atomic<bool> configured[64];  // once per device; racing threads repeat an idempotent call
+  int device = 0;
+  cudaGetDevice(&device);
+  if (device < 0 || device >= 64 || !configured[device].load(std::memory_order_acquire)) {
+    cudaError_t e = cudaFuncSetAttribute(spmv_row_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SHARED_X_FLOATS * 4);
+    if (e != cudaSuccess) return e;
+    if (device >= 0 && device < 64) configured[device].store(true, std::memory_order_release);
+  }
+  return launch_chained(spmv_row_stream_kernel, (unsigned)dev.sm_count, SHARED_X_THREADS, SHARED_X_FLOATS * 4, s,
+                        a.rows, a.nnz, a.row_ptr, a.col_idx, a.val, a.x, a.y);
+}
+
+enum class RowForm { REFERENCE, SHORT_ROWS, STREAM };
+
+// wave-per-row keeps a warp per row, on its own grid, for rows of some 50 positions in matrices below 4 M nonzeros, where
+// the longest rows decide (20,000 ragged rows of 30: 6.4 us against 7.6), and for rows of more than 100 unless x is
+// staged; block-per-row keeps a block per row there, and on few rows.
+RowForm row_form(const CsrSpmvArgs &a, bool block_per_row) {
+  if (!aligned16(a.col_idx) || !aligned16(a.val) || a.rows == 0) return RowForm::REFERENCE;
+  if (a.nnz > 2147483647LL - 65536) return RowForm::REFERENCE;  // positions of a step reach past a row's end
+  const int64_t mean = a.nnz / a.rows;
+  if (block_per_row && a.rows < 148 * 8) return RowForm::REFERENCE;
+  if (mean <= 24 || (mean <= 100 && (block_per_row || a.nnz >= 4000000))) return RowForm::SHORT_ROWS;
+  return mean > 100 && stages_x(a) ? RowForm::STREAM : RowForm::REFERENCE;
+}
+
+}  // namespace
+
+int64_t row_mapping_physical_grid(int64_t rows, int64_t cols, int64_t nnz, bool block_per_row, int block,
+                                  const DeviceInfo &dev) {
+  switch (row_form({rows, cols, nnz}, block_per_row)) {
+    case RowForm::STREAM: return dev.sm_count;
+    case RowForm::SHORT_ROWS: {
+      const int64_t blocks = ceil_div(rows, ROWS_THREADS / lanes_per_short_row(nnz / rows));
+      return blocks < (int64_t)dev.sm_count * 8 ? blocks : (int64_t)dev.sm_count * 8;
+    }
+    case RowForm::REFERENCE: break;
+  }
+  return max1(block_per_row ? rows : ceil_div(rows, block / 32));
+}
+
+cudaError_t launch_spmv_wave_per_row(const CsrSpmvArgs &a, int block, const DeviceInfo &dev, cudaStream_t s,
                                      int64_t *launches) {
-  const bool vec_ok = aligned16(a.col_idx) && aligned16(a.val);
-  launch_chained(spmv_wave_per_row_kernel, grid_of(ceil_div(a.rows, block / 32)), block, 0, s,
-      a.rows, a.row_ptr, a.col_idx, a.val, a.x, a.y, vec_ok);
   ++*launches;
+  switch (row_form(a, false)) {
+    case RowForm::SHORT_ROWS: return launch_short_rows(a, dev, s);
+    case RowForm::STREAM: return launch_row_stream(a, dev, s);
+    case RowForm::REFERENCE: break;
+  }
+  spmv_wave_per_row_kernel<<<grid_of(ceil_div(a.rows, block / 32)), block, 0, s>>>(
+      a.rows, a.row_ptr, a.col_idx, a.val, a.x, a.y, aligned16(a.col_idx) && aligned16(a.val));
   return cudaGetLastError();
 }
 
-cudaError_t launch_spmv_block_per_row(const CsrSpmvArgs &a, int block, cudaStream_t s,
+cudaError_t launch_spmv_block_per_row(const CsrSpmvArgs &a, int block, const DeviceInfo &dev, cudaStream_t s,
                                       int64_t *launches) {
-  const bool vec_ok = aligned16(a.col_idx) && aligned16(a.val);
-  spmv_block_per_row_kernel<<<grid_of(a.rows), block, 0, s>>>(a.rows, a.row_ptr, a.col_idx,
-                                                               a.val, a.x, a.y, vec_ok);
   ++*launches;
+  switch (row_form(a, true)) {
+    case RowForm::SHORT_ROWS: return launch_short_rows(a, dev, s);
+    case RowForm::STREAM: return launch_row_stream(a, dev, s);
+    case RowForm::REFERENCE: break;
+  }
+  spmv_block_per_row_kernel<<<grid_of(a.rows), block, 0, s>>>(a.rows, a.row_ptr, a.col_idx, a.val, a.x, a.y,
+                                                              aligned16(a.col_idx) && aligned16(a.val));
   return cudaGetLastError();
 }
 

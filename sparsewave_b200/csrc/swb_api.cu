@@ -493,12 +493,12 @@ int swb_launch_shape_query(swb_context *ctx, const swb_options *o, int64_t rows,
       case SWB_WAVE_PER_ROW:
         r.work_units = rows;
         r.logical_grid = max1(ceil_div(rows, B / 32));
-        r.physical_grid = r.logical_grid;
+        r.physical_grid = swb::row_mapping_physical_grid(rows, rows, nnz, false, (int)B, dev);  // as of a square matrix
         break;
       case SWB_BLOCK_PER_ROW:
         r.work_units = rows;
         r.logical_grid = max1(rows);
-        r.physical_grid = r.logical_grid;
+        r.physical_grid = swb::row_mapping_physical_grid(rows, rows, nnz, true, (int)B, dev);
         break;
       case SWB_THREAD_PER_POSITION:
         r.work_units = ceil_div(nnz, o->position_chunk_size);
@@ -580,8 +580,8 @@ static int spmv_impl(swb_context *ctx, const swb_options *o, int64_t rows, int64
   cudaError_t e = cudaSuccess;
   switch (o->mapping) {
     case SWB_THREAD_PER_ROW: e = swb::launch_spmv_thread_per_row(a, stream, &ctx->launches); break;
-    case SWB_WAVE_PER_ROW: e = swb::launch_spmv_wave_per_row(a, B, stream, &ctx->launches); break;
-    case SWB_BLOCK_PER_ROW: e = swb::launch_spmv_block_per_row(a, B, stream, &ctx->launches); break;
+    case SWB_WAVE_PER_ROW: e = swb::launch_spmv_wave_per_row(a, B, ctx->dev, stream, &ctx->launches); break;
+    case SWB_BLOCK_PER_ROW: e = swb::launch_spmv_block_per_row(a, B, ctx->dev, stream, &ctx->launches); break;
     case SWB_THREAD_PER_POSITION:
       e = swb::launch_spmv_thread_per_position(a, B, o->position_chunk_size,
                                                o->position_reduction == SWB_REDUCTION_SEGMENTED, trace,

@@ -1,0 +1,42 @@
+"""wave-per-row and block-per-row SpMV: a group of lanes per short row, and the stream of rows with x in shared memory."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from tests.helpers import assert_within_bound, dev
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(ctx, opts, lens, cols, seed, grid_below=None):
+    rng = np.random.default_rng(seed)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = rng.integers(0, cols, rp[-1]).astype(np.int32)
+    v, x = rng.uniform(-1, 1, rp[-1]).astype(np.float32), rng.uniform(-1, 1, cols).astype(np.float32)
+    y = torch.full((len(lens),), 9.0, device="cuda")
+    ctx.spmv(opts, dev(rp), dev(ci), dev(v), dev(x), y)
+    assert_within_bound(y.cpu().numpy(), oracle.csr_spmv(rp, ci, v, x, parallel=True), oracle.csr_abs_bound(rp, ci, v, x))
+    if grid_below:
+        assert ctx.launch_shape(opts, len(lens), int(rp[-1])).physical_grid < grid_below
+
+
+@pytest.mark.parametrize("mapping", ["wave-per-row", "block-per-row"])
+@pytest.mark.parametrize("mean", [1, 20, 24, 40, 50, 90])  # 4, 8 and 16 lanes per row
+def test_short_rows(ctx, mapping, mean):
+    rng = np.random.default_rng(mean)
+    # more rows than groups of lanes in the grid; rows below, at and above what a group and a warp take at once
+    lens = rng.integers(0, 2 * mean + 1, 160000 if mean < 30 else 90000)
+    lens[rng.integers(0, len(lens), 40)] = [0, 1, 3, 4, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 513, 1000, 5000,
+                                            8191] * 2
+    lens[-1] = 3
+    _check(ctx, f"spmv-mapping={mapping}", lens, 3000, mean, grid_below=148 * 8 + 1)
+
+
+@pytest.mark.parametrize("mapping", ["wave-per-row", "block-per-row"])
+@pytest.mark.parametrize("cols", [49153, 70001, 196608])
+def test_rows_with_x_in_shared_memory(ctx, mapping, cols):
+    rng = np.random.default_rng(cols)
+    lens = rng.integers(0, 400, 4 * cols * 1000000 // 49152 // 200 * 5 // 4 + 100)
+    lens[[0, 5, -1]] = 0, 20000, 1
+    _check(ctx, f"spmv-mapping={mapping}", lens, cols, cols)
