@@ -810,9 +810,25 @@ cudaError_t launch_spmv_block_per_row(const CsrSpmvArgs &a, int block, const Dev
   return cudaGetLastError();
 }
 
+namespace {
+
+// col and val start the same number of elements past a 16-byte boundary: what the span kernel reads.
+inline bool spans_fit(const CsrSpmvArgs &a) {
+  const uintptr_t col_off = reinterpret_cast<uintptr_t>(a.col_idx) & 15u, val_off = reinterpret_cast<uintptr_t>(a.val) & 15u;
+  return col_off == val_off && col_off % 4 == 0 && a.nnz > 0;
+}
+
+}  // namespace
+
 cudaError_t launch_spmv_thread_per_position(const CsrSpmvArgs &a, int block, int64_t chunk,
-                                            bool segmented, const PositionTrace &trace,
+                                            bool segmented, const PositionTrace &trace, const DeviceInfo &dev,
                                             cudaStream_t s, int64_t *launches) {
+  // Without a trace the schedule shows only in the order of the sums: the span kernel deals the positions to warps instead,
+  // which read col and val coalesced whatever the chunk size (23 M power-law nonzeros: atomic chunk 1 330 -> 114 us,
+  // segmented chunk 8 150 -> 114; 1 M ragged rows of 60, atomic: 812 -> 262).
+  if (!trace.enabled() && spans_fit(a))
+    return launch_spmv_wave_per_position(a, kThreadPerPositionSpanBlock, wave_per_position_auto_batch(a.nnz, kThreadPerPositionSpanBlock, dev),
+                                         trace, s, launches, nullptr, nullptr, nullptr, dev);
   if (!a.accumulate) {
     cudaError_t e = launch_fill_zero(a.y, a.rows, block, s, launches);
     if (e != cudaSuccess) return e;
@@ -881,6 +897,17 @@ size_t band_scratch_bytes(const BandPlan &plan) {
   return 256 + 2 * (size_t)plan.cap * 4 + (size_t)(plan.bands + 1) * (size_t)plan.cap * 4;
 }
 
+namespace {
+
+template <bool TRACE, int MAX_BLOCK>
+auto span_kernel(int64_t cols, int64_t nnz) {
+  // 1 MB of x: beyond it L1 holds too little of it; 32 M nonzeros: 256 MB of streams, twice the L2
+  return cols <= 262144 || nnz < 32000000 ? spmv_wave_span_kernel<TRACE, MAX_BLOCK, true>
+                                          : spmv_wave_span_kernel<TRACE, MAX_BLOCK, false>;
+}
+
+}  // namespace
+
 cudaError_t launch_spmv_wave_per_position(const CsrSpmvArgs &a, int block, int64_t batch,
                                           const PositionTrace &trace, cudaStream_t s,
                                           int64_t *launches, int64_t *physical_grid,
@@ -894,9 +921,8 @@ cudaError_t launch_spmv_wave_per_position(const CsrSpmvArgs &a, int block, int64
   // the register-capped instantiation.
   // col and val views that start the same number of elements past a 16-byte boundary take the span kernel
   // too (it reads from that boundary); other misalignments take the scalar kernel.
-  const uintptr_t col_off = reinterpret_cast<uintptr_t>(a.col_idx) & 15u, val_off = reinterpret_cast<uintptr_t>(a.val) & 15u;
-  const bool span = batch >= 2 && col_off == val_off && col_off % 4 == 0 && a.nnz > 0;
-  const int shift = span ? (int)(col_off / 4) : 0;
+  const bool span = batch >= 2 && spans_fit(a);
+  const int shift = span ? (int)((reinterpret_cast<uintptr_t>(a.col_idx) & 15u) / 4) : 0;
   const bool banded = span && shift == 0 && band && band_scratch && !trace.enabled();
   int long_min = 0;
   int *count = nullptr, *long_rows = nullptr, *strides = nullptr, *tab = nullptr;
@@ -950,7 +976,7 @@ cudaError_t launch_spmv_wave_per_position(const CsrSpmvArgs &a, int block, int64
 #define SWB_WPP(TR, MB)                                                                   \
   do {                                                                                    \
     if (span)                                                                             \
-      cudaLaunchKernelEx(&cfg, spmv_wave_span_kernel<TR, MB>, a.rows, a.nnz, waves, batch, a.row_ptr, a.col_idx, \
+      cudaLaunchKernelEx(&cfg, span_kernel<TR, MB>(a.cols, a.nnz), a.rows, a.nnz, waves, batch, a.row_ptr, a.col_idx, \
                          a.val, a.x, a.y, trace, long_min, shift);                         \
     else                                                                                  \
       launch_chained(spmv_wave_per_position_kernel<TR, MB>, (unsigned)grid, block, smem, s,            \

@@ -42,6 +42,12 @@
 
 constexpr int SPAN_CHUNK = 128;
 
+template <bool CACHE_X>
+__device__ __forceinline__ float gather_of(const float *p) {
+  if constexpr (CACHE_X) return __ldg(p);
+  else return ld_x(p);
+}
+
 template <bool TRACE>
 struct SpanEmit {
   float *y;
@@ -56,7 +62,12 @@ struct SpanEmit {
   }
 };
 
-template <bool TRACE, int MAX_BLOCK>
+// CACHE_X: x goes through L1, with no eviction priority in L2.  Gathers of a small x that bypass L1 queue up on few L2 lines
+// (16.8 M gathers of an x of 64 KB: 27 us through L1, 119 without), and the kernel needs 32 registers instead of 40, so
+// that all warps of an SM are in flight, which short rows need (500,000 ragged rows of 20: 58.5 us against 63.3).  Large
+// matrices take neither: their streams would push x out of L2, and long spans fill the memory system with fewer warps
+// (92 M power-law nonzeros: 404 -> 397 us).
+template <bool TRACE, int MAX_BLOCK, bool CACHE_X>
 __global__ void __launch_bounds__(MAX_BLOCK) spmv_wave_span_kernel(
     int64_t rows, int64_t nnz, int64_t wave_count, int64_t batch, const int32_t *__restrict__ row_ptr,
     const int32_t *__restrict__ col, const float *__restrict__ val, const float *__restrict__ x,
@@ -145,10 +156,10 @@ __global__ void __launch_bounds__(MAX_BLOCK) spmv_wave_span_kernel(
     load_chunk(cb + SPAN_CHUNK, cn, vn);
     const bool m0 = p0 + 0 >= sb && p0 + 0 < ce, m1 = p0 + 1 >= sb && p0 + 1 < ce;
     const bool m2 = p0 + 2 >= sb && p0 + 2 < ce, m3 = p0 + 3 >= sb && p0 + 3 < ce;
-    const float q0 = m0 ? mul(v.x, ld_x(x + c.x)) : 0.0f;
-    const float q1 = m1 ? mul(v.y, ld_x(x + c.y)) : 0.0f;
-    const float q2 = m2 ? mul(v.z, ld_x(x + c.z)) : 0.0f;
-    const float q3 = m3 ? mul(v.w, ld_x(x + c.w)) : 0.0f;
+    const float q0 = m0 ? mul(v.x, gather_of<CACHE_X>(x + c.x)) : 0.0f;
+    const float q1 = m1 ? mul(v.y, gather_of<CACHE_X>(x + c.y)) : 0.0f;
+    const float q2 = m2 ? mul(v.z, gather_of<CACHE_X>(x + c.z)) : 0.0f;
+    const float q3 = m3 ? mul(v.w, gather_of<CACHE_X>(x + c.w)) : 0.0f;
 
     if (next_b >= ce) {
       // The whole chunk lies in row R.
