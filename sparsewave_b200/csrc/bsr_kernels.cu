@@ -72,24 +72,24 @@ __device__ __forceinline__ void store(__nv_bfloat16 *p, const float (&v)[n]) {
 constexpr int TILE_THREADS = 128;
 template <int n> struct Count { static constexpr int value = n; };
 
-// BS: the block size where it is a constant (TR = BS rows, K = BS or 4 local columns per load), or 0: any bs, tiles of
-// TR = 8 rows.  WIDE: block values are aligned for loads of K.
-template <typename T, int BS, int V, bool WIDE>
-__global__ void __launch_bounds__(TILE_THREADS, BS == 4 ? 7 : 1) bsr_spmm_row_tile_kernel(int64_t brows, int64_t N, int64_t block_size, int tiles,
+// BS: the block size where it is a constant (K = BS or 4 local columns per load), or 0: any bs.  TR rows per thread.
+// WIDE: block values are aligned for loads of K.
+template <typename T, int BS, int TR, int V, bool WIDE>
+__global__ void __launch_bounds__(TILE_THREADS, BS == 4 && TR == 4 ? 7 : 1) bsr_spmm_row_tile_kernel(int64_t brows, int64_t N, int64_t block_size, int tiles,
                                                                 const int32_t *__restrict__ brp,
                                                                 const int32_t *__restrict__ bci,
                                                                 const T *__restrict__ bv, const T *__restrict__ B,
                                                                 T *__restrict__ C) {
   after_previous_kernel();
-  constexpr int TR = BS ? BS : 8;
+  constexpr bool WHOLE = BS == TR;  // one tile per block row
   constexpr int K = BS ? (BS % 4 == 0 ? 4 : BS) : 4;
-  constexpr bool AHEAD = BS == 3 || BS == 4 || BS == 8;  // rows of B requested a step ahead of their sums
+  constexpr bool AHEAD = (BS == 3 || BS == 4 || BS == 8) && WHOLE;  // rows of B requested a step ahead of their sums
   const int64_t bs = BS ? BS : block_size, G = N / V;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t unit = t / G, g = t - unit * G;
-  const int64_t brow = BS ? unit : unit / tiles;
+  const int64_t brow = WHOLE ? unit : unit / tiles;
   if (brow >= brows) return;
-  const int r0 = BS ? 0 : (int)(unit - brow * tiles) * TR;
+  const int r0 = WHOLE ? 0 : (int)(unit - brow * tiles) * TR;
   const T *Bt = B + g * V;
   float acc[TR][V];
 #pragma unroll
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(TILE_THREADS, BS == 4 ? 7 : 1) bsr_spmm_row_ti
 #pragma unroll
     for (int r = 0; r < TR; ++r) {
       // a tile that reaches past the block repeats its last row, which is not stored
-      const int64_t row = BS ? r : (r0 + r < bs ? r0 + r : bs - 1);
+      const int64_t row = WHOLE ? r : BS ? r0 + r : (r0 + r < bs ? r0 + r : bs - 1);
       float aw[W];
       const T *p = a + row * bs + lc;
       if constexpr (WIDE && W > 1) {
@@ -174,15 +174,15 @@ __global__ void __launch_bounds__(TILE_THREADS, BS == 4 ? 7 : 1) bsr_spmm_row_ti
     if (BS || r0 + r < bs) store<V>(C + (brow * bs + r0 + r) * N + g * V, acc[r]);
 }
 
-template <typename T, int BS, int V>
+template <typename T, int BS, int TR, int V>
 cudaError_t launch_tiles(const BsrSpmmArgs &a, cudaStream_t s) {
-  const int64_t bs = a.block_size, brows = a.rows / bs, tiles = BS ? 1 : ceil_div(bs, 8);
+  const int64_t bs = a.block_size, brows = a.rows / bs, tiles = ceil_div(bs, TR);
   unsigned grid = 0;  // refused, not truncated, beyond the CUDA grid limit
   if (!grid_dim(ceil_div(brows * tiles * (a.n_rhs / V), TILE_THREADS), &grid)) return cudaErrorInvalidConfiguration;
   // loads of K values start at multiples of K from an aligned base (K divides bs where BS is constant)
   const bool wide = reinterpret_cast<uintptr_t>(a.block_values) % (4 * sizeof(T)) == 0 && (BS == 2 || bs % 4 == 0);
 #define SWB_BSR(WIDE)                                                                                             \
-  launch_chained(bsr_spmm_row_tile_kernel<T, BS, V, WIDE>, grid, TILE_THREADS, 0, s,                                                    \
+  launch_chained(bsr_spmm_row_tile_kernel<T, BS, TR, V, WIDE>, grid, TILE_THREADS, 0, s,                          \
       brows, a.n_rhs, bs, (int)tiles, a.block_row_ptr, a.block_col_idx, static_cast<const T *>(a.block_values), \
       static_cast<const T *>(a.B), static_cast<T *>(a.C))
   if (wide) SWB_BSR(true); else SWB_BSR(false);
@@ -191,15 +191,15 @@ cudaError_t launch_tiles(const BsrSpmmArgs &a, cudaStream_t s) {
 }
 
 template <typename T, int V>
-cudaError_t launch_columns(const BsrSpmmArgs &a, cudaStream_t s) {
+cudaError_t launch_columns(const BsrSpmmArgs &a, bool few, cudaStream_t s) {
   switch (a.block_size) {
-    case 1: return launch_tiles<T, 1, V>(a, s);
-    case 2: return launch_tiles<T, 2, V>(a, s);
-    case 3: return launch_tiles<T, 3, V>(a, s);
-    case 4: return launch_tiles<T, 4, V>(a, s);
-    case 8: return launch_tiles<T, 8, V>(a, s);
+    case 1: return launch_tiles<T, 1, 1, V>(a, s);
+    case 2: return launch_tiles<T, 2, 2, V>(a, s);
+    case 3: return launch_tiles<T, 3, 3, V>(a, s);
+    case 4: return few ? launch_tiles<T, 4, 2, V>(a, s) : launch_tiles<T, 4, 4, V>(a, s);
+    case 8: return few ? launch_tiles<T, 8, 2, V>(a, s) : launch_tiles<T, 8, 8, V>(a, s);
   }
-  return launch_tiles<T, 0, V>(a, s);
+  return few ? launch_tiles<T, 0, 2, V>(a, s) : launch_tiles<T, 0, 8, V>(a, s);
 }
 
 template <typename T>
@@ -207,13 +207,15 @@ cudaError_t launch(const BsrSpmmArgs &a, cudaStream_t s, int64_t *launches) {
   ++*launches;
   // As many columns per thread, up to four, as rows of B and C are aligned to; small blocks keep 65,536 threads, enough to
   // hide the gathers (larger ones have more rows of B in flight per thread: 16 x 16 blocks, 20 per block row, N = 64
-  // 77 us with four columns, 176 with one).
+  // 77 us with four columns, 176 with one).  Two rows per thread where eight would leave less than 20,000 threads
+  // (201 block rows of 52 blocks of 32 x 32, N = 24: 207 us with eight, 122 with two).
   const uintptr_t at = reinterpret_cast<uintptr_t>(a.B) | reinterpret_cast<uintptr_t>(a.C);
   int V = a.n_rhs % 4 == 0 && at % (4 * sizeof(T)) == 0 ? 4 : a.n_rhs % 2 == 0 && at % (2 * sizeof(T)) == 0 ? 2 : 1;
   if (a.block_size <= 8)
     while (V > 1 && a.rows / a.block_size * (a.n_rhs / V) < 65536) V /= 2;
-  if (V == 4) return launch_columns<T, 4>(a, s);
-  return V == 2 ? launch_columns<T, 2>(a, s) : launch_columns<T, 1>(a, s);
+  const bool few = a.rows / a.block_size * ceil_div(a.block_size, 8) * (a.n_rhs / V) < 20000;
+  if (V == 4) return launch_columns<T, 4>(a, few, s);
+  return V == 2 ? launch_columns<T, 2>(a, few, s) : launch_columns<T, 1>(a, few, s);
 }
 
 }  // namespace

@@ -26,7 +26,7 @@ def _check(ctx, opts, lens, cols, seed, grid_below=None):
 def test_short_rows(ctx, mapping, mean):
     rng = np.random.default_rng(mean)
     # more rows than groups of lanes in the grid; rows below, at and above what a group and a warp take at once
-    lens = rng.integers(0, 2 * mean + 1, 160000 if mean < 30 else 90000)
+    lens = rng.integers(0, 2 * mean + 1, 160000 if mean < 30 else 120000)
     lens[rng.integers(0, len(lens), 40)] = [0, 1, 3, 4, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 513, 1000, 5000,
                                             8191] * 2
     lens[-1] = 3
