@@ -503,7 +503,9 @@ int swb_launch_shape_query(swb_context *ctx, const swb_options *o, int64_t rows,
       case SWB_THREAD_PER_POSITION:
         r.work_units = ceil_div(nnz, o->position_chunk_size);
         r.logical_grid = max1(ceil_div(r.work_units, B));
-        r.physical_grid = r.logical_grid;
+        r.physical_grid = swb::wave_per_position_physical_grid(
+            nnz, swb::kThreadPerPositionSpanBlock,
+            swb::wave_per_position_auto_batch(nnz, swb::kThreadPerPositionSpanBlock, dev));
         r.kernels = 2;
         break;
       case SWB_WAVE_PER_POSITION: {
@@ -584,7 +586,7 @@ static int spmv_impl(swb_context *ctx, const swb_options *o, int64_t rows, int64
     case SWB_BLOCK_PER_ROW: e = swb::launch_spmv_block_per_row(a, B, ctx->dev, stream, &ctx->launches); break;
     case SWB_THREAD_PER_POSITION:
       e = swb::launch_spmv_thread_per_position(a, B, o->position_chunk_size,
-                                               o->position_reduction == SWB_REDUCTION_SEGMENTED, trace,
+                                               o->position_reduction == SWB_REDUCTION_SEGMENTED, trace, ctx->dev,
                                                stream, &ctx->launches);
       break;
     case SWB_WAVE_PER_POSITION: {

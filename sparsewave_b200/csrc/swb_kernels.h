@@ -85,8 +85,9 @@ int64_t row_mapping_physical_grid(int64_t rows, int64_t cols, int64_t nnz, bool 
 // --- SpMV position mappings (each also launches the zero fill)
 cudaError_t launch_spmv_thread_per_position(const CsrSpmvArgs &a, int block,
                                             int64_t chunk, bool segmented,
-                                            const PositionTrace &trace,
+                                            const PositionTrace &trace, const DeviceInfo &dev,
                                             cudaStream_t s, int64_t *launches);
+constexpr int kThreadPerPositionSpanBlock = 128;  // threads per block of its untraced form (aligned arrays)
 // Long rows of a large matrix through shared-memory bands of x (spmv_band.cuh): `bands` bands of columns,
 // rows of at least `long_min` positions, room for `cap` such rows in the scratch memory.
 struct BandPlan {
