@@ -790,16 +790,29 @@ int swb_check_csr_host(swb_context *ctx, int64_t rows, int64_t cols, int64_t nnz
   if (st != SWB_OK) return st;
   if (!row_ptr || (nnz > 0 && !col_idx)) return fail(ctx, SWB_ERR_INVALID_ARGUMENT, "csr: NULL operand pointer");
   if (row_ptr[0] != 0) return fail(ctx, SWB_ERR_INVALID_DATA, "row offsets must start at 0, but got %d", row_ptr[0]);
-  for (int64_t r = 0; r < rows; ++r)
-    if (row_ptr[r + 1] < row_ptr[r])
-      return fail(ctx, SWB_ERR_INVALID_DATA, "row offsets must be non-decreasing, but row %lld has %d > %d",
-                  (long long)r, row_ptr[r], row_ptr[r + 1]);
+  // Both arrays are looked over in pieces without an exit inside (the compiler vectorises that), a bad piece entry by entry.
+  constexpr int64_t kPiece = 8192;
+  for (int64_t r0 = 0; r0 < rows; r0 += kPiece) {
+    const int64_t r1 = r0 + kPiece < rows ? r0 + kPiece : rows;
+    int32_t bad = 0;
+    for (int64_t r = r0; r < r1; ++r) bad |= row_ptr[r + 1] < row_ptr[r];
+    for (int64_t r = r0; bad && r < r1; ++r)
+      if (row_ptr[r + 1] < row_ptr[r])
+        return fail(ctx, SWB_ERR_INVALID_DATA, "row offsets must be non-decreasing, but row %lld has %d > %d",
+                    (long long)r, row_ptr[r], row_ptr[r + 1]);
+  }
   if (row_ptr[rows] != nnz)
     return fail(ctx, SWB_ERR_INVALID_DATA, "last row offset must equal NNZ, but got %d and %lld", row_ptr[rows], (long long)nnz);
-  for (int64_t p = 0; p < nnz; ++p)
-    if (col_idx[p] < 0 || col_idx[p] >= cols)
-      return fail(ctx, SWB_ERR_INVALID_DATA, "column index %d at position %lld is out of bounds for %lld columns",
-                  col_idx[p], (long long)p, (long long)cols);
+  const int32_t limit = (int32_t)cols;  // cols <= the int32 maximum
+  for (int64_t p0 = 0; p0 < nnz; p0 += kPiece) {
+    const int64_t p1 = p0 + kPiece < nnz ? p0 + kPiece : nnz;
+    int32_t bad = 0;
+    for (int64_t p = p0; p < p1; ++p) bad |= (col_idx[p] < 0) | (col_idx[p] >= limit);
+    for (int64_t p = p0; bad && p < p1; ++p)
+      if (col_idx[p] < 0 || col_idx[p] >= cols)
+        return fail(ctx, SWB_ERR_INVALID_DATA, "column index %d at position %lld is out of bounds for %lld columns",
+                    col_idx[p], (long long)p, (long long)cols);
+  }
   return SWB_OK;
 }
 
@@ -925,15 +938,15 @@ int swb_bsr_spmm_bf16_host(swb_context *ctx, const swb_options *o, int64_t rows,
 // their device-to-host copy on a second stream as soon as its kernels are done.  A panel starts at a row
 // whose first position is a multiple of 4 (of 32 where one is near), so the col/val slices keep the
 // 16-byte alignment the vectorised kernels ask for.  Environment: SWB_RESIDENT_PANEL_NNZ (nnz per panel
-// that makes a matrix worth cutting, default 20000000) and SWB_RESIDENT_PANEL_BYTES (result bytes per
-// panel below which a call runs uncut, default 524288), both read at upload.
+// that makes a matrix worth cutting, default 8000000) and SWB_RESIDENT_PANEL_BYTES (result bytes per
+// panel below which a call runs uncut, default 262144), both read at upload.
 constexpr int kMaxPanels = 8;
 
 // Column parts.  A large matrix is also stored as two matrices over the same rows, one with the entries
 // whose column lies below a cut (36 % of the columns by default) and one with the rest.  A call on a mapping that can accumulate then sends
 // the first half of the dense operand, runs the first matrix while the second half is still on its way,
 // and adds the second matrix (cut into row panels, as above) on top.  SWB_RESIDENT_SPLIT_NNZ: nnz from
-// which a matrix is stored this way (default 40000000; it doubles the matrix's device memory).
+// which a matrix is stored this way (default 3000000; it doubles the matrix's device memory).
 struct CsrPart {
   int64_t nnz = 0;
   int32_t *row_ptr = nullptr, *col_idx = nullptr;
@@ -989,7 +1002,8 @@ void free_part(CsrPart &p) {
   p = CsrPart();
 }
 
-// Copies one CSR matrix to the device and, when panel_nnz > 0, plans and stores its row panels.
+// Copies one CSR matrix to the device (col_idx NULL: only its row offsets; the entries are written there later) and, when
+// panel_nnz > 0, plans and stores its row panels.
 cudaError_t upload_part(CsrPart &p, int64_t rows, int64_t nnz, const int32_t *row_ptr, const int32_t *col_idx,
                         const float *val, int64_t panel_nnz) {
   p.nnz = nnz;
@@ -999,8 +1013,8 @@ cudaError_t upload_part(CsrPart &p, int64_t rows, int64_t nnz, const int32_t *ro
   if (e == cudaSuccess) e = cudaMalloc(&p.col_idx, (size_t)(nnz > 0 ? nnz : 1) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&p.val, (size_t)(nnz > 0 ? nnz : 1) * 4);
   if (e == cudaSuccess) e = cudaMemcpy(p.row_ptr, row_ptr, (size_t)(rows + 1) * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && nnz > 0) e = cudaMemcpy(p.col_idx, col_idx, (size_t)nnz * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && nnz > 0) e = cudaMemcpy(p.val, val, (size_t)nnz * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && nnz > 0 && col_idx) e = cudaMemcpy(p.col_idx, col_idx, (size_t)nnz * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && nnz > 0 && col_idx) e = cudaMemcpy(p.val, val, (size_t)nnz * 4, cudaMemcpyHostToDevice);
   if (e != cudaSuccess || panel_nnz <= 0 || rows <= 0 || nnz <= 0) return e;
   const int count = plan_panels(rows, nnz, row_ptr, panel_nnz, p.panel_row);
   if (count <= 1) return e;
@@ -1041,11 +1055,11 @@ static int csr_upload_impl(swb_context *ctx, int64_t rows, int64_t cols, int64_t
   if (nnz > 0 && !val) return fail(ctx, SWB_ERR_INVALID_ARGUMENT, "csr upload: NULL operand pointer");
   swb_csr_handle *h = new swb_csr_handle();
   h->rows = rows; h->cols = cols; h->nnz = nnz;
-  h->panel_min_bytes = env_i64("SWB_RESIDENT_PANEL_BYTES", 512 * 1024);
-  const int64_t panel_nnz = plain ? 0 : env_i64("SWB_RESIDENT_PANEL_NNZ", 20000000);
+  h->panel_min_bytes = env_i64("SWB_RESIDENT_PANEL_BYTES", 256 * 1024);
+  const int64_t panel_nnz = plain ? 0 : env_i64("SWB_RESIDENT_PANEL_NNZ", 8000000);
   cudaError_t e = upload_part(h->whole, rows, nnz, row_ptr, col_idx, val, panel_nnz);
 
-  if (!plain && e == cudaSuccess && rows > 0 && cols >= 2 && nnz >= env_i64("SWB_RESIDENT_SPLIT_NNZ", 40000000)) {
+  if (!plain && e == cudaSuccess && rows > 0 && cols >= 2 && nnz >= env_i64("SWB_RESIDENT_SPLIT_NNZ", 3000000)) {
     // The two column parts, each a CSR matrix over all rows with the entries in their original order.  They
     // are an optimisation: without the host or device memory for them the matrix stays resident uncut.
     // Where the columns are cut: the first part should finish computing about when the rest of the operand
@@ -1057,28 +1071,26 @@ static int csr_upload_impl(swb_context *ctx, int64_t rows, int64_t cols, int64_t
     int64_t mid = (int64_t)((__int128)cols * percent / 100);
     mid -= mid % 4;  // the second part of the operand starts 16-byte aligned
     if (mid < 1) mid = 1;
+    int32_t *d_below = nullptr;
     try {
-      std::vector<int32_t> rp_lo(rows + 1, 0), rp_hi(rows + 1, 0);
-      for (int64_t r = 0; r < rows; ++r) {
-        int32_t below = 0;
-        for (int32_t p = row_ptr[r]; p < row_ptr[r + 1]; ++p) below += col_idx[p] < mid;
-        rp_lo[r + 1] = rp_lo[r] + below;
-        rp_hi[r + 1] = rp_hi[r] + (row_ptr[r + 1] - row_ptr[r] - below);
+      std::vector<int32_t> below(rows), rp_lo(rows + 1, 0), rp_hi(rows + 1, 0);
+      cudaError_t es = cudaMalloc(&d_below, (size_t)rows * 4);
+      if (es == cudaSuccess)
+        es = swb::launch_count_below(rows, h->whole.row_ptr, h->whole.col_idx, (int32_t)mid, d_below, nullptr);
+      if (es == cudaSuccess) es = cudaMemcpy(below.data(), d_below, (size_t)rows * 4, cudaMemcpyDeviceToHost);
+      for (int64_t r = 0; es == cudaSuccess && r < rows; ++r) {
+        rp_lo[r + 1] = rp_lo[r] + below[r];
+        rp_hi[r + 1] = rp_hi[r] + (row_ptr[r + 1] - row_ptr[r] - below[r]);
       }
-      const int64_t nnz_lo = rp_lo[rows], nnz_hi = rp_hi[rows];
-      std::vector<int32_t> ci_lo(nnz_lo), ci_hi(nnz_hi);
-      std::vector<float> v_lo(nnz_lo), v_hi(nnz_hi);
-      for (int64_t r = 0; r < rows; ++r) {
-        int64_t a = rp_lo[r], b = rp_hi[r];
-        for (int32_t p = row_ptr[r]; p < row_ptr[r + 1]; ++p) {
-          if (col_idx[p] < mid) { ci_lo[a] = col_idx[p]; v_lo[a++] = val[p]; }
-          else { ci_hi[b] = col_idx[p]; v_hi[b++] = val[p]; }
-        }
-      }
-      cudaError_t es = upload_part(h->low, rows, nnz_lo, rp_lo.data(), ci_lo.data(), v_lo.data(), 0);
+      if (es == cudaSuccess) es = upload_part(h->low, rows, rp_lo[rows], rp_lo.data(), nullptr, nullptr, 0);
       // the second part finishes the result, so it is the one cut into row panels (about as many as the whole)
       if (es == cudaSuccess)
-        es = upload_part(h->high, rows, nnz_hi, rp_hi.data(), ci_hi.data(), v_hi.data(), (panel_nnz + 1) / 2);
+        es = upload_part(h->high, rows, rp_hi[rows], rp_hi.data(), nullptr, nullptr, (panel_nnz + 1) / 2);
+      if (es == cudaSuccess)
+        es = swb::launch_split_columns(rows, h->whole.row_ptr, h->whole.col_idx, h->whole.val, (int32_t)mid,
+                                       h->low.row_ptr, h->high.row_ptr, h->low.col_idx, h->low.val, h->high.col_idx,
+                                       h->high.val, nullptr);
+      if (es == cudaSuccess) es = cudaStreamSynchronize(nullptr);  // the host calls use streams of their own
       if (es == cudaSuccess) {
         h->split = true;
         h->split_col = mid;
@@ -1088,6 +1100,7 @@ static int csr_upload_impl(swb_context *ctx, int64_t rows, int64_t cols, int64_t
     } catch (const std::bad_alloc &) {
       // no host memory for the temporary copies: the matrix stays uncut
     }
+    cudaFree(d_below);
     if (!h->split) {
       free_part(h->low);
       free_part(h->high);
@@ -1185,7 +1198,17 @@ int resident_host_call(swb_context *ctx, const swb_options *o, const swb_csr_han
   st = ensure_copy_stream(ctx);
   if (st != SWB_OK) return st;
   cudaError_t e = cudaSuccess;
-  if (!halves) {
+  if (!halves && can_accumulate && !o->accumulate) {
+    // the result is cleared while the operand travels, and the panels only add to it
+    cudaStream_t up = ctx->upload_stream;
+    e = cudaMemcpyAsync(d_dense, dense_host, dense_bytes, cudaMemcpyHostToDevice, up);
+    if (e == cudaSuccess) e = cudaEventRecord(ctx->upload_done[0], up);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_out, 0, out_bytes, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ctx->upload_done[0], 0);
+    swb_options add = *o;
+    add.accumulate = 1;
+    if (e == cudaSuccess) st = run_panels_with_copy(ctx, &add, h->whole, width, d_out, out_host, e, launch);
+  } else if (!halves) {
     e = cudaMemcpyAsync(d_dense, dense_host, dense_bytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) st = run_panels_with_copy(ctx, o, h->whole, width, d_out, out_host, e, launch);
   } else {

@@ -125,6 +125,13 @@ cudaError_t launch_spmm_thread_per_position(const CsrSpmmArgs &a, int block,
                                             int64_t chunk, cudaStream_t s,
                                             int64_t *launches);
 
+// --- column parts of an uploaded matrix (csr_split.cu): entries per row below the cut, then the two parts
+cudaError_t launch_count_below(int64_t rows, const int32_t *row_ptr, const int32_t *col, int32_t cut, int32_t *below,
+                               cudaStream_t s);
+cudaError_t launch_split_columns(int64_t rows, const int32_t *row_ptr, const int32_t *col, const float *val, int32_t cut,
+                                 const int32_t *low_ptr, const int32_t *high_ptr, int32_t *low_col, float *low_val,
+                                 int32_t *high_col, float *high_val, cudaStream_t s);
+
 // --- BSR SpMM
 cudaError_t launch_bsr_spmm_thread_per_output_f32(const BsrSpmmArgs &a, cudaStream_t s, int64_t *launches);
 cudaError_t launch_bsr_spmm_thread_per_output_bf16(const BsrSpmmArgs &a, cudaStream_t s, int64_t *launches);
