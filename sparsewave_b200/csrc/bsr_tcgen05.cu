@@ -1,4 +1,4 @@
-// BSR SpMM for 16x16 bf16 blocks on the Blackwell tensor cores:
+// BSR SpMM for 16x16 bf16 blocks (and 8x8, 32x32: Shape below) on the Blackwell tensor cores:
 // TMA (cp.async.bulk.tensor) -> shared memory -> tcgen05.mma -> TMEM -> tcgen05.ld.
 //
 // Reference arithmetic (ThreadPerOutputBSRSpMMPattern, SparseWaveToGPU.cpp:560-665):
@@ -55,31 +55,46 @@ namespace {
 
 constexpr int TILE_N = 256;                  // right-hand-side columns per CTA (two MMA M = 128 halves)
 constexpr int HALF_N = 128;
-// One block per stage, three stages (28 KiB of shared memory, seven CTAs per SM): on the 5 %-dense
-// 1024 x 1024 block grid with 512 columns, 69.7 us; (2,2) 75.7, (2,3) 80.0, (1,2) 78.7, (1,4) 84.0, (4,2) 86.0.
-// What counts is the number of CTAs in flight per SM, each being one serial chain of copies.
-#ifndef SWB_BSR_CHUNK
-#define SWB_BSR_CHUNK 1
-#endif
-#ifndef SWB_BSR_STAGES
-#define SWB_BSR_STAGES 3
-#endif
-constexpr int CHUNK = SWB_BSR_CHUNK;         // blocks per pipeline stage
-constexpr int STAGES = SWB_BSR_STAGES;
-constexpr int BOX_BYTES = 16 * 64 * 2;       // 2048: 64 columns x 16 rows
-constexpr int HALF_SLAB = 2 * BOX_BYTES;     // 4096: one 16 x 128 bf16 slab (one accumulator's operand)
-constexpr int SLAB_BYTES = 2 * HALF_SLAB;    // 8192: 16 x 256
-constexpr int BLOCK_BYTES = 16 * 16 * 2;     // 512
-constexpr int STAGE_SLABS = CHUNK * SLAB_BYTES;
-// slabs first (1024-aligned), then blocks, padded so that the next stage's slabs are 1024-aligned again
-constexpr int STAGE_BYTES = (STAGE_SLABS + CHUNK * BLOCK_BYTES + 1023) / 1024 * 1024;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;         // + alignment slack
-constexpr int TMEM_COLS = 32;                // two accumulators of 16 columns
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
 constexpr int PRODUCER_THREAD = 128;         // lane 0 of warp 4 issues the TMA copies
 constexpr int MMA_THREAD = 160;              // lane 0 of warp 5 issues the MMAs
 constexpr int THREADS = 192;
-static_assert(STAGE_BYTES % 1024 == 0, "stages must keep the 1024-byte alignment of the swizzled slabs");
+constexpr int MAX_STAGES = 8;
+
+// A pipeline step: one block of 16 x 16 or 32 x 32, or two blocks of 8 x 8 side by side along k.
+template <int BS>
+struct Shape {
+  static constexpr int BLOCKS = BS == 8 ? 2 : 1;            // blocks per step
+  static constexpr int K = BS * BLOCKS;                     // rows of B per step: 16 or 32
+  static constexpr int BOX_BYTES = BS * 64 * 2;             // 64 columns x BS rows of B
+  static constexpr int GROUP_BYTES = K * 64 * 2;            // 64 columns x K rows
+  static constexpr int HALF_BYTES = 2 * GROUP_BYTES;        // one accumulator's operand
+  static constexpr int SLAB_BYTES = 2 * HALF_BYTES;
+  static constexpr int VALUE_BYTES = BS * BS * 2;           // one block
+  static constexpr int MMA_N = BS == 32 ? 32 : 16;          // at least 16 with M = 128: 8 rows are padded with zeros
+  static constexpr int TMEM_COLS = 2 * MMA_N;               // two accumulators
+  // slabs first (1024-aligned), then the blocks, padded so that the next stage's slabs are 1024-aligned again
+  static constexpr int STAGE_BYTES = (SLAB_BYTES + (BS == 8 ? 512 : VALUE_BYTES) + 1023) / 1024 * 1024;
+  // Block operand, K-major: rows of 32 or 64 bytes swizzled within themselves, or (8 x 8) unswizzled core matrices of
+  // 8 rows x 16 bytes, each of which is one block: 128 bytes to the next along k, 256 bytes to the (zero) rows 8 - 15.
+  static constexpr uint32_t LAYOUT = BS == 32 ? 4u : BS == 16 ? 6u : 0u;
+  static constexpr uint32_t LBO = BS == 8 ? 128u : 16u;
+  static constexpr uint32_t SBO = BS == 32 ? 512u : 256u;
+};
+
+// Stages of a launch.  What fills the path from L2 is the number of copies in flight per SM: with CTAs enough, three
+// stages (28 KiB for 16 x 16 blocks, seven CTAs per SM: 1024 x 1024 blocks at 5 %, 512 columns 69.7 us; two stages 78.7,
+// four 84.0); with fewer, the shared memory that is left over goes into more stages.
+template <int BS>
+int stages_for(int64_t grid, int sm_count) {
+  int64_t per_sm = (grid + sm_count - 1) / sm_count;
+  if (per_sm > 7) per_sm = 7;
+  const int64_t fit = 210 * 1024 / (per_sm > 0 ? per_sm : 1) / Shape<BS>::STAGE_BYTES;
+  const int least = BS == 32 ? 2 : 3;
+  return fit < least ? least : fit > MAX_STAGES ? MAX_STAGES : (int)fit;
+}
+template <int BS>
+constexpr int smem_bytes(int stages) { return stages * Shape<BS>::STAGE_BYTES + 1024; }  // + alignment slack
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -87,7 +102,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 
 // Shared-memory matrix descriptor, version 1 (Blackwell): bits [0,14) address
 // >> 4, [16,30) leading byte offset >> 4, [32,46) stride byte offset >> 4,
-// [46,48) version, [61,64) layout type (2 = 128-byte swizzle, 6 = 32-byte).
+// [46,48) version, [61,64) layout type (0 = none, 2 = 128-byte swizzle, 4 = 64-byte, 6 = 32-byte).
 __device__ __forceinline__ uint64_t make_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes,
                                               uint32_t layout) {
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16) |
@@ -97,7 +112,9 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t addr, uint32_t lbo_bytes,
 // Instruction descriptor for kind::f16: D f32 (bits 4-5 = 1), A and B bf16
 // (bits 7-9 and 10-12 = 1), A MN-major (bit 15), B K-major (bit 16 = 0),
 // N >> 3 at bits 17-22, M >> 4 at bits 24-28.
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
+constexpr uint32_t instruction_descriptor(uint32_t n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+}
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
@@ -121,15 +138,18 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
       : "memory");
 }
 
-// PER_CTA_STATUS: raise status[blockIdx.x] instead of status[0] when a wait gives up.
-template <bool PER_CTA_STATUS>
-__global__ void __launch_bounds__(THREADS) bsr16_spmm_tcgen05_kernel(
+// PER_CTA_STATUS: raise status[blockIdx.x] instead of status[0] when a wait gives up.  STAGES: the number of stages where
+// it is a constant, or 0: `run_stages` of them.
+template <bool PER_CTA_STATUS, int BS, int STAGES>
+__global__ void __launch_bounds__(THREADS) bsr_spmm_tcgen05_kernel(
     const __grid_constant__ CUtensorMap map_B, const __grid_constant__ CUtensorMap map_A, int64_t n_tiles,
-    int64_t N, const int32_t *__restrict__ brp, const int32_t *__restrict__ bci, __nv_bfloat16 *__restrict__ C,
-    int *status) {
+    int64_t N, int cols, int value_rows, int run_stages, const int32_t *__restrict__ brp, const int32_t *__restrict__ bci,
+    __nv_bfloat16 *__restrict__ C, int *status) {
+  using S = Shape<BS>;
+  const int stages = STAGES ? STAGES : run_stages;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bar_full[STAGES];
-  __shared__ __align__(8) uint64_t bar_empty[STAGES];
+  __shared__ __align__(8) uint64_t bar_full[STAGES ? STAGES : MAX_STAGES];
+  __shared__ __align__(8) uint64_t bar_empty[STAGES ? STAGES : MAX_STAGES];
   __shared__ __align__(8) uint64_t bar_done;
   __shared__ uint32_t tmem_slot;
   __shared__ int failed;
@@ -145,13 +165,13 @@ __global__ void __launch_bounds__(THREADS) bsr16_spmm_tcgen05_kernel(
 
   if (nblk == 0) {  // empty block row: C = 0
     for (int64_t col = (int64_t)n0 + tid; col < N && col < (int64_t)n0 + TILE_N; col += THREADS)
-      for (int r = 0; r < 16; ++r) C[(br * 16 + r) * N + col] = __float2bfloat16_rn(0.0f);
+      for (int r = 0; r < BS; ++r) C[(br * BS + r) * N + col] = __float2bfloat16_rn(0.0f);
     return;
   }
 
   if (tid == 0) {
     failed = 0;
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_full[s])) : "memory");
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_empty[s])) : "memory");
     }
@@ -162,72 +182,76 @@ __global__ void __launch_bounds__(THREADS) bsr16_spmm_tcgen05_kernel(
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                 "r"(TMEM_COLS)
+                 "r"(S::TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if constexpr (BS == 8) {  // rows 8 - 15 of the block operand, which no copy writes
+    for (int i = tid; i < stages * 64; i += THREADS)
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(stage0 + (uint32_t)(i / 64) * S::STAGE_BYTES + S::SLAB_BYTES + 256u +
+                                                   (uint32_t)(i % 64) * 4u), "r"(0u) : "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
-  const int nchunks = (nblk + CHUNK - 1) / CHUNK;
+  const int steps = (nblk + S::BLOCKS - 1) / S::BLOCKS;
 
   if (tid == PRODUCER_THREAD) {
-    for (int i = 0; i < nchunks; ++i) {
-      const int s = i % STAGES;
-      if (i >= STAGES && !mbar_wait(smem_u32(&bar_empty[s]), ((i / STAGES) - 1) & 1u)) {
-        failed = 1;  // the MMAs of chunk i - STAGES never released this stage
+    for (int i = 0, s = 0, round = 0; i < steps; ++i) {
+      if (round > 0 && !mbar_wait(smem_u32(&bar_empty[s]), (uint32_t)(round - 1) & 1u)) {
+        failed = 1;  // the MMAs of step i - stages never released this stage
         atomicExch(status + (PER_CTA_STATUS ? blockIdx.x : 0), 1);
         break;
       }
-      const int first = start + i * CHUNK;
-      const int count = min(CHUNK, end - first);
-      int bcs[CHUNK];
+      const int first = start + i * S::BLOCKS;
+      int y_B[S::BLOCKS], y_A[S::BLOCKS];  // first rows in B and among the block values; past a row's blocks: zeros
 #pragma unroll
-      for (int j = 0; j < CHUNK; ++j) bcs[j] = (j < count) ? __ldg(bci + first + j) : 0;
+      for (int j = 0; j < S::BLOCKS; ++j) {
+        const bool in = first + j < end;
+        y_B[j] = in ? __ldg(bci + first + j) * BS : cols;
+        y_A[j] = in ? (first + j) * BS : value_rows;
+      }
       const uint32_t full = smem_u32(&bar_full[s]);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full),
-                   "r"((uint32_t)count * (uint32_t)(halves * HALF_SLAB + BLOCK_BYTES))
+                   "r"((uint32_t)(halves * S::HALF_BYTES + S::BLOCKS * S::VALUE_BYTES))
                    : "memory");
-      const uint32_t sbase = stage0 + (uint32_t)s * STAGE_BYTES;
+      const uint32_t base = stage0 + (uint32_t)s * S::STAGE_BYTES;
 #pragma unroll
-      for (int j = 0; j < CHUNK; ++j) {
-        if (j >= count) break;
-        const uint32_t slab = sbase + (uint32_t)j * SLAB_BYTES;
-        tma_load_2d(slab, &map_B, n0, bcs[j] * 16, full);
-        tma_load_2d(slab + BOX_BYTES, &map_B, n0 + 64, bcs[j] * 16, full);
-        if (halves == 2) {
-          tma_load_2d(slab + 2 * BOX_BYTES, &map_B, n0 + 128, bcs[j] * 16, full);
-          tma_load_2d(slab + 3 * BOX_BYTES, &map_B, n0 + 192, bcs[j] * 16, full);
-        }
-        tma_load_2d(sbase + STAGE_SLABS + (uint32_t)j * BLOCK_BYTES, &map_A, 0, (first + j) * 16, full);
+      for (int j = 0; j < S::BLOCKS; ++j) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+          if (g < 2 || halves == 2)
+            tma_load_2d(base + (uint32_t)(g * S::GROUP_BYTES + j * S::BOX_BYTES), &map_B, n0 + 64 * g, y_B[j], full);
+        tma_load_2d(base + (uint32_t)(S::SLAB_BYTES + j * S::VALUE_BYTES), &map_A, 0, y_A[j], full);
       }
+      if (++s == stages) { s = 0; ++round; }
     }
   } else if (tid == MMA_THREAD) {
     bool ok = true;
-    for (int c = 0; c < nchunks; ++c) {
-      const int s = c % STAGES;
-      ok = mbar_wait(smem_u32(&bar_full[s]), (c / STAGES) & 1u);
+    for (int c = 0, s = 0, round = 0; c < steps; ++c) {
+      ok = mbar_wait(smem_u32(&bar_full[s]), (uint32_t)round & 1u);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t sbase = stage0 + (uint32_t)s * STAGE_BYTES;
-      const int count = min(CHUNK, nblk - c * CHUNK);
-      for (int j = 0; j < count; ++j) {
-        const uint64_t bdesc = make_desc(sbase + STAGE_SLABS + (uint32_t)j * BLOCK_BYTES, 16u, 256u, 6u);
-        const uint32_t accumulate = (c > 0 || j > 0) ? 1u : 0u;
-        for (int h = 0; h < halves; ++h) {
-          const uint64_t adesc = make_desc(sbase + (uint32_t)j * SLAB_BYTES + (uint32_t)h * HALF_SLAB, 2048u, 1024u, 2u);
+      const uint32_t base = stage0 + (uint32_t)s * S::STAGE_BYTES;
+      for (int h = 0; h < halves; ++h) {
+#pragma unroll
+        for (int k = 0; k < S::K / 16; ++k) {  // 16 rows of a slab are 2048 bytes, 16 values of a block row 32
+          const uint64_t adesc = make_desc(base + (uint32_t)(h * S::HALF_BYTES + k * 2048), S::GROUP_BYTES, 1024u, 2u);
+          const uint64_t bdesc = make_desc(base + (uint32_t)(S::SLAB_BYTES + k * 32), S::LBO, S::SBO, S::LAYOUT);
           asm volatile(
               "{\n\t.reg .pred p;\n\t"
               "setp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem + (uint32_t)h * 16u),
-              "l"(adesc), "l"(bdesc), "r"(IDESC), "r"(accumulate)
+              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem + (uint32_t)(h * S::MMA_N)),
+              "l"(adesc), "l"(bdesc), "r"(instruction_descriptor(S::MMA_N)), "r"((c > 0 || k > 0) ? 1u : 0u)
               : "memory");
         }
       }
-      const uint32_t arrive_on = (c == nchunks - 1) ? smem_u32(&bar_done) : smem_u32(&bar_empty[s]);
+      const uint32_t arrive_on = (c == steps - 1) ? smem_u32(&bar_done) : smem_u32(&bar_empty[s]);
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(arrive_on)
                    : "memory");
+      if (++s == stages) { s = 0; ++round; }
     }
     if (!ok) {
       failed = 1;
@@ -250,27 +274,31 @@ __global__ void __launch_bounds__(THREADS) bsr16_spmm_tcgen05_kernel(
   if (done_ok && !failed && warp < 4) {
     // TMEM lane m of accumulator h = column n0 + 128 h + m of C; this warp reads lanes 32 warp .. +32
     for (int h = 0; h < halves; ++h) {
-      uint32_t v[16];
-      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)h * 16u;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-          "%15}, [%16];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-            "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(taddr)
-          : "memory");
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       const int64_t col = (int64_t)n0 + h * HALF_N + warp * 32 + lane;
-      if (col < N) {
 #pragma unroll
-        for (int r = 0; r < 16; ++r) C[(br * 16 + r) * N + col] = __float2bfloat16_rn(__uint_as_float(v[r]));
+      for (int r0 = 0; r0 < BS; r0 += 16) {
+        uint32_t v[16];
+        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(h * S::MMA_N + r0);
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+            "%15}, [%16];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(taddr)
+            : "memory");
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (col < N) {
+#pragma unroll
+          for (int r = 0; r < (BS < 16 ? BS : 16); ++r)
+            C[(br * BS + r0 + r) * N + col] = __float2bfloat16_rn(__uint_as_float(v[r]));
+        }
       }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TMEM_COLS) : "memory");
 }
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -305,44 +333,74 @@ bool make_map_2d(CUtensorMap *map, const void *base, uint64_t inner, uint64_t ou
 
 }  // namespace
 
-bool bsr16_tcgen05_supported(const BsrSpmmArgs &a) {
+bool bsr_tcgen05_supported(const BsrSpmmArgs &a) {
   // TMA needs 16-byte aligned bases and row pitches.
-  // ... and 32-bit box coordinates: block rows of the value matrix (nnzb * 16) and B's extents.
-  if (a.nnzb > 2147483647LL / 16 || a.cols > 2147483647LL || a.n_rhs > 2147483647LL - 256) return false;
-  return a.block_size == 16 && a.n_rhs % 8 == 0 && a.nnzb > 0 && a.cols > 0 &&
+  // ... and 32-bit box coordinates: block rows of the value matrix (nnzb * block size) and B's extents.
+  if (a.block_size != 8 && a.block_size != 16 && a.block_size != 32) return false;
+  if (a.nnzb > 2147483647LL / a.block_size || a.cols > 2147483647LL - 64 || a.n_rhs > 2147483647LL - 256) return false;
+  return a.n_rhs % 8 == 0 && a.nnzb > 0 && a.cols > 0 &&
          (reinterpret_cast<uintptr_t>(a.B) & 15u) == 0 && (reinterpret_cast<uintptr_t>(a.block_values) & 15u) == 0;
 }
 
-cudaError_t launch_bsr16_spmm_tcgen05(const BsrSpmmArgs &a, int *status_flag, const DeviceInfo &dev,
-                                      cudaStream_t s, int64_t *launches) {
-  (void)dev;
-  // Once per device; racing host threads at worst repeat the (idempotent) attribute call.
+// 16 x 16 and 32 x 32 blocks always gain; 8 x 8 half fill the MMA and a block row is little work for a CTA: they gain from
+// some 96 columns (2,048 block rows of 32, N = 128: 74 -> 32 us), not below (8,000 block rows of 8, N = 64: 45 us on the
+// CUDA cores, 67 here).
+bool bsr_tcgen05_pays(const BsrSpmmArgs &a) { return a.block_size != 8 || a.n_rhs >= 96; }
+
+namespace {
+
+// Opts a kernel into its largest shared memory, once per device; racing threads repeat an idempotent call.
+template <bool PER_CTA_STATUS, int BS, int STAGES>
+cudaError_t configure() {
   static std::atomic<bool> configured[64];
   int device = 0;
   cudaGetDevice(&device);
-  if (device < 0 || device >= 64 || !configured[device].load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(bsr16_spmm_tcgen05_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    if (device >= 0 && device < 64) configured[device].store(true, std::memory_order_release);
-  }
-  const int64_t brows = a.rows / 16;
-  if (brows == 0) return cudaSuccess;
-  const int64_t n_tiles = ceil_div(a.n_rhs, TILE_N);
-  const int64_t grid = brows * n_tiles;
-  if (grid > 2147483647LL) return cudaErrorInvalidConfiguration;
+  if (device >= 0 && device < 64 && configured[device].load(std::memory_order_acquire)) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(bsr_spmm_tcgen05_kernel<PER_CTA_STATUS, BS, STAGES>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       smem_bytes<BS>(STAGES ? STAGES : MAX_STAGES));
+  if (e == cudaSuccess && device >= 0 && device < 64) configured[device].store(true, std::memory_order_release);
+  return e;
+}
+
+template <bool PER_CTA_STATUS, int BS, int STAGES>
+cudaError_t launch_stages(const BsrSpmmArgs &a, int *status, int stages, int64_t grid, int64_t n_tiles, cudaStream_t s) {
+  cudaError_t e = configure<PER_CTA_STATUS, BS, STAGES>();
+  if (e != cudaSuccess) return e;
   CUtensorMap map_B, map_A;
-  // B: cols x N bf16, boxes of 64 columns x 16 rows, 128-byte swizzle.
-  if (!make_map_2d(&map_B, a.B, (uint64_t)a.n_rhs, (uint64_t)a.cols, 64, 16, CU_TENSOR_MAP_SWIZZLE_128B))
+  // B: cols x N bf16, boxes of 64 columns x BS rows, 128-byte swizzle; block values: (nnzb * BS) x BS, one box per block.
+  if (!make_map_2d(&map_B, a.B, (uint64_t)a.n_rhs, (uint64_t)a.cols, 64, BS, CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !make_map_2d(&map_A, a.block_values, BS, (uint64_t)a.nnzb * BS, BS, BS,
+                   BS == 8 ? CU_TENSOR_MAP_SWIZZLE_NONE : BS == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B))
     return cudaErrorInvalidValue;
-  // Block values as (nnzb*16) x 16 bf16, one 16 x 16 box per block, 32-byte swizzle.
-  if (!make_map_2d(&map_A, a.block_values, 16, (uint64_t)a.nnzb * 16, 16, 16, CU_TENSOR_MAP_SWIZZLE_32B))
-    return cudaErrorInvalidValue;
-  launch_chained(bsr16_spmm_tcgen05_kernel<false>, (unsigned)grid, THREADS, SMEM_BYTES, s,
-      map_B, map_A, n_tiles, a.n_rhs, a.block_row_ptr, a.block_col_idx, static_cast<__nv_bfloat16 *>(a.C),
-      status_flag);
-  ++*launches;
+  launch_chained(bsr_spmm_tcgen05_kernel<PER_CTA_STATUS, BS, STAGES>, (unsigned)grid, THREADS,
+                 (size_t)smem_bytes<BS>(stages), s, map_B, map_A, n_tiles, a.n_rhs, (int)a.cols, (int)(a.nnzb * BS), stages,
+                 a.block_row_ptr, a.block_col_idx, static_cast<__nv_bfloat16 *>(a.C), status);
   return cudaGetLastError();
+}
+
+template <bool PER_CTA_STATUS, int BS>
+cudaError_t launch_tcgen05(const BsrSpmmArgs &a, int *status, int sm_count, cudaStream_t s) {
+  const int64_t n_tiles = ceil_div(a.n_rhs, TILE_N), grid = a.rows / BS * n_tiles;
+  if (grid == 0) return cudaSuccess;
+  if (grid > 2147483647LL) return cudaErrorInvalidConfiguration;
+  const int stages = stages_for<BS>(grid, sm_count);
+  if (stages == 3) return launch_stages<PER_CTA_STATUS, BS, 3>(a, status, stages, grid, n_tiles, s);
+  return launch_stages<PER_CTA_STATUS, BS, 0>(a, status, stages, grid, n_tiles, s);
+}
+
+}  // namespace
+
+cudaError_t launch_bsr_spmm_tcgen05(const BsrSpmmArgs &a, int *status_flag, const DeviceInfo &dev, cudaStream_t s,
+                                    int64_t *launches) {
+  if (a.rows == 0) return cudaSuccess;
+  ++*launches;
+  switch (a.block_size) {
+    case 8: return launch_tcgen05<false, 8>(a, status_flag, dev.sm_count, s);
+    case 16: return launch_tcgen05<false, 16>(a, status_flag, dev.sm_count, s);
+    case 32: return launch_tcgen05<false, 32>(a, status_flag, dev.sm_count, s);
+  }
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace swb
@@ -451,7 +509,7 @@ extern "C" __attribute__((visibility("default"))) int swb_bsr16_spmm_bf16_static
   if (!block_row_ptr || (nnzb > 0 && (!block_col_idx || !block_values)) || (cols > 0 && !B) || (rows > 0 && !C))
     return static_fail(kInvalidArgument, "bsr_spmm: NULL operand pointer");
   BsrSpmmArgs a{rows, cols, nnzb, 16, n_rhs, block_row_ptr, block_col_idx, block_values, B, C};
-  if (!bsr16_tcgen05_supported(a))
+  if (!bsr_tcgen05_supported(a))
     return static_fail(kUnsupported,
                        "the static-scratch BSR entry point needs at least one block, a column count that is a "
                        "multiple of 8 and 16-byte aligned block values and right-hand side");
@@ -468,18 +526,11 @@ extern "C" __attribute__((visibility("default"))) int swb_bsr16_spmm_bf16_static
   StaticStatusSlot *slot = nullptr;
   int *status = static_status_address(&e, &slot);
   if (!status) return static_fail(kCuda, cudaGetErrorString(e));
-  e = cudaFuncSetAttribute(bsr16_spmm_tcgen05_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-  if (e != cudaSuccess) return static_fail(kCuda, cudaGetErrorString(e));
-  CUtensorMap map_B, map_A;
-  if (!make_map_2d(&map_B, B, (uint64_t)n_rhs, (uint64_t)cols, 64, 16, CU_TENSOR_MAP_SWIZZLE_128B) ||
-      !make_map_2d(&map_A, block_values, 16, (uint64_t)nnzb * 16, 16, 16, CU_TENSOR_MAP_SWIZZLE_32B))
-    return static_fail(kCuda, "could not encode the TMA tensor maps");
   // The words keep the previous call's outcome: clear the ones this call uses.
   e = cudaMemsetAsync(status, 0, (size_t)grid * sizeof(int), s);
   if (e != cudaSuccess) return static_fail(kCuda, cudaGetErrorString(e));
-  launch_chained(bsr16_spmm_tcgen05_kernel<true>, (unsigned)grid, THREADS, SMEM_BYTES, s,
-      map_B, map_A, n_tiles, n_rhs, block_row_ptr, block_col_idx, reinterpret_cast<__nv_bfloat16 *>(C), status);
-  e = cudaGetLastError();
+  e = launch_tcgen05<true, 16>(a, status, DeviceInfo().sm_count, s);
+  if (e == cudaErrorInvalidValue) return static_fail(kCuda, "could not encode the TMA tensor maps");
   if (e != cudaSuccess) return static_fail(kCuda, cudaGetErrorString(e));
   slot->last_grid.store(grid, std::memory_order_release);
   if (gave_up_ctas) {

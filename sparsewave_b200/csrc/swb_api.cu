@@ -774,8 +774,8 @@ int swb_bsr_spmm_bf16(swb_context *ctx, const swb_options *o, int64_t rows, int6
   swb::BsrSpmmArgs a{rows, cols, nnzb, bs, n_rhs, brp, bci, bv, B, C};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e;
-  if (swb::bsr16_tcgen05_supported(a))
-    e = swb::launch_bsr16_spmm_tcgen05(a, ctx->status_flag, ctx->dev, s, &ctx->launches);
+  if (swb::bsr_tcgen05_supported(a) && swb::bsr_tcgen05_pays(a))
+    e = swb::launch_bsr_spmm_tcgen05(a, ctx->status_flag, ctx->dev, s, &ctx->launches);
   else
     e = swb::launch_bsr_spmm_thread_per_output_bf16(a, s, &ctx->launches);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "bsr_spmm launch");

@@ -1,0 +1,37 @@
+"""BSR SpMM on the tensor cores for blocks of 8 x 8 (two per step), 16 x 16 and 32 x 32."""
+import pytest
+import torch
+
+from sparsewave_b200 import workloads as W
+from tests.helpers import assert_bf16_close
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bs", [8, 16, 32])
+@pytest.mark.parametrize("n", [8, 64, 72, 96, 128, 136, 256, 264, 520])
+@pytest.mark.parametrize("rows,density", [(1, 1.0), (40, 0.12), (3, 0.9), (700, 0.2)])
+def test_shapes(ctx, bs, n, rows, density):
+    """Empty block rows, odd and even block counts, fewer and more steps than stages, one and two halves of a tile, few and
+    many CTAs per SM."""
+    if rows == 700 and (n > 136 or bs == 32):
+        pytest.skip("covered by the smaller sizes")
+    a = W.random_bsr(rows, 37, bs, density, seed=bs + n + rows)
+    B = W.dense_normal((37 * bs, n), seed=n)
+    C = ctx.bsr_spmm("", a.block_row_ptr.cuda(), a.block_col_idx.cuda(), a.block_values.cuda(), B.cuda(), bs)
+    assert ctx.device_status() == 0
+    assert_bf16_close(C, a.block_row_ptr.numpy(), a.block_col_idx.numpy(), a.block_values.view(torch.uint16).numpy(),
+                      B.view(torch.uint16).numpy(), bs)
+
+
+@pytest.mark.parametrize("bs", [8, 16, 32])
+def test_values_of_other_block_rows_do_not_leak(ctx, bs):
+    brp = torch.tensor([0, 1, 4, 7, 9], dtype=torch.int32)  # odd counts before, at and after the poisoned row
+    bci = torch.tensor([2, 0, 1, 2, 0, 1, 2, 0, 3], dtype=torch.int32)
+    values = torch.ones(9 * bs * bs, dtype=torch.bfloat16)
+    values[4 * bs * bs:7 * bs * bs] = float("nan")
+    B = torch.ones((4 * bs, 128), dtype=torch.bfloat16)
+    B[3 * bs:] = float("inf")
+    C = ctx.bsr_spmm("", brp.cuda(), bci.cuda(), values.cuda(), B.cuda(), bs).float().cpu()
+    assert torch.equal(C[:bs], torch.full((bs, 128), float(bs))) and torch.equal(C[bs:2 * bs], torch.full((bs, 128), 3.0 * bs))
+    assert bool(C[2 * bs:3 * bs].isnan().all()) and bool(C[3 * bs:].isinf().all())
