@@ -626,22 +626,28 @@ cudaError_t launch_rows_as(const CsrSpmmArgs &a, cudaStream_t s, int64_t per = 0
   return cudaGetLastError();
 }
 
-// Runs of columns per lane: enough that 32 lanes hold the row of C, else column tiles (the widest odd row without
-// tiles, 224 columns, takes seven single columns per lane).
+// Runs of columns per lane for M runs of V columns: the fewest lane slots (column tiles x runs), the larger number of runs
+// where two take as many; and from 33 runs so that two rows fit a warp.  150,000 ragged rows of 15 (us with 2 / 3 / 4 / 5
+// runs): N = 35 84 / 69 / 66 / 75, N = 63 87 / 107 / 80 / 100, N = 75 - / 108 / 117 / 101, N = 147 - / 222 / 256 / 177,
+// N = 187 - / 248 / 277 / 321; N = 66 (V = 2) 100 / 92 / 93; N = 132 (V = 4) 177 / 154.
 inline int runs_per_lane(int64_t M, int V) {
-  if (M <= 96) return (int)(M > 0 ? ceil_div(M, 32) : 1);
-  return V > 1 || M <= 128 ? 4 : M <= 160 ? 5 : 7;
+  if (M <= 32) return 1;
+  if (M <= 48) return 3;
+  if (V == 1 && M <= 80) return M <= 64 ? 4 : 5;
+  int best = V == 1 ? 5 : V == 2 ? 4 : 3;  // more runs than this spill registers
+  for (int R = best - 1; R >= (V == 1 ? 3 : 2); --R)
+    if (ceil_div(M, 32 * R) * R < ceil_div(M, 32 * best) * best) best = R;
+  return best;
 }
 
 template <int V>
 cudaError_t launch_rows_columns(const CsrSpmmArgs &a, cudaStream_t s) {
-  switch (runs_per_lane(a.n_rhs / V, V)) {
-    case 1: return launch_rows_as<V, 1, V <= 2 ? 8 : 4>(a, s);
-    case 2: return launch_rows_as<V, 2, 4>(a, s);
-    case 3: return launch_rows_as<V, 3, 4>(a, s);
-    case 4: return launch_rows_as<V, 4, 4>(a, s);
-  }
-  if constexpr (V == 1) return a.n_rhs <= 160 ? launch_rows_as<V, 5, 4>(a, s) : launch_rows_as<V, 7, 4>(a, s);
+  const int R = runs_per_lane(a.n_rhs / V, V);
+  if (R == 1) return launch_rows_as<V, 1, V <= 2 ? 8 : 4>(a, s);
+  if (R == 3) return launch_rows_as<V, 3, 4>(a, s);
+  if constexpr (V > 1) if (R == 2) return launch_rows_as<V, 2, 4>(a, s);
+  if constexpr (V < 4) if (R == 4) return launch_rows_as<V, 4, 4>(a, s);
+  if constexpr (V == 1) if (R == 5) return launch_rows_as<V, 5, 4>(a, s);
   return cudaErrorInvalidValue;
 }
 
@@ -668,7 +674,7 @@ inline bool few_rows(int64_t rows, int64_t n_rhs) { return rows <= 8192 || (rows
 
 cudaError_t launch_rows(const CsrSpmmArgs &a, cudaStream_t s) {
   if (takes_row_products(a.rows, a.n_rhs)) return launch_row_products(a, s);
-  if (a.n_rhs > 0x3fffffffLL) return launch_rows_as<1, 7, 4, uint64_t>(a, s);
+  if (a.n_rhs > 0x3fffffffLL) return launch_rows_as<1, 5, 4, uint64_t>(a, s);
   const int V = columns_per_lane(a.rows, a.nnz, a.n_rhs, reinterpret_cast<uintptr_t>(a.B) | reinterpret_cast<uintptr_t>(a.C));
   if (few_rows(a.rows, a.n_rhs)) return V == 2 ? launch_rows_as<2, 1, 8>(a, s) : launch_rows_as<1, 1, 16>(a, s);
   if (V == 4) return launch_rows_columns<4>(a, s);

@@ -17,8 +17,15 @@
 
 constexpr int STAGE_THREADS = 128, STAGE_POSITIONS = 1536, STAGE_ROWS = 256;
 
+// Blocks per SM: as many as the rows of B in flight and the sums leave registers for.  One block too many spills inside the
+// loop and costs a factor of two (40,000 rows of 20, N = 187, seven columns per lane in 64 registers: 242 us).
+constexpr int stage_min_blocks(int V, int R, int Q) {
+  const int words = V * R;
+  return words <= 3 || (words == 4 && R == 1) ? (Q > 8 ? 8 : 10) : words <= 5 ? 8 : words <= 8 ? 6 : 5;
+}
+
 template <int V, int R, int Q, typename Pitch>
-__global__ void __launch_bounds__(STAGE_THREADS, V * R > 4 || Q > 8 ? 8 : 10)
+__global__ void __launch_bounds__(STAGE_THREADS, stage_min_blocks(V, R, Q))
     spmm_staged_rows_kernel(int64_t rows, int64_t N, Pitch pitch, int G, int rows_per_block, int64_t tiles,
                             const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col,
                             const float *__restrict__ val, const float *__restrict__ B, float *__restrict__ C,

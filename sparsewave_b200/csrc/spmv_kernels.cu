@@ -706,7 +706,8 @@ cudaError_t launch_row_products(const CsrSpmmArgs &a, cudaStream_t s) {
 }
 
 int64_t row_products_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs) {
-  return max1(ceil_div(rows, product_rows_per_block(rows, nnz, n_rhs)));
+  return max1(ceil_div(rows, products_once(rows, nnz, n_rhs) ? product_rows_per_block<ProductsOnce>(rows, nnz, n_rhs)
+                                                             : product_rows_per_block<ProductsMany>(rows, nnz, n_rhs)));
 }
 
 cudaError_t launch_spmv_thread_per_row(const CsrSpmvArgs &a, cudaStream_t s, int64_t *launches) {

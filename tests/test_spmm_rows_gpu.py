@@ -9,8 +9,8 @@ from tests.helpers import assert_within_bound, dev, random_csr
 
 pytestmark = pytest.mark.gpu
 
-# one, two and four columns per lane; 1 to 7 runs of them; the last width without column tiles and the first with
-WIDTHS = [1, 2, 3, 4, 5, 8, 31, 32, 33, 64, 66, 96, 97, 100, 128, 129, 161, 224, 225, 256, 260, 512, 516]
+# one, two and four columns per lane; 1 to 5 runs of them; the last widths without column tiles and the first with
+WIDTHS = [1, 2, 3, 4, 5, 8, 31, 32, 33, 35, 63, 64, 66, 75, 96, 97, 100, 128, 129, 130, 132, 161, 187, 198, 224, 225, 256, 260, 300, 321, 512, 516]
 
 
 def _spmm(ctx, opts, rp, ci, v, B, C=None):
