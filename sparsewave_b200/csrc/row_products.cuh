@@ -20,9 +20,10 @@
 // Threads of a block, most rows of a block, and products of a tile before padding.  Where 512 threads and 4,096 products per
 // block cover the matrix with four blocks per SM, all of it is in flight at once and evenly spread (206,501 ragged rows of 6:
 // 12.0 -> 9.7 us a call against blocks of 256, of which some SMs get six and others five).  Larger matrices take blocks of
-// 128 and tiles of 2,048, whose gaps between gathers and sums interleave better (1 M ragged rows of 10: 52.4 -> 51.0).
+// 128 and tiles of 2,048, whose gaps between gathers and sums interleave better (1 M ragged rows of 10: 52.4 -> 51.0); with
+// several columns those hold too few positions, and blocks are of 256 (404,892 banded rows of 19, N = 4: 49 -> 46).
 struct ProductsOnce { static constexpr int THREADS = 512, WORDS = 4096; };
-struct ProductsMany { static constexpr int THREADS = 128, WORDS = 2048; };
+template <int N> struct ProductsMany { static constexpr int THREADS = N == 1 ? 128 : 256, WORDS = N == 1 ? 2048 : 4096; };
 
 template <int W> struct Words;  // what one load brings
 template <> struct Words<1> { using T = float; };
@@ -154,5 +155,5 @@ cudaError_t launch_row_products_in(const CsrSpmmArgs &a, cudaStream_t s) {
 template <int N, int W>
 cudaError_t launch_row_products_of(const CsrSpmmArgs &a, cudaStream_t s) {
   return products_once(a.rows, a.nnz, N) ? launch_row_products_in<N, W, ProductsOnce>(a, s)
-                                         : launch_row_products_in<N, W, ProductsMany>(a, s);
+                                         : launch_row_products_in<N, W, ProductsMany<N>>(a, s);
 }

@@ -155,6 +155,7 @@ __global__ void spmv_wave_per_row_kernel(int64_t rows, const int32_t *__restrict
                                          const float *__restrict__ val,
                                          const float *__restrict__ x, float *__restrict__ y,
                                          bool vec_ok) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -175,6 +176,7 @@ __global__ void spmv_block_per_row_kernel(int64_t rows, const int32_t *__restric
                                           const float *__restrict__ val,
                                           const float *__restrict__ x, float *__restrict__ y,
                                           bool vec_ok) {
+  after_previous_kernel();
   __shared__ float wave_sums[32];
   const int64_t row = blockIdx.x;
   if (row >= rows) return;  // uniform for the block
@@ -707,7 +709,8 @@ cudaError_t launch_row_products(const CsrSpmmArgs &a, cudaStream_t s) {
 
 int64_t row_products_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs) {
   return max1(ceil_div(rows, products_once(rows, nnz, n_rhs) ? product_rows_per_block<ProductsOnce>(rows, nnz, n_rhs)
-                                                             : product_rows_per_block<ProductsMany>(rows, nnz, n_rhs)));
+                             : n_rhs == 1 ? product_rows_per_block<ProductsMany<1>>(rows, nnz, n_rhs)
+                                          : product_rows_per_block<ProductsMany<2>>(rows, nnz, n_rhs)));
 }
 
 cudaError_t launch_spmv_thread_per_row(const CsrSpmvArgs &a, cudaStream_t s, int64_t *launches) {
@@ -793,7 +796,7 @@ cudaError_t launch_spmv_wave_per_row(const CsrSpmvArgs &a, int block, const Devi
     case RowForm::STREAM: return launch_row_stream(a, dev, s);
     case RowForm::REFERENCE: break;
   }
-  spmv_wave_per_row_kernel<<<grid_of(ceil_div(a.rows, block / 32)), block, 0, s>>>(
+  launch_chained(spmv_wave_per_row_kernel, grid_of(ceil_div(a.rows, block / 32)), block, 0, s,
       a.rows, a.row_ptr, a.col_idx, a.val, a.x, a.y, aligned16(a.col_idx) && aligned16(a.val));
   return cudaGetLastError();
 }
@@ -806,8 +809,8 @@ cudaError_t launch_spmv_block_per_row(const CsrSpmvArgs &a, int block, const Dev
     case RowForm::STREAM: return launch_row_stream(a, dev, s);
     case RowForm::REFERENCE: break;
   }
-  spmv_block_per_row_kernel<<<grid_of(a.rows), block, 0, s>>>(a.rows, a.row_ptr, a.col_idx, a.val, a.x, a.y,
-                                                              aligned16(a.col_idx) && aligned16(a.val));
+  launch_chained(spmv_block_per_row_kernel, grid_of(a.rows), block, 0, s, a.rows, a.row_ptr, a.col_idx, a.val, a.x, a.y,
+                 aligned16(a.col_idx) && aligned16(a.val));
   return cudaGetLastError();
 }
 
