@@ -643,6 +643,9 @@ inline int runs_per_lane(int64_t M, int V) {
 template <int V>
 cudaError_t launch_rows_columns(const CsrSpmmArgs &a, cudaStream_t s) {
   const int R = runs_per_lane(a.n_rhs / V, V);
+  // Twelve positions a step take most short rows at once (285,639 rows of 10, N = 9: 41 us with eight, 36 with twelve; 100,000
+  // ragged rows of 6, N = 13: 18.0 and 16.3); from 16 they only add masked ones.
+  if constexpr (V == 1) if (R == 1 && a.nnz <= 12 * a.rows) return launch_rows_as<V, 1, 12>(a, s);
   if (R == 1) return launch_rows_as<V, 1, V <= 2 ? 8 : 4>(a, s);
   if (R == 3) return launch_rows_as<V, 3, 4>(a, s);
   if constexpr (V > 1) if (R == 2) return launch_rows_as<V, 2, 4>(a, s);
@@ -693,7 +696,7 @@ int64_t rows_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs) {  // 16-by
 // rows many times longer than usual in a small matrix are one lane group's chain there, while a warp per row splits
 // them.  Measured against the kernels with a warp or part of one per row:
 //   N = 16, 32, 64, 128 (300,000 ragged rows of 5: 41 -> 29, 69 -> 45, 110 -> 89, 184 -> 141 us), with the sizes and mean
-//   lengths up to which each wins; N = 8 and rows of 50 and more do not gain;
+//   lengths up to which each wins; N = 8 and long rows do not gain (154,183 ragged rows of 36, N = 32: 106 us there, 111 here);
 //   other multiples of 4 from 12 to 124 (150,000 rows of 20, N = 100: 182 -> 126 us; 15,000 rows of 20, N = 24: a draw);
 //   the rest up to 512 columns, which else read B by single columns (250,001 rows of 20, N = 50: 664 -> 128 us;
 //   102,040 rows of 20, N = 147: 742 -> 145 us; 15,000 rows of 20, N = 7: 10 us there against 13 here).
@@ -704,7 +707,7 @@ inline bool tile_takes_staged_rows(int64_t rows, int64_t nnz, int64_t N) {
     case 2: case 3: return rows > 8192;  // products summed per row: 300,000 rows of 20, N = 1: 113 -> 37 us
     case 4: case 8: case 256: case 384: case 512: return false;
     case 16: return outputs >= 2500000 && mean <= 14;
-    case 32: return outputs >= 4000000 && mean <= 48;
+    case 32: return outputs >= 4000000 && mean <= 32;
     case 64: return outputs >= 6000000 && mean <= 48;
     case 128: return outputs >= 8000000;
   }

@@ -59,3 +59,18 @@ def test_wave_per_row_tile_takes_the_rows_kernel(ctx, rows, mean, n):
     C = torch.ones((rows, n), device="cuda")
     _spmm(ctx, opts + " accumulate=1", rp, ci, v, dev(B), C)
     assert_within_bound(C.cpu().numpy(), want + 1.0, bound + 1.0)
+
+
+@pytest.mark.parametrize("n", [5, 17, 31, 32])
+@pytest.mark.parametrize("mean", [10, 11, 24])  # one or several steps of 12 positions, steps of 8
+def test_steps_of_many_rows(ctx, mean, n):
+    rows = 40000
+    rng = np.random.default_rng(mean + n)
+    lens = rng.integers(0, 2 * mean + 1, rows)
+    lens[:64] = np.arange(64)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = rng.integers(0, 900, rp[-1]).astype(np.int32)
+    v = rng.uniform(-1, 1, rp[-1]).astype(np.float32)
+    B = rng.uniform(-1, 1, (900, n)).astype(np.float32)
+    Bu = torch.empty(B.size + 1, device="cuda")[1:].view(B.shape).copy_(torch.from_numpy(B))
+    assert np.array_equal(_spmm(ctx, "", rp, ci, v, Bu).cpu().numpy(), oracle.csr_spmm(rp, ci, v, B, parallel=True))
