@@ -201,8 +201,9 @@ SWB_API int swb_bsr_spmm_f32(swb_context *ctx, const swb_options *opts,
 
 /* sparsewave.bsr_spmm on bf16 blocks with f32 accumulation and bf16 output
  * (the op requires one element type, SparseWaveOps.cpp:355-360).  Values are
- * raw bf16 bit patterns.  block_size 16 runs on the tcgen05 tensor cores;
- * other block sizes use the thread-per-output kernel. */
+ * raw bf16 bit patterns.  Blocks of 16 and 32 (and of 8 from 96 columns) on aligned
+ * operands with n_rhs a multiple of 8 run on the tcgen05 tensor cores, the others
+ * on the thread-per-output kernel. */
 SWB_API int swb_bsr_spmm_bf16(swb_context *ctx, const swb_options *opts,
                               int64_t rows, int64_t cols, int64_t nnzb,
                               int64_t block_size, int64_t n_rhs,
