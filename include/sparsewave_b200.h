@@ -284,7 +284,7 @@ SWB_API int swb_bsr_spmm_bf16_host(swb_context *ctx, const swb_options *opts,
  * copy y (or C) out and synchronise.  Large matrices are cut into row panels
  * at upload (swb_plan_row_panels) and the rows of the result start their copy
  * to the host as soon as their panel is done, while later panels compute;
- * matrices of 3 M nonzeros or more (SWB_RESIDENT_SPLIT_NNZ) are also kept as
+ * matrices of 4.5 M nonzeros or more (SWB_RESIDENT_SPLIT_NNZ) are also kept as
  * two column parts (twice the device memory) so that the first part computes
  * while the rest of the dense operand is still being copied in.  Use
  * pinned host buffers to benefit.  The handle belongs to the context's device

@@ -946,7 +946,7 @@ constexpr int kMaxPanels = 8;
 // whose column lies below a cut (36 % of the columns by default) and one with the rest.  A call on a mapping that can accumulate then sends
 // the first half of the dense operand, runs the first matrix while the second half is still on its way,
 // and adds the second matrix (cut into row panels, as above) on top.  SWB_RESIDENT_SPLIT_NNZ: nnz from
-// which a matrix is stored this way (default 3000000; it doubles the matrix's device memory).
+// which a matrix is stored this way (default 4500000; it doubles the matrix's device memory).
 struct CsrPart {
   int64_t nnz = 0;
   int32_t *row_ptr = nullptr, *col_idx = nullptr;
@@ -1059,7 +1059,7 @@ static int csr_upload_impl(swb_context *ctx, int64_t rows, int64_t cols, int64_t
   const int64_t panel_nnz = plain ? 0 : env_i64("SWB_RESIDENT_PANEL_NNZ", 8000000);
   cudaError_t e = upload_part(h->whole, rows, nnz, row_ptr, col_idx, val, panel_nnz);
 
-  if (!plain && e == cudaSuccess && rows > 0 && cols >= 2 && nnz >= env_i64("SWB_RESIDENT_SPLIT_NNZ", 3000000)) {
+  if (!plain && e == cudaSuccess && rows > 0 && cols >= 2 && nnz >= env_i64("SWB_RESIDENT_SPLIT_NNZ", 4500000)) {
     // The two column parts, each a CSR matrix over all rows with the entries in their original order.  They
     // are an optimisation: without the host or device memory for them the matrix stays resident uncut.
     // Where the columns are cut: the first part should finish computing about when the rest of the operand

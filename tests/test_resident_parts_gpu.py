@@ -1,4 +1,4 @@
-"""Resident matrices at the sizes where they are stored as two column parts and cut into row panels by default."""
+"""Resident matrices stored as two column parts and cut into row panels."""
 import numpy as np
 import pytest
 
@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("rows,cols,max_len", [(150001, 150001, 65536), (700000, 40, 20), (600000, 300007, 3000)])
-def test_column_parts_made_on_the_device(ctx, rows, cols, max_len):
+def test_column_parts_made_on_the_device(ctx, monkeypatch, rows, cols, max_len):
+    monkeypatch.setenv("SWB_RESIDENT_SPLIT_NNZ", "3000000")
     a = W.zipf_csr(rows, cols, 1.2 if cols == 40 else 1.6, 1, max_len, seed=rows, device="cuda")
     assert a.nnz > 3_000_000
     rp, ci, v = a.numpy()
