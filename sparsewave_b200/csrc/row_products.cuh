@@ -58,14 +58,16 @@ __global__ void __launch_bounds__(Shape::THREADS)
   float sum[N];  // of outputs tid, tid + PRODUCT_THREADS, ... (rows_per_block <= PRODUCT_THREADS)
 #pragma unroll
   for (int k = 0; k < N; ++k) sum[k] = 0.0f;
-  for (int tile = first; tile < last; tile += TILE) {
-    const int items = (last - tile < TILE ? last - tile : TILE) * ITEMS;
+  // unsigned: behind the last tile of a matrix of up to 2^31 - 1 nonzeros `tile` passes the int32 maximum
+  for (unsigned tile = first; tile < (unsigned)last; tile += TILE) {
+    const int items = (last - tile < TILE ? (int)(last - tile) : TILE) * ITEMS;
     for (int i0 = tid; i0 < items; i0 += PER * PRODUCT_THREADS) {
       int c[PER];
       float v[PER];
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
-        const int i = i0 + k * PRODUCT_THREADS, p = tile + i / ITEMS;
+        const int i = i0 + k * PRODUCT_THREADS;
+        const unsigned p = tile + i / ITEMS;
         c[k] = i < items ? ld_stream(col + p) : 0;
         v[k] = i < items ? ld_stream(val + p) : 0.0f;
       }
@@ -102,7 +104,7 @@ __global__ void __launch_bounds__(Shape::THREADS)
       const int o = tid + k * PRODUCT_THREADS;
       if (o < count * N) {
         const int r = o / N, j = o - r * N;
-        int p = offsets[r] - tile, end = offsets[r + 1] - tile;
+        int p = (int)(offsets[r] - tile), end = (int)(offsets[r + 1] - tile);
         if (p < 0) p = 0;
         if (end > TILE) end = TILE;
         float s = sum[k];

@@ -101,3 +101,24 @@ def test_bsr16_bf16_outputs_past_2_pow_31_elements(ctx):
         # one bf16 ulp around the fp32 sum, plus the slack of the accumulation order where terms cancel
         excess = (got - expected).abs() - (2.0 ** -7) * expected.abs() - 1e-2 * (2.0 ** -6) * bound
         assert float(excess.max()) <= 0, f"block rows {b0}..{b1}"
+
+
+def _up_to_the_last_position(nnz, row_length):
+    """Rows of `row_length` positions up to position `nnz`, columns p % 5, values 1; the sum of x = 0, 1, 2, 3, 4 over each row."""
+    rows = -(-nnz // row_length)
+    ends = torch.clamp(torch.arange(rows + 1, device="cuda") * row_length, max=nnz)
+    col = torch.arange(nnz, dtype=torch.int32, device="cuda").remainder_(5)
+    below = ends // 5 * 10 + (ends % 5) * (ends % 5 - 1) // 2  # sum of p % 5 over the positions before
+    return ends.to(torch.int32), col, torch.ones(nnz, device="cuda"), (below[1:] - below[:-1]).float()
+
+
+def test_row_products_up_to_the_last_position(ctx):
+    # tiles of 2048 positions: the one behind the last would start past the int32 maximum.  Sums are whole numbers: exact.
+    row_ptr, col, val, expected = _up_to_the_last_position((1 << 31) - 1, 2048)
+    x = torch.arange(5, dtype=torch.float32, device="cuda")
+    assert torch.equal(ctx.spmv("", row_ptr, col, val, x), expected)
+    row_ptr[-1] -= 256  # SpMM takes up to 2^31 - 257 nonzeros
+    expected[-1] -= (torch.arange((1 << 31) - 257, (1 << 31) - 1, device="cuda") % 5).sum()
+    C = ctx.spmm("", row_ptr, col[:-256], val[:-256], torch.stack([x, 2 * x, 3 * x, -x], 1).contiguous())
+    assert torch.equal(C, torch.stack([expected, 2 * expected, 3 * expected, -expected], 1))
+    assert ctx.device_status() == 0
