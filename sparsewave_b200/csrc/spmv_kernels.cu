@@ -104,8 +104,8 @@ __device__ __forceinline__ float strided_row_partial(int start, int end, int who
   float sum = 0.0f;
   if (vec_ok && end - start >= VEC_MIN) {
     const int a0 = (start + 3) & ~3;  // first 16-byte aligned position
-    int p = start + who;
-    if (p < a0) sum = add(sum, mul(ld_stream(val + p), __ldg(x + ld_stream(col + p))));
+    unsigned p = (unsigned)start + who;
+    if (p < (unsigned)a0) sum = add(sum, mul(ld_stream(val + p), __ldg(x + ld_stream(col + p))));
     const int g1 = end >> 2;
     const int4 *col4 = reinterpret_cast<const int4 *>(col);
     const float4 *val4 = reinterpret_cast<const float4 *>(val);
@@ -127,21 +127,23 @@ __device__ __forceinline__ float strided_row_partial(int start, int end, int who
       sum = add(sum, mul(va.x, xa0)); sum = add(sum, mul(va.y, xa1));
       sum = add(sum, mul(va.z, xa2)); sum = add(sum, mul(va.w, xa3));
     }
-    p = (g1 << 2) + who;
-    if (p < end) sum = add(sum, mul(ld_stream(val + p), __ldg(x + ld_stream(col + p))));
+    p = (unsigned)(g1 << 2) + who;
+    if (p < (unsigned)end) sum = add(sum, mul(ld_stream(val + p), __ldg(x + ld_stream(col + p))));
     return sum;
   }
   // Reference traversal: p = start + who, step count
-  // (buildStridedPositionRange, SparseGPUUtils.cpp:70-78), two loads in flight.
-  int p = start + who;
-  for (; p + count < end; p += 2 * count) {
+  // (buildStridedPositionRange, SparseGPUUtils.cpp:70-78), two loads in flight.  Positions are unsigned: up to two strides
+  // past the end of a row they exceed the int32 maximum where the matrix has nearly 2^31 nonzeros.
+  unsigned p = (unsigned)start + who;
+  const unsigned stop = end;
+  for (; p + count < stop; p += 2 * count) {
     int c0 = ld_stream(col + p), c1 = ld_stream(col + p + count);
     float v0 = ld_stream(val + p), v1 = ld_stream(val + p + count);
     float x0 = __ldg(x + c0), x1 = __ldg(x + c1);
     sum = add(sum, mul(v0, x0));
     sum = add(sum, mul(v1, x1));
   }
-  if (p < end) sum = add(sum, mul(ld_stream(val + p), __ldg(x + ld_stream(col + p))));
+  if (p < stop) sum = add(sum, mul(ld_stream(val + p), __ldg(x + ld_stream(col + p))));
   return sum;
 }
 

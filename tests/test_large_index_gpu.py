@@ -122,3 +122,14 @@ def test_row_products_up_to_the_last_position(ctx):
     C = ctx.spmm("", row_ptr, col[:-256], val[:-256], torch.stack([x, 2 * x, 3 * x, -x], 1).contiguous())
     assert torch.equal(C, torch.stack([expected, 2 * expected, 3 * expected, -expected], 1))
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("row_length", [64, 2048])  # below and above the rows that take 128-bit loads
+def test_row_mappings_up_to_the_last_position(ctx, row_length):
+    # strides of up to 1024 threads past the last positions of the matrix
+    row_ptr, col, val, expected = _up_to_the_last_position((1 << 31) - 1, row_length)
+    x = torch.arange(5, dtype=torch.float32, device="cuda")
+    for opts in ("spmv-mapping=wave-per-row spmv-block-size=128", "spmv-mapping=block-per-row spmv-block-size=64",
+                 "spmv-mapping=block-per-row spmv-block-size=1024"):
+        assert torch.equal(ctx.spmv(opts, row_ptr, col, val, x), expected), opts
+    assert ctx.device_status() == 0
