@@ -142,8 +142,8 @@ __global__ void __launch_bounds__(TILE_THREADS, BS == 4 && TR == 4 ? 7 : 1) bsr_
     };
     if (AHEAD) request(bc, 0);
     for (int bp = start; bp < end; ++bp, a += block) {
-      const int after = bp + 2 < end ? __ldg(bci + bp + 2) : next;
-      if (AHEAD && bp + 3 < end) asm volatile("prefetch.global.L1 [%0];" ::"l"(a + 3 * block));
+      const int after = end - bp > 2 ? __ldg(bci + bp + 2) : next;
+      if (AHEAD && end - bp > 3) asm volatile("prefetch.global.L1 [%0];" ::"l"(a + 3 * block));
 #pragma unroll
       for (int lc = 0; lc < whole; lc += K) {
         if (!AHEAD) request(bc, lc);

@@ -133,3 +133,12 @@ def test_row_mappings_up_to_the_last_position(ctx, row_length):
                  "spmv-mapping=block-per-row spmv-block-size=1024"):
         assert torch.equal(ctx.spmv(opts, row_ptr, col, val, x), expected), opts
     assert ctx.device_status() == 0
+
+
+def test_bsr_blocks_up_to_the_last_position(ctx):
+    # 2^31 - 1 blocks of 1 x 1: block columns are read two blocks ahead of the last one
+    brp, bci, bv, expected = _up_to_the_last_position((1 << 31) - 1, 2048)
+    x = torch.arange(5, dtype=torch.float32, device="cuda")
+    C = ctx.bsr_spmm("", brp, bci, bv, torch.stack([x, 2 * x, 3 * x, -x], 1).contiguous(), 1)
+    assert torch.equal(C, torch.stack([expected, 2 * expected, 3 * expected, -expected], 1))
+    assert ctx.device_status() == 0
