@@ -622,6 +622,13 @@ inline RowsShape rows_shape(int64_t rows, int64_t nnz, int64_t M, int R) {
   return h;
 }
 
+// Positions of a row that its group of lanes takes; the block takes the rest.  Above what a block holds in all (some 640
+// positions), so that ordinary blocks need not look for such rows, and above the length of ordinary rows.
+inline int long_row_of(int64_t rows, int64_t nnz) {
+  const int64_t mean = rows > 0 ? nnz / rows : 0;
+  return mean <= 128 ? 1024 : mean < 0x0fffffff ? (int)(8 * mean) : 0x7fffffff;
+}
+
 // `per` > 0: rows per block, instead of the rule above.
 template <int V, int R, int Q, typename Pitch = uint32_t>
 cudaError_t launch_rows_as(const CsrSpmmArgs &a, cudaStream_t s, int64_t per = 0) {
@@ -629,7 +636,8 @@ cudaError_t launch_rows_as(const CsrSpmmArgs &a, cudaStream_t s, int64_t per = 0
   if (per > 0) h.per = per;
   SWB_GRID(grid, ceil_div(a.rows, h.per) * h.tiles);
   launch_chained(spmm_staged_rows_kernel<V, R, Q, Pitch>, grid, STAGE_THREADS, 0, s,
-      a.rows, a.n_rhs, (Pitch)(a.n_rhs * 4), h.G, (int)h.per, h.tiles, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
+      a.rows, a.n_rhs, (Pitch)(a.n_rhs * 4), h.G, (int)h.per, h.tiles, long_row_of(a.rows, a.nnz),
+      a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
   return cudaGetLastError();
 }
 
@@ -699,9 +707,9 @@ int64_t rows_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs) {  // 16-by
   return max1(ceil_div(rows, h.per) * h.tiles);
 }
 
-// Whether wave-per-row-tile takes the staged-rows kernel.  It wins where there are rows enough to balance the blocks;
-// rows many times longer than usual in a small matrix are one lane group's chain there, while a warp per row splits
-// them.  Measured against the kernels with a warp or part of one per row:
+// Whether wave-per-row-tile takes the staged-rows kernel.  It wins where there are rows enough to balance the blocks.  A
+// row many times longer than usual is one block's work there (200,000 power-law rows of up to 63,402, N = 32 / 50 / 64 / 128:
+// 1.46 / 2.39 / 2.21 / 3.73 ms, with a warp or part of one per row 3.95 / 2.10 / 2.76 / 6.12).  Measured against those kernels:
 //   N = 16, 32, 64, 128 (300,000 ragged rows of 5: 41 -> 29, 69 -> 45, 110 -> 89, 184 -> 141 us), with the sizes and mean
 //   lengths up to which each wins; N = 8 and long rows do not gain (154,183 ragged rows of 36, N = 32: 106 us there, 111 here);
 //   other multiples of 4 from 12 to 124 (150,000 rows of 20, N = 100: 182 -> 126 us; 15,000 rows of 20, N = 24: a draw);

@@ -74,3 +74,39 @@ def test_steps_of_many_rows(ctx, mean, n):
     B = rng.uniform(-1, 1, (900, n)).astype(np.float32)
     Bu = torch.empty(B.size + 1, device="cuda")[1:].view(B.shape).copy_(torch.from_numpy(B))
     assert np.array_equal(_spmm(ctx, "", rp, ci, v, Bu).cpu().numpy(), oracle.csr_spmm(rp, ci, v, B, parallel=True))
+
+
+@pytest.mark.parametrize("n", [5, 9, 16, 32, 35, 50, 63, 75, 66, 132, 198, 256, 300])  # 1, 2, 4 columns x 1 to 5 runs
+def test_rows_that_the_block_finishes(ctx, n):
+    # a group takes 1,024 positions of a row, the block the rest in tiles of up to 128: ends of both, several in a block
+    lens = np.full(9000, 3)
+    lens[[0, 1, 2, 3, 40, 41, 4500, 8999]] = 1024, 1025, 1151, 1153, 1026, 1280, 7000, 3333
+    rng = np.random.default_rng(n)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = rng.integers(0, 1300, rp[-1]).astype(np.int32)
+    v = rng.uniform(-1, 1, rp[-1]).astype(np.float32)
+    B = rng.uniform(-1, 1, (1300, n)).astype(np.float32)
+    want = oracle.csr_spmm(rp, ci, v, B, parallel=True)
+    assert np.array_equal(_spmm(ctx, "", rp, ci, v, dev(B)).cpu().numpy(), want)
+    C = torch.ones((9000, n), device="cuda")
+    _spmm(ctx, "spmm-mapping=wave-per-row-tile spmm-tile-size=8 accumulate=1", rp, ci, v, dev(B), C)
+    assert_within_bound(C.cpu().numpy(), want + 1.0, oracle.csr_abs_bound(rp, ci, v, B) + 1.0)
+
+
+@pytest.mark.parametrize("opts", ["", "spmm-mapping=wave-per-row-tile spmm-tile-size=16 spmm-block-size=256"])
+def test_a_very_long_row_is_not_one_chain(ctx, opts):
+    # 64 columns, 200,000 rows of 10 and one of 65,536: as a chain of one group of lanes it takes 125 ns a position
+    lens = torch.full((200000,), 10, device="cuda")
+    lens[777] = 65536
+    rp = torch.nn.functional.pad(torch.cumsum(lens, 0), (1, 0)).int()
+    ci = torch.randint(0, 200000, (int(rp[-1]),), device="cuda", dtype=torch.int32)
+    v, B = torch.rand(ci.numel(), device="cuda"), torch.rand((200000, 64), device="cuda")
+    times = []
+    for _ in range(4):
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        begin.record()
+        ctx.spmm(opts, rp, ci, v, B)
+        end.record()
+        end.synchronize()
+        times.append(begin.elapsed_time(end))
+    assert min(times) < 65536 * 80e-6  # ms
