@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(SHARED_X_THREADS, 1)
   after_previous_kernel();
   for (int i = threadIdx.x; i < SHARED_X_FLOATS / 4; i += SHARED_X_THREADS)
     staged_x[i] = __ldg(reinterpret_cast<const float4 *>(x) + i);
-  const uint32_t staged = static_cast<uint32_t>(__cvta_generic_to_shared(staged_x));
+  uint32_t staged = static_cast<uint32_t>(__cvta_generic_to_shared(staged_x));
   const int lane = threadIdx.x & 31;
   const int warps = (int)((gridDim.x * blockDim.x) >> 5);
   struct Step { int64_t row; int s, e, q; };  // row, its bounds, first position of the step (a multiple of 4)
@@ -152,6 +152,9 @@ __global__ void __launch_bounds__(SHARED_X_THREADS, 1)
   Quad b = load(next);
   advance();
   __syncthreads();
+  // A gather reads shared memory, but says to the compiler only that it depends on its operands: `staged` comes from here on
+  // from behind the barrier, and so do the gathers.
+  asm volatile("" : "+r"(staged) : : "memory");
   float4 g = gather(a.c);
   float sum = 0.0f;
   while (now.row < rows) {

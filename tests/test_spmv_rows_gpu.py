@@ -40,3 +40,15 @@ def test_rows_with_x_in_shared_memory(ctx, mapping, cols):
     lens = rng.integers(0, 400, 4 * cols * 1000000 // 49152 // 200 * 5 // 4 + 100)
     lens[[0, 5, -1]] = 0, 20000, 1
     _check(ctx, f"spmv-mapping={mapping}", lens, cols, cols)
+
+
+@pytest.mark.parametrize("mapping", ["wave-per-row", "block-per-row"])
+@pytest.mark.parametrize("rows", [65536, 81921, 122880])
+def test_square_matrices_take_the_stream_of_rows(ctx, mapping, rows):
+    # one block of 1,024 threads per SM: the launch shape says that x is staged
+    rng = np.random.default_rng(rows)
+    lens = rng.integers(60, 200, rows)
+    lens[[0, 7, -1]] = 0, 9001, 1
+    opts = f"spmv-mapping={mapping}"
+    assert ctx.launch_shape(opts, rows, int(lens.sum())).physical_grid == torch.cuda.get_device_properties(0).multi_processor_count
+    _check(ctx, opts, lens, rows, rows)
