@@ -28,6 +28,13 @@ __device__ __forceinline__ Quad load_quad(const int32_t *__restrict__ col, const
   return t;
 }
 
+// Columns of a quad as far as they are the row's, which is [s, e).  The others, which may belong to no row at all (spare
+// capacity of the arrays, rows of a larger matrix in front of this one's and behind), are not used as an index into x.
+__device__ __forceinline__ int4 own_columns(const int4 &c, int q, int s, int e) {
+  return make_int4(q >= s && q < e ? c.x : 0, q + 1 >= s && q + 1 < e ? c.y : 0, q + 2 >= s && q + 2 < e ? c.z : 0,
+                   q + 3 >= s && q + 3 < e ? c.w : 0);
+}
+
 // Sum of the products of a quad's positions inside [s, e); g: x at its columns.
 __device__ __forceinline__ float quad_sum(const float4 &v, const float4 &g, int q, int s, int e) {
   const float p0 = q >= s && q < e ? mul(v.x, g.x) : 0.0f;
@@ -57,7 +64,8 @@ __global__ void __launch_bounds__(ROWS_THREADS)
   };
   auto load = [&](int q, int e) { return load_quad(col, val, nnz, q, e); };
   auto sum_of = [&](const Quad &t, int q, int s, int e) {
-    return quad_sum(t.v, make_float4(__ldg(x + t.c.x), __ldg(x + t.c.y), __ldg(x + t.c.z), __ldg(x + t.c.w)), q, s, e);
+    const int4 c = own_columns(t.c, q, s, e);
+    return quad_sum(t.v, make_float4(__ldg(x + c.x), __ldg(x + c.y), __ldg(x + c.z), __ldg(x + c.w)), q, s, e);
   };
   int s, e, s1, e1;
   int64_t r = warp * (32 / L) + lane / L;
@@ -141,7 +149,8 @@ __global__ void __launch_bounds__(SHARED_X_THREADS, 1)
     }
   };
   auto load = [&](const Step &t) { return load_quad(col, val, nnz, t.q + 4 * lane, t.e); };
-  auto gather = [&](const int4 &c) {
+  auto gather = [&](const Quad &t, const Step &of) {
+    const int4 c = own_columns(t.c, of.q + 4 * lane, of.s, of.e);
     return make_float4(gather_x(x, staged, c.x), gather_x(x, staged, c.y), gather_x(x, staged, c.z),
                        gather_x(x, staged, c.w));
   };
@@ -155,13 +164,13 @@ __global__ void __launch_bounds__(SHARED_X_THREADS, 1)
   // A gather reads shared memory, but says to the compiler only that it depends on its operands: `staged` comes from here on
   // from behind the barrier, and so do the gathers.
   asm volatile("" : "+r"(staged) : : "memory");
-  float4 g = gather(a.c);
+  float4 g = gather(a, now);
   float sum = 0.0f;
   while (now.row < rows) {
     const Step fresh = ahead;
     const Quad c = load(fresh);
     advance();
-    const float4 gn = gather(b.c);
+    const float4 gn = gather(b, next);
     sum = add(sum, quad_sum(a.v, g, now.q + 4 * lane, now.s, now.e));
     if (now.q + 128 >= now.e) {
       sum = warp_sum(sum);

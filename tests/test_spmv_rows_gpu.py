@@ -52,3 +52,22 @@ def test_square_matrices_take_the_stream_of_rows(ctx, mapping, rows):
     opts = f"spmv-mapping={mapping}"
     assert ctx.launch_shape(opts, rows, int(lens.sum())).physical_grid == torch.cuda.get_device_properties(0).multi_processor_count
     _check(ctx, opts, lens, rows, rows)
+
+
+@pytest.mark.parametrize("mapping", ["wave-per-row", "block-per-row"])
+@pytest.mark.parametrize("rows,low,high", [(50000, 0, 30), (65536, 90, 170)])  # groups of lanes; stream of rows
+def test_entries_outside_the_rows_belong_to_another_x(ctx, mapping, rows, low, high):
+    # a range of rows of a larger matrix with spare capacity behind it: the entries around the range lie past the end of x.
+    # (x is the front of a larger buffer, so that a kernel that read there all the same would do no harm.)
+    rng = np.random.default_rng(rows)
+    lens = rng.integers(low, high, rows)
+    rp = (5 + np.concatenate([[0], np.cumsum(lens)])).astype(np.int32)
+    ci = rng.integers(rows, rows + 4096, rp[-1] + 7).astype(np.int32)
+    ci[rp[0]:rp[-1]] = rng.integers(0, rows, rp[-1] - rp[0])
+    v = rng.uniform(-1, 1, len(ci)).astype(np.float32)
+    xs = np.full(rows + 4096, np.nan, np.float32)
+    xs[:rows] = rng.uniform(-1, 1, rows)
+    y = ctx.spmv(f"spmv-mapping={mapping}", dev(rp), dev(ci), dev(v), dev(xs)[:rows]).cpu().numpy()
+    own = slice(rp[0], rp[-1])
+    want = oracle.csr_spmv(rp - rp[0], ci[own], v[own], xs[:rows], parallel=True)
+    assert_within_bound(y, want, oracle.csr_abs_bound(rp - rp[0], ci[own], v[own], xs[:rows]))
