@@ -28,19 +28,19 @@ __device__ __forceinline__ Quad load_quad(const int32_t *__restrict__ col, const
   return t;
 }
 
+__device__ __forceinline__ bool inside(int p, int s, int e) { return (unsigned)(p - s) < (unsigned)(e - s); }  // s <= e
+
 // Columns of a quad as far as they are the row's, which is [s, e).  The others, which may belong to no row at all (spare
 // capacity of the arrays, rows of a larger matrix in front of this one's and behind), are not used as an index into x.
 __device__ __forceinline__ int4 own_columns(const int4 &c, int q, int s, int e) {
-  return make_int4(q >= s && q < e ? c.x : 0, q + 1 >= s && q + 1 < e ? c.y : 0, q + 2 >= s && q + 2 < e ? c.z : 0,
-                   q + 3 >= s && q + 3 < e ? c.w : 0);
+  return make_int4(inside(q, s, e) ? c.x : 0, inside(q + 1, s, e) ? c.y : 0, inside(q + 2, s, e) ? c.z : 0,
+                   inside(q + 3, s, e) ? c.w : 0);
 }
 
 // Sum of the products of a quad's positions inside [s, e); g: x at its columns.
 __device__ __forceinline__ float quad_sum(const float4 &v, const float4 &g, int q, int s, int e) {
-  const float p0 = q >= s && q < e ? mul(v.x, g.x) : 0.0f;
-  const float p1 = q + 1 >= s && q + 1 < e ? mul(v.y, g.y) : 0.0f;
-  const float p2 = q + 2 >= s && q + 2 < e ? mul(v.z, g.z) : 0.0f;
-  const float p3 = q + 3 >= s && q + 3 < e ? mul(v.w, g.w) : 0.0f;
+  const float p0 = inside(q, s, e) ? mul(v.x, g.x) : 0.0f, p1 = inside(q + 1, s, e) ? mul(v.y, g.y) : 0.0f;
+  const float p2 = inside(q + 2, s, e) ? mul(v.z, g.z) : 0.0f, p3 = inside(q + 3, s, e) ? mul(v.w, g.w) : 0.0f;
   return add(add(p0, p1), add(p2, p3));
 }
 
