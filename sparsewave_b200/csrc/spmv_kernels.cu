@@ -732,8 +732,11 @@ template <int L>
 cudaError_t launch_rows_of(const CsrSpmvArgs &a, const DeviceInfo &dev, cudaStream_t s) {
   int64_t blocks = ceil_div(a.rows, ROWS_THREADS / L);
   if (blocks > (int64_t)dev.sm_count * 8) blocks = (int64_t)dev.sm_count * 8;
+  // Warps of neighbouring rows share sectors of col and val, and all blocks stay for the last turn where there are one or two:
+  // apart only where that is 3 % or less (100,000 ragged rows of 22: 17 %; 250,000 rows of 3: 13 %).
+  const bool apart = a.rows >= 150000 && a.nnz >= 12 * a.rows;
   return launch_chained(spmv_rows_kernel<L>, grid_of(blocks), ROWS_THREADS, 0, s, a.rows, a.nnz, a.row_ptr, a.col_idx,
-                        a.val, a.x, a.y);
+                        a.val, a.x, a.y, apart);
 }
 
 // Lanes per row so that a row of mean length is in flight at once.
@@ -757,8 +760,11 @@ cudaError_t launch_row_stream(const CsrSpmvArgs &a, const DeviceInfo &dev, cudaS
     if (e != cudaSuccess) return e;
     if (device >= 0 && device < 64) configured[device].store(true, std::memory_order_release);
   }
+  // what the block takes at a time, and above ordinary rows
+  const int64_t mean = a.nnz / a.rows;
+  const int longest = mean <= 1024 ? 8192 : mean < 0x0fffffff ? (int)(8 * mean) : 0x7fffffff;
   return launch_chained(spmv_row_stream_kernel, (unsigned)dev.sm_count, SHARED_X_THREADS, SHARED_X_FLOATS * 4, s,
-                        a.rows, a.nnz, a.row_ptr, a.col_idx, a.val, a.x, a.y);
+                        a.rows, a.nnz, a.row_ptr, a.col_idx, a.val, a.x, a.y, longest);
 }
 
 enum class RowForm { REFERENCE, SHORT_ROWS, STREAM };

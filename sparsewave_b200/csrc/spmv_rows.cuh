@@ -3,6 +3,7 @@
 #pragma once
 
 constexpr int ROWS_THREADS = 256;
+constexpr int ROWS_LONGEST = 2048;      // positions of a row that a warp takes: what the block takes at a time
 constexpr int SHARED_X_FLOATS = 49152;  // 192 KB
 constexpr int SHARED_X_THREADS = 1024;  // one block per SM
 
@@ -44,28 +45,81 @@ __device__ __forceinline__ float quad_sum(const float4 &v, const float4 &g, int 
   return add(add(p0, p1), add(p2, p3));
 }
 
+// Rows that the warps of a block have left out, because they are far longer than the others, by the whole block, one at a
+// time.  `row_of(i)` is the block's i-th row, in any order, `end(i)` whether there is none from i on.  A sum depends on its
+// row alone.
+template <int THREADS, typename Gather, typename RowOf, typename End>
+__device__ __forceinline__ void sum_rows_left_out(int most, int64_t rows, int64_t nnz, const int32_t *__restrict__ row_ptr,
+                                                  const int32_t *__restrict__ col, const float *__restrict__ val,
+                                                  float *__restrict__ y, Gather gather, RowOf row_of, End end) {
+  __shared__ unsigned found[THREADS / 32];  // of THREADS rows looked at
+  __shared__ float sums[THREADS / 32];
+  const int tid = threadIdx.x;
+  for (int i0 = 0; !end(i0); i0 += THREADS) {
+    const int64_t r = row_of(i0 + tid);
+    const unsigned mask = __ballot_sync(FULL, r < rows && __ldg(row_ptr + r + 1) - __ldg(row_ptr + r) > most);
+    if ((tid & 31) == 0) found[tid >> 5] = mask;
+    __syncthreads();
+    for (int w = 0; w < THREADS / 32; ++w) {
+      for (unsigned todo = found[w]; todo != 0; todo &= todo - 1) {
+        const int64_t row = row_of(i0 + 32 * w + __ffs(todo) - 1);
+        const int s = __ldg(row_ptr + row), e = __ldg(row_ptr + row + 1);
+        float sum = 0.0f;
+        int p = (s & ~3) + 4 * tid;
+        for (; p + 4 * THREADS < e; p += 8 * THREADS) {
+          const Quad t = load_quad(col, val, nnz, p, e), u = load_quad(col, val, nnz, p + 4 * THREADS, e);
+          const float4 g = gather(own_columns(t.c, p, s, e)), h = gather(own_columns(u.c, p + 4 * THREADS, s, e));
+          sum = add(sum, add(quad_sum(t.v, g, p, s, e), quad_sum(u.v, h, p + 4 * THREADS, s, e)));
+        }
+        if (p < e) {
+          const Quad t = load_quad(col, val, nnz, p, e);
+          sum = add(sum, quad_sum(t.v, gather(own_columns(t.c, p, s, e)), p, s, e));
+        }
+        sum = warp_sum(sum);
+        if ((tid & 31) == 0) sums[tid >> 5] = sum;
+        __syncthreads();
+        if (tid < 32) {
+          sum = warp_sum(tid < THREADS / 32 ? sums[tid] : 0.0f);
+          if (tid == 0) y[row] = sum;
+        }
+        __syncthreads();
+      }
+    }
+    __syncthreads();  // `found` is written again
+  }
+}
+
 // A warp per short row leaves most lanes without a position, a block per row even more, and both pay the chain row offset
 // -> col/val -> x -> reduction for every row.  Here L = 4 to 16 lanes take a row in 16-byte quads of four positions, two
-// quads per lane (8 L positions) in flight; the grid fills the GPU once, a group walks rows a grid apart and requests the
-// next row's quads (and the offsets of the one behind it) before it sums this one.  Rows of more than 16 L positions
-// are finished by the whole warp.  Large matrices are then bound by the gather of x from L2 (253 G/s): 700,000 rows of 40
+// quads per lane (8 L positions) in flight; the grid is eight blocks per SM, of which four run at a time (64 registers), a
+// group walks rows a grid apart and requests the next row's quads (and the offsets of the one behind it) before it sums this
+// one.  Rows of more than 16 L positions are finished by the whole warp, and rows of more than ROWS_LONGEST are left to the
+// block, which takes eight times as many positions at once, in the end: as one warp's, a row of 65,536 is 256 steps (4 M
+// power-law rows 775 -> 540 us; 300,000 rows of 10 with eight of 65,536 183 -> 37).  Large matrices are then bound by the gather of x from L2 (253 G/s): 700,000 rows of 40
 // 165 -> 112 us, 1 M ragged rows of 16 149 -> 82 us, 400,000 rows of 70 (block-per-row) 220 -> 114 us.
 template <int L>
 __global__ void __launch_bounds__(ROWS_THREADS)
     spmv_rows_kernel(int64_t rows, int64_t nnz, const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col,
-                     const float *__restrict__ val, const float *__restrict__ x, float *__restrict__ y) {
+                     const float *__restrict__ val, const float *__restrict__ x, float *__restrict__ y, bool apart) {
+  __shared__ bool left_out;  // some row
+  if (threadIdx.x == 0) left_out = false;
+  __syncthreads();
   after_previous_kernel();
   const int lane = threadIdx.x & 31, l = lane % L;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  constexpr int WARPS = ROWS_THREADS / 32;
+  // `apart`: the warps of a block lie a grid apart, so that neighbouring rows, which are long together where rows are sorted
+  // by length, are other blocks' (1 M sorted power-law rows 2260 -> 460 us)
+  auto warp_of = [&](int w) { return apart ? (int64_t)w * gridDim.x + blockIdx.x : (int64_t)blockIdx.x * WARPS + w; };
+  const int64_t warp = warp_of(threadIdx.x >> 5);
   const int64_t stride = (((int64_t)gridDim.x * blockDim.x) >> 5) * (32 / L);
   auto bounds = [&](int64_t r, int &s, int &e) {  // empty past the last row
     s = r < rows ? __ldg(row_ptr + r) : 0;
     e = r < rows ? __ldg(row_ptr + r + 1) : 0;
   };
   auto load = [&](int q, int e) { return load_quad(col, val, nnz, q, e); };
+  auto gather = [&](const int4 &c) { return make_float4(__ldg(x + c.x), __ldg(x + c.y), __ldg(x + c.z), __ldg(x + c.w)); };
   auto sum_of = [&](const Quad &t, int q, int s, int e) {
-    const int4 c = own_columns(t.c, q, s, e);
-    return quad_sum(t.v, make_float4(__ldg(x + c.x), __ldg(x + c.y), __ldg(x + c.z), __ldg(x + c.w)), q, s, e);
+    return quad_sum(t.v, gather(own_columns(t.c, q, s, e)), q, s, e);
   };
   int s, e, s1, e1;
   int64_t r = warp * (32 / L) + lane / L;
@@ -77,6 +131,10 @@ __global__ void __launch_bounds__(ROWS_THREADS)
     bounds(r + 2 * stride, s2, e2);
     const Quad an = load((s1 & ~3) + 4 * l, e1), bn = load((s1 & ~3) + 4 * (l + L), e1);
     const int q = (s & ~3) + 4 * l;
+    if (e - s > ROWS_LONGEST) {  // no position, then: the zero that is stored is overwritten in the end
+      left_out = true;
+      e = s;
+    }
     const bool is_long = e - s > 16 * L;
     float sum = 0.0f;
     if (q < e) sum = sum_of(a, q, s, e);
@@ -102,6 +160,15 @@ __global__ void __launch_bounds__(ROWS_THREADS)
     s = s1; e = e1; s1 = s2; e1 = e2;
     a = an; b = bn;
   }
+  __syncthreads();
+  if (!left_out) return;
+  constexpr int TURN = ROWS_THREADS / L;  // rows of the block in one turn of its warps
+  auto row_of = [&](int i) {
+    const int w = i % TURN / (32 / L), k = i % (32 / L);
+    return warp_of(w) * (32 / L) + k + i / TURN * stride;
+  };
+  sum_rows_left_out<ROWS_THREADS>(ROWS_LONGEST, rows, nnz, row_ptr, col, val, y, gather, row_of,
+                                  [&](int i) { return i / TURN * stride >= rows; });
 }
 
 // Longer rows are bound by the gather of x alone.  L1 serves two of them per clock and SM while x fits it (570 G/s), but
@@ -109,7 +176,8 @@ __global__ void __launch_bounds__(ROWS_THREADS)
 // shared memory, once per SM, and only the others are gathered through L1.  One block of 32 warps fits an SM: a warp
 // takes rows a grid apart as one stream of steps of 128 positions and requests the quads of the next step before it
 // gathers for it, and gathers before it sums this one, across the ends of rows.  (Requesting further ahead takes more
-// registers than 1,024 threads have.)  65,536 rows of 256: 60 -> 33 us; 100,000 ragged rows of 200: 77 -> 73;
+// registers than 1,024 threads have.)  Rows of more than `longest` positions are left to the block (180,000 rows of 150 with
+// eight of 65,536: 400 -> 119 us).  65,536 rows of 256: 60 -> 34 us; 100,000 ragged rows of 200: 77 -> 73;
 // 150,000: 134 -> 121.
 __device__ __forceinline__ float gather_x(const float *__restrict__ x, uint32_t staged, int c) {
   float v;  // one of two predicated loads: a branch would split the warp at every gather
@@ -121,8 +189,11 @@ __device__ __forceinline__ float gather_x(const float *__restrict__ x, uint32_t 
 __global__ void __launch_bounds__(SHARED_X_THREADS, 1)
     spmv_row_stream_kernel(int64_t rows, int64_t nnz, const int32_t *__restrict__ row_ptr,
                            const int32_t *__restrict__ col, const float *__restrict__ val, const float *__restrict__ x,
-                           float *__restrict__ y) {
+                           float *__restrict__ y, int longest) {
   extern __shared__ float4 staged_x[];
+  __shared__ bool left_out;  // some row
+  if (threadIdx.x == 0) left_out = false;
+  __syncthreads();
   after_previous_kernel();
   for (int i = threadIdx.x; i < SHARED_X_FLOATS / 4; i += SHARED_X_THREADS)
     staged_x[i] = __ldg(reinterpret_cast<const float4 *>(x) + i);
@@ -133,6 +204,10 @@ __global__ void __launch_bounds__(SHARED_X_THREADS, 1)
   auto bounds = [&](int64_t r, int &s, int &e) {
     s = r < rows ? __ldg(row_ptr + r) : 0;
     e = r < rows ? __ldg(row_ptr + r + 1) : 0;
+    if (e - s > longest) {  // no position, as above
+      left_out = true;
+      e = s;
+    }
   };
   Step ahead;
   int ns, ne;  // bounds of the row behind that step's
@@ -149,11 +224,11 @@ __global__ void __launch_bounds__(SHARED_X_THREADS, 1)
     }
   };
   auto load = [&](const Step &t) { return load_quad(col, val, nnz, t.q + 4 * lane, t.e); };
-  auto gather = [&](const Quad &t, const Step &of) {
-    const int4 c = own_columns(t.c, of.q + 4 * lane, of.s, of.e);
+  auto gather_of = [&](const int4 &c) {
     return make_float4(gather_x(x, staged, c.x), gather_x(x, staged, c.y), gather_x(x, staged, c.z),
                        gather_x(x, staged, c.w));
   };
+  auto gather = [&](const Quad &t, const Step &of) { return gather_of(own_columns(t.c, of.q + 4 * lane, of.s, of.e)); };
   Step now = ahead;
   Quad a = load(now);
   advance();
@@ -181,4 +256,10 @@ __global__ void __launch_bounds__(SHARED_X_THREADS, 1)
     a = b; b = c;
     now = next; next = fresh;
   }
+  __syncthreads();
+  if (!left_out) return;
+  sum_rows_left_out<SHARED_X_THREADS>(
+      longest, rows, nnz, row_ptr, col, val, y, gather_of,
+      [&](int i) { return (int64_t)blockIdx.x * 32 + (i & 31) + (int64_t)(i >> 5) * warps; },
+      [&](int i) { return (int64_t)(i >> 5) * warps >= rows; });
 }

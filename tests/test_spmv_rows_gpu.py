@@ -71,3 +71,36 @@ def test_entries_outside_the_rows_belong_to_another_x(ctx, mapping, rows, low, h
     own = slice(rp[0], rp[-1])
     want = oracle.csr_spmv(rp - rp[0], ci[own], v[own], xs[:rows], parallel=True)
     assert_within_bound(y, want, oracle.csr_abs_bound(rp - rp[0], ci[own], v[own], xs[:rows]))
+
+
+@pytest.mark.parametrize("mapping", ["wave-per-row", "block-per-row"])
+@pytest.mark.parametrize("rows,low,high", [(100000, 0, 8), (90000, 20, 50), (170000, 30, 80), (120000, 30, 100), (81920, 100, 160)])
+def test_rows_that_the_block_takes(ctx, mapping, rows, low, high):
+    # limits of 2,048 (groups of lanes) and 8,192 (stream of rows); steps of two quads per thread; several in one block
+    rng = np.random.default_rng(rows)
+    lens = rng.integers(low, high, rows)
+    edges = [2047, 2048, 2049, 2052, 4095, 4097, 8191, 8192, 8193, 8200, 16384, 16389, 30001]
+    lens[:len(edges)] = edges
+    lens[rng.integers(100, rows - 1, len(edges))] = edges
+    lens[-1] = 9000
+    _check(ctx, f"spmv-mapping={mapping}", lens, rows, rows)
+
+
+@pytest.mark.parametrize("mapping", ["wave-per-row", "block-per-row"])
+def test_rows_sorted_by_length(ctx, mapping):
+    # 64 rows of 65,536 in front of 500,000 of 8: as eight rows of one warp each they take 3 ms
+    lens = torch.full((500000,), 8, device="cuda")
+    lens[:64] = 65536
+    rp = torch.nn.functional.pad(torch.cumsum(lens, 0), (1, 0)).int()
+    ci = torch.randint(0, 500000, (int(rp[-1]),), device="cuda", dtype=torch.int32)
+    v, x = torch.ones(ci.numel(), device="cuda"), torch.ones(500000, device="cuda")
+    times = []
+    for _ in range(4):
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        begin.record()
+        y = ctx.spmv(f"spmv-mapping={mapping}", rp, ci, v, x)
+        end.record()
+        end.synchronize()
+        times.append(begin.elapsed_time(end))
+    assert torch.equal(y, lens.float())
+    assert min(times) < 1.0  # ms
