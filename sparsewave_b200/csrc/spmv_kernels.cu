@@ -770,15 +770,17 @@ cudaError_t launch_row_stream(const CsrSpmvArgs &a, const DeviceInfo &dev, cudaS
 enum class RowForm { REFERENCE, SHORT_ROWS, STREAM };
 
 // wave-per-row keeps a warp per row, on its own grid, for rows of some 50 positions in matrices below 4 M nonzeros, where
-// the longest rows decide (20,000 ragged rows of 30: 6.4 us against 7.6), and for rows of more than 100 unless x is
-// staged; block-per-row keeps a block per row there, and on few rows.
+// the longest rows decide (20,000 ragged rows of 30: 6.4 us against 7.6), for rows of 51 to 100 below 10 M (100,000 ragged
+// rows of 95: 38 us against 43; 250,000 equal rows of 95: 101 against 88), and for longer ones except where x
+// is staged and lies between 256 KB, which L1 still holds (50,000 ragged rows of 500: 61 us against 79), and 512 KB (160,000
+// ragged rows of 200: 117 against 132).  block-per-row keeps a block per row for long rows with no staged x, and on few rows.
 RowForm row_form(const CsrSpmvArgs &a, bool block_per_row) {
   if (!aligned16(a.col_idx) || !aligned16(a.val) || a.rows == 0) return RowForm::REFERENCE;
   if (a.nnz > 2147483647LL - 65536) return RowForm::REFERENCE;  // positions of a step reach past a row's end
   const int64_t mean = a.nnz / a.rows;
   if (block_per_row && a.rows < 148 * 8) return RowForm::REFERENCE;
-  if (mean <= 24 || (mean <= 100 && (block_per_row || a.nnz >= 4000000))) return RowForm::SHORT_ROWS;
-  return mean > 100 && stages_x(a) ? RowForm::STREAM : RowForm::REFERENCE;
+  if (mean <= 24 || (mean <= 100 && (block_per_row || a.nnz >= (mean <= 50 ? 4000000 : 10000000)))) return RowForm::SHORT_ROWS;
+  return mean > 100 && stages_x(a) && (block_per_row || (a.cols >= 65536 && a.cols <= 131072)) ? RowForm::STREAM : RowForm::REFERENCE;
 }
 
 }  // namespace

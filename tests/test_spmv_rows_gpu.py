@@ -104,3 +104,14 @@ def test_rows_sorted_by_length(ctx, mapping):
         times.append(begin.elapsed_time(end))
     assert torch.equal(y, lens.float())
     assert min(times) < 1.0  # ms
+
+
+@pytest.mark.parametrize("rows,mean", [(60000, 70), (100000, 95), (110000, 95), (250000, 95), (60000, 130), (131072, 120), (140000, 120)])
+def test_wave_per_row_on_both_sides_of_its_limits(ctx, rows, mean):
+    # a warp per row on the reference's grid, or groups of lanes (up to eight blocks per SM) and one block per SM
+    lens = np.random.default_rng(mean).integers(mean - 30, mean + 30, rows)
+    nnz = int(lens.sum())
+    grid = ctx.launch_shape("spmv-mapping=wave-per-row spmv-block-size=128", rows, nnz).physical_grid
+    takes_others = nnz >= 10000000 if mean <= 100 else 65536 <= rows <= 131072
+    assert (grid < rows // 4) == takes_others
+    _check(ctx, "spmv-mapping=wave-per-row spmv-block-size=128", lens, rows, mean)
