@@ -731,10 +731,14 @@ inline bool tile_takes_staged_rows(int64_t rows, int64_t nnz, int64_t N) {
   return outputs >= 256000;
 }
 
-// Rows per block of that kernel for N = 64 and short rows: those of a block of the (row, tile) units, with half a warp or
-// a warp per row; 0: the kernel's own rule.
+// Rows per block of that kernel for N = 64 and short rows: from blocks of 256 on those of a block of the (row, tile) units, half
+// a warp or a warp per row, which is the grid that such a launch is known by.  Against the kernel's own rule (0: some 50 to
+// 128 rows) it costs with blocks of 256 up to 39 % on very short rows (1 M ragged rows of 3: 236 us against 170; of 5: 300
+// against 227; of 12: 520 against 448) and gains up to 14 % (100,000 equal rows of 10: 24.3 against 28.3); with blocks of 512
+// and 1,024 the two are within 10 %.  Blocks of 128 would have 4 or 8 rows and cost up to twice the time (300,000 ragged rows
+// of 3: 95 against 52).
 inline int64_t tile_rows_per_block(int64_t N, int64_t mean, int block) {
-  return N == 64 && mean <= 13 && block >= 128 ? (mean <= 12 ? 2 : 1) * (block / 32) : 0;
+  return N == 64 && mean <= 13 && block >= 256 ? (mean <= 12 ? 2 : 1) * (block / 32) : 0;
 }
 
 template <int G, int L>

@@ -160,6 +160,13 @@ def test_launch_shapes_follow_reference_grid_arithmetic():
     assert (s.work_units, s.physical_grid) == (16000, 250)
 
 
+def test_small_blocks_do_not_shrink_the_blocks_of_short_rows():
+    # wave-per-row-tile, N = 64, short rows: a block of 256 or more names its rows, smaller ones take those of the kernel's rule
+    grids = [swb.launch_shape(f"spmm-mapping=wave-per-row-tile spmm-tile-size=16 spmm-block-size={b}", 300000, 900000, 64).physical_grid
+             for b in (64, 128, 256, 1024)]
+    assert grids[0] == grids[1] < 300000 // 64 and grids[2:] == [300000 // 16, 300000 // 64 + 1]
+
+
 def test_shard_rows_by_nnz():
     rp = np.array([0, 10, 10, 30, 31, 100, 100, 120], np.int32)
     b = swb.shard_rows_by_nnz(rp, 4)
