@@ -18,6 +18,32 @@ __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b);
 #include "spmm_columns.cuh"
 #include "spmm_staged_rows.cuh"
 
+// The reference's schedule itself: a thread per output, element = blockIdx * blockDim + threadIdx, row = element / N.  On very
+// short rows there is nothing to stage and little to wait for; see takes_outputs.
+__global__ void __launch_bounds__(256)
+    spmm_thread_per_output_kernel(int64_t rows, uint32_t N, const int32_t *__restrict__ row_ptr,
+                                  const int32_t *__restrict__ col, const float *__restrict__ val,
+                                  const float *__restrict__ B, float *__restrict__ C) {
+  after_previous_kernel();
+  const int64_t first = (int64_t)blockIdx.x * 256, r0 = first / N;  // the same for the block
+  const uint32_t from = (uint32_t)(first - r0 * N) + threadIdx.x;
+  const int64_t row = r0 + from / N;
+  if (row >= rows) return;
+  const float *Bj = B + from % N;
+  int p = row_ptr[row];
+  const int end = row_ptr[row + 1];
+  float sum = 0.0f;
+  for (; end - p >= 4; p += 4) {
+    const int c0 = __ldg(col + p), c1 = __ldg(col + p + 1), c2 = __ldg(col + p + 2), c3 = __ldg(col + p + 3);
+    const float v0 = __ldg(val + p), v1 = __ldg(val + p + 1), v2 = __ldg(val + p + 2), v3 = __ldg(val + p + 3);
+    const float b0 = __ldg(Bj + (int64_t)c0 * N), b1 = __ldg(Bj + (int64_t)c1 * N);
+    const float b2 = __ldg(Bj + (int64_t)c2 * N), b3 = __ldg(Bj + (int64_t)c3 * N);
+    sum = add(add(add(add(sum, mul(v0, b0)), mul(v1, b1)), mul(v2, b2)), mul(v3, b3));
+  }
+  for (; p < end; ++p) sum = add(sum, mul(__ldg(val + p), __ldg(Bj + (int64_t)__ldg(col + p) * N)));
+  C[first + threadIdx.x] = sum;
+}
+
 // ---------------------------------------------------------------------------
 // wave-per-row-tile (WavePerRowTileSpMMPattern, SparseWaveToGPU.cpp:1057-1256)
 // tiles = ceil(N / T); unit = blockIdx * (blockDim/32) + threadIdx/32;
@@ -690,6 +716,21 @@ inline int columns_per_lane(int64_t rows, int64_t nnz, int64_t n_rhs, uintptr_t 
 // ... and whether each lane keeps to one run, with more positions a step.
 inline bool few_rows(int64_t rows, int64_t n_rhs) { return rows <= 8192 || (rows <= 32768 && n_rhs <= 32); }
 
+// Whether thread-per-output takes a thread per output: where that wins on rows of equal length, which have no longest row to
+// wait for, by more than it loses on ragged ones.  Measured (time against the kernels below, equal / ragged rows): N = 2
+// 0.83 to 0.92 / 0.97 to 1.12, N = 3 0.72 to 0.91 / 0.89 to 1.07 with up to 12 positions a row (1 M equal rows of 12: 82 -> 59
+// us), from 16 on 1.0 to 1.2; up to 4 positions a row: 2,048 to 8,000 rows, N = 33 to 128 0.45 to 0.77 / 0.66 to 1.08 (N = 200
+// 1.0 / 1.1), 9,000 to 32,000 rows, N = 5 to 32 0.49 to 0.95 / 0.74 to 1.27, up to 600,000 rows, N = 5, 7, 9, whose rows are
+// read by single columns, 0.61 to 0.81 / 0.90 to 1.20.  What is left to the kernels below can still be slower than a thread per
+// output on equal rows (N = 5 to 10 with 6 to 24 positions by up to 1.5), by less than ragged rows of the same size gain.
+inline bool takes_outputs(int64_t rows, int64_t nnz, int64_t n_rhs) {
+  if (n_rhs == 2 || n_rhs == 3) return rows >= 262144 && nnz < 13 * rows;
+  if (nnz >= 5 * rows) return false;
+  if (rows <= 8192) return n_rhs > 32 && n_rhs <= 128;
+  if (rows <= 32768) return n_rhs >= 5 && n_rhs <= 32;
+  return rows <= 700000 && (n_rhs == 5 || n_rhs == 7 || n_rhs == 9);
+}
+
 cudaError_t launch_rows(const CsrSpmmArgs &a, cudaStream_t s) {
   if (takes_row_products(a.rows, a.n_rhs)) return launch_row_products(a, s);
   if (a.n_rhs > 0x3fffffffLL) return launch_rows_as<1, 5, 4, uint64_t>(a, s);
@@ -773,6 +814,12 @@ cudaError_t launch_row_of_tiles(const CsrSpmmArgs &a, int block, cudaStream_t s)
 
 cudaError_t launch_spmm_thread_per_output(const CsrSpmmArgs &a, cudaStream_t s, int64_t *launches) {
   ++*launches;
+  if (takes_outputs(a.rows, a.nnz, a.n_rhs)) {
+    SWB_GRID(grid, ceil_div(a.rows * a.n_rhs, 256));
+    launch_chained(spmm_thread_per_output_kernel, grid, 256, 0, s, a.rows, (uint32_t)a.n_rhs, a.row_ptr, a.col_idx, a.val,
+                   a.B, a.C);
+    return cudaGetLastError();
+  }
   return launch_rows(a, s);
 }
 
@@ -828,7 +875,7 @@ cudaError_t launch_spmm_wave_per_row_tile(const CsrSpmmArgs &a, int block, int t
 }
 
 int64_t thread_per_output_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs) {
-  return rows_physical_grid(rows, nnz, n_rhs);
+  return takes_outputs(rows, nnz, n_rhs) ? max1(ceil_div(rows * n_rhs, 256)) : rows_physical_grid(rows, nnz, n_rhs);
 }
 
 int64_t wave_per_row_tile_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs, int block, int tile) {

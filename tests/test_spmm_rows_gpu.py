@@ -110,3 +110,20 @@ def test_a_very_long_row_is_not_one_chain(ctx, opts):
         end.synchronize()
         times.append(begin.elapsed_time(end))
     assert min(times) < 65536 * 80e-6  # ms
+
+
+@pytest.mark.parametrize("rows,most,n,outputs", [
+    (262144, 9, 2, True), (262144, 24, 3, True), (262143, 9, 3, False), (262144, 28, 2, False), (8192, 7, 33, True),
+    (8192, 7, 128, True), (8192, 7, 129, False), (8193, 7, 33, False), (8193, 7, 5, True), (32768, 8, 32, True), (32769, 7, 9, True),
+    (32769, 7, 8, False), (9000, 11, 16, False), (8000, 2, 100, True)])
+def test_thread_per_output_on_very_short_rows(ctx, rows, most, n, outputs):
+    # a thread per output in blocks of 256, which start and end inside a row; both sides of each limit
+    rng = np.random.default_rng(rows + n)
+    lens = rng.integers(0, most + 1, rows)
+    lens[[0, 5, -1]] = 0, 700, 5
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = rng.integers(0, 800, rp[-1]).astype(np.int32)
+    v = rng.uniform(-1, 1, rp[-1]).astype(np.float32)
+    B = rng.uniform(-1, 1, (800, n)).astype(np.float32)
+    assert (ctx.launch_shape("", rows, int(rp[-1]), n).physical_grid == -(-rows * n // 256)) == outputs
+    assert np.array_equal(_spmm(ctx, "", rp, ci, v, dev(B)).cpu().numpy(), oracle.csr_spmm(rp, ci, v, B, parallel=True))
