@@ -13,6 +13,7 @@ import subprocess
 import sys
 import sysconfig
 from concurrent.futures import ThreadPoolExecutor
+from importlib import metadata
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -120,11 +121,22 @@ def build_loaders(verbose: bool = False) -> Path:
 
 BINDING_SRC = CSRC / "binding" / "swb_torch_binding.cpp"
 BINDING = LIBDIR / "swb_torch.so"
+BINDING_FOR = LIBDIR / "swb_torch.for"  # the torch and Python that the extension was built against
+
+
+def _binding_target() -> str:
+    return f"torch {metadata.version('torch')}, python {sys.version}"
+
+
+def binding_is_stale() -> bool:
+    """Also when torch or Python were exchanged: the object links torch's C++ interface, which changes with it."""
+    return (_stale(BINDING, [BINDING_SRC, ROOT / "include" / "sparsewave_b200.h", Path(__file__)])
+            or not BINDING_FOR.exists() or BINDING_FOR.read_text() != _binding_target())
 
 
 def build_binding(verbose: bool = False) -> Path:
     """CPython extension over torch tensors and the C ABI (g++; host code only): the operator calls of api.Context."""
-    if _stale(BINDING, [BINDING_SRC, ROOT / "include" / "sparsewave_b200.h", Path(__file__)]):
+    if binding_is_stale():
         import torch
         torch_dir = Path(torch.__file__).resolve().parent
         cuda = Path(_nvcc()).resolve().parent.parent
@@ -140,6 +152,7 @@ def build_binding(verbose: bool = False) -> Path:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
         os.replace(fresh, BINDING)
+        BINDING_FOR.write_text(_binding_target())
     return BINDING
 
 
