@@ -83,7 +83,25 @@ typedef enum swb_spmm_mapping {
 
 /* Option block.  Names, defaults and ranges follow Passes.td:160-176,207-241
  * and Pipelines.h:114-190.  A wave is a CUDA warp, so wave_size must be 32 for
- * every cooperative mapping. */
+ * every cooperative mapping.
+ *
+ * All values are checked as the reference checks them.  A mapping fixes what
+ * is summed in which way (thread-per-row, thread-per-output and BSR: in
+ * position order, bit for bit the sequential loop; the others: in any order);
+ * the kernel behind it chooses its own launch shape where that is faster, and
+ * then these values have no effect on the launch:
+ *   - block_size with thread-per-row; spmm_block_size with thread-per-output
+ *     and BSR;
+ *   - block_size, position_chunk_size and position_reduction with
+ *     thread-per-position SpMV, whose positions are dealt to warps in spans
+ *     (all values give the same schedule).  They do shape the launch in
+ *     swb_spmv_position_trace, and where col_idx and val start a different
+ *     number of elements past a 16-byte boundary;
+ *   - block_size with wave-per-row and block-per-row where rows are dealt to
+ *     groups of lanes or to one block per SM, and spmm_block_size and
+ *     spmm_tile_size with wave-per-row-tile where the tiles of a row are one
+ *     pass or blocks stage their rows.
+ * swb_launch_shape_query reports both shapes. */
 typedef struct swb_options {
   int32_t mapping;                  /* swb_spmv_mapping, default thread-per-row  */
   int32_t position_reduction;       /* swb_position_reduction, default atomic    */
@@ -151,7 +169,11 @@ SWB_API int swb_options_validate(swb_context *ctx, const swb_options *opts);
 
 /* sparsewave.spmv (SparseWaveOps.td:17-52): y[r] = sum_p val[p] * x[col[p]]
  * over p in [row_ptr[r], row_ptr[r+1]).  row_ptr has rows+1 entries, col_idx
- * and val have nnz entries, x has cols entries, y has rows entries. */
+ * and val have nnz entries, x has cols entries, y has rows entries.  The row
+ * mappings use the entries of the rows only: row_ptr[0] may be above 0 and
+ * row_ptr[rows] below nnz, and what the other entries hold is not looked at.
+ * At most 2^31 - 1 nonzeros, 2^31 - 65537 with the position mappings
+ * (SWB_ERR_UNSUPPORTED beyond). */
 SWB_API int swb_spmv(swb_context *ctx, const swb_options *opts, int64_t rows,
                      int64_t cols, int64_t nnz, const int32_t *row_ptr,
                      const int32_t *col_idx, const float *val, const float *x,
@@ -453,7 +475,10 @@ SWB_API int64_t swb_row_at_position(const int32_t *row_ptr,
 /* Launch geometry of an operator under `opts`: the reference's logical grid
  * and block (SparseGPUUtils.cpp:11-59, SparseWaveToGPU.cpp:380,
  * SparsePositionScheduling.cpp:340-350), the number of kernels per call and
- * the physical CUDA grid this library launches.  n_rhs == 0 selects SpMV. */
+ * the physical CUDA grid this library launches.  n_rhs == 0 selects SpMV.
+ * The number of columns is not an argument: for wave-per-row and block-per-row
+ * SpMV, whose kernel also depends on the size of x, the physical grid is that
+ * of a square matrix. */
 typedef struct swb_launch_shape {
   int64_t logical_grid;   /* blocks the reference would launch            */
   int64_t logical_block;  /* threads per block                            */

@@ -69,6 +69,8 @@ __device__ __forceinline__ void store(__nv_bfloat16 *p, const float (&v)[n]) {
   }
 }
 
+// 4 x 4 blocks with four rows per thread: 72 registers, so that seven blocks fit an SM, at the price of 48 (f32) and 32 (bf16)
+// bytes of spills with aligned block values and four columns.
 constexpr int TILE_THREADS = 128;
 template <int n> struct Count { static constexpr int value = n; };
 

@@ -1,5 +1,5 @@
 // Sequential row sums over products formed in position order by the whole block: thread-per-row SpMV and SpMM with up to
-// four right-hand sides (included by spmv_kernels.cu inside namespace swb::{anonymous}).
+// four right-hand sides, eight on few rows (included by spmv_kernels.cu inside namespace swb::{anonymous}).
 //
 // The reference mapping gives a thread a row, so that lanes read col and val a row length apart: 32 sectors a load, each
 // fetched for four bytes, and a chain of dependent loads as long as the longest row.  Here a block owns a run of rows,
@@ -19,7 +19,9 @@
 
 // Threads of a block, most rows of a block, and products of a tile before padding.  Where 512 threads and 4,096 products per
 // block cover the matrix with four blocks per SM, all of it is in flight at once and evenly spread (206,501 ragged rows of 6:
-// 12.0 -> 9.7 us a call against blocks of 256, of which some SMs get six and others five).  Larger matrices take blocks of
+// 12.0 -> 9.7 us a call against blocks of 256, of which some SMs get six and others five).  (Three blocks fit an SM with N = 3
+// and unaligned 4, which take 40 registers, and two with N = 5 to 7 and unaligned 8, which take 56 to 64 and run on up to
+// 8,192 rows only; the rest waits.)  Larger matrices take blocks of
 // 128 and tiles of 2,048, whose gaps between gathers and sums interleave better (1 M ragged rows of 10: 52.4 -> 51.0); with
 // several columns those hold too few positions, and blocks are of 256 (404,892 banded rows of 19, N = 4: 49 -> 46).
 struct ProductsOnce { static constexpr int THREADS = 512, WORDS = 4096; };

@@ -70,7 +70,7 @@ cudaError_t launch_coo_spmv_thread_per_nonzero(int64_t rows, int64_t nnz, const 
 
 // --- SpMV row mappings
 cudaError_t launch_spmv_thread_per_row(const CsrSpmvArgs &a, cudaStream_t s, int64_t *launches);
-// Sequential row sums for n_rhs = 1 to 4 (row_products.cuh); also SpMM.
+// Sequential row sums for n_rhs = 1 to 8 (row_products.cuh); also SpMM.
 cudaError_t launch_row_products(const CsrSpmmArgs &a, cudaStream_t s);
 int64_t row_products_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs);
 cudaError_t launch_spmv_wave_per_row(const CsrSpmvArgs &a, int block, const DeviceInfo &dev,
@@ -78,7 +78,7 @@ cudaError_t launch_spmv_wave_per_row(const CsrSpmvArgs &a, int block, const Devi
 cudaError_t launch_spmv_block_per_row(const CsrSpmvArgs &a, int block, const DeviceInfo &dev,
                                       cudaStream_t s, int64_t *launches);
 
-// CUDA blocks of the two (for 16-byte aligned arrays).
+// CUDA blocks of the two (for 16-byte aligned arrays); swb_launch_shape_query asks for a square matrix.
 int64_t row_mapping_physical_grid(int64_t rows, int64_t cols, int64_t nnz, bool block_per_row, int block,
                                   const DeviceInfo &dev);
 

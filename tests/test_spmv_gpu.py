@@ -242,3 +242,26 @@ def test_gather_probe_adds_every_product(ctx):
     want = float((a.values[:n].double() * x[a.col_idx[:n].long()].double()).sum())
     scale = float((a.values[:n].double() * x[a.col_idx[:n].long()].double()).abs().sum())
     assert abs(float(sink.double().sum()) - want) <= 1e-5 * scale
+
+
+@pytest.mark.parametrize("rows", [3000, 1 << 18])  # one partition of positions per warp; spans of several
+def test_thread_per_position_options_name_one_schedule(ctx, rows):
+    """Chunk size, reduction and block size are checked, but untraced calls deal positions to warps whatever they say: whole
+    numbers come out exact under all of them, and the launch is that of wave-per-position with blocks of 128, whose rows and
+    segments the trace shows (with its batch for the same number of nonzeros)."""
+    a, x = W.config_c3(device="cuda", rows=rows)
+    v, x = torch.sign(a.values), torch.round(3 * x)
+    rp, ci = a.row_ptr.cpu().numpy(), a.col_idx.cpu().numpy()
+    want = oracle.csr_spmv(rp, ci, v.cpu().numpy(), x.cpu().numpy())
+    nnz = len(ci)
+    spans = ctx.launch_shape("spmv-mapping=wave-per-position spmv-block-size=128", rows, nnz).physical_grid
+    for chunk in (1, 7, 64):
+        for reduction in ("atomic", "segmented"):
+            for block in (32, 100, 1024):
+                opts = (f"spmv-mapping=thread-per-position spmv-position-chunk-size={chunk} "
+                        f"spmv-position-reduction={reduction} spmv-block-size={block}")
+                assert np.array_equal(ctx.spmv(opts, a.row_ptr, a.col_idx, v, x).cpu().numpy(), want)
+                assert ctx.launch_shape(opts, rows, nnz).physical_grid == spans
+    y, row, _, _ = ctx.spmv_position_trace("spmv-mapping=wave-per-position spmv-block-size=128", a.row_ptr, a.col_idx, v, x)
+    assert np.array_equal(y.cpu().numpy(), want)
+    assert np.array_equal(row.cpu().numpy(), np.repeat(np.arange(rows), np.diff(rp)))
