@@ -12,31 +12,33 @@
 //   D[m, r] (+)= sum_k  Bt[m, k] * At[k, r],   m = column, k = lc,
 // one tcgen05.mma of shape M=128, N=16, K=16 per nonzero block, all blocks of
 // the block row accumulating into one 128-lane x 16-column f32 tile in TMEM.
-// A CTA owns one block row and a tile of 256 right-hand-side columns, i.e. two
-// such accumulators side by side in TMEM (columns 0-15 and 16-31), so that each
-// block and each block-column index is fetched once per 256 columns.
+// A unit of work is one block row and a tile of 128 or 256 right-hand-side
+// columns, i.e. one or two such accumulators side by side in TMEM, so that each
+// block and each block-column index is fetched once per tile.
 //   - MMA operand A = a 16 x 128 slab B[bci*16 .. +16, n .. n+128).  Row k is
-//     contiguous along m: MN-major.  Two TMA boxes of 64 columns x 16 rows with
-//     the 128-byte swizzle land it as the canonical MN-major SWIZZLE_128B layout
+//     contiguous along m: MN-major.  TMA boxes of 64 columns x 16 rows with the
+//     128-byte swizzle land it as the canonical MN-major SWIZZLE_128B layout
 //     (128-byte rows, 1024 bytes between groups of 8 k rows = stride byte
-//     offset, 2048 bytes between the two 64-column halves = leading byte
-//     offset).  Columns past N are zero-filled by the TMA unit; a tile whose
-//     second 128 columns lie wholly past N skips them.
-//   - MMA operand B = the block itself, [r][lc] row-major: K-major.  One TMA box
-//     of 16 x 16 with the 32-byte swizzle over the block values viewed as a
+//     offset, 2048 bytes between 64-column groups = leading byte offset).  A
+//     tile of whole groups is one copy (a map of 64 columns x rows x groups).
+//   - MMA operand B = the block itself, [r][lc] row-major: K-major.  A TMA box
+//     of 16 columns with the 32-byte swizzle over the block values viewed as a
 //     (nnzb*16) x 16 matrix lands it as the canonical K-major SWIZZLE_32B layout
 //     (32-byte rows, 256 bytes between groups of 8 rows = stride byte offset).
 //     Both accumulators' MMAs read the same copy.
-// The slab rows are gathered by block-column index, four boxes per block.
 //
-// Pipeline.  Lane 0 of warp 4 is the producer: per chunk of blocks it waits for
-// the stage's `empty` mbarrier, loads the chunk's block-column indices, arms the
-// stage's `full` mbarrier with the byte count and issues the TMA copies.  Lane 0
-// of warp 5 issues the MMAs: it waits for `full`, issues the chunk's MMAs and
-// lets tcgen05.commit arrive on `empty` when they have read their operands, so
-// index loads and copies of later chunks never wait behind a commit.  After the
-// last chunk the commit arrives on `done`; warps 0-3 then read both accumulators
-// with tcgen05.ld (each warp its own 32 TMEM lanes), round to bf16 and store C.
+// Pipeline.  Persistent CTAs, three (256 columns) to five per SM, walk the units.  A stage holds a group of four 16 x 16
+// blocks (two of 32 x 32, eight of 8 x 8) with their slabs.  Lanes 0 of warps 4 - 7 copy: each takes its blocks of every
+// group, block columns held 32 at a time in the warp's lanes and requested ahead.  Lane 0 of warp 8 issues the group's MMAs
+// and lets tcgen05.commit arrive on `empty`.  There are two sets of accumulators: while warps 0 - 3 read one with tcgen05.ld,
+// round to bf16 and store C, the MMAs of the next unit fill the other.
+//
+// What bounds it is the path from L2 (13 TB/s of slabs and blocks), and below that the fixed cost of a step: a stage with one
+// MMA takes its thread some 500 clocks and its copies 300 (wait, arrive, issue, commit), whatever its size.  Hence groups,
+// several copying warps and persistence: with one block per stage, one copying thread and a CTA per unit, 3,419 block rows of
+// 8, N = 128 took 29.6 us (now 19.0), 847 of 16, N = 256 20.0 (15.2), 128 of 32, N = 512 21.3 (12.2), 1,024 of 51, N = 512
+// 63.4 (59.4).  Tried: a CTA per unit with these stages (65.8 on the last), 1 or 2 CTAs per SM with deeper rings (142, 77),
+// two chains of accumulators (no change).
 //
 // Every mbarrier wait is bounded: when one runs out the kernel raises the
 // status word, frees its TMEM columns and returns.
@@ -53,48 +55,55 @@
 namespace swb {
 namespace {
 
-constexpr int TILE_N = 256;                  // right-hand-side columns per CTA (two MMA M = 128 halves)
-constexpr int HALF_N = 128;
+constexpr int HALF_N = 128;                  // right-hand-side columns of an MMA (M); a CTA takes one or two such halves
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
-constexpr int PRODUCER_THREAD = 128;         // lane 0 of warp 4 issues the TMA copies
-constexpr int MMA_THREAD = 160;              // lane 0 of warp 5 issues the MMAs
-constexpr int THREADS = 192;
-constexpr int MAX_STAGES = 8;
+constexpr int STORE_WARPS = 4;               // warps 0 - 3 store C
+constexpr int COPY_WARP = 4;                 // the first of up to four warps whose lanes 0 issue the TMA copies
+constexpr int MMA_THREAD = 256;              // lane 0 of the last warp issues the MMAs
+constexpr int THREADS = 288;
+constexpr int MAX_STAGES = 16;
+constexpr unsigned FULL = 0xffffffffu;
 
-// A pipeline step: one block of 16 x 16 or 32 x 32, or two blocks of 8 x 8 side by side along k.
-template <int BS>
+// A stage: GROUP blocks of a block row, their slabs of B and the blocks themselves.
+template <int BS, int HALVES>
 struct Shape {
-  static constexpr int BLOCKS = BS == 8 ? 2 : 1;            // blocks per step
-  static constexpr int K = BS * BLOCKS;                     // rows of B per step: 16 or 32
+  static constexpr int GROUP = 64 / BS;                     // blocks per stage
+  static constexpr int COPY_WARPS = GROUP < 4 ? GROUP : 4;  // warps that issue its copies
+  static constexpr int MMA_BLOCKS = BS == 8 ? 2 : 1;        // blocks per MMA: two of 8 x 8 side by side along k
   static constexpr int BOX_BYTES = BS * 64 * 2;             // 64 columns x BS rows of B
-  static constexpr int GROUP_BYTES = K * 64 * 2;            // 64 columns x K rows
-  static constexpr int HALF_BYTES = 2 * GROUP_BYTES;        // one accumulator's operand
-  static constexpr int SLAB_BYTES = 2 * HALF_BYTES;
+  static constexpr int SLAB_BYTES = 2 * HALVES * BOX_BYTES; // a block's rows of B
   static constexpr int VALUE_BYTES = BS * BS * 2;           // one block
   static constexpr int MMA_N = BS == 32 ? 32 : 16;          // at least 16 with M = 128: 8 rows are padded with zeros
-  static constexpr int TMEM_COLS = 2 * MMA_N;               // two accumulators
-  // slabs first (1024-aligned), then the blocks, padded so that the next stage's slabs are 1024-aligned again
-  static constexpr int STAGE_BYTES = (SLAB_BYTES + (BS == 8 ? 512 : VALUE_BYTES) + 1023) / 1024 * 1024;
+  static constexpr int TMEM_COLS = 2 * HALVES * MMA_N;      // two sets of accumulators: 32, 64 or 128 columns
+  static constexpr int VALUES_AT = GROUP * SLAB_BYTES;      // slabs first (1024-aligned), then the blocks, then (8 x 8) zeros
+  static constexpr int ZEROS_AT = VALUES_AT + GROUP * VALUE_BYTES;
+  static constexpr int STAGE_BYTES = ZEROS_AT + (BS == 8 ? GROUP * VALUE_BYTES : 0);  // a multiple of 1024
   // Block operand, K-major: rows of 32 or 64 bytes swizzled within themselves, or (8 x 8) unswizzled core matrices of
-  // 8 rows x 16 bytes, each of which is one block: 128 bytes to the next along k, 256 bytes to the (zero) rows 8 - 15.
+  // 8 rows x 16 bytes, each of which is one block: 128 bytes to the next along k, rows 8 - 15 among the zeros.
   static constexpr uint32_t LAYOUT = BS == 32 ? 4u : BS == 16 ? 6u : 0u;
   static constexpr uint32_t LBO = BS == 8 ? 128u : 16u;
-  static constexpr uint32_t SBO = BS == 32 ? 512u : 256u;
+  static constexpr uint32_t SBO = BS == 32 ? 512u : BS == 16 ? 256u : (uint32_t)(GROUP * VALUE_BYTES);
 };
 
-// Stages of a launch.  What fills the path from L2 is the number of copies in flight per SM: with CTAs enough, three
-// stages (28 KiB for 16 x 16 blocks, seven CTAs per SM: 1024 x 1024 blocks at 5 %, 512 columns 69.7 us; two stages 78.7,
-// four 84.0); with fewer, the shared memory that is left over goes into more stages.
-template <int BS>
-int stages_for(int64_t grid, int sm_count) {
-  int64_t per_sm = (grid + sm_count - 1) / sm_count;
-  if (per_sm > 7) per_sm = 7;
-  const int64_t fit = 210 * 1024 / (per_sm > 0 ? per_sm : 1) / Shape<BS>::STAGE_BYTES;
-  const int least = BS == 32 ? 2 : 3;
-  return fit < least ? least : fit > MAX_STAGES ? MAX_STAGES : (int)fit;
+template <int BS, int HALVES>
+constexpr int most_stages() {
+  return 215 * 1024 / Shape<BS, HALVES>::STAGE_BYTES < MAX_STAGES ? 215 * 1024 / Shape<BS, HALVES>::STAGE_BYTES : MAX_STAGES;
 }
-template <int BS>
-constexpr int smem_bytes(int stages) { return stages * Shape<BS>::STAGE_BYTES + 1024; }  // + alignment slack
+// CTAs per SM, and the stages of each: the shared memory of an SM shared out among the CTAs that run on it.  More CTAs gain
+// more than more stages each (1,024 x 1,024 16 x 16 blocks at 5 %, N = 512: one CTA of six stages 142 us, two of three 77,
+// three of two 59); their accumulators fit the 512 columns of TMEM.
+template <int BS, int HALVES>
+int ctas_per_sm(int64_t units, int sm_count, int *stages) {
+  constexpr int MOST = HALVES == 2 ? 3 : BS == 32 ? 4 : 5;
+  static_assert(MOST * Shape<BS, HALVES>::TMEM_COLS <= 512 && 222 * 1024 / MOST - 1024 >= 2 * Shape<BS, HALVES>::STAGE_BYTES, "");
+  int64_t per_sm = (units + sm_count - 1) / sm_count;
+  if (per_sm > MOST) per_sm = MOST;
+  const int fit = (222 * 1024 / (int)per_sm - 1024) / Shape<BS, HALVES>::STAGE_BYTES;
+  *stages = fit > most_stages<BS, HALVES>() ? most_stages<BS, HALVES>() : fit;
+  return (int)per_sm;
+}
+template <int BS, int HALVES>
+constexpr int smem_bytes(int stages) { return stages * Shape<BS, HALVES>::STAGE_BYTES + 1024; }  // + alignment slack
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -131,6 +140,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return false;
 }
 
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+
+// Arrives on `bar` when the MMAs issued so far have completed.
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
@@ -138,47 +163,38 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
       : "memory");
 }
 
-// PER_CTA_STATUS: raise status[blockIdx.x] instead of status[0] when a wait gives up.  STAGES: the number of stages where
-// it is a constant, or 0: `run_stages` of them.
-template <bool PER_CTA_STATUS, int BS, int STAGES>
+// PER_UNIT_STATUS: raise status[unit] instead of status[0] when a wait gives up.
+template <bool PER_UNIT_STATUS, int BS, int HALVES>
 __global__ void __launch_bounds__(THREADS) bsr_spmm_tcgen05_kernel(
-    const __grid_constant__ CUtensorMap map_B, const __grid_constant__ CUtensorMap map_A, int64_t n_tiles,
-    int64_t N, int cols, int value_rows, int run_stages, const int32_t *__restrict__ brp, const int32_t *__restrict__ bci,
+    const __grid_constant__ CUtensorMap map_slab, const __grid_constant__ CUtensorMap map_box,
+    const __grid_constant__ CUtensorMap map_block, const __grid_constant__ CUtensorMap map_group, int64_t units, int64_t n_tiles,
+    int64_t N, int cols, int value_rows, int stages, const int32_t *__restrict__ brp, const int32_t *__restrict__ bci,
     __nv_bfloat16 *__restrict__ C, int *status) {
-  using S = Shape<BS>;
-  const int stages = STAGES ? STAGES : run_stages;
+  using S = Shape<BS, HALVES>;
+  constexpr int TILE_N = HALVES * HALF_N;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bar_full[STAGES ? STAGES : MAX_STAGES];
-  __shared__ __align__(8) uint64_t bar_empty[STAGES ? STAGES : MAX_STAGES];
-  __shared__ __align__(8) uint64_t bar_done;
+  __shared__ __align__(8) uint64_t bar_full[MAX_STAGES], bar_empty[MAX_STAGES];  // a stage has landed; has been read
+  __shared__ __align__(8) uint64_t bar_sums[2], bar_stored[2];  // an accumulator pair is complete; has been read
   __shared__ uint32_t tmem_slot;
   __shared__ int failed;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t br = blockIdx.x / n_tiles;
-  const int n0 = (int)((blockIdx.x % n_tiles) * TILE_N);
-  const int halves = ((int64_t)n0 + HALF_N < N) ? 2 : 1;  // the second 128 columns may lie wholly past N
   const uint32_t stage0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   after_previous_kernel();
-  const int start = brp[br], end = brp[br + 1];
-  const int nblk = end - start;
-
-  if (nblk == 0) {  // empty block row: C = 0
-    for (int64_t col = (int64_t)n0 + tid; col < N && col < (int64_t)n0 + TILE_N; col += THREADS)
-      for (int r = 0; r < BS; ++r) C[(br * BS + r) * N + col] = __float2bfloat16_rn(0.0f);
-    return;
-  }
-
   if (tid == 0) {
     failed = 0;
     for (int s = 0; s < stages; ++s) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_full[s])) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_empty[s])) : "memory");
+      mbar_init(smem_u32(&bar_full[s]), S::COPY_WARPS);
+      mbar_init(smem_u32(&bar_empty[s]), 1);
     }
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar_done)) : "memory");
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(smem_u32(&bar_sums[a]), 1);
+      mbar_init(smem_u32(&bar_stored[a]), STORE_WARPS);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_B) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_A) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_slab) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_block) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_group) : "memory");
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
@@ -187,116 +203,210 @@ __global__ void __launch_bounds__(THREADS) bsr_spmm_tcgen05_kernel(
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if constexpr (BS == 8) {  // rows 8 - 15 of the block operand, which no copy writes
-    for (int i = tid; i < stages * 64; i += THREADS)
-      asm volatile("st.shared.u32 [%0], %1;" ::"r"(stage0 + (uint32_t)(i / 64) * S::STAGE_BYTES + S::SLAB_BYTES + 256u +
-                                                   (uint32_t)(i % 64) * 4u), "r"(0u) : "memory");
+    constexpr int WORDS = (S::STAGE_BYTES - S::ZEROS_AT) / 4;
+    for (int i = tid; i < stages * WORDS; i += THREADS)
+      asm volatile("st.shared.u32 [%0], %1;" ::"r"(stage0 + (uint32_t)(i / WORDS * S::STAGE_BYTES + S::ZEROS_AT + i % WORDS * 4)),
+                   "r"(0u) : "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
-  const int steps = (nblk + S::BLOCKS - 1) / S::BLOCKS;
 
-  if (tid == PRODUCER_THREAD) {
-    for (int i = 0, s = 0, round = 0; i < steps; ++i) {
-      if (round > 0 && !mbar_wait(smem_u32(&bar_empty[s]), (uint32_t)(round - 1) & 1u)) {
-        failed = 1;  // the MMAs of step i - stages never released this stage
-        atomicExch(status + (PER_CTA_STATUS ? blockIdx.x : 0), 1);
-        break;
-      }
-      const int first = start + i * S::BLOCKS;
-      int y_B[S::BLOCKS], y_A[S::BLOCKS];  // first rows in B and among the block values; past a row's blocks: zeros
+  // All roles walk the CTA's units in the same order.  The offsets of a unit's block row are loaded a unit ahead.
+  const int64_t first_unit = blockIdx.x, stride = gridDim.x;
+  auto bounds = [&](int64_t unit) {
+    if (unit >= units) return make_int2(0, 0);
+    const int32_t *p = brp + unit / n_tiles;
+    return make_int2(__ldg(p), __ldg(p + 1));
+  };
+  auto gave_up = [&](int64_t unit) {
+    failed = 1;
+    atomicExch(status + (PER_UNIT_STATUS ? unit : 0), 1);
+  };
+  if (warp >= COPY_WARP && warp < COPY_WARP + S::COPY_WARPS) {
+    // Each of these warps copies its share of every group: blocks `mine`, mine + COPY_WARPS, ...  Lane l holds the block column
+    // of the l-th of 32 blocks, and of the 32 behind them or of the next unit's first.
+    const int mine = warp - COPY_WARP;
+    auto column = [&](int2 b, int p) { return b.x + p + lane < b.y ? __ldg(bci + b.x + p + lane) : 0; };
+    int2 b = bounds(first_unit), after = bounds(first_unit + stride);
+    int s = 0, round = 0;
+    int next_unit = column(b, 0);
+    bool ok = true;
+    for (int64_t unit = first_unit; ok && unit < units; unit += stride) {
+      const int n0 = (int)(unit % n_tiles) * TILE_N;
+      // The tile's boxes of 64 columns that reach into B.  One copy takes them all unless the last is a part of one: then, and
+      // where there is one, each is a copy.  The others are not copied (or zeros): what lies in their place makes accumulator
+      // lanes that are not stored.
+      const int boxes = N - n0 >= TILE_N ? 2 * HALVES : (int)(N - n0 + 63) / 64;
+      const bool one_copy = boxes > 1 && (N - n0 >= TILE_N || N % 64 == 0);
+      const uint32_t block_bytes = (one_copy ? 2 * HALVES : boxes) * S::BOX_BYTES;
+      int here = next_unit, ahead = column(b, 32);
+      next_unit = column(after, 0);
+      const int2 after2 = bounds(unit + 2 * stride);
+      const int nblk = b.y - b.x;
+      for (int p = 0; p < nblk; p += S::GROUP) {
+        ok = round == 0 || mbar_wait(smem_u32(&bar_empty[s]), (uint32_t)(round - 1) & 1u);
+        ok = __all_sync(FULL, ok);
+        if (!ok) {  // the MMAs that read this stage last never released it
+          if (lane == 0) gave_up(unit);
+          break;
+        }
+        if (p != 0 && p % 32 == 0) { here = ahead; ahead = column(b, p + 32); }
+        constexpr int SHARE = S::GROUP / S::COPY_WARPS;
+        int block_column[SHARE];
 #pragma unroll
-      for (int j = 0; j < S::BLOCKS; ++j) {
-        const bool in = first + j < end;
-        y_B[j] = in ? __ldg(bci + first + j) * BS : cols;
-        y_A[j] = in ? (first + j) * BS : value_rows;
-      }
-      const uint32_t full = smem_u32(&bar_full[s]);
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full),
-                   "r"((uint32_t)(halves * S::HALF_BYTES + S::BLOCKS * S::VALUE_BYTES))
-                   : "memory");
-      const uint32_t base = stage0 + (uint32_t)s * S::STAGE_BYTES;
+        for (int i = 0; i < SHARE; ++i) block_column[i] = __shfl_sync(FULL, here, (p + mine + i * S::COPY_WARPS) & 31);
+        if (lane == 0) {
+          const uint32_t full = smem_u32(&bar_full[s]), base = stage0 + (uint32_t)s * S::STAGE_BYTES;
+          const int left = nblk - p < S::GROUP ? nblk - p : S::GROUP;
+          const bool group = left == S::GROUP;  // all values are one copy, this warp's if it is the first
+          const int copies = (left + S::MMA_BLOCKS - 1) / S::MMA_BLOCKS * S::MMA_BLOCKS;  // past a row's blocks: zeros
+          const int share = group ? SHARE : (copies - mine + S::COPY_WARPS - 1) / S::COPY_WARPS;
+          const uint32_t bytes = share * block_bytes + (group ? (mine == 0 ? S::GROUP : 0) : share) * S::VALUE_BYTES;
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(bytes) : "memory");
+          if (group && mine == 0) tma_load_2d(base + S::VALUES_AT, &map_group, 0, (b.x + p) * BS, full);
 #pragma unroll
-      for (int j = 0; j < S::BLOCKS; ++j) {
+          for (int i = 0; i < SHARE; ++i) {
+            if (i >= share) break;
+            const int j = mine + i * S::COPY_WARPS;
+            const int y_B = j < left ? block_column[i] * BS : cols;
+            const uint32_t slab = base + (uint32_t)(j * S::SLAB_BYTES);
+            if (one_copy) {
+              tma_load_3d(slab, &map_slab, 0, y_B, n0 / 64, full);
+            } else {
 #pragma unroll
-        for (int g = 0; g < 4; ++g)
-          if (g < 2 || halves == 2)
-            tma_load_2d(base + (uint32_t)(g * S::GROUP_BYTES + j * S::BOX_BYTES), &map_B, n0 + 64 * g, y_B[j], full);
-        tma_load_2d(base + (uint32_t)(S::SLAB_BYTES + j * S::VALUE_BYTES), &map_A, 0, y_A[j], full);
+              for (int g = 0; g < 2 * HALVES; ++g)
+                if (g < boxes) tma_load_2d(slab + (uint32_t)(g * S::BOX_BYTES), &map_box, n0 + 64 * g, y_B, full);
+            }
+            if (!group)
+              tma_load_2d(base + (uint32_t)(S::VALUES_AT + j * S::VALUE_BYTES), &map_block, 0,
+                          j < left ? (b.x + p + j) * BS : value_rows, full);
+          }
+        }
+        __syncwarp();
+        if (++s == stages) { s = 0; ++round; }
       }
-      if (++s == stages) { s = 0; ++round; }
+      b = after;
+      after = after2;
+    }
+    // the last arrivals on `empty` before the shared memory goes back
+    for (int i = 0; ok && i < stages; ++i) {
+      if (s == 0) { s = stages; --round; }
+      --s;
+      if (round < 0) break;
+      ok = mbar_wait(smem_u32(&bar_empty[s]), (uint32_t)round & 1u);
     }
   } else if (tid == MMA_THREAD) {
+    int2 b = bounds(first_unit);
+    int s = 0, round = 0, made = 0;  // accumulator pairs begun
     bool ok = true;
-    for (int c = 0, s = 0, round = 0; c < steps; ++c) {
-      ok = mbar_wait(smem_u32(&bar_full[s]), (uint32_t)round & 1u);
-      if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t base = stage0 + (uint32_t)s * S::STAGE_BYTES;
-      for (int h = 0; h < halves; ++h) {
+    for (int64_t unit = first_unit; ok && unit < units; unit += stride) {
+      const int2 after = bounds(unit + stride);
+      const int nblk = b.y - b.x;
+      if (nblk > 0) {
+        const int halves = HALVES == 2 && (unit % n_tiles) * TILE_N + HALF_N < N ? 2 : 1;
+        const uint32_t sums = tmem + (uint32_t)((made & 1) * HALVES * S::MMA_N);
+        ok = made < 2 || mbar_wait(smem_u32(&bar_stored[made & 1]), (uint32_t)(made / 2 - 1) & 1u);
+        for (int p = 0; ok && p < nblk; p += S::GROUP) {
+          ok = mbar_wait(smem_u32(&bar_full[s]), (uint32_t)round & 1u);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t base = stage0 + (uint32_t)s * S::STAGE_BYTES;
 #pragma unroll
-        for (int k = 0; k < S::K / 16; ++k) {  // 16 rows of a slab are 2048 bytes, 16 values of a block row 32
-          const uint64_t adesc = make_desc(base + (uint32_t)(h * S::HALF_BYTES + k * 2048), S::GROUP_BYTES, 1024u, 2u);
-          const uint64_t bdesc = make_desc(base + (uint32_t)(S::SLAB_BYTES + k * 32), S::LBO, S::SBO, S::LAYOUT);
-          asm volatile(
-              "{\n\t.reg .pred p;\n\t"
-              "setp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem + (uint32_t)(h * S::MMA_N)),
-              "l"(adesc), "l"(bdesc), "r"(instruction_descriptor(S::MMA_N)), "r"((c > 0 || k > 0) ? 1u : 0u)
-              : "memory");
+          for (int j = 0; j < S::GROUP; j += S::MMA_BLOCKS) {
+            if (p + j >= nblk) break;
+#pragma unroll
+            for (int h = 0; h < HALVES; ++h) {
+              if (h >= halves) break;
+#pragma unroll
+              for (int k = 0; k < BS * S::MMA_BLOCKS / 16; ++k) {  // 16 rows of a box are 2048 bytes, 16 values of a block row 32
+                const uint64_t adesc = make_desc(base + (uint32_t)(j * S::SLAB_BYTES + h * 2 * S::BOX_BYTES + k * 2048),
+                                                 S::BOX_BYTES, BS == 8 ? S::SLAB_BYTES : 1024u, 2u);
+                const uint64_t bdesc = make_desc(base + (uint32_t)(S::VALUES_AT + j * S::VALUE_BYTES + k * 32), S::LBO, S::SBO,
+                                                 S::LAYOUT);
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\t"
+                    "setp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(sums + (uint32_t)(h * S::MMA_N)),
+                    "l"(adesc), "l"(bdesc), "r"(instruction_descriptor(S::MMA_N)), "r"((p > 0 || j > 0 || k > 0) ? 1u : 0u)
+                    : "memory");
+              }
+            }
+          }
+          mma_commit(smem_u32(&bar_empty[s]));
+          if (p + S::GROUP >= nblk) mma_commit(smem_u32(&bar_sums[made & 1]));
+          if (++s == stages) { s = 0; ++round; }
+        }
+        if (!ok) gave_up(unit);
+        ++made;
+      }
+      b = after;
+    }
+  } else if (warp < STORE_WARPS) {
+    int2 b = bounds(first_unit);
+    int made = 0;
+    for (int64_t unit = first_unit; unit < units; unit += stride) {
+      const int2 after = bounds(unit + stride);
+      const int64_t br = unit / n_tiles;
+      const int n0 = (int)(unit - br * n_tiles) * TILE_N;
+      const bool empty = b.x == b.y;  // C = 0
+      const int halves = HALVES == 2 && (int64_t)n0 + HALF_N < N ? 2 : 1;
+      const uint32_t sums = tmem + (uint32_t)((made & 1) * HALVES * S::MMA_N) + ((uint32_t)(warp * 32) << 16);
+      if (!empty) {
+        const bool ok = mbar_wait(smem_u32(&bar_sums[made & 1]), (uint32_t)(made / 2) & 1u);
+        if (!__all_sync(FULL, ok)) {
+          if (lane == 0) gave_up(unit);
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      // TMEM lane m of accumulator h = column n0 + 128 h + m of C; this warp reads lanes 32 warp .. +32
+      uint32_t v[HALVES][BS < 16 ? 16 : BS];
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h)
+#pragma unroll
+        for (int r0 = 0; r0 < BS; r0 += 16) {
+          if (empty || h >= halves) {
+#pragma unroll
+            for (int r = 0; r < 16; ++r) v[h][r0 + r] = 0;
+          } else {
+            uint32_t *w = &v[h][r0];
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+                "%15}, [%16];"
+                : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]),
+                  "=r"(w[8]), "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
+                : "r"(sums + (uint32_t)(h * S::MMA_N + r0))
+                : "memory");
+          }
+        }
+      if (!empty) {
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_stored[made & 1])) : "memory");
+        ++made;
+      }
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h) {
+        const int64_t col = (int64_t)n0 + h * HALF_N + warp * 32 + lane;
+        if (col < N) {
+          __nv_bfloat16 *out = C + br * BS * N + col;
+#pragma unroll
+          for (int r = 0; r < BS; ++r) out[r * N] = __float2bfloat16_rn(__uint_as_float(v[h][r]));
         }
       }
-      const uint32_t arrive_on = (c == steps - 1) ? smem_u32(&bar_done) : smem_u32(&bar_empty[s]);
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(arrive_on)
-                   : "memory");
-      if (++s == stages) { s = 0; ++round; }
-    }
-    if (!ok) {
-      failed = 1;
-      atomicExch(status + (PER_CTA_STATUS ? blockIdx.x : 0), 1);
-      // Release the waiters below.
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_done)) : "memory");
+      b = after;
     }
   }
-  // The four epilogue warps wait for the last MMA (or for the failure release).
-  bool done_ok = warp < 4 ? mbar_wait(smem_u32(&bar_done), 0u) : true;
-  done_ok = __syncthreads_and(done_ok);
+  __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (!done_ok && tid == 0) atomicExch(status + (PER_CTA_STATUS ? blockIdx.x : 0), 1);
-  if (!done_ok || failed) {
+  if (failed) {
     // A wait gave up with copies or MMAs of this CTA possibly still in flight: give them a bounded time (1 ms)
     // to land before the shared memory and the TMEM columns go back to the SM.
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   }
-
-  if (done_ok && !failed && warp < 4) {
-    // TMEM lane m of accumulator h = column n0 + 128 h + m of C; this warp reads lanes 32 warp .. +32
-    for (int h = 0; h < halves; ++h) {
-      const int64_t col = (int64_t)n0 + h * HALF_N + warp * 32 + lane;
-#pragma unroll
-      for (int r0 = 0; r0 < BS; r0 += 16) {
-        uint32_t v[16];
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(h * S::MMA_N + r0);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-            "%15}, [%16];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(taddr)
-            : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (col < N) {
-#pragma unroll
-          for (int r = 0; r < (BS < 16 ? BS : 16); ++r)
-            C[(br * BS + r0 + r) * N + col] = __float2bfloat16_rn(__uint_as_float(v[r]));
-        }
-      }
-    }
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TMEM_COLS) : "memory");
 }
@@ -331,6 +441,19 @@ bool make_map_2d(CUtensorMap *map, const void *base, uint64_t inner, uint64_t ou
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// B as groups of 64 columns: 64 elements, `rows` rows, n / 64 groups; a box of `box_rows` rows of `groups` groups.
+bool make_map_3d(CUtensorMap *map, const void *base, uint64_t n, uint64_t rows, uint32_t box_rows, uint32_t groups) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return false;
+  cuuint64_t dims[3] = {64, rows, n / 64};
+  cuuint64_t strides[2] = {n * 2, 128};  // bytes between rows, between groups
+  cuuint32_t box[3] = {64, box_rows, groups};
+  cuuint32_t elem[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(base), dims, strides, box, elem,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 }  // namespace
 
 bool bsr_tcgen05_supported(const BsrSpmmArgs &a) {
@@ -350,43 +473,59 @@ bool bsr_tcgen05_pays(const BsrSpmmArgs &a) { return a.block_size != 8 || a.n_rh
 namespace {
 
 // Opts a kernel into its largest shared memory, once per device; racing threads repeat an idempotent call.
-template <bool PER_CTA_STATUS, int BS, int STAGES>
+template <bool PER_UNIT_STATUS, int BS, int HALVES>
 cudaError_t configure() {
   static std::atomic<bool> configured[64];
   int device = 0;
   cudaGetDevice(&device);
   if (device >= 0 && device < 64 && configured[device].load(std::memory_order_acquire)) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(bsr_spmm_tcgen05_kernel<PER_CTA_STATUS, BS, STAGES>,
+  cudaError_t e = cudaFuncSetAttribute(bsr_spmm_tcgen05_kernel<PER_UNIT_STATUS, BS, HALVES>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       smem_bytes<BS>(STAGES ? STAGES : MAX_STAGES));
+                                       smem_bytes<BS, HALVES>(most_stages<BS, HALVES>()));
   if (e == cudaSuccess && device >= 0 && device < 64) configured[device].store(true, std::memory_order_release);
   return e;
 }
 
-template <bool PER_CTA_STATUS, int BS, int STAGES>
-cudaError_t launch_stages(const BsrSpmmArgs &a, int *status, int stages, int64_t grid, int64_t n_tiles, cudaStream_t s) {
-  cudaError_t e = configure<PER_CTA_STATUS, BS, STAGES>();
+template <bool PER_UNIT_STATUS, int BS, int HALVES>
+cudaError_t launch_halves(const BsrSpmmArgs &a, int *status, int sm_count, cudaStream_t s) {
+  const int64_t n_tiles = ceil_div(a.n_rhs, HALVES * HALF_N), units = a.rows / BS * n_tiles;
+  if (units == 0) return cudaSuccess;
+  cudaError_t e = configure<PER_UNIT_STATUS, BS, HALVES>();
   if (e != cudaSuccess) return e;
-  CUtensorMap map_B, map_A;
-  // B: cols x N bf16, boxes of 64 columns x BS rows, 128-byte swizzle; block values: (nnzb * BS) x BS, one box per block.
-  if (!make_map_2d(&map_B, a.B, (uint64_t)a.n_rhs, (uint64_t)a.cols, 64, BS, CU_TENSOR_MAP_SWIZZLE_128B) ||
-      !make_map_2d(&map_A, a.block_values, BS, (uint64_t)a.nnzb * BS, BS, BS,
-                   BS == 8 ? CU_TENSOR_MAP_SWIZZLE_NONE : BS == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B))
+  CUtensorMap map_slab, map_box, map_block, map_group;
+  // B: cols x N bf16, boxes of 64 columns x BS rows, 128-byte swizzle, one or (in whole groups of 64 columns) a tile's; block
+  // values: (nnzb * BS) x BS, boxes of one block and of a group.
+  const auto swizzle = BS == 8 ? CU_TENSOR_MAP_SWIZZLE_NONE : BS == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B;
+  if (!make_map_2d(&map_box, a.B, (uint64_t)a.n_rhs, (uint64_t)a.cols, 64, BS, CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !make_map_2d(&map_block, a.block_values, BS, (uint64_t)a.nnzb * BS, BS, BS, swizzle) ||
+      !make_map_2d(&map_group, a.block_values, BS, (uint64_t)a.nnzb * BS, BS, 64, swizzle))
     return cudaErrorInvalidValue;
-  launch_chained(bsr_spmm_tcgen05_kernel<PER_CTA_STATUS, BS, STAGES>, (unsigned)grid, THREADS,
-                 (size_t)smem_bytes<BS>(stages), s, map_B, map_A, n_tiles, a.n_rhs, (int)a.cols, (int)(a.nnzb * BS), stages,
-                 a.block_row_ptr, a.block_col_idx, static_cast<__nv_bfloat16 *>(a.C), status);
+  if (a.n_rhs < 64)
+    map_slab = map_box;  // not used: no tile has two boxes
+  else if (!make_map_3d(&map_slab, a.B, (uint64_t)a.n_rhs, (uint64_t)a.cols, BS, 2 * HALVES))
+    return cudaErrorInvalidValue;
+  int stages;
+  const int per_sm = ctas_per_sm<BS, HALVES>(units, sm_count, &stages);
+  const int64_t grid = units < (int64_t)per_sm * sm_count ? units : (int64_t)per_sm * sm_count;
+  launch_chained(bsr_spmm_tcgen05_kernel<PER_UNIT_STATUS, BS, HALVES>, (unsigned)grid, THREADS,
+                 (size_t)smem_bytes<BS, HALVES>(stages), s, map_slab, map_box, map_block, map_group, units, n_tiles, a.n_rhs,
+                 (int)a.cols, (int)(a.nnzb * BS), stages, a.block_row_ptr, a.block_col_idx,
+                 static_cast<__nv_bfloat16 *>(a.C), status);
   return cudaGetLastError();
 }
 
-template <bool PER_CTA_STATUS, int BS>
+template <bool PER_UNIT_STATUS, int BS>
 cudaError_t launch_tcgen05(const BsrSpmmArgs &a, int *status, int sm_count, cudaStream_t s) {
-  const int64_t n_tiles = ceil_div(a.n_rhs, TILE_N), grid = a.rows / BS * n_tiles;
-  if (grid == 0) return cudaSuccess;
-  if (grid > 2147483647LL) return cudaErrorInvalidConfiguration;
-  const int stages = stages_for<BS>(grid, sm_count);
-  if (stages == 3) return launch_stages<PER_CTA_STATUS, BS, 3>(a, status, stages, grid, n_tiles, s);
-  return launch_stages<PER_CTA_STATUS, BS, 0>(a, status, stages, grid, n_tiles, s);
+  // Tiles of 256 columns fetch a block once for two accumulators; tiles of 128 where the second would be empty or nearly so,
+  // and where 256 leave too few units (403 block rows of 9, N = 480: 13.2 us with 256, 12.4 with 128; 1,024 of 51, N = 512:
+  // 59 and 64).  A block of 32 x 32 is large beside its slab, but two tiles' slabs leave room for one stage only (47.7 us
+  // with 128, 80 with 256 on 512 block rows of 32, N = 512).  The status words of the static entry point are per 256 columns.
+  const int64_t pairs = a.rows / BS * ceil_div(a.n_rhs, 2 * HALF_N), tail = a.n_rhs % (2 * HALF_N);
+  const bool narrow = BS == 32 || a.n_rhs <= HALF_N || (tail > 0 && tail <= 64) || pairs < 6 * (int64_t)sm_count;
+  if constexpr (!PER_UNIT_STATUS)
+    if (narrow) return launch_halves<PER_UNIT_STATUS, BS, 1>(a, status, sm_count, s);
+  if constexpr (BS != 32) return launch_halves<PER_UNIT_STATUS, BS, 2>(a, status, sm_count, s);
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace
@@ -513,7 +652,7 @@ extern "C" __attribute__((visibility("default"))) int swb_bsr16_spmm_bf16_static
     return static_fail(kUnsupported,
                        "the static-scratch BSR entry point needs at least one block, a column count that is a "
                        "multiple of 8 and 16-byte aligned block values and right-hand side");
-  const int64_t n_tiles = ceil_div(n_rhs, TILE_N);
+  const int64_t n_tiles = ceil_div(n_rhs, 2 * HALF_N);
   const int64_t grid = (rows / 16) * n_tiles;
   if (grid > SWB_STATIC_MAX_CTAS)
     return static_fail(kCapacity,

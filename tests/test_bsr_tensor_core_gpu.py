@@ -35,3 +35,19 @@ def test_values_of_other_block_rows_do_not_leak(ctx, bs):
     C = ctx.bsr_spmm("", brp.cuda(), bci.cuda(), values.cuda(), B.cuda(), bs).float().cpu()
     assert torch.equal(C[:bs], torch.full((bs, 128), float(bs))) and torch.equal(C[bs:2 * bs], torch.full((bs, 128), 3.0 * bs))
     assert bool(C[2 * bs:3 * bs].isnan().all()) and bool(C[3 * bs:].isinf().all())
+
+
+@pytest.mark.parametrize("bs,rows,n", [(16, 3, 128), (16, 1900, 128), (16, 1000, 320), (16, 700, 232), (16, 1300, 512),
+                                       (32, 450, 64), (32, 1500, 72), (32, 300, 200), (8, 2100, 256), (8, 4400, 440)])
+def test_several_units_per_cta(ctx, bs, rows, n):
+    """Persistent CTAs: one to nine units each, with empty block rows, whole and partial groups, and both tile widths."""
+    counts = torch.tensor([0, 1, 2, 3, 4, 5, 9, 0, 16, 35])[torch.arange(rows) % 10]
+    brp = torch.zeros(rows + 1, dtype=torch.int32)
+    brp[1:] = torch.cumsum(counts, 0)
+    cols = 37
+    bci = torch.cat([torch.randperm(cols, generator=torch.Generator().manual_seed(i))[:c].sort()[0] for i, c in enumerate(counts)])
+    values = W.dense_normal((int(brp[-1]) * bs, bs), seed=bs).view(-1)
+    B = W.dense_normal((cols * bs, n), seed=n)
+    C = ctx.bsr_spmm("", brp.cuda(), bci.int().cuda(), values.cuda(), B.cuda(), bs)
+    assert ctx.device_status() == 0
+    assert_bf16_close(C, brp.numpy(), bci.int().numpy(), values.view(torch.uint16).numpy(), B.view(torch.uint16).numpy(), bs)
