@@ -465,10 +465,18 @@ bool bsr_tcgen05_supported(const BsrSpmmArgs &a) {
          (reinterpret_cast<uintptr_t>(a.B) & 15u) == 0 && (reinterpret_cast<uintptr_t>(a.block_values) & 15u) == 0;
 }
 
-// 16 x 16 and 32 x 32 blocks always gain; 8 x 8 half fill the MMA and a block row is little work for a CTA: they gain from
-// some 96 columns (2,048 block rows of 32, N = 128: 74 -> 32 us), not below (8,000 block rows of 8, N = 64: 45 us on the
-// CUDA cores, 67 here).
-bool bsr_tcgen05_pays(const BsrSpmmArgs &a) { return a.block_size != 8 || a.n_rhs >= 96; }
+// Against the mma.sync kernel, which reads its operands from global memory and takes any size: this one where a tile of
+// columns is well filled and there are units enough for persistent CTAs (times: mma.sync, here).  16 x 16: whole groups of 64
+// columns (1,024 block rows of 51, N = 512: 133, 59 us; 3,419 of 8, N = 128: 24.7, 19.0), or a last tile of 96 columns or more
+// (846 of 9, N = 496: 25.2, 19.6), but N = 264 leaves tiles of 8 columns (6,651 units of 6: 25, 30) and N = 64 half a tile
+// (1,025 of 7: 6.1, 8.8).  32 x 32: from 64 columns (1,331 of 5, N = 64: 11.7, 10.8; 94 units, N = 88: 6.8, 13.7).  8 x 8, half
+// of whose MMA is padding: from 256 columns on many units (6,105 of 13, N = 256: 57, 40; N = 184: 39, 47).
+bool bsr_tcgen05_pays(const BsrSpmmArgs &a) {
+  const int64_t n = a.n_rhs, units = a.rows / a.block_size * ceil_div(n, HALF_N), tail = n % (2 * HALF_N);
+  if (a.block_size == 32) return n >= HALF_N ? units >= 200 : n >= 64 && units >= 400;
+  if (a.block_size == 16) return n >= HALF_N && (n % 64 == 0 || (tail >= 96 && units >= 1000));
+  return n >= 2 * HALF_N && (n % 64 == 0 ? units >= 4000 : n >= 400 && units >= 13000);
+}
 
 namespace {
 
@@ -668,7 +676,10 @@ extern "C" __attribute__((visibility("default"))) int swb_bsr16_spmm_bf16_static
   // The words keep the previous call's outcome: clear the ones this call uses.
   e = cudaMemsetAsync(status, 0, (size_t)grid * sizeof(int), s);
   if (e != cudaSuccess) return static_fail(kCuda, cudaGetErrorString(e));
-  e = launch_tcgen05<true, 16>(a, status, DeviceInfo().sm_count, s);
+  // The kernel that the regular entry point would choose, so that both give the same bits; the one without tcgen05 never waits.
+  int64_t launches = 0;
+  e = bsr_tcgen05_pays(a) ? launch_tcgen05<true, 16>(a, status, DeviceInfo().sm_count, s)
+                          : launch_bsr_spmm_mma(a, DeviceInfo(), s, &launches);
   if (e == cudaErrorInvalidValue) return static_fail(kCuda, "could not encode the TMA tensor maps");
   if (e != cudaSuccess) return static_fail(kCuda, cudaGetErrorString(e));
   slot->last_grid.store(grid, std::memory_order_release);

@@ -776,6 +776,8 @@ int swb_bsr_spmm_bf16(swb_context *ctx, const swb_options *o, int64_t rows, int6
   cudaError_t e;
   if (swb::bsr_tcgen05_supported(a) && swb::bsr_tcgen05_pays(a))
     e = swb::launch_bsr_spmm_tcgen05(a, ctx->status_flag, ctx->dev, s, &ctx->launches);
+  else if (a.block_size == 8 || a.block_size == 16 || a.block_size == 32)
+    e = swb::launch_bsr_spmm_mma(a, ctx->dev, s, &ctx->launches);
   else
     e = swb::launch_bsr_spmm_thread_per_output_bf16(a, s, &ctx->launches);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "bsr_spmm launch");

@@ -135,10 +135,12 @@ cudaError_t launch_split_columns(int64_t rows, const int32_t *row_ptr, const int
 // --- BSR SpMM
 cudaError_t launch_bsr_spmm_thread_per_output_f32(const BsrSpmmArgs &a, cudaStream_t s, int64_t *launches);
 cudaError_t launch_bsr_spmm_thread_per_output_bf16(const BsrSpmmArgs &a, cudaStream_t s, int64_t *launches);
-// 8x8, 16x16 and 32x32 bf16 blocks on the tcgen05 tensor cores.  `status_flag` is a device
+// 8x8, 16x16 and 32x32 bf16 blocks with warp-level MMAs: any number of columns and alignment.
+cudaError_t launch_bsr_spmm_mma(const BsrSpmmArgs &a, const DeviceInfo &dev, cudaStream_t s, int64_t *launches);
+// The same blocks on the tcgen05 tensor cores.  `status_flag` is a device
 // int the kernel sets non-zero when one of its bounded waits gives up.
 bool bsr_tcgen05_supported(const BsrSpmmArgs &a);
-bool bsr_tcgen05_pays(const BsrSpmmArgs &a);  // faster there than thread-per-output
+bool bsr_tcgen05_pays(const BsrSpmmArgs &a);  // faster there than launch_bsr_spmm_mma
 cudaError_t launch_bsr_spmm_tcgen05(const BsrSpmmArgs &a, int *status_flag, const DeviceInfo &dev, cudaStream_t s,
                                     int64_t *launches);
 
