@@ -27,11 +27,11 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int MMA_WARPS = 8;
 
-template <int BS, int T>
+template <int BS, int T, int V>
 struct Fragments {
   static constexpr int ROWS = BS == 32 ? 8 : 4;   // rows of B per lane and step
   static constexpr int TILES = BS / 8;            // n8 tiles of block rows
-  uint32_t slab[ROWS][T];                         // 2 T adjacent columns each
+  uint32_t slab[ROWS][T + (V == 0)];              // 2 T adjacent columns each (V = 0: the words that hold them)
   uint32_t block[TILES][ROWS / 2];                // block row 8 u + g, the lane's ROWS columns
 };
 
@@ -67,6 +67,17 @@ __device__ __forceinline__ void load_row(uint32_t (&w)[T], const __nv_bfloat16 *
     }
   }
 }
+// The T + 1 aligned words that hold 2 T adjacent elements, of which the first `valid` matter (`odd`: they start in the middle
+// of a word).  A word that holds one of those lies in B, which has an even number of elements and starts at a word.
+template <int T>
+__device__ __forceinline__ void load_words(uint32_t (&w)[T + 1], const __nv_bfloat16 *p, int odd, int valid) {
+  const unsigned *word = reinterpret_cast<const unsigned *>(p - odd);
+#pragma unroll
+  for (int i = 0; i <= T; ++i) {
+    w[i] = 0;
+    if (valid > 0 && 2 * i - odd < valid && (i < T || odd)) w[i] = __ldg(word + i);
+  }
+}
 template <int T, int V>
 __device__ __forceinline__ void store_row(__nv_bfloat16 *p, const uint32_t (&w)[T], int valid) {
   if constexpr (V == 8) {
@@ -95,13 +106,14 @@ __device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uin
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// V: elements per load of a row of B.  WIDE: block values are aligned for loads of a lane's ROWS.
+// V: elements per load of a row of B, or 0: N is odd and B starts at a word, so that rows in turn start at a word and in the
+// middle of one.  WIDE: block values are aligned for loads of a lane's ROWS.
 template <int BS, int T, int V, bool WIDE>
 __global__ void __launch_bounds__(32 * MMA_WARPS, 2)
     bsr_spmm_mma_kernel(int64_t units, int tiles, int split, int64_t N, const int32_t *__restrict__ brp,
                         const int32_t *__restrict__ bci, const __nv_bfloat16 *__restrict__ bv,
                         const __nv_bfloat16 *__restrict__ B, __nv_bfloat16 *__restrict__ C) {
-  using F = Fragments<BS, T>;
+  using F = Fragments<BS, T, V>;
   constexpr int BLOCKS = BS == 8 ? 2 : 1;  // blocks per step
   constexpr int BATCH = 32 / BLOCKS;       // steps whose block columns the warp holds
   after_previous_kernel();
@@ -144,7 +156,10 @@ __global__ void __launch_bounds__(32 * MMA_WARPS, 2)
     const bool in = BS != 8 || p < end;  // the second block of a last step may be missing: zeros
     const __nv_bfloat16 *b = Bt + (int64_t)bc * BS * N;
 #pragma unroll
-    for (int r = 0; r < F::ROWS; ++r) load_row<T, V>(f.slab[r], b + r * N, in ? valid : 0);
+    for (int r = 0; r < F::ROWS; ++r) {
+      if constexpr (V == 0) load_words<T>(f.slab[r], b + r * N, r & 1, in ? valid : 0);
+      else load_row<T, V>(f.slab[r], b + r * N, in ? valid : 0);
+    }
     const __nv_bfloat16 *a = bv + (int64_t)p * (BS * BS) + g * BS + (BS == 8 ? 4 * (q & 1) : F::ROWS * q);
 #pragma unroll
     for (int u = 0; u < F::TILES; ++u) load_row<F::ROWS / 2, WIDE ? F::ROWS : 1>(f.block[u], a + u * 8 * BS, in ? F::ROWS : 0);
@@ -154,10 +169,14 @@ __global__ void __launch_bounds__(32 * MMA_WARPS, 2)
     for (int r = 0; r < F::ROWS; r += 4)
 #pragma unroll
       for (int t = 0; t < T; ++t) {
-        const uint32_t a0 = __byte_perm(f.slab[r][t], f.slab[r + 1][t], 0x5410);
-        const uint32_t a1 = __byte_perm(f.slab[r][t], f.slab[r + 1][t], 0x7632);
-        const uint32_t a2 = __byte_perm(f.slab[r + 2][t], f.slab[r + 3][t], 0x5410);
-        const uint32_t a3 = __byte_perm(f.slab[r + 2][t], f.slab[r + 3][t], 0x7632);
+        uint32_t x[4];  // columns 2 t and 2 t + 1 of four rows
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if constexpr (V == 0) x[i] = i & 1 ? __byte_perm(f.slab[r + i][t], f.slab[r + i][t + 1], 0x5432) : f.slab[r + i][t];
+          else x[i] = f.slab[r + i][t];
+        }
+        const uint32_t a0 = __byte_perm(x[0], x[1], 0x5410), a1 = __byte_perm(x[0], x[1], 0x7632);
+        const uint32_t a2 = __byte_perm(x[2], x[3], 0x5410), a3 = __byte_perm(x[2], x[3], 0x7632);
 #pragma unroll
         for (int u = 0; u < F::TILES; ++u) mma(acc[u][t], a0, a1, a2, a3, f.block[u][r / 2], f.block[u][r / 2 + 1]);
       }
@@ -203,7 +222,7 @@ __global__ void __launch_bounds__(32 * MMA_WARPS, 2)
         const __nv_bfloat162 h = __floats2bfloat162_rn(acc[u][t][r], acc[u][t][2 + r]);
         w[t] = *reinterpret_cast<const uint32_t *>(&h);
       }
-      store_row<T, V>(C + (brow * BS + 8 * u + 2 * q + r) * N + col0, w, valid);
+      store_row<T, V ? V : 1>(C + (brow * BS + 8 * u + 2 * q + r) * N + col0, w, valid);
     }
 }
 
@@ -234,14 +253,18 @@ cudaError_t launch_bs(const BsrSpmmArgs &a, int sm_count, cudaStream_t s) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(a.B) | reinterpret_cast<uintptr_t>(a.C) | (uintptr_t)(a.n_rhs * 2);
   const int64_t n = a.n_rhs;
   // 64 columns per warp, fewer for narrow B; two-byte loads and the 32 rows of a large block leave registers for 32
-  // (706 block rows of 9, N = 302: 22.9 us with 64, 19.5 with 32).
-  const int T = n <= 16 ? 1 : n <= 32 || BS == 32 || at % 4 != 0 ? 2 : 4;
-  if (T == 1) return at % 4 == 0 ? launch_wide<BS, 1, 2>(a, sm_count, s) : launch_wide<BS, 1, 1>(a, sm_count, s);
+  // (706 block rows of 9, N = 302 off a word: 22.9 us with 64, 19.5 with 32).
+  const bool words = n % 2 == 1 && reinterpret_cast<uintptr_t>(a.B) % 4 == 0;
+  const int T = n <= 16 ? 1 : n <= 32 || BS == 32 || (at % 4 != 0 && !words) ? 2 : 4;
+  if (T == 1)
+    return words ? launch_wide<BS, 1, 0>(a, sm_count, s) : at % 4 == 0 ? launch_wide<BS, 1, 2>(a, sm_count, s)
+                                                                     : launch_wide<BS, 1, 1>(a, sm_count, s);
   if (T == 2)
-    return at % 8 == 0 ? launch_wide<BS, 2, 4>(a, sm_count, s) : at % 4 == 0 ? launch_wide<BS, 2, 2>(a, sm_count, s)
-                                                                             : launch_wide<BS, 2, 1>(a, sm_count, s);
+    return words ? launch_wide<BS, 2, 0>(a, sm_count, s) : at % 8 == 0 ? launch_wide<BS, 2, 4>(a, sm_count, s)
+           : at % 4 == 0 ? launch_wide<BS, 2, 2>(a, sm_count, s) : launch_wide<BS, 2, 1>(a, sm_count, s);
   if constexpr (BS != 32)
-    return at % 16 == 0 ? launch_wide<BS, 4, 8>(a, sm_count, s) : at % 8 == 0 ? launch_wide<BS, 4, 4>(a, sm_count, s)
+    return words ? launch_wide<BS, 4, 0>(a, sm_count, s) : at % 16 == 0 ? launch_wide<BS, 4, 8>(a, sm_count, s)
+           : at % 8 == 0 ? launch_wide<BS, 4, 4>(a, sm_count, s)
                                                                              : launch_wide<BS, 4, 2>(a, sm_count, s);
   return cudaErrorInvalidValue;
 }
