@@ -8,7 +8,8 @@
 // order, bit for bit.  Block values are the same for all threads of a block row (one L1 access per load), rows of B are
 // read V columns at a time.  With products and sums separate instructions the floor of 4 x 4 blocks is the FP32 pipe,
 // then the gather of slabs of B from L2.  4 x 4 f32 blocks, 16,384 block rows of 24, N = 32: 180 -> 43 us (11 us of FP32
-// pipe, 18 us of L2); 8 x 8, 8,192 block rows of 12, N = 64: 304 -> 70 us; 32 x 32 bf16, N = 64: 740 -> 245 us.
+// pipe, 18 us of L2); 8 x 8, 8,192 block rows of 12, N = 64: 304 -> 70 us; 32 x 32 bf16, N = 64: 740 -> 245 us.  f32 blocks of 4 x 4
+// and 8 x 8 with enough outputs go on to groups of lanes (bsr_rows.cuh).
 #include <cuda_bf16.h>
 
 #include "swb_chain.cuh"
@@ -204,6 +205,8 @@ cudaError_t launch_columns(const BsrSpmmArgs &a, bool few, cudaStream_t s) {
   return few ? launch_tiles<T, 0, 2, V>(a, s) : launch_tiles<T, 0, 8, V>(a, s);
 }
 
+#include "bsr_rows.cuh"
+
 template <typename T>
 cudaError_t launch(const BsrSpmmArgs &a, cudaStream_t s, int64_t *launches) {
   ++*launches;
@@ -213,6 +216,11 @@ cudaError_t launch(const BsrSpmmArgs &a, cudaStream_t s, int64_t *launches) {
   // (201 block rows of 52 blocks of 32 x 32, N = 24: 207 us with eight, 122 with two).
   const uintptr_t at = reinterpret_cast<uintptr_t>(a.B) | reinterpret_cast<uintptr_t>(a.C);
   int V = a.n_rhs % 4 == 0 && at % (4 * sizeof(T)) == 0 ? 4 : a.n_rhs % 2 == 0 && at % (2 * sizeof(T)) == 0 ? 2 : 1;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    cudaError_t e = cudaSuccess;
+    if (a.block_size == 4 && try_groups<4>(a, V, s, &e)) return e;
+    if (a.block_size == 8 && try_groups<8>(a, V, s, &e)) return e;
+  }
   if (a.block_size <= 8)
     while (V > 1 && a.rows / a.block_size * (a.n_rhs / V) < 65536) V /= 2;
   const bool few = a.rows / a.block_size * ceil_div(a.block_size, 8) * (a.n_rhs / V) < 20000;
