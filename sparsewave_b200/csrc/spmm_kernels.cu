@@ -625,6 +625,18 @@ cudaError_t launch_tile(const CsrSpmmArgs &a, int block, int T, cudaStream_t s) 
 // instead of a warp) 1.02 -> 0.53 ms.
 constexpr int64_t positions_per_lane_group(int G) { return G == 1 ? 6 : G == 2 ? 12 : G <= 8 ? 16 : 12; }
 
+// ... and doubled for few rows, which leave the GPU idle, so that the time is that of the longest row: up to 200,000 lanes (42
+// warps per SM) where a row's lanes have less than a mean row in flight (four positions per group), up to 100,000 where less
+// than two.  Ragged rows (times in a CUDA graph): 3,476 of 16, N = 32 16.8 -> 4.3 us; 10,651 of 16, N = 16 17.4 -> 7.9; 4,963 of 39, N = 8
+// 12.5 -> 5.8; equal rows 0.8 to 1.1, the shortest 1.3 (11,917 of 6, N = 32: 2.8 -> 3.6).  More lanes lose on short rows (12,068
+// of 7, N = 16 with 380,000: 5.0 -> 7.4).
+inline int lanes_per_row(int64_t rows, int64_t mean, int G) {
+  int lanes = G > 4 ? G : 4;
+  while (lanes < 32 && (int64_t)(lanes / G) * positions_per_lane_group(G) < mean) lanes *= 2;
+  while (lanes < 32 && (lanes / G * 4 < mean ? rows * lanes <= 100000 : lanes / G * 4 < 2 * mean && rows * lanes <= 50000)) lanes *= 2;
+  return lanes;
+}
+
 // ---- launches of the staged-rows kernel -------------------------------------------------------
 
 // Lanes per row and rows per block for M runs of columns, R of them per lane.
@@ -794,9 +806,7 @@ cudaError_t launch_subwarp(const CsrSpmmArgs &a, int block, cudaStream_t s) {
 template <int G>
 cudaError_t launch_row_of_tiles(const CsrSpmmArgs &a, int block, cudaStream_t s) {
   const int64_t mean = a.rows > 0 ? a.nnz / a.rows : 0;
-  int lanes = G > 4 ? G : 4;
-  constexpr int64_t kPerGroup = positions_per_lane_group(G);
-  while (lanes < 32 && (int64_t)(lanes / G) * kPerGroup < mean) lanes *= 2;
+  const int lanes = lanes_per_row(a.rows, mean, G);
   if constexpr (G <= 4) if (lanes == 4) return launch_subwarp<G, 4>(a, block, s);
   if constexpr (G <= 8) if (lanes == 8) return launch_subwarp<G, 8>(a, block, s);
   if (lanes == 16) return launch_subwarp<G, 16>(a, block, s);
@@ -892,8 +902,7 @@ int64_t wave_per_row_tile_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs
   if (!pow2_row) return max1(ceil_div(rows * ceil_div(n_rhs, tile), wpb));
   if (n_rhs > 64) return max1(ceil_div(rows, wpb));
   const int64_t G = n_rhs / 4, mean = rows > 0 ? nnz / rows : 0;
-  int64_t lanes = G > 4 ? G : 4;
-  while (lanes < 32 && G<=16 && (lanes / G) * positions_per_lane_group((int)G) < mean) lanes *= 2;
+  const int lanes = lanes_per_row(rows, mean, (int)G);
   return max1(ceil_div(ceil_div(rows, 32 / lanes), wpb));
 }
 
