@@ -17,6 +17,7 @@ __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b);
 // bit-identical to the CPU CSR loop.
 #include "spmm_columns.cuh"
 #include "spmm_staged_rows.cuh"
+#include "spmm_team_rows.cuh"
 
 // The reference's schedule itself: a thread per output, element = blockIdx * blockDim + threadIdx, row = element / N.  On very
 // short rows there is nothing to stage and little to wait for; see takes_outputs.
@@ -794,6 +795,49 @@ inline int64_t tile_rows_per_block(int64_t N, int64_t mean, int block) {
   return N == 64 && mean <= 13 && block >= 256 ? (mean <= 12 ? 2 : 1) * (block / 32) : 0;
 }
 
+// Columns per lane, lanes per tile and warps per row of a team, or no warps where the team kernel is not for these sizes: N that
+// is no power of two up to 128, not the staged-rows kernel's, and few rows.  The other kernels' lanes deal with one column at a
+// time of a tile, for all positions at once: they keep what fills their tiles well (tiles of 8 and up to 40 columns: 3,076
+// ragged rows of 9, N = 35 5.8 us, here 10.7; tiles of 16 and 17 to 48 columns: 2,451 rows of 12, N = 39 5.3, 6.4), long rows of
+// odd N (8,533 of 35, N = 25: 19.4, 25.6) and up to 8 columns in narrow tiles (3,706 ragged rows of 17, N = 5 in tiles of 4: 3.6,
+// 4.7); a warp per row
+// (spmm_wave_per_row_any_kernel) keeps short rows and more than 4,736 (5,900 of 27, N = 40: 4.9, 6.5).  Fewer than 1,024 rows
+// keep the (row, tile) units, which spread a row's columns over more warps.  A row gets a second and a third and fourth warp while
+// a warp has not three mean rows' positions in flight and all warps are one wave, or not one mean row and they are three
+// (4,164 ragged rows of 40, N = 18: 12.9 us with one warp, 10.2 with two; 2,172 of 64, N = 19: 44, 27 and with four 15.5).
+struct Team {
+  int V, G, S;
+  int64_t tiles;
+};
+
+inline Team team_of(int64_t rows, int64_t nnz, int64_t N, int tile, uintptr_t alignment_bits) {
+  Team t{1, 0, 0, 0};
+  if (rows < 1024 || N > 512) return t;
+  const int64_t mean = nnz / rows;
+  const int V = N % 4 == 0 && alignment_bits % 16 == 0 ? 4 : N % 2 == 0 && alignment_bits % 8 == 0 ? 2 : 1;
+  const bool any = N % 4 == 0 && N >= 12 && N < 128 && mean >= 8;
+  if (rows > (any ? 4736 : 8192) || (any && mean < 24) || (V == 1 && mean > 16)) return t;
+  if (N <= 8 && tile < (N <= 4 ? 32 : 16)) return t;
+  if (!any && ((tile == 8 && N <= 40) || (tile == 16 && N > 16 && N <= 48))) return t;
+  t.V = V;
+  const int64_t M = N / t.V;
+  t.tiles = ceil_div(M, 32);
+  t.G = (int)ceil_div(M, t.tiles);
+  const int64_t units = rows * t.tiles, in_flight = 32 / t.G * team_positions(t.V);
+  t.S = 1;
+  while (t.S < 4 && t.S * in_flight < 3 * mean && units * t.S <= (t.S * in_flight < mean ? 13000 : 4750)) t.S *= 2;
+  return t;
+}
+
+template <int V>
+cudaError_t launch_team_rows(const CsrSpmmArgs &a, const Team &t, cudaStream_t s) {
+  const int64_t units = a.rows * t.tiles;
+  SWB_GRID(grid, ceil_div(units, TEAM_THREADS / 32 / t.S));
+  launch_chained(spmm_team_rows_kernel<V>, grid, TEAM_THREADS, 0, s, units, a.n_rhs, (uint32_t)(a.n_rhs * 4), t.G, t.S, t.tiles,
+                 a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
+  return cudaGetLastError();
+}
+
 template <int G, int L>
 cudaError_t launch_subwarp(const CsrSpmmArgs &a, int block, cudaStream_t s) {
   const int64_t warps = ceil_div(a.rows, 32 / L);
@@ -856,6 +900,10 @@ cudaError_t launch_spmm_wave_per_row_tile(const CsrSpmmArgs &a, int block, int t
       launch_chained(spmm_wave_per_row_wide_kernel<4>, grid, block, 0, s, a.rows, N, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
     return cudaGetLastError();
   }
+  const Team team = pow2_row ? Team{1, 0, 0, 0}
+                             : team_of(a.rows, a.nnz, N, tile, reinterpret_cast<uintptr_t>(a.B) | reinterpret_cast<uintptr_t>(a.C));
+  if (team.S > 0)
+    return team.V == 4 ? launch_team_rows<4>(a, team, s) : team.V == 2 ? launch_team_rows<2>(a, team, s) : launch_team_rows<1>(a, team, s);
   // other multiples of 4 up to 124 (rows of B of 12, 20, 24 ... floats) where a matrix row has enough positions
   // for a warp: one warp per row as well
   if (N >= 12 && N < 128 && N % 4 == 0 && !pow2_row && a.rows > 0 && a.nnz / a.rows >= 8 && aligned16(a.B) &&
@@ -897,6 +945,8 @@ int64_t wave_per_row_tile_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs
   }
   const bool pow2_row = n_rhs >= 4 && n_rhs <= 128 && (n_rhs & (n_rhs - 1)) == 0;
   if (n_rhs == 256 || n_rhs == 384 || n_rhs == 512) return max1(ceil_div(rows, wpb));
+  const Team team = pow2_row ? Team{1, 0, 0, 0} : team_of(rows, nnz, n_rhs, tile, 0);
+  if (team.S > 0) return max1(ceil_div(rows * team.tiles, TEAM_THREADS / 32 / team.S));
   if (n_rhs >= 12 && n_rhs < 128 && n_rhs % 4 == 0 && !pow2_row && rows > 0 && nnz / rows >= 8)
     return max1(ceil_div(rows, wpb));
   if (!pow2_row) return max1(ceil_div(rows * ceil_div(n_rhs, tile), wpb));
