@@ -7,7 +7,7 @@
 // both operands agree.  Lane (g, q) = (lane / 4, lane % 4) takes adjacent local columns ROWS q .. ROWS q + ROWS - 1 and
 // adjacent columns 2 T g .. 2 T g + 2 T - 1: its share of the block values is one load per 8 rows, its share of a row of B one
 // load of up to 16 bytes, and its results are adjacent columns of C.  Pairs of rows of B are interleaved by byte permutes.
-// The next step's loads are in flight during this step's MMAs, block columns are held 32 at a time by the warp's lanes.
+// The next steps' loads are in flight during this step's MMAs, block columns are held 32 at a time by the warp's lanes.
 // Where block rows are few, up to eight warps share one and its parts are added up through shared memory in their order.
 //
 // What bounds it: launch and latency on small calls, L1 on large ones (eight lanes of a load touch four lines, some 64 lookups
@@ -26,6 +26,12 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int MMA_WARPS = 8;
+// Steps in hand (one being multiplied, the others' loads in flight) and CTAs per SM that registers are kept for.  Narrow B leaves
+// registers for more of both: 1,628 block rows of 14 blocks of 16 x 16, N = 24 9.8 -> 6.8 us with three CTAs; 2,970 of 52, N = 8
+// 36.9 -> 30.0 with three steps and CTAs (37.6 with four CTAs of two steps, 37.1 with two of four).
+// 8 x 8 blocks then have three CTAs for four: 2,744 block rows of 54, N = 16 15.3 -> 12.7, but 7,454 of 44, N = 8 20.7 -> 24.0.
+constexpr int mma_depth(int bs, int T) { return bs == 32 || T > 1 ? 2 : 3; }
+constexpr int mma_ctas(int bs, int T, int V) { return bs < 32 && T == 1 ? 3 : bs == 16 && T == 2 && V > 1 ? 3 : 2; }
 
 template <int BS, int T, int V>
 struct Fragments {
@@ -109,7 +115,7 @@ __device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uin
 // V: elements per load of a row of B, or 0: N is odd and B starts at a word, so that rows in turn start at a word and in the
 // middle of one.  WIDE: block values are aligned for loads of a lane's ROWS.
 template <int BS, int T, int V, bool WIDE>
-__global__ void __launch_bounds__(32 * MMA_WARPS, 2)
+__global__ void __launch_bounds__(32 * MMA_WARPS, mma_ctas(BS, T, V))
     bsr_spmm_mma_kernel(int64_t units, int tiles, int split, int64_t N, const int32_t *__restrict__ brp,
                         const int32_t *__restrict__ bci, const __nv_bfloat16 *__restrict__ bv,
                         const __nv_bfloat16 *__restrict__ B, __nv_bfloat16 *__restrict__ C) {
@@ -184,16 +190,18 @@ __global__ void __launch_bounds__(32 * MMA_WARPS, 2)
   if (k0 < k1) {
     here = column(k0);
     ahead = column(k0 + BATCH);
-    F f0, f1;
-    load(f0, k0);
-    int k = k0;
-    while (true) {
-      if (k + 1 < k1) load(f1, k + 1);
-      compute(f0);
-      if (++k >= k1) break;
-      if (k + 1 < k1) load(f0, k + 1);
-      compute(f1);
-      if (++k >= k1) break;
+    constexpr int DEPTH = mma_depth(BS, T);
+    F f[DEPTH];
+#pragma unroll
+    for (int d = 0; d < DEPTH - 1; ++d)
+      if (k0 + d < k1) load(f[d], k0 + d);
+    for (int k = k0; k < k1;) {
+#pragma unroll
+      for (int d = 0; d < DEPTH; ++d) {
+        if (k + DEPTH - 1 < k1) load(f[(d + DEPTH - 1) % DEPTH], k + DEPTH - 1);
+        compute(f[d]);
+        if (++k >= k1) break;
+      }
     }
   }
   if (split > 1) {  // the parts' sums, added up by the unit's first warp in order
