@@ -796,15 +796,17 @@ inline int64_t tile_rows_per_block(int64_t N, int64_t mean, int block) {
 }
 
 // Columns per lane, lanes per tile and warps per row of a team, or no warps where the team kernel is not for these sizes: N that
-// is no power of two up to 128, not the staged-rows kernel's, and few rows.  The other kernels' lanes deal with one column at a
-// time of a tile, for all positions at once: they keep what fills their tiles well (tiles of 8 and up to 40 columns: 3,076
-// ragged rows of 9, N = 35 5.8 us, here 10.7; tiles of 16 and 17 to 48 columns: 2,451 rows of 12, N = 39 5.3, 6.4), long rows of
-// odd N (8,533 of 35, N = 25: 19.4, 25.6) and up to 8 columns in narrow tiles (3,706 ragged rows of 17, N = 5 in tiles of 4: 3.6,
-// 4.7); a warp per row
-// (spmm_wave_per_row_any_kernel) keeps short rows and more than 4,736 (5,900 of 27, N = 40: 4.9, 6.5).  Fewer than 1,024 rows
-// keep the (row, tile) units, which spread a row's columns over more warps.  A row gets a second and a third and fourth warp while
-// a warp has not three mean rows' positions in flight and all warps are one wave, or not one mean row and they are three
-// (4,164 ragged rows of 40, N = 18: 12.9 us with one warp, 10.2 with two; 2,172 of 64, N = 19: 44, 27 and with four 15.5).
+// is no power of two up to 128, not the staged-rows kernel's, and few rows.  The (row, tile) kernel's lanes deal with one column
+// of a tile at a time, for all positions at once, which fills tiles well that are about as wide as N.  It keeps
+//   tiles of 8 and up to 40 columns, of 16 and 17 to 48 (3,076 ragged rows of 9, N = 35 5.8 us, 10.7 here; 2,451 of 12,
+//   N = 39 5.3, 6.4), and up to 8 columns in narrower tiles (3,706 ragged rows of 17, N = 5 in tiles of 4: 3.6, 4.7);
+//   odd N with more than 16 a row (8,533 of 35, N = 25 in tiles of 4: 19.4, 25.6), unless rows are long and tiles wide
+//   (6,244 ragged rows of 35, N = 29 in tiles of 32: 49.5, 19.6; 1,961 of 31, N = 93 37.2, 17.6);
+//   fewer than 1,024 rows, whose columns it spreads over more warps.
+// A warp per row (spmm_wave_per_row_any_kernel) keeps short rows and more than 4,736 (5,900 of 27, N = 40: 4.9, 6.5).  A row gets
+// a second and then a third and fourth warp while a warp has not three mean rows' positions in flight and all warps are one
+// wave, or not one mean row and they are three (4,164 ragged rows of 40, N = 18: 12.9 us with one warp, 10.2 with two; 2,172 of
+// 64, N = 19: 44, 27 and with four 15.5).
 struct Team {
   int V, G, S;
   int64_t tiles;
@@ -816,7 +818,8 @@ inline Team team_of(int64_t rows, int64_t nnz, int64_t N, int tile, uintptr_t al
   const int64_t mean = nnz / rows;
   const int V = N % 4 == 0 && alignment_bits % 16 == 0 ? 4 : N % 2 == 0 && alignment_bits % 8 == 0 ? 2 : 1;
   const bool any = N % 4 == 0 && N >= 12 && N < 128 && mean >= 8;
-  if (rows > (any ? 4736 : 8192) || (any && mean < 24) || (V == 1 && mean > 16)) return t;
+  if (rows > (any ? 4736 : 8192) || (any && mean < 24)) return t;
+  if (V == 1 && mean > 16 && (mean < 30 || tile < (N >= 64 ? 8 : 32))) return t;
   if (N <= 8 && tile < (N <= 4 ? 32 : 16)) return t;
   if (!any && ((tile == 8 && N <= 40) || (tile == 16 && N > 16 && N <= 48))) return t;
   t.V = V;
