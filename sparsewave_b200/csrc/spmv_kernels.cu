@@ -874,13 +874,16 @@ int64_t wave_per_position_auto_batch(int64_t nnz, int block, const DeviceInfo &d
   // Spans long enough that the one row search per span is amortised, short enough that the warps fill the
   // SMs many times over.  Measured on a power-law SpMV: 92 M nonzeros want 32 to 48 partitions per span
   // (0.397 ms; 0.400 at 64, 0.413 at 16), a quarter of it 12 to 16 (0.110 ms; 0.115 at 9), an eighth 8 (0.059 ms;
-  // 0.065 at 4, 0.062 at 16).  Small problems keep at least 16 warps per SM.
+  // 0.065 at 4, 0.062 at 16).  Small problems are bound by latency and by the set-up of their warps; two partitions cost no more
+  // than one, which goes to the kernel of the reference's schedule.  Times in a CUDA graph with 1, 2, 4 and 8: 16,000 nonzeros
+  // 4.3, 4.3, 4.6, 6.5 us; 92,824 power-law ones 5.5, 4.6, 4.7, 6.4; 127,998 in rows of 4 8.2, 5.0, 5.1, 7.1; 479,980 in rows of
+  // 60 -, 6.3, 5.5, 6.6; 959,979 -, 10.4, 7.1, 7.4; 1,279,994 in rows of 20 -, 14.7, 11.2, 10.3.
   const int64_t waves = wave_position_wave_count(nnz, block);
   int64_t batch = waves / ((int64_t)dev.sm_count * 64 * 6);
   if (batch > 48) batch = 48;
   if (batch < 8) {
-    const int64_t by_occupancy = waves / ((int64_t)dev.sm_count * 16);
-    batch = by_occupancy < 8 ? by_occupancy : 8;
+    const int64_t per_sm = waves / dev.sm_count;
+    batch = per_sm < 7 ? 1 : per_sm < 42 ? 2 : per_sm < 243 ? 4 : 8;
   }
   if (batch < 1) batch = 1;
   return batch;
