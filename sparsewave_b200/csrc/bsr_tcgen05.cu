@@ -467,22 +467,28 @@ bool bsr_tcgen05_supported(const BsrSpmmArgs &a) {
 
 // Against the mma.sync kernel, which reads its operands from global memory and takes any size: this one where a tile of
 // columns is well filled and there are units enough for persistent CTAs (times: mma.sync, here).
-// 16 x 16: whole groups of 64 columns from 128 on (1,500 block rows of 40, N = 192 61.7, 38.2 us; 3,419 of 8, N = 128 24.7, 19.0);
-// 80, 96 and 112 columns but for short block rows (1,500 of 40, N = 96 45.6, 27.2; 3,800 of 8, N = 80 22.3, 22.0), 64 and 72 on
-// long ones (1,500 of 40, N = 64 31.6, 26.2; 3,800 of 8 17.3, 21.7); a last tile of 32 columns or more (300 of 30, N = 336 22.8,
-// 15.3; 447 of 39, N = 160 25.3, 17.5; of short rows only 96 of 256: 2,941 of 4, N = 296 26.6, 32.3); with less in the last tile
-// on many units (264 columns, 3,800 of 8: 60.7, 52.8, 900 of 12: 18.1, 19.8; 136 columns, 3,800 of 25: 86.6, 70.4, 2,271 of 12:
-// 25.2, 27.9).  Rows of B that are no multiple of 32 bytes cost the copies more (N = 104, 2,177 of 17: 24.1, 26.9; N = 88, 557 of
-// 16: 9.4, 10.4).  32 x 32: from 64 columns (1,331 of 5, N = 64: 11.7, 10.8; 94 units, N = 88: 6.8, 13.7).  8 x 8, half of whose MMA
-// is padding: whole groups of 64 from 128 on (1,500 of 40, N = 128 29.6, 17.3; 4,000 of 10 19.2, 18.8), others from 400 on many
-// units (N = 184: 39, 47).
+// 16 x 16: whole groups of 64 columns from 128 on (1,500 block rows of 40, N = 192 61.7, 38.2 us; 3,419 of 8, N = 128 24.7,
+// 19.0; but 70 of 30, N = 256 6.2, 9.0 and 150 of 5, N = 512 5.9, 7.1; 683 of 10, N = 128 10.5, 8.6); 80, 96 and 112 columns
+// but for short block rows (1,500 of 40, N = 96 45.6, 27.2; 3,800 of 8, N = 80 22.3, 22.0; 1,187 of 6, N = 88 7.7, 9.4), 64
+// and 72 on long ones (1,500 of 40, N = 64 31.6, 26.2; 3,800 of 8 17.3, 21.7); a last tile of 32 columns or more (300 of 30, N
+// = 336 22.8, 15.3; 447 of 39, N = 160 25.3, 17.5; of short rows only 96 of 256: 2,941 of 4, N = 296 26.6, 32.3); with less in
+// the last tile on many units (264 columns, 3,800 of 8: 60.7, 52.8, 900 of 12: 18.1, 19.8; 136 columns, 3,800 of 25: 86.6,
+// 70.4, 2,271 of 12: 25.2, 27.9).  Rows of B that are no multiple of 32 bytes cost the copies more (N = 104, 2,177 of 17:
+// 24.1, 26.9; N = 88, 557 of 16: 9.4, 10.4).
+// 32 x 32: from 64 columns (1,331 of 5, N = 64: 11.7, 10.8; 489 of 15, N = 96 16.1, 12.3; 94 units, N = 88: 6.8, 13.7).
+// 8 x 8, half of whose MMA is padding: whole groups of 64 from 128 on, on long block rows (500 of 40, N = 256 17.6, 12.4) or
+// many units without a last tile of 64 (4,000 of 10, N = 128 19.2, 18.8, N = 320 40.5, 47.9), others from 400 (N = 184: 39,
+// 47).
 bool bsr_tcgen05_pays(const BsrSpmmArgs &a) {
   const int64_t n = a.n_rhs, brows = a.rows / a.block_size, units = brows * ceil_div(n, HALF_N), tail = n % HALF_N;
   const int64_t mean = brows > 0 ? a.nnzb / brows : 0;
   if (a.block_size == 32) return n >= HALF_N ? units >= 200 : n >= 64 && units >= 400;
-  if (a.block_size == 8) return n >= HALF_N && (n % 64 == 0 ? units >= 1500 : n >= 400 && units >= 13000);
+  if (a.block_size == 8) {
+    if (n < HALF_N || n % 64 != 0) return n >= 400 && units >= 13000;
+    return mean >= 24 ? units >= 450 : n % (2 * HALF_N) != 64 && units >= 1500;
+  }
   if (n < HALF_N) return n >= 80 ? n % 16 == 0 && units >= 600 && mean >= 8 : n >= 64 && mean >= 30 && units >= 1000;
-  if (n % 64 == 0) return true;
+  if (n % 64 == 0) return units >= (mean >= 16 ? 150 : mean >= 8 ? 350 : 700);
   const bool filled = n % (2 * HALF_N) >= 96 && units >= 1000;
   if (n < HALF_N + 16) return units >= 6000 && mean >= 16;
   if (mean < 8 || (n < 2 * HALF_N && (tail < 32 || n % 16 != 0))) return filled;

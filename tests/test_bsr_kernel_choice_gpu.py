@@ -10,7 +10,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("bs,brows,per,n", [(16, 599, 9, 80), (16, 600, 8, 96), (16, 610, 7, 112), (16, 600, 9, 104), (16, 1000, 30, 72),
                                             (16, 300, 9, 160), (16, 300, 9, 168), (16, 1334, 9, 264), (16, 200, 8, 296), (16, 3000, 16, 136),
-                                            (8, 1500, 6, 128), (8, 750, 5, 192), (8, 1499, 6, 128)])
+                                            (8, 1500, 6, 128), (8, 750, 5, 192), (8, 1499, 6, 128),
+                                            (8, 450, 24, 128), (8, 500, 5, 320), (16, 150, 16, 128), (16, 75, 17, 256), (16, 175, 5, 512),
+                                            (32, 84, 9, 264), (32, 400, 16, 72), (32, 400, 5, 72)])
 def test_both_sides(ctx, bs, brows, per, n):
     cols = 40
     gen = torch.Generator().manual_seed(brows + n)
