@@ -2,19 +2,25 @@
 // fragments: any number of columns, any alignment, few block rows as well as many (arithmetic as in bsr_tcgen05.cu).
 //
 // A warp owns a block row and 16 T columns and forms the product transposed, so that one instruction shape fits all block
-// sizes: mma.sync.m16n8k16 with m = 16 columns of B, n = 8 rows of a block, k = 16 local columns (two 8 x 8 blocks, one
+// sizes: mma.sync.m16n8k16 with m = 16 columns of B, n = 8 rows of a block, k = 16 local columns (a step: two 8 x 8 blocks, one
 // 16 x 16 block, half of a 32 x 32 block).  Which local column is which k, and which column of B which m, is free as long as
-// both operands agree.  Lane (g, q) = (lane / 4, lane % 4) takes adjacent local columns ROWS q .. ROWS q + ROWS - 1 and
+// both operands agree.  Lane (g, q) = (lane / 4, lane % 4) takes adjacent local columns 4 q .. 4 q + 3 of a step and
 // adjacent columns 2 T g .. 2 T g + 2 T - 1: its share of the block values is one load per 8 rows, its share of a row of B one
 // load of up to 16 bytes, and its results are adjacent columns of C.  Pairs of rows of B are interleaved by byte permutes.
 // The next steps' loads are in flight during this step's MMAs, block columns are held 32 at a time by the warp's lanes.
-// Where block rows are few, up to eight warps share one and its parts are added up through shared memory in their order.
+//
+// Every output is one chain of MMAs over its block row's steps in storage order, as in bsr_tcgen05.cu, so that its bits depend
+// on its block row and its column alone: not on how many block rows or columns the call has, which kernel takes it, alignment
+// or the device.  Where block rows are few, a team of up to eight warps shares one all the same: its members load the steps in
+// turn and hand them over in shared memory, and each of the first members adds up its share of the block row's rows.
 //
 // What bounds it: launch and latency on small calls, L1 on large ones (eight lanes of a load touch four lines, some 64 lookups
 // for 2 KB of B; ncu: L1 data pipe 67 %, tensor pipe 18 % on 1,024 block rows of 51, N = 512), which bsr_tcgen05.cu then takes.
 // Tried: the same loads through a ring in shared memory (178 us against 134 on that size).  Before, on the CUDA cores or with
-// tcgen05 at any size: 123 block rows of 61 blocks of 32 x 32, N = 2 138 -> 6.2 us; 382 of 27, N = 29 111 -> 17.6; 1,438 of 15
-// blocks of 8 x 8, N = 80 30.6 -> 10.4; 73 of 36 blocks of 16 x 16, N = 88 18.5 -> 5.9.
+// tcgen05 at any size: 123 block rows of 61 blocks of 32 x 32, N = 2 132 -> 12.4 us; 382 of 27, N = 29 105 -> 19.6; 1,438 of 15
+// blocks of 8 x 8, N = 80 30.0 -> 10.1; 90 of 36 blocks of 16 x 16, N = 88 17.5 -> 7.9.  One chain has its price where few
+// warps have much to add up: a block row in parts with sums of their own, added up at the end, took 5.8, 12.1, 10.4 and 5.8 us.
+// Tried for teams: two rounds' loads in flight (spills; 1.09 times the time over 170 sizes), a barrier per step (1.13).
 #include <cuda_bf16.h>
 
 #include "swb_chain.cuh"
@@ -27,19 +33,22 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int MMA_WARPS = 8;
 // Steps in hand (one being multiplied, the others' loads in flight) and CTAs per SM that registers are kept for.  Narrow B leaves
-// registers for more of both: 1,628 block rows of 14 blocks of 16 x 16, N = 24 9.8 -> 6.8 us with three CTAs; 2,970 of 52, N = 8
-// 36.9 -> 30.0 with three steps and CTAs (37.6 with four CTAs of two steps, 37.1 with two of four).
-// 8 x 8 blocks then have three CTAs for four: 2,744 block rows of 54, N = 16 15.3 -> 12.7, but 7,454 of 44, N = 8 20.7 -> 24.0.
+// registers for more of both: 2,970 block rows of 52 blocks of 16 x 16, N = 8 36.9 -> 30.4 us with three steps and CTAs (37.6
+// with four CTAs of two steps, 37.1 with two of four).  8 x 8 blocks then need no more than 64 registers, which is four CTAs.
 constexpr int mma_depth(int bs, int T) { return bs == 32 || T > 1 ? 2 : 3; }
+// Steps that each member of a team has in flight and hands over at a time: 48 KB of shared memory for eight members.
+constexpr int team_steps(int bs, int T) { return T == 4 ? 2 : bs == 32 && T == 2 ? 3 : 4; }
 constexpr int mma_ctas(int bs, int T, int V) { return bs < 32 && T == 1 ? 3 : bs == 16 && T == 2 && V > 1 ? 3 : 2; }
 
-template <int BS, int T, int V>
+// H: a lane's share of one step (1) or of both of a 32 x 32 block (2), which lie 16 rows of B and local columns apart.
+template <int BS, int T, int V, int H>
 struct Fragments {
-  static constexpr int ROWS = BS == 32 ? 8 : 4;   // rows of B per lane and step
-  static constexpr int TILES = BS / 8;            // n8 tiles of block rows
-  uint32_t slab[ROWS][T + (V == 0)];              // 2 T adjacent columns each (V = 0: the words that hold them)
-  uint32_t block[TILES][ROWS / 2];                // block row 8 u + g, the lane's ROWS columns
+  static constexpr int TILES = BS / 8;  // n8 tiles of block rows
+  uint32_t slab[H][4][T + (V == 0)];    // four rows of B, 2 T adjacent columns each (V = 0: the words that hold them)
+  uint32_t block[H][TILES][2];          // block row 8 u + g, four local columns
 };
+// Words per lane of a step as its MMAs take it: four for every 16 columns of B, two for every 8 rows of blocks.
+constexpr int step_words(int bs, int T) { return 4 * T + bs / 4; }
 
 // 2 T adjacent elements as loads of V (those at or past `valid` are zeros), two to a word.
 template <int T, int V>
@@ -113,19 +122,23 @@ __device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uin
 }
 
 // V: elements per load of a row of B, or 0: N is odd and B starts at a word, so that rows in turn start at a word and in the
-// middle of one.  WIDE: block values are aligned for loads of a lane's ROWS.
-template <int BS, int T, int V, bool WIDE>
-__global__ void __launch_bounds__(32 * MMA_WARPS, mma_ctas(BS, T, V))
-    bsr_spmm_mma_kernel(int64_t units, int tiles, int split, int64_t N, const int32_t *__restrict__ brp,
+// middle of one.  WIDE: block values are aligned for loads of a lane's four.  TEAM: several warps share a unit, 2, 4 or 8 but
+// no fewer than there are tiles of 8 rows in a block.
+template <int BS, int T, int V, bool WIDE, bool TEAM>
+__global__ void __launch_bounds__(32 * MMA_WARPS, TEAM ? 2 : mma_ctas(BS, T, V))
+    bsr_spmm_mma_kernel(int64_t units, int tiles, int team_warps, int64_t N, const int32_t *__restrict__ brp,
                         const int32_t *__restrict__ bci, const __nv_bfloat16 *__restrict__ bv,
                         const __nv_bfloat16 *__restrict__ B, __nv_bfloat16 *__restrict__ C) {
-  using F = Fragments<BS, T, V>;
-  constexpr int BLOCKS = BS == 8 ? 2 : 1;  // blocks per step
-  constexpr int BATCH = 32 / BLOCKS;       // steps whose block columns the warp holds
+  constexpr int H = BS == 32 && !TEAM ? 2 : 1;
+  using F = Fragments<BS, T, V, H>;
+  // Steps of this kernel per two blocks, and those whose block columns the warp holds.
+  constexpr int PER_TWO = BS == 8 ? 1 : BS == 16 || H == 2 ? 2 : 4, BATCH = 16 * PER_TWO;
+  constexpr int DEPTH = TEAM ? team_steps(BS, T) : mma_depth(BS, T);
+  constexpr int WORDS = step_words(BS, T);
   after_previous_kernel();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
-  const int part = warp % split;
-  const int64_t unit = (int64_t)blockIdx.x * (MMA_WARPS / split) + warp / split;
+  const int split = TEAM ? team_warps : 1, team = warp / split, member = warp % split;
+  const int64_t unit = (int64_t)blockIdx.x * (MMA_WARPS / split) + team;
   const bool active = unit < units;
   const int64_t brow = active ? unit / tiles : 0;
   const int64_t col0 = (active ? unit - brow * tiles : 0) * (16 * T) + g * (2 * T);
@@ -135,93 +148,128 @@ __global__ void __launch_bounds__(32 * MMA_WARPS, mma_ctas(BS, T, V))
     start = brp[brow];
     end = brp[brow + 1];
   }
-  const int steps = (end - start + BLOCKS - 1) / BLOCKS;
-  const int share = (steps + split - 1) / split;
-  const int k0 = part * share, k1 = k0 + share < steps ? k0 + share : steps;
+  const int steps = BS == 8 ? (end - start + 1) / 2 : (end - start) * (PER_TWO / 2);
 
-  float acc[F::TILES][T][4];
+  constexpr int SUMS = TEAM ? 1 : F::TILES;  // tiles of 8 rows that the warp adds up: all, or (the first warps of a team) one
+  float acc[SUMS][T][4];
 #pragma unroll
-  for (int u = 0; u < F::TILES; ++u)
+  for (int u = 0; u < SUMS; ++u)
 #pragma unroll
     for (int t = 0; t < T; ++t)
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[u][t][i] = 0.0f;
 
-  const __nv_bfloat16 *Bt = B + col0 + (int64_t)(BS == 8 ? 4 * (q & 1) : F::ROWS * q) * N;
+  const int local = BS == 8 ? 4 * (q & 1) : 4 * q;  // the lane's first local column of a step
+  const int second = BS == 8 ? q >> 1 : 0;          // which of a step's two blocks it reads
+  const __nv_bfloat16 *Bt = B + col0 + (int64_t)local * N;
+  auto block_of = [&](int k) { return PER_TWO == 1 ? 2 * k : PER_TWO == 2 ? k : k >> 1; };
   auto column = [&](int k) {  // block columns of the steps from k on
-    const int p = start + k * BLOCKS + lane;
+    const int p = start + block_of(k) + lane;
     return p < end ? __ldg(bci + p) : 0;
   };
-  int here = 0, ahead = 0;
-  auto load = [&](F &f, int k) {
-    const int i = k - k0;
-    if (i % BATCH == 0 && i != 0) { here = ahead; ahead = column(k + BATCH); }
-    const int j = BS == 8 ? q >> 1 : 0;
-    const int bc = __shfl_sync(FULL, here, (i % BATCH) * BLOCKS + j);
-    const int p = start + k * BLOCKS + j;
+  int here = column(0), ahead = column(BATCH);
+  auto load = [&](F &f, int k) {  // called for k = member, member + split, ... (a batch is a multiple of every split)
+    const int i = k % BATCH;
+    if (i == member && k != member) { here = ahead; ahead = column(k - i + BATCH); }
+    const int bc = __shfl_sync(FULL, here, block_of(i) + second);
+    const int p = start + block_of(k) + second;
+    const int from = PER_TWO == 4 ? 16 * (k & 1) : 0;
     const bool in = BS != 8 || p < end;  // the second block of a last step may be missing: zeros
-    const __nv_bfloat16 *b = Bt + (int64_t)bc * BS * N;
+    const __nv_bfloat16 *b = Bt + ((int64_t)bc * BS + from) * N;
 #pragma unroll
-    for (int r = 0; r < F::ROWS; ++r) {
-      if constexpr (V == 0) load_words<T>(f.slab[r], b + r * N, r & 1, in ? valid : 0);
-      else load_row<T, V>(f.slab[r], b + r * N, in ? valid : 0);
-    }
-    const __nv_bfloat16 *a = bv + (int64_t)p * (BS * BS) + g * BS + (BS == 8 ? 4 * (q & 1) : F::ROWS * q);
+    for (int h = 0; h < H; ++h)
 #pragma unroll
-    for (int u = 0; u < F::TILES; ++u) load_row<F::ROWS / 2, WIDE ? F::ROWS : 1>(f.block[u], a + u * 8 * BS, in ? F::ROWS : 0);
-  };
-  auto compute = [&](const F &f) {
-#pragma unroll
-    for (int r = 0; r < F::ROWS; r += 4)
-#pragma unroll
-      for (int t = 0; t < T; ++t) {
-        uint32_t x[4];  // columns 2 t and 2 t + 1 of four rows
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if constexpr (V == 0) x[i] = i & 1 ? __byte_perm(f.slab[r + i][t], f.slab[r + i][t + 1], 0x5432) : f.slab[r + i][t];
-          else x[i] = f.slab[r + i][t];
-        }
-        const uint32_t a0 = __byte_perm(x[0], x[1], 0x5410), a1 = __byte_perm(x[0], x[1], 0x7632);
-        const uint32_t a2 = __byte_perm(x[2], x[3], 0x5410), a3 = __byte_perm(x[2], x[3], 0x7632);
-#pragma unroll
-        for (int u = 0; u < F::TILES; ++u) mma(acc[u][t], a0, a1, a2, a3, f.block[u][r / 2], f.block[u][r / 2 + 1]);
+      for (int r = 0; r < 4; ++r) {
+        if constexpr (V == 0) load_words<T>(f.slab[h][r], b + (16 * h + r) * N, r & 1, in ? valid : 0);
+        else load_row<T, V>(f.slab[h][r], b + (16 * h + r) * N, in ? valid : 0);
       }
+    const __nv_bfloat16 *a = bv + (int64_t)p * (BS * BS) + g * BS + from + local;
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+#pragma unroll
+      for (int u = 0; u < F::TILES; ++u) load_row<2, WIDE ? 4 : 1>(f.block[h][u], a + u * 8 * BS + 16 * h, in ? 4 : 0);
   };
-  if (k0 < k1) {
-    here = column(k0);
-    ahead = column(k0 + BATCH);
-    constexpr int DEPTH = mma_depth(BS, T);
-    F f[DEPTH];
+  auto columns_of = [&](const F &f, int h, int t, uint32_t (&a)[4]) {  // the MMA's operand of columns 2 t and 2 t + 1
+    uint32_t x[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if constexpr (V == 0) x[i] = i & 1 ? __byte_perm(f.slab[h][i][t], f.slab[h][i][t + 1], 0x5432) : f.slab[h][i][t];
+      else x[i] = f.slab[h][i][t];
+    }
+    a[0] = __byte_perm(x[0], x[1], 0x5410); a[1] = __byte_perm(x[0], x[1], 0x7632);
+    a[2] = __byte_perm(x[2], x[3], 0x5410); a[3] = __byte_perm(x[2], x[3], 0x7632);
+  };
+  F f[DEPTH];
+  if constexpr (!TEAM) {
 #pragma unroll
     for (int d = 0; d < DEPTH - 1; ++d)
-      if (k0 + d < k1) load(f[d], k0 + d);
-    for (int k = k0; k < k1;) {
+      if (d < steps) load(f[d], d);
+    for (int k = 0; k < steps;) {
 #pragma unroll
       for (int d = 0; d < DEPTH; ++d) {
-        if (k + DEPTH - 1 < k1) load(f[(d + DEPTH - 1) % DEPTH], k + DEPTH - 1);
-        compute(f[d]);
-        if (++k >= k1) break;
+        if (k + DEPTH - 1 < steps) load(f[(d + DEPTH - 1) % DEPTH], k + DEPTH - 1);
+#pragma unroll
+        for (int h = 0; h < H; ++h)
+#pragma unroll
+          for (int t = 0; t < T; ++t) {
+            uint32_t a[4];
+            columns_of(f[d], h, t, a);
+#pragma unroll
+            for (int u = 0; u < F::TILES; ++u) mma(acc[u][t], a[0], a[1], a[2], a[3], f[d].block[h][u][0], f[d].block[h][u][1]);
+          }
+        if (++k >= steps) break;
       }
     }
-  }
-  if (split > 1) {  // the parts' sums, added up by the unit's first warp in order
-    constexpr int WORDS = F::TILES * T * 4;
-    extern __shared__ __align__(16) float partial[];
-    float *mine = partial + (warp - warp / split - 1) * (WORDS * 32) + lane;
-    if (part > 0) {
+  } else {
+    // A round: each member puts its steps, every split-th one, into the team's shared memory; behind a barrier the first members
+    // add them up, in order, for a tile of 8 rows each, while the next round's loads are in flight.
+    extern __shared__ __align__(16) uint4 handed[];
+    constexpr int STEP = WORDS * 8;  // quads
+    uint4 *steps_of_team = handed + team * split * (DEPTH * STEP);
+    auto meet = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(32 * split) : "memory"); };
+    auto load_round = [&](int k) {
 #pragma unroll
-      for (int i = 0; i < WORDS; ++i) mine[i * 32] = acc[i / (4 * T)][i / 4 % T][i % 4];
+      for (int d = 0; d < DEPTH; ++d)
+        if (k + d * split < steps) load(f[d], k + d * split);
+    };
+    load_round(member);
+    for (int first = 0; first < steps; first += DEPTH * split) {
+#pragma unroll
+      for (int d = 0; d < DEPTH; ++d) {
+        if (first + d * split + member < steps) {
+          uint4 *mine = steps_of_team + (d * split + member) * STEP;
+#pragma unroll
+          for (int t = 0; t < T; ++t) {
+            uint32_t a[4];
+            columns_of(f[d], 0, t, a);
+            mine[t * 32 + lane] = make_uint4(a[0], a[1], a[2], a[3]);
+          }
+          uint2 *blocks = reinterpret_cast<uint2 *>(mine + T * 32);
+#pragma unroll
+          for (int u = 0; u < F::TILES; ++u) blocks[u * 32 + lane] = make_uint2(f[d].block[0][u][0], f[d].block[0][u][1]);
+        }
+      }
+      meet();
+      load_round(first + DEPTH * split + member);
+      if (member < F::TILES) {
+        const int n = steps - first < DEPTH * split ? steps - first : DEPTH * split;
+        const uint4 *step = steps_of_team;
+#pragma unroll 4
+        for (int j = 0; j < n; ++j, step += STEP) {
+          const uint2 v = reinterpret_cast<const uint2 *>(step + T * 32)[member * 32 + lane];
+#pragma unroll
+          for (int t = 0; t < T; ++t) {
+            const uint4 a = step[t * 32 + lane];
+            mma(acc[0][t], a.x, a.y, a.z, a.w, v.x, v.y);
+          }
+        }
+      }
+      if (first + DEPTH * split < steps) meet();
     }
-    __syncthreads();
-    if (part > 0) return;
-    mine += WORDS * 32;
-    for (int s = 1; s < split; ++s, mine += WORDS * 32)
-#pragma unroll
-      for (int i = 0; i < WORDS; ++i) acc[i / (4 * T)][i / 4 % T][i % 4] += mine[i * 32];
   }
-  if (!active) return;
+  if (!active || (TEAM && member >= F::TILES)) return;
 #pragma unroll
-  for (int u = 0; u < F::TILES; ++u)
+  for (int u = 0; u < SUMS; ++u) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       uint32_t w[T];
@@ -230,29 +278,34 @@ __global__ void __launch_bounds__(32 * MMA_WARPS, mma_ctas(BS, T, V))
         const __nv_bfloat162 h = __floats2bfloat162_rn(acc[u][t][r], acc[u][t][2 + r]);
         w[t] = *reinterpret_cast<const uint32_t *>(&h);
       }
-      store_row<T, V ? V : 1>(C + (brow * BS + 8 * u + 2 * q + r) * N + col0, w, valid);
+      store_row<T, V ? V : 1>(C + (brow * BS + 8 * (TEAM ? member : u) + 2 * q + r) * N + col0, w, valid);
     }
+  }
 }
 
 template <int BS, int T, int V, bool WIDE>
 cudaError_t launch_mma(const BsrSpmmArgs &a, int sm_count, cudaStream_t s) {
   const int64_t tiles = ceil_div(a.n_rhs, 16 * T), units = a.rows / BS * tiles;
-  // Parts of a block row: while there are fewer than 16 warps per SM and a part keeps 64 rows of B (140 block rows of 47 blocks
-  // of 16 x 16, N = 4: 17.5 us whole, 4.7 in eight parts; 303 of 5, N = 504: 8.0 whole, 13.2 in four).
+  // Warps of a block row: more while the GPU has no more than ten per SM and each has a step, and at least one for every tile of
+  // 8 rows (16 x 16, N = 8, us with 1, 2, 4 and 8 warps: 80 block rows of 30 9.9, 7.0, 4.9, 3.9; 300 of 20 8.3, 5.4, 4.4, 4.8;
+  // 600 of 12 6.6, 4.8, 5.4, 6.1; 2,000 of 20 11.0, 11.4, 13.9, 17.5; 32 x 32, N = 48: 80 of 30 19.8 and, with four and eight, 13.6,
+  // 11.1; 1,000 of 20 23.4, 40.7, 43.0).
   int split = 1;
-  while (split < MMA_WARPS && units * split < (int64_t)sm_count * 16 && a.nnzb * BS * BS >= split * 64 * a.rows) split *= 2;
+  while (split < MMA_WARPS && units * split * 2 <= (int64_t)sm_count * 10 && a.nnzb * BS * BS >= split * 16 * a.rows) split *= 2;
+  if (split > 1 && split < BS / 8) split = BS / 8;
   unsigned grid = 0;
   if (!grid_dim(ceil_div(units * split, MMA_WARPS), &grid)) return cudaErrorInvalidConfiguration;
-  const size_t smem = (size_t)(MMA_WARPS - MMA_WARPS / split) * (BS / 8 * T * 4 * 32) * 4;
-  launch_chained(bsr_spmm_mma_kernel<BS, T, V, WIDE>, grid, 32 * MMA_WARPS, smem, s, units, (int)tiles, split, a.n_rhs,
-                 a.block_row_ptr, a.block_col_idx, static_cast<const __nv_bfloat16 *>(a.block_values),
-                 static_cast<const __nv_bfloat16 *>(a.B), static_cast<__nv_bfloat16 *>(a.C));
+  const size_t smem = split > 1 ? MMA_WARPS * team_steps(BS, T) * step_words(BS, T) * 32 * 4 : 0;  // at most 48 KB
+  launch_chained(split > 1 ? bsr_spmm_mma_kernel<BS, T, V, WIDE, true> : bsr_spmm_mma_kernel<BS, T, V, WIDE, false>, grid,
+                 32 * MMA_WARPS, smem, s, units, (int)tiles, split, a.n_rhs, a.block_row_ptr, a.block_col_idx,
+                 static_cast<const __nv_bfloat16 *>(a.block_values), static_cast<const __nv_bfloat16 *>(a.B),
+                 static_cast<__nv_bfloat16 *>(a.C));
   return cudaGetLastError();
 }
 
 template <int BS, int T, int V>
 cudaError_t launch_wide(const BsrSpmmArgs &a, int sm_count, cudaStream_t s) {
-  const bool wide = reinterpret_cast<uintptr_t>(a.block_values) % (BS == 32 ? 16 : 8) == 0;
+  const bool wide = reinterpret_cast<uintptr_t>(a.block_values) % 8 == 0;
   return wide ? launch_mma<BS, T, V, true>(a, sm_count, s) : launch_mma<BS, T, V, false>(a, sm_count, s);
 }
 
