@@ -28,7 +28,7 @@
 //     Both accumulators' MMAs read the same copy.
 //
 // Pipeline.  Persistent CTAs, three (256 columns) to five per SM, walk the units.  A stage holds a group of four 16 x 16
-// blocks (two of 32 x 32, eight of 8 x 8) with their slabs.  Lanes 0 of warps 4 - 7 copy: each takes its blocks of every
+// blocks (two of 32 x 32, one with 256 columns; eight of 8 x 8) with their slabs.  Lanes 0 of warps 4 - 7 copy: each takes its blocks of every
 // group, block columns held 32 at a time in the warp's lanes and requested ahead.  Lane 0 of warp 8 issues the group's MMAs
 // and lets tcgen05.commit arrive on `empty`.  There are two sets of accumulators: while warps 0 - 3 read one with tcgen05.ld,
 // round to bf16 and store C, the MMAs of the next unit fill the other.
@@ -67,7 +67,7 @@ constexpr unsigned FULL = 0xffffffffu;
 // A stage: GROUP blocks of a block row, their slabs of B and the blocks themselves.
 template <int BS, int HALVES>
 struct Shape {
-  static constexpr int GROUP = 64 / BS;                     // blocks per stage
+  static constexpr int GROUP = BS == 32 && HALVES == 2 ? 1 : 64 / BS;  // blocks per stage
   static constexpr int COPY_WARPS = GROUP < 4 ? GROUP : 4;  // warps that issue its copies
   static constexpr int MMA_BLOCKS = BS == 8 ? 2 : 1;        // blocks per MMA: two of 8 x 8 side by side along k
   static constexpr int BOX_BYTES = BS * 64 * 2;             // 64 columns x BS rows of B
@@ -94,7 +94,7 @@ constexpr int most_stages() {
 // three of two 59); their accumulators fit the 512 columns of TMEM.
 template <int BS, int HALVES>
 int ctas_per_sm(int64_t units, int sm_count, int *stages) {
-  constexpr int MOST = HALVES == 2 ? 3 : BS == 32 ? 4 : 5;
+  constexpr int MOST = BS == 32 ? 4 : HALVES == 2 ? 3 : 5;
   static_assert(MOST * Shape<BS, HALVES>::TMEM_COLS <= 512 && 222 * 1024 / MOST - 1024 >= 2 * Shape<BS, HALVES>::STAGE_BYTES, "");
   int64_t per_sm = (units + sm_count - 1) / sm_count;
   if (per_sm > MOST) per_sm = MOST;
@@ -363,38 +363,46 @@ __global__ void __launch_bounds__(THREADS) bsr_spmm_tcgen05_kernel(
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       }
       // TMEM lane m of accumulator h = column n0 + 128 h + m of C; this warp reads lanes 32 warp .. +32
-      uint32_t v[HALVES][BS < 16 ? 16 : BS];
+      // (two accumulators of 32 columns after one another, for registers that leave room for three CTAs).
+      constexpr int ROWS = BS < 16 ? 16 : BS, AT_ONCE = BS == 32 ? 1 : HALVES;
 #pragma unroll
-      for (int h = 0; h < HALVES; ++h)
+      for (int h0 = 0; h0 < HALVES; h0 += AT_ONCE) {
+        uint32_t v[AT_ONCE][ROWS];
 #pragma unroll
-        for (int r0 = 0; r0 < BS; r0 += 16) {
-          if (empty || h >= halves) {
+        for (int h = 0; h < AT_ONCE; ++h)
 #pragma unroll
-            for (int r = 0; r < 16; ++r) v[h][r0 + r] = 0;
-          } else {
+          for (int r0 = 0; r0 < ROWS; r0 += 16) {
             uint32_t *w = &v[h][r0];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-                "%15}, [%16];"
-                : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]),
-                  "=r"(w[8]), "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
-                : "r"(sums + (uint32_t)(h * S::MMA_N + r0))
-                : "memory");
+            if (empty || h0 + h >= halves) {
+#pragma unroll
+              for (int r = 0; r < 16; ++r) w[r] = 0;
+            } else {
+              asm volatile(
+                  "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+                  "%15}, [%16];"
+                  : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]),
+                    "=r"(w[8]), "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
+                  : "r"(sums + (uint32_t)((h0 + h) * S::MMA_N + r0))
+                  : "memory");
+            }
+          }
+        if (!empty) {
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (h0 + AT_ONCE == HALVES) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            if (lane == 0)
+              asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_stored[made & 1])) : "memory");
+            ++made;
           }
         }
-      if (!empty) {
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_stored[made & 1])) : "memory");
-        ++made;
-      }
 #pragma unroll
-      for (int h = 0; h < HALVES; ++h) {
-        const int64_t col = (int64_t)n0 + h * HALF_N + warp * 32 + lane;
-        if (col < N) {
-          __nv_bfloat16 *out = C + br * BS * N + col;
+        for (int h = 0; h < AT_ONCE; ++h) {
+          const int64_t col = (int64_t)n0 + (h0 + h) * HALF_N + warp * 32 + lane;
+          if (col < N) {
+            __nv_bfloat16 *out = C + br * BS * N + col;
 #pragma unroll
-          for (int r = 0; r < BS; ++r) out[r * N] = __float2bfloat16_rn(__uint_as_float(v[h][r]));
+            for (int r = 0; r < BS; ++r) out[r * N] = __float2bfloat16_rn(__uint_as_float(v[h][r]));
+          }
         }
       }
       b = after;
@@ -523,7 +531,7 @@ cudaError_t launch_halves(const BsrSpmmArgs &a, int *status, int sm_count, cudaS
   const auto swizzle = BS == 8 ? CU_TENSOR_MAP_SWIZZLE_NONE : BS == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B;
   if (!make_map_2d(&map_box, a.B, (uint64_t)a.n_rhs, (uint64_t)a.cols, 64, BS, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !make_map_2d(&map_block, a.block_values, BS, (uint64_t)a.nnzb * BS, BS, BS, swizzle) ||
-      !make_map_2d(&map_group, a.block_values, BS, (uint64_t)a.nnzb * BS, BS, 64, swizzle))
+      !make_map_2d(&map_group, a.block_values, BS, (uint64_t)a.nnzb * BS, BS, Shape<BS, HALVES>::GROUP * BS, swizzle))
     return cudaErrorInvalidValue;
   if (a.n_rhs < 64)
     map_slab = map_box;  // not used: no tile has two boxes
@@ -543,14 +551,15 @@ template <bool PER_UNIT_STATUS, int BS>
 cudaError_t launch_tcgen05(const BsrSpmmArgs &a, int *status, int sm_count, cudaStream_t s) {
   // Tiles of 256 columns fetch a block once for two accumulators; tiles of 128 where the second would be empty or nearly so,
   // and where 256 leave too few units (403 block rows of 9, N = 480: 13.2 us with 256, 12.4 with 128; 1,024 of 51, N = 512:
-  // 59 and 64).  A block of 32 x 32 is large beside its slab, but two tiles' slabs leave room for one stage only (47.7 us
-  // with 128, 80 with 256 on 512 block rows of 32, N = 512).  The status words of the static entry point are per 256 columns.
-  const int64_t pairs = a.rows / BS * ceil_div(a.n_rhs, 2 * HALF_N), tail = a.n_rhs % (2 * HALF_N);
-  const bool narrow = BS == 32 || a.n_rhs <= HALF_N || (tail > 0 && tail <= 64) || pairs < 6 * (int64_t)sm_count;
+  // 59 and 64).  32 x 32 has one block per stage with 256, which only many whole tiles make up for (us with 128 and 256: 2,000
+  // block rows of 30, N = 512 157, 134; 900 of 20 56.8, 50.5; 2,000 of 6, N = 192 26.0, 22.4; but 700 of 20, N = 512 41.9, 44.8;
+  // 2,000 of 30, N = 384 115, 123, N = 200 115, 120).  The status words of the static entry point are per 256 columns.
+  const int64_t n = a.n_rhs, pairs = a.rows / BS * ceil_div(n, 2 * HALF_N), tail = n % (2 * HALF_N);
+  const bool narrow = BS == 32 ? n % 64 != 0 || (tail > 0 && tail < 192) || pairs < 10 * (int64_t)sm_count
+                               : n <= HALF_N || (tail > 0 && tail <= 64) || pairs < 6 * (int64_t)sm_count;
   if constexpr (!PER_UNIT_STATUS)
     if (narrow) return launch_halves<PER_UNIT_STATUS, BS, 1>(a, status, sm_count, s);
-  if constexpr (BS != 32) return launch_halves<PER_UNIT_STATUS, BS, 2>(a, status, sm_count, s);
-  return cudaErrorInvalidValue;
+  return launch_halves<PER_UNIT_STATUS, BS, 2>(a, status, sm_count, s);
 }
 
 }  // namespace

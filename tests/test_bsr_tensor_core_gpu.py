@@ -38,7 +38,7 @@ def test_values_of_other_block_rows_do_not_leak(ctx, bs):
 
 
 @pytest.mark.parametrize("bs,rows,n", [(16, 3, 128), (16, 1900, 128), (16, 1000, 320), (16, 700, 232), (16, 1300, 512),
-                                       (32, 450, 64), (32, 1500, 72), (32, 300, 200), (8, 2100, 256), (8, 4400, 440)])
+                                       (32, 450, 64), (32, 1500, 72), (32, 300, 200), (8, 2100, 256), (8, 4400, 440), (32, 1600, 192), (32, 2100, 256)])
 def test_several_units_per_cta(ctx, bs, rows, n):
     """Persistent CTAs: one to nine units each, with empty block rows, whole and partial groups, and both tile widths."""
     counts = torch.tensor([0, 1, 2, 3, 4, 5, 9, 0, 16, 35])[torch.arange(rows) % 10]
