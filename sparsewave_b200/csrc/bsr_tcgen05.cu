@@ -473,34 +473,29 @@ bool bsr_tcgen05_supported(const BsrSpmmArgs &a) {
          (reinterpret_cast<uintptr_t>(a.B) & 15u) == 0 && (reinterpret_cast<uintptr_t>(a.block_values) & 15u) == 0;
 }
 
-// Against the mma.sync kernel, which reads its operands from global memory and takes any size: this one where a tile of
-// columns is well filled and there are units enough for persistent CTAs (times: mma.sync, here).
-// 16 x 16: whole groups of 64 columns from 128 on (1,500 block rows of 40, N = 192 61.7, 38.2 us; 3,419 of 8, N = 128 24.7,
-// 19.0; but 70 of 30, N = 256 6.2, 9.0 and 150 of 5, N = 512 5.9, 7.1; 683 of 10, N = 128 10.5, 8.6); 80, 96 and 112 columns
-// but for short block rows (1,500 of 40, N = 96 45.6, 27.2; 3,800 of 8, N = 80 22.3, 22.0; 1,187 of 6, N = 88 7.7, 9.4), 64
-// and 72 on long ones (1,500 of 40, N = 64 31.6, 26.2; 3,800 of 8 17.3, 21.7); a last tile of 32 columns or more (300 of 30, N
-// = 336 22.8, 15.3; 447 of 39, N = 160 25.3, 17.5; of short rows only 96 of 256: 2,941 of 4, N = 296 26.6, 32.3); with less in
-// the last tile on many units (264 columns, 3,800 of 8: 60.7, 52.8, 900 of 12: 18.1, 19.8; 136 columns, 3,800 of 25: 86.6,
-// 70.4, 2,271 of 12: 25.2, 27.9).  Rows of B that are no multiple of 32 bytes cost the copies more (N = 104, 2,177 of 17:
-// 24.1, 26.9; N = 88, 557 of 16: 9.4, 10.4).
-// 32 x 32: from 64 columns (1,331 of 5, N = 64: 11.7, 10.8; 489 of 15, N = 96 16.1, 12.3; 94 units, N = 88: 6.8, 13.7).
-// 8 x 8, half of whose MMA is padding: whole groups of 64 from 128 on, on long block rows (500 of 40, N = 256 17.6, 12.4) or
-// many units without a last tile of 64 (4,000 of 10, N = 128 19.2, 18.8, N = 320 40.5, 47.9), others from 400 (N = 184: 39,
-// 47).
-bool bsr_tcgen05_pays(const BsrSpmmArgs &a) {
-  const int64_t n = a.n_rhs, brows = a.rows / a.block_size, units = brows * ceil_div(n, HALF_N), tail = n % HALF_N;
-  const int64_t mean = brows > 0 ? a.nnzb / brows : 0;
-  if (a.block_size == 32) return n >= HALF_N ? units >= 200 : n >= 64 && units >= 400;
-  if (a.block_size == 8) {
-    if (n < HALF_N || n % 64 != 0) return n >= 400 && units >= 13000;
-    return mean >= 24 ? units >= 450 : n % (2 * HALF_N) != 64 && units >= 1500;
-  }
-  if (n < HALF_N) return n >= 80 ? n % 16 == 0 && units >= 600 && mean >= 8 : n >= 64 && mean >= 30 && units >= 1000;
-  if (n % 64 == 0) return units >= (mean >= 16 ? 150 : mean >= 8 ? 350 : 700);
-  const bool filled = n % (2 * HALF_N) >= 96 && units >= 1000;
-  if (n < HALF_N + 16) return units >= 6000 && mean >= 16;
-  if (mean < 8 || (n < 2 * HALF_N && (tail < 32 || n % 16 != 0))) return filled;
-  return units >= (tail >= 32 ? 600 : 4000) || filled;
+// Against the mma.sync kernel, which reads its operands from global memory and takes any size: this one where a tile of columns
+// is well filled, there is a unit for every SM and block rows are long enough to fill the pipeline.  Both give the same bits, so
+// that the line only decides the time.  Measured on 80 to 5,000 block rows of 5 to 40 (us with mma.sync, here):
+//   32 x 32: 300 block rows of 24, N = 64 19.5, 14.2; 1,200 of 12, N = 136 33.6, 33.5, N = 256 57.0, 28.3; from 104 columns on
+//   less than a unit per SM too (80 of 24, N = 128 17.2, 11.8; of 6, N = 104 5.9, 6.5).
+//   16 x 16: whole groups of 64 columns from 128 on whatever the rows' length (300 of 6, N = 128 6.9, 5.9; 1,200 of 30, N = 256
+//   53.9, 26.9; but 80 of 6, N = 128 3.2, 4.4; 600 of 6, N = 192 8.5, 9.3); others from 8 blocks a row on (1,200 of 12, N = 160
+//   19.1, 16.7; of 5 10.9, 11.7), with rows of B that are no multiple of 32 bytes from 12 (150 of 40, N = 136 16.0, 11.1; 600 of 24
+//   16.7, 18.5; 1,200 of 30 32.0, 31.7); 64 columns from 12 a row and two units per SM on (300 of 24 10.5, 8.7; 150 of 12 4.5, 6.0).
+//   8 x 8, half of whose MMA is padding: whole groups of 64 columns from 128 on and rows of 20 blocks (300 of 24, N = 256 11.1, 8.8,
+//   N = 192 8.2, 9.2; 1,200 of 30, N = 128 20.7, 12.6; but 2,500 of 20, N = 264 33.2, 43.3), or many units of whole tiles (5,000
+//   of 8, N = 512 78.1, 48.3; 1,200 of 12, N = 256 14.1, 11.9; 600 of 6 6.4, 8.3).
+bool bsr_tcgen05_pays(const BsrSpmmArgs &a, int sm_count) {
+  const int64_t n = a.n_rhs, brows = a.rows / a.block_size, units = brows * ceil_div(n, HALF_N);
+  if (n < 64 || brows == 0) return false;
+  if (a.block_size == 32) return n >= 104 || units >= sm_count;
+  if (units < sm_count) return false;
+  const int64_t mean = a.nnzb / brows;
+  const bool groups = n >= HALF_N && n % 64 == 0;
+  if (a.block_size == 8) return groups && (mean >= 20 || (mean >= 8 && n % (2 * HALF_N) == 0 && units >= 8 * (int64_t)sm_count));
+  if (groups) return true;
+  if (n < 72) return mean >= 12 && units >= 2 * (int64_t)sm_count;
+  return mean >= (n > HALF_N && n % 16 != 0 ? 12 : 8);
 }
 
 namespace {
@@ -526,16 +521,14 @@ cudaError_t launch_halves(const BsrSpmmArgs &a, int *status, int sm_count, cudaS
   cudaError_t e = configure<PER_UNIT_STATUS, BS, HALVES>();
   if (e != cudaSuccess) return e;
   CUtensorMap map_slab, map_box, map_block, map_group;
-  // B: cols x N bf16, boxes of 64 columns x BS rows, 128-byte swizzle, one or (in whole groups of 64 columns) a tile's; block
+  // B: cols x N bf16 (N at least 64), boxes of 64 columns x BS rows, 128-byte swizzle, one or (in whole groups of 64 columns) a tile's; block
   // values: (nnzb * BS) x BS, boxes of one block and of a group.
   const auto swizzle = BS == 8 ? CU_TENSOR_MAP_SWIZZLE_NONE : BS == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B;
   if (!make_map_2d(&map_box, a.B, (uint64_t)a.n_rhs, (uint64_t)a.cols, 64, BS, CU_TENSOR_MAP_SWIZZLE_128B) ||
       !make_map_2d(&map_block, a.block_values, BS, (uint64_t)a.nnzb * BS, BS, BS, swizzle) ||
       !make_map_2d(&map_group, a.block_values, BS, (uint64_t)a.nnzb * BS, BS, Shape<BS, HALVES>::GROUP * BS, swizzle))
     return cudaErrorInvalidValue;
-  if (a.n_rhs < 64)
-    map_slab = map_box;  // not used: no tile has two boxes
-  else if (!make_map_3d(&map_slab, a.B, (uint64_t)a.n_rhs, (uint64_t)a.cols, BS, 2 * HALVES))
+  if (!make_map_3d(&map_slab, a.B, (uint64_t)a.n_rhs, (uint64_t)a.cols, BS, 2 * HALVES))
     return cudaErrorInvalidValue;
   int stages;
   const int per_sm = ctas_per_sm<BS, HALVES>(units, sm_count, &stages);
@@ -702,10 +695,11 @@ extern "C" __attribute__((visibility("default"))) int swb_bsr16_spmm_bf16_static
   // The words keep the previous call's outcome: clear the ones this call uses.
   e = cudaMemsetAsync(status, 0, (size_t)grid * sizeof(int), s);
   if (e != cudaSuccess) return static_fail(kCuda, cudaGetErrorString(e));
-  // The kernel that the regular entry point would choose, so that both give the same bits; the one without tcgen05 never waits.
+  // The kernel that the regular entry point would choose, but for the SM count, which costs a call here; both kernels give the
+  // same bits, and the one without tcgen05 never gives up.
   int64_t launches = 0;
-  e = bsr_tcgen05_pays(a) ? launch_tcgen05<true, 16>(a, status, DeviceInfo().sm_count, s)
-                          : launch_bsr_spmm_mma(a, DeviceInfo(), s, &launches);
+  e = bsr_tcgen05_pays(a, DeviceInfo().sm_count) ? launch_tcgen05<true, 16>(a, status, DeviceInfo().sm_count, s)
+                                                     : launch_bsr_spmm_mma(a, DeviceInfo(), s, &launches);
   if (e == cudaErrorInvalidValue) return static_fail(kCuda, "could not encode the TMA tensor maps");
   if (e != cudaSuccess) return static_fail(kCuda, cudaGetErrorString(e));
   slot->last_grid.store(grid, std::memory_order_release);
