@@ -200,8 +200,9 @@ cudaError_t launch_columns(const BsrSpmmArgs &a, bool few, cudaStream_t s) {
     case 2: return launch_tiles<T, 2, 2, V>(a, s);
     case 3: return launch_tiles<T, 3, 3, V>(a, s);
     case 4: return few ? launch_tiles<T, 4, 2, V>(a, s) : launch_tiles<T, 4, 4, V>(a, s);
-    case 8: return few ? launch_tiles<T, 8, 2, V>(a, s) : launch_tiles<T, 8, 8, V>(a, s);
   }
+  if constexpr (sizeof(T) == sizeof(float))  // 8 x 8 blocks in bf16 run on tensor cores
+    if (a.block_size == 8) return few ? launch_tiles<T, 8, 2, V>(a, s) : launch_tiles<T, 8, 8, V>(a, s);
   return few ? launch_tiles<T, 0, 2, V>(a, s) : launch_tiles<T, 0, 8, V>(a, s);
 }
 
