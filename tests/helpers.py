@@ -65,6 +65,19 @@ def dev(a, dtype=None):
     return t.cuda()
 
 
+def launched(call):
+    """The result of `call` and the names of the library's kernels that it launched, e.g. "bsr_spmm_tcgen05_kernel<false, 16, 1>";
+    None for the names where no profiler is to be had."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as profile:
+        result = call()
+        torch.cuda.synchronize()
+    names = [e.name for e in profile.events()]
+    if not any("(" in name for name in names):
+        return result, None
+    return result, [name.split("::")[-1].split(">(")[0] + ">" if ">(" in name else name.split("::")[-1].split("(")[0]
+                    for name in (n.replace("(anonymous namespace)::", "") for n in names) if "swb::" in name]
+
+
 def assert_within_bound(actual, expected, bound, rel=1e-5):
     """|actual - expected| <= rel * sum|a*x| per output element."""
     actual = np.asarray(actual, dtype=np.float64)

@@ -1,4 +1,5 @@
-"""bf16 BSR SpMM on both sides of the lines between the tensor-core kernels, against the oracle."""
+"""bf16 BSR SpMM of sizes with short, long and ragged last tiles of columns on both tensor-core kernels, against the oracle (the line
+between the two, by kernel name: test_bsr_tcgen05_gpu.py)."""
 import pytest
 import torch
 

@@ -1,4 +1,5 @@
-"""BSR SpMM on the tensor cores for blocks of 8 x 8 (two per step), 16 x 16 and 32 x 32."""
+"""BSR SpMM on the tensor cores for blocks of 8 x 8 (two per step), 16 x 16 and 32 x 32, in whichever of the two kernels the sizes
+lead to (few block rows: warp-level MMAs; the tcgen05 kernel by name: test_bsr_tcgen05_gpu.py)."""
 import pytest
 import torch
 

@@ -75,6 +75,14 @@ def test_spmm_any_shape_any_option(ctx, case, n, opts):
     assert_within_bound(C.cpu().numpy(), oracle.csr_spmm(rp, ci, v, B), oracle.csr_abs_bound(rp, ci, v, B))
 
 
+@settings(max_examples=15, deadline=None, derandomize=True, suppress_health_check=[HealthCheck.function_scoped_fixture])
+@given(brows=st.integers(150, 1000), bcols=st.integers(1, 40), n64=st.integers(2, 5), density=st.floats(0.01, 0.3),
+       seed=st.integers(0, 10 ** 6))
+def test_bsr16_many_block_rows_any_shape(ctx, brows, bcols, n64, density, seed):
+    """A unit of work for every SM: the tcgen05 kernel (the test below stays below that)."""
+    test_bsr16_tensor_core_any_shape.hypothesis.inner_test(ctx, brows, bcols, 8 * n64, density, seed)
+
+
 @settings(max_examples=25, deadline=None, derandomize=True, suppress_health_check=[HealthCheck.function_scoped_fixture])
 @given(brows=st.integers(1, 40), bcols=st.integers(1, 40), n8=st.integers(1, 40), density=st.floats(0.0, 0.6),
        seed=st.integers(0, 10 ** 6))

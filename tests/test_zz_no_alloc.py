@@ -2,8 +2,9 @@
 (swb_bsr16_spmm_bf16_static: no context, status words in a fixed array inside
 the library).  It must give the same bits as the regular context-based entry
 point, on two calls in a row that share the fixed array, and it must refuse
-what does not fit.  Collected last on purpose: a failure here stops nothing
-else."""
+what does not fit.  These sizes run on warp-level MMAs, which never wait; the
+kernel with a status word per unit is in test_bsr_tcgen05_gpu.py.  Collected
+last on purpose: a failure here stops nothing else."""
 import pytest
 import torch
 
