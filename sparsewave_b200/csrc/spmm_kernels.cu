@@ -629,12 +629,15 @@ constexpr int64_t positions_per_lane_group(int G) { return G == 1 ? 6 : G == 2 ?
 // ... and doubled for few rows, which leave the GPU idle, so that the time is that of the longest row: up to 200,000 lanes (42
 // warps per SM) where a row's lanes have less than a mean row in flight (four positions per group), up to 100,000 where less
 // than two.  Ragged rows (times in a CUDA graph): 3,476 of 16, N = 32 16.8 -> 4.3 us; 10,651 of 16, N = 16 17.4 -> 7.9; 4,963 of 39, N = 8
-// 12.5 -> 5.8; equal rows 0.8 to 1.1, the shortest 1.3 (11,917 of 6, N = 32: 2.8 -> 3.6).  More lanes lose on short rows (12,068
-// of 7, N = 16 with 380,000: 5.0 -> 7.4).
+// 12.5 -> 5.8; equal rows 0.8 to 1.1.  More lanes lose on short rows (12,068 of 7, N = 16 with 380,000: 5.0 -> 7.4), and on equal
+// rows below eight positions (6,090 of 6, N = 64 2.7 -> 3.7, ragged 7.3 -> 4.2) or above 15,000 rows (18,489 of 15, N = 16 4.1 -> 5.2,
+// ragged 17.1 -> 11.7), which therefore keep theirs.
 inline int lanes_per_row(int64_t rows, int64_t mean, int G) {
   int lanes = G > 4 ? G : 4;
   while (lanes < 32 && (int64_t)(lanes / G) * positions_per_lane_group(G) < mean) lanes *= 2;
-  while (lanes < 32 && (lanes / G * 4 < mean ? rows * lanes <= 100000 : lanes / G * 4 < 2 * mean && rows * lanes <= 50000)) lanes *= 2;
+  while (lanes < 32 && ((lanes / G * 4 < mean && mean >= 8 && rows <= 15000 && rows * lanes <= 100000) ||
+                        (lanes / G * 4 < 2 * mean && rows * lanes <= 50000)))
+    lanes *= 2;
   return lanes;
 }
 

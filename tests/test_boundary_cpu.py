@@ -123,6 +123,15 @@ def test_row_search_matches_oracle_with_empty_rows():
         assert rp[r] <= p < rp[r + 1]
 
 
+@pytest.mark.parametrize("rows,mean,n,rows_per_warp", [
+    (15000, 15, 16, 4), (15001, 15, 16, 8),  # up to 15,000 rows a second group of lanes for a row of 15
+    (6000, 8, 64, 1), (6000, 7, 64, 2), (3000, 7, 64, 1),  # below eight positions only up to 50,000 lanes
+    (11917, 6, 32, 4), (5000, 16, 32, 1)])
+def test_lanes_per_row_of_few_rows(rows, mean, n, rows_per_warp):
+    shape = swb.launch_shape("spmm-mapping=wave-per-row-tile spmm-tile-size=16 spmm-block-size=256", rows, mean * rows, n)
+    assert shape.physical_grid == -(-rows // (8 * rows_per_warp))
+
+
 def test_launch_shapes_follow_reference_grid_arithmetic():
     # SparseGPUUtils.cpp:11-59, SparseWaveToGPU.cpp:380, SparsePositionScheduling.cpp:340-350
     s = swb.launch_shape("mapping=thread-per-row block-size=128", rows=4096, nnz=65536)
