@@ -809,14 +809,18 @@ inline int64_t tile_rows_per_block(int64_t N, int64_t mean, int block) {
 // A warp per row (spmm_wave_per_row_any_kernel) keeps short rows and more than 4,736 (5,900 of 27, N = 40: 4.9, 6.5).  A row gets
 // a second and then a third and fourth warp while a warp has not three mean rows' positions in flight and all warps are one
 // wave, or not one mean row and they are three (4,164 ragged rows of 40, N = 18: 12.9 us with one warp, 10.2 with two; 2,172 of
-// 64, N = 19: 44, 27 and with four 15.5).
+// 64, N = 19: 44, 27 and with four 15.5).  With four columns per lane, two warps in blocks of 128 threads take the place of four
+// that would be more than one wave, where they have half a mean row in flight: equal rows pay for warps that they do not need
+// (us without teams, with four warps and with two, equal and ragged rows: 4,736 of 28, N = 40 4.9, 8.3, 5.6 and 15.0, 9.3, 7.5; 3,151 of
+// 35, N = 36 4.3, 6.1, 4.8 and 16.8, 8.0, 7.6; 4,600 of 60, N = 28 6.8, 8.3, 6.0 and 18.5, 10.7, 11.1).
 struct Team {
   int V, G, S;
   int64_t tiles;
+  int threads;
 };
 
 inline Team team_of(int64_t rows, int64_t nnz, int64_t N, int tile, uintptr_t alignment_bits) {
-  Team t{1, 0, 0, 0};
+  Team t{1, 0, 0, 0, TEAM_THREADS};
   if (rows < 1024 || N > 512) return t;
   const int64_t mean = nnz / rows;
   const int V = N % 4 == 0 && alignment_bits % 16 == 0 ? 4 : N % 2 == 0 && alignment_bits % 8 == 0 ? 2 : 1;
@@ -832,14 +836,18 @@ inline Team team_of(int64_t rows, int64_t nnz, int64_t N, int tile, uintptr_t al
   const int64_t units = rows * t.tiles, in_flight = 32 / t.G * team_positions(t.V);
   t.S = 1;
   while (t.S < 4 && t.S * in_flight < 3 * mean && units * t.S <= (t.S * in_flight < mean ? 13000 : 4750)) t.S *= 2;
+  if (V == 4 && t.S == 4 && 4 * units > 148 * 64 && 4 * in_flight >= mean) {
+    t.S = 2;
+    t.threads = TEAM_THREADS / 2;
+  }
   return t;
 }
 
 template <int V>
 cudaError_t launch_team_rows(const CsrSpmmArgs &a, const Team &t, cudaStream_t s) {
   const int64_t units = a.rows * t.tiles;
-  SWB_GRID(grid, ceil_div(units, TEAM_THREADS / 32 / t.S));
-  launch_chained(spmm_team_rows_kernel<V>, grid, TEAM_THREADS, 0, s, units, a.n_rhs, (uint32_t)(a.n_rhs * 4), t.G, t.S, t.tiles,
+  SWB_GRID(grid, ceil_div(units, t.threads / 32 / t.S));
+  launch_chained(spmm_team_rows_kernel<V>, grid, t.threads, 0, s, units, a.n_rhs, (uint32_t)(a.n_rhs * 4), t.G, t.S, t.tiles,
                  a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
   return cudaGetLastError();
 }
@@ -906,7 +914,7 @@ cudaError_t launch_spmm_wave_per_row_tile(const CsrSpmmArgs &a, int block, int t
       launch_chained(spmm_wave_per_row_wide_kernel<4>, grid, block, 0, s, a.rows, N, a.row_ptr, a.col_idx, a.val, a.B, a.C, a.accumulate);
     return cudaGetLastError();
   }
-  const Team team = pow2_row ? Team{1, 0, 0, 0}
+  const Team team = pow2_row ? Team{1, 0, 0, 0, 0}
                              : team_of(a.rows, a.nnz, N, tile, reinterpret_cast<uintptr_t>(a.B) | reinterpret_cast<uintptr_t>(a.C));
   if (team.S > 0)
     return team.V == 4 ? launch_team_rows<4>(a, team, s) : team.V == 2 ? launch_team_rows<2>(a, team, s) : launch_team_rows<1>(a, team, s);
@@ -951,8 +959,8 @@ int64_t wave_per_row_tile_physical_grid(int64_t rows, int64_t nnz, int64_t n_rhs
   }
   const bool pow2_row = n_rhs >= 4 && n_rhs <= 128 && (n_rhs & (n_rhs - 1)) == 0;
   if (n_rhs == 256 || n_rhs == 384 || n_rhs == 512) return max1(ceil_div(rows, wpb));
-  const Team team = pow2_row ? Team{1, 0, 0, 0} : team_of(rows, nnz, n_rhs, tile, 0);
-  if (team.S > 0) return max1(ceil_div(rows * team.tiles, TEAM_THREADS / 32 / team.S));
+  const Team team = pow2_row ? Team{1, 0, 0, 0, 0} : team_of(rows, nnz, n_rhs, tile, 0);
+  if (team.S > 0) return max1(ceil_div(rows * team.tiles, team.threads / 32 / team.S));
   if (n_rhs >= 12 && n_rhs < 128 && n_rhs % 4 == 0 && !pow2_row && rows > 0 && nnz / rows >= 8)
     return max1(ceil_div(rows, wpb));
   if (!pow2_row) return max1(ceil_div(rows * ceil_div(n_rhs, tile), wpb));

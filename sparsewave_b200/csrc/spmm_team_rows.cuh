@@ -8,7 +8,7 @@
 // Requesting a step's positions beside the rows of B of the step before gains nothing: the loads' issue is what counts.
 #pragma once
 
-constexpr int TEAM_THREADS = 256;
+constexpr int TEAM_THREADS = 256;  // or half of them
 constexpr int team_positions(int V) { return V == 4 ? 4 : 8; }  // in flight per group
 
 // A position's column and value where k < n, as predicated loads (see spmm_columns.cuh).
@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(TEAM_THREADS)
   constexpr int Q = team_positions(V);
   __shared__ __align__(16) float s_sums[TEAM_THREADS * V];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, team = warp / S, member = warp - team * S;
-  const int64_t unit = (int64_t)blockIdx.x * (TEAM_THREADS / 32 / S) + team;
+  const int64_t unit = (int64_t)blockIdx.x * (int)(blockDim.x / 32 / S) + team;
   const int per_warp = 32 / G, group = lane / G, l = lane - group * G;
   const int64_t row = tiles == 1 ? unit : unit / tiles, first_col = tiles == 1 ? 0 : (unit - row * tiles) * G * V;
   const int groups = S * per_warp, mine = member * per_warp + group;

@@ -13,7 +13,8 @@ OPTIONS = "spmm-mapping=wave-per-row-tile spmm-tile-size=32 spmm-block-size=256"
     (1024, 5, 5, 1, 1), (1100, 12, 19, 1, 4), (2400, 12, 33, 2, 2), (6001, 7, 9, 1, 1), (1025, 12, 511, 16, 1),
     (1100, 40, 29, 1, 4),  # a column per lane
     (1100, 30, 2, 1, 1), (1100, 40, 62, 1, 4), (3000, 31, 130, 3, 2), (8192, 3, 22, 1, 1),  # two
-    (4736, 28, 40, 1, 4), (3500, 40, 12, 1, 2), (1024, 6, 68, 1, 4)])  # four
+    (4736, 28, 40, 1, 4), (3500, 40, 12, 1, 2), (1024, 6, 68, 1, 4),  # four
+    (3001, 26, 36, 1, 4), (4100, 60, 28, 1, 4)])  # two warps per row in blocks of half the size: the grid of four
 def test_few_rows(ctx, rows, mean, n, tiles, warps):
     rng = np.random.default_rng(rows + n)
     lens = np.minimum(rng.geometric(1 / (mean + 1), rows) - 1, 900)
