@@ -2,16 +2,17 @@
 // swb::{anonymous}).
 //
 // With products and sums rounded separately the operator is bound by issue slots: the threads of bsr_spmm_row_tile_kernel
-// spent one of two on loads, addresses and branches (16,384 block rows of 24 blocks of 4 x 4, N = 32: 25.6 M instructions for
+// spent one of two on loads, addresses and branches (16,384 block rows of 24 blocks of 4 x 4, N = 32: 26.3 M instructions for
 // 12.6 M products and sums).  Here a group of lanes copies its block row's blocks and block columns to shared memory with
 // cp.async, a chunk of four or eight blocks ahead, so that a step has no load but its rows of B and broadcasts from shared
-// memory, and two adjacent columns are one packed instruction: 14.0 M instructions.  The rows of B of a step are requested
-// together; what hides them is other warps.  Every output is added up by one lane in storage order, bit for bit.
+// memory, and two adjacent columns are one packed instruction: 15.6 M instructions with four columns per lane, 19.3 M with two.
+// The rows of B of a step are requested together; what hides them is other warps.  Every output is added up by one lane in
+// storage order, bit for bit.
 //
-// 16,384 block rows of 24, N = 32: 40.2 -> 31 us; 8 x 8, 2,953 of 29, N = 96 76 -> 57, 7,427 of 10, N = 208 125 -> 97,
-// 4 x 4, 7,430 of 5, N = 472 56 -> 44, 111 of 33, N = 360 16.2 -> 10.8; geometric mean over 60 sizes 0.85.  What remains is the end: the longest block rows
-// run on in a few warps.  Blocks of 2 x 2 have too little to add per block (14,720 of 5, N = 56: 7.4 us with the other
-// kernel, 7.9 to 15 here).
+// 16,384 block rows of 24, N = 32: 43.0 -> 32.6 us in a row of calls; 8 x 8, 2,953 of 29, N = 96 76 -> 57, 7,427 of 10, N = 208
+// 125 -> 97, 4 x 4, 7,430 of 5, N = 472 56 -> 44, 111 of 33, N = 360 16.2 -> 10.8; geometric mean over 60 sizes 0.87.  What
+// remains is the end: the longest block rows run on in a few warps.  Blocks of 2 x 2 have too little to add per block (14,720 of
+// 5, N = 56: 7.4 us with the other kernel, 7.9 to 15 here).
 #pragma once
 
 constexpr int GROUP_THREADS = 64;
@@ -207,16 +208,19 @@ cudaError_t launch_groups(const BsrSpmmArgs &a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// V: the columns per lane that B and C are aligned for.  Four where that leaves 130,000 lanes, two above 45,000, one above
-// 20,000 (times with four, two and one: 1,476 block rows of 20 of 4 x 4, N = 448 26, 28, 38 us; 3,461 of 48, N = 136 58, 55,
-// 66; 2,081 of 53, N = 32 27, 18, 17).  With fewer, threads that read their operands themselves, two rows each, start sooner
-// (204 block rows of 40 of 8 x 8, N = 88: 15.9 us, here 21.9; 374 of 13 of 4 x 4, N = 16: 5.1, here 6.2).  Groups below eight
-// lanes would crowd shared memory.
+// V: the columns per lane that B and C are aligned for.  Four where that leaves 24 warps for every one of 148 SMs, 32 warps with up
+// to 64 columns, whose warps hold several block rows and run as long as the longest; two above 45,000 lanes, one above 20,000
+// (time with four columns against two, over 100 sizes of 6 to 24 blocks a row: up to 64 columns 1.02 to 1.25 below 120,000 lanes,
+// 1.03 at 131,072 (16,384 of 24 of 4 x 4, N = 32: 30.8 and 30.0 us), 0.93 to 1.01 from 160,000 on; more columns 0.85 to 1.15 from
+// 90,000 to 110,000, 0.86 to 1.04 at 115,000, 0.73 to 0.94 above; two and one: 2,081 of 53, N = 32 18 and 17 us, 1,476 of 20, N =
+// 448 28 and 38).  With fewer lanes, threads that read their operands themselves, two rows each, start sooner (204 block rows of 40
+// of 8 x 8, N = 88: 15.9 us, here 21.9; 374 of 13 of 4 x 4, N = 16: 5.1, here 6.2).  Groups below eight lanes would crowd shared
+// memory.
 template <int BS>
 bool try_groups(const BsrSpmmArgs &a, int V, cudaStream_t s, cudaError_t *e) {
   const int64_t brows = a.rows / BS, n = a.n_rhs;
   if (n < 8 || brows * n < 20000) return false;
-  if (V == 4 && n >= 32 && brows * (n / 4) >= 130000) *e = launch_groups<BS, 4>(a, s);
+  if (V == 4 && n >= 32 && brows * (n / 4) >= 148 * 32 * (n <= 64 ? 32 : 24)) *e = launch_groups<BS, 4>(a, s);
   else if (V >= 2 && n >= 16 && brows * (n / 2) >= 45000) *e = launch_groups<BS, 2>(a, s);
   else *e = launch_groups<BS, 1>(a, s);
   return true;

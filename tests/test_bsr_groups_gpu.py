@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("bs", [4, 8])
 @pytest.mark.parametrize("brows,n", [(1, 8), (1, 20000), (620, 33), (600, 64), (2500, 9), (2300, 43), (1700, 54), (4200, 124), (5700, 16),
-                                     (16300, 32)])
+                                     (16300, 32), (19000, 32), (3650, 124), (3700, 124)])
 def test_groups(ctx, bs, brows, n):
     """Empty block rows, parts of chunks, whole chunks and more; columns that fill a tile, leave lanes idle, make several tiles."""
     counts = torch.tensor([0, 1, 3, 4, 5, 8, 9, 0, 17, 2])[(torch.arange(brows) * 7 + brows) % 10]
