@@ -9,10 +9,10 @@
 // load of up to 16 bytes, and its results are adjacent columns of C.  Pairs of rows of B are interleaved by byte permutes.
 // The next steps' loads are in flight during this step's MMAs, block columns are held 32 at a time by the warp's lanes.
 //
-// Every output is one chain of MMAs over its block row's steps in storage order, as in bsr_tcgen05.cu, so that its bits depend
-// on its block row and its column alone: not on how many block rows or columns the call has, which kernel takes it, alignment
-// or the device.  Where block rows are few, a team of up to eight warps shares one all the same: its members load the steps in
-// turn and hand them over in shared memory, and each of the first members adds up its share of the block row's rows.
+// Every output is added up over its block row's steps in storage order, as one chain of MMAs or (bsr_chain_sums) as f32 sums of
+// steps, so that a part of a matrix has the bits of the whole, whichever kernel takes either.  Where block rows are few, a team
+// of up to eight warps shares one all the same: its members load the steps in turn and hand them over in shared memory, and each
+// of the first members adds up its share of the block row's rows.
 //
 // What bounds it: launch and latency on small calls, L1 on large ones (eight lanes of a load touch four lines, some 64 lookups
 // for 2 KB of B; ncu: L1 data pipe 67 %, tensor pipe 18 % on 1,024 block rows of 51, N = 512), which bsr_tcgen05.cu then takes.
@@ -120,11 +120,24 @@ __device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uin
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// A step's 16 products added to the sums: by the tensor core, or (its sums are cut off, not rounded) as a sum of their own that
+// is then added, rounded to nearest.
+template <bool CHAIN>
+__device__ __forceinline__ void add_step(float (&sum)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if constexpr (CHAIN) {
+    mma(sum, a[0], a[1], a[2], a[3], b0, b1);
+  } else {
+    float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    mma(d, a[0], a[1], a[2], a[3], b0, b1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[i] += d[i];
+  }
+}
 
 // V: elements per load of a row of B, or 0: N is odd and B starts at a word, so that rows in turn start at a word and in the
 // middle of one.  WIDE: block values are aligned for loads of a lane's four.  TEAM: several warps share a unit, 2, 4 or 8 but
 // no fewer than there are tiles of 8 rows in a block.
-template <int BS, int T, int V, bool WIDE, bool TEAM>
+template <int BS, int T, int V, bool WIDE, bool TEAM, bool CHAIN>
 __global__ void __launch_bounds__(32 * MMA_WARPS, TEAM ? 2 : mma_ctas(BS, T, V))
     bsr_spmm_mma_kernel(int64_t units, int tiles, int team_warps, int64_t N, const int32_t *__restrict__ brp,
                         const int32_t *__restrict__ bci, const __nv_bfloat16 *__restrict__ bv,
@@ -215,7 +228,7 @@ __global__ void __launch_bounds__(32 * MMA_WARPS, TEAM ? 2 : mma_ctas(BS, T, V))
             uint32_t a[4];
             columns_of(f[d], h, t, a);
 #pragma unroll
-            for (int u = 0; u < F::TILES; ++u) mma(acc[u][t], a[0], a[1], a[2], a[3], f[d].block[h][u][0], f[d].block[h][u][1]);
+            for (int u = 0; u < F::TILES; ++u) add_step<CHAIN>(acc[u][t], a, f[d].block[h][u][0], f[d].block[h][u][1]);
           }
         if (++k >= steps) break;
       }
@@ -254,13 +267,14 @@ __global__ void __launch_bounds__(32 * MMA_WARPS, TEAM ? 2 : mma_ctas(BS, T, V))
       if (member < F::TILES) {
         const int n = steps - first < DEPTH * split ? steps - first : DEPTH * split;
         const uint4 *step = steps_of_team;
-#pragma unroll 4
+#pragma unroll CHAIN || T < 4 ? 4 : 2
         for (int j = 0; j < n; ++j, step += STEP) {
           const uint2 v = reinterpret_cast<const uint2 *>(step + T * 32)[member * 32 + lane];
 #pragma unroll
           for (int t = 0; t < T; ++t) {
-            const uint4 a = step[t * 32 + lane];
-            mma(acc[0][t], a.x, a.y, a.z, a.w, v.x, v.y);
+            const uint4 w = step[t * 32 + lane];
+            const uint32_t a[4] = {w.x, w.y, w.z, w.w};
+            add_step<CHAIN>(acc[0][t], a, v.x, v.y);
           }
         }
       }
@@ -283,7 +297,7 @@ __global__ void __launch_bounds__(32 * MMA_WARPS, TEAM ? 2 : mma_ctas(BS, T, V))
   }
 }
 
-template <int BS, int T, int V, bool WIDE>
+template <int BS, int T, int V, bool WIDE, bool CHAIN = false>
 cudaError_t launch_mma(const BsrSpmmArgs &a, int sm_count, cudaStream_t s) {
   const int64_t tiles = ceil_div(a.n_rhs, 16 * T), units = a.rows / BS * tiles;
   // Warps of a block row: more while the GPU has no more than ten per SM and each has a step, and at least one for every tile of
@@ -296,8 +310,8 @@ cudaError_t launch_mma(const BsrSpmmArgs &a, int sm_count, cudaStream_t s) {
   unsigned grid = 0;
   if (!grid_dim(ceil_div(units * split, MMA_WARPS), &grid)) return cudaErrorInvalidConfiguration;
   const size_t smem = split > 1 ? MMA_WARPS * team_steps(BS, T) * step_words(BS, T) * 32 * 4 : 0;  // at most 48 KB
-  launch_chained(split > 1 ? bsr_spmm_mma_kernel<BS, T, V, WIDE, true> : bsr_spmm_mma_kernel<BS, T, V, WIDE, false>, grid,
-                 32 * MMA_WARPS, smem, s, units, (int)tiles, split, a.n_rhs, a.block_row_ptr, a.block_col_idx,
+  launch_chained(split > 1 ? bsr_spmm_mma_kernel<BS, T, V, WIDE, true, CHAIN> : bsr_spmm_mma_kernel<BS, T, V, WIDE, false, CHAIN>,
+                 grid, 32 * MMA_WARPS, smem, s, units, (int)tiles, split, a.n_rhs, a.block_row_ptr, a.block_col_idx,
                  static_cast<const __nv_bfloat16 *>(a.block_values), static_cast<const __nv_bfloat16 *>(a.B),
                  static_cast<__nv_bfloat16 *>(a.C));
   return cudaGetLastError();
@@ -313,6 +327,8 @@ template <int BS>
 cudaError_t launch_bs(const BsrSpmmArgs &a, int sm_count, cudaStream_t s) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(a.B) | reinterpret_cast<uintptr_t>(a.C) | (uintptr_t)(a.n_rhs * 2);
   const int64_t n = a.n_rhs;
+  if (bsr_chain_sums(a) && reinterpret_cast<uintptr_t>(a.C) % 16 == 0)  // 64 columns and more, all aligned
+    return launch_mma<BS, BS == 32 ? 2 : 4, BS == 32 ? 4 : 8, true, true>(a, sm_count, s);
   // 64 columns per warp, fewer for narrow B; two-byte loads and the 32 rows of a large block leave registers for 32
   // (706 block rows of 9, N = 302 off a word: 22.9 us with 64, 19.5 with 32).
   const bool words = n % 2 == 1 && reinterpret_cast<uintptr_t>(a.B) % 4 == 0;

@@ -464,13 +464,25 @@ bool make_map_3d(CUtensorMap *map, const void *base, uint64_t n, uint64_t rows, 
 
 }  // namespace
 
+namespace {
+bool aligned_for_tma(const BsrSpmmArgs &a) {  // 16-byte aligned bases and row pitches
+  return a.n_rhs % 8 == 0 && (reinterpret_cast<uintptr_t>(a.B) & 15u) == 0 &&
+         (reinterpret_cast<uintptr_t>(a.block_values) & 15u) == 0;
+}
+}  // namespace
+
+// Whether an output is one chain of MMAs, whose sums are cut off and not rounded, in this kernel and in the mma.sync one: by what
+// does not change with the number of block rows or blocks, so that a part of a matrix has the bits of the whole.  The kernels on
+// CUDA cores that used to take the other calls rounded every sum to nearest, and so does the mma.sync kernel there (f32 sums of
+// products that cancel, root mean square over that of the sum, 400 blocks of 16 x 16 a block row: 6.7e-7 on CUDA cores,
+// 3.4e-7 with sums of 16 added, 6.1e-6 as a chain; the rounding to bf16 is 1.1e-3).
+bool bsr_chain_sums(const BsrSpmmArgs &a) { return a.n_rhs >= (a.block_size == 8 ? 96 : 64) && aligned_for_tma(a); }
+
 bool bsr_tcgen05_supported(const BsrSpmmArgs &a) {
-  // TMA needs 16-byte aligned bases and row pitches.
   // ... and 32-bit box coordinates: block rows of the value matrix (nnzb * block size) and B's extents.
   if (a.block_size != 8 && a.block_size != 16 && a.block_size != 32) return false;
   if (a.nnzb > 2147483647LL / a.block_size || a.cols > 2147483647LL - 64 || a.n_rhs > 2147483647LL - 256) return false;
-  return a.n_rhs % 8 == 0 && a.nnzb > 0 && a.cols > 0 &&
-         (reinterpret_cast<uintptr_t>(a.B) & 15u) == 0 && (reinterpret_cast<uintptr_t>(a.block_values) & 15u) == 0;
+  return a.nnzb > 0 && a.cols > 0 && aligned_for_tma(a);
 }
 
 // Against the mma.sync kernel, which reads its operands from global memory and takes any size: this one where a tile of columns
@@ -487,7 +499,8 @@ bool bsr_tcgen05_supported(const BsrSpmmArgs &a) {
 //   of 8, N = 512 78.1, 48.3; 1,200 of 12, N = 256 14.1, 11.9; 600 of 6 6.4, 8.3).
 bool bsr_tcgen05_pays(const BsrSpmmArgs &a, int sm_count) {
   const int64_t n = a.n_rhs, brows = a.rows / a.block_size, units = brows * ceil_div(n, HALF_N);
-  if (n < 64 || brows == 0) return false;
+  if (!bsr_chain_sums(a) || !bsr_tcgen05_supported(a) || brows == 0) return false;
+  if (reinterpret_cast<uintptr_t>(a.C) % 16 != 0) return true;  // the mma.sync kernel has chains for aligned C only
   if (a.block_size == 32) return n >= 104 || units >= sm_count;
   if (units < sm_count) return false;
   const int64_t mean = a.nnzb / brows;

@@ -774,7 +774,7 @@ int swb_bsr_spmm_bf16(swb_context *ctx, const swb_options *o, int64_t rows, int6
   swb::BsrSpmmArgs a{rows, cols, nnzb, bs, n_rhs, brp, bci, bv, B, C};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e;
-  if (swb::bsr_tcgen05_supported(a) && swb::bsr_tcgen05_pays(a, ctx->dev.sm_count))
+  if (swb::bsr_tcgen05_pays(a, ctx->dev.sm_count))
     e = swb::launch_bsr_spmm_tcgen05(a, ctx->status_flag, ctx->dev, s, &ctx->launches);
   else if (a.block_size == 8 || a.block_size == 16 || a.block_size == 32)
     e = swb::launch_bsr_spmm_mma(a, ctx->dev, s, &ctx->launches);

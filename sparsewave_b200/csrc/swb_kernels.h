@@ -139,8 +139,9 @@ cudaError_t launch_bsr_spmm_thread_per_output_bf16(const BsrSpmmArgs &a, cudaStr
 cudaError_t launch_bsr_spmm_mma(const BsrSpmmArgs &a, const DeviceInfo &dev, cudaStream_t s, int64_t *launches);
 // The same blocks on the tcgen05 tensor cores.  `status_flag` is a device
 // int the kernel sets non-zero when one of its bounded waits gives up.
+bool bsr_chain_sums(const BsrSpmmArgs &a);  // the tensor cores' own chain of sums, in both kernels
 bool bsr_tcgen05_supported(const BsrSpmmArgs &a);
-bool bsr_tcgen05_pays(const BsrSpmmArgs &a, int sm_count);  // faster there than launch_bsr_spmm_mma
+bool bsr_tcgen05_pays(const BsrSpmmArgs &a, int sm_count);  // and supported; faster there than launch_bsr_spmm_mma
 cudaError_t launch_bsr_spmm_tcgen05(const BsrSpmmArgs &a, int *status_flag, const DeviceInfo &dev, cudaStream_t s,
                                     int64_t *launches);
 
