@@ -17,10 +17,11 @@
 // What bounds it: launch and latency on small calls, L1 on large ones (eight lanes of a load touch four lines, some 64 lookups
 // for 2 KB of B; ncu: L1 data pipe 67 %, tensor pipe 18 % on 1,024 block rows of 51, N = 512), which bsr_tcgen05.cu then takes.
 // Tried: the same loads through a ring in shared memory (178 us against 134 on that size).  Before, on the CUDA cores or with
-// tcgen05 at any size: 123 block rows of 61 blocks of 32 x 32, N = 2 132 -> 12.4 us; 382 of 27, N = 29 105 -> 19.6; 1,438 of 15
-// blocks of 8 x 8, N = 80 30.0 -> 10.1; 90 of 36 blocks of 16 x 16, N = 88 17.5 -> 7.9.  One chain has its price where few
-// warps have much to add up: a block row in parts with sums of their own, added up at the end, took 5.8, 12.1, 10.4 and 5.8 us.
-// Tried for teams: two rounds' loads in flight (spills; 1.09 times the time over 170 sizes), a barrier per step (1.13).
+// tcgen05 at any size: 123 block rows of 61 blocks of 32 x 32, N = 2 132 -> 12.0 us; 382 of 27, N = 29 105 -> 19.9; 1,438 of 15
+// blocks of 8 x 8, N = 80 30.0 -> 10.0; 90 of 36 blocks of 16 x 16, N = 88 17.5 -> 7.9.  Sums in storage order have
+// their price where few warps have much to add up: a block row in parts with sums of their own, added up at the end, took 5.8,
+// 12.1, 10.4 and 5.8 us.  Tried for teams: two rounds' loads in flight (spills; 1.09 times the time over 170 sizes), a barrier per
+// step (1.13), sums of steps handed over in place of operands (1.00 to 1.2).
 #include <cuda_bf16.h>
 
 #include "swb_chain.cuh"
@@ -300,13 +301,14 @@ __global__ void __launch_bounds__(32 * MMA_WARPS, TEAM ? 2 : mma_ctas(BS, T, V))
 template <int BS, int T, int V, bool WIDE, bool CHAIN = false>
 cudaError_t launch_mma(const BsrSpmmArgs &a, int sm_count, cudaStream_t s) {
   const int64_t tiles = ceil_div(a.n_rhs, 16 * T), units = a.rows / BS * tiles;
-  // Warps of a block row: more while the GPU has no more than ten per SM and each has a step, and at least one for every tile of
-  // 8 rows (16 x 16, N = 8, us with 1, 2, 4 and 8 warps: 80 block rows of 30 9.9, 7.0, 4.9, 3.9; 300 of 20 8.3, 5.4, 4.4, 4.8;
-  // 600 of 12 6.6, 4.8, 5.4, 6.1; 2,000 of 20 11.0, 11.4, 13.9, 17.5; 32 x 32, N = 48: 80 of 30 19.8 and, with four and eight, 13.6,
-  // 11.1; 1,000 of 20 23.4, 40.7, 43.0).
+  // Warps of a block row: more while the GPU has no more than ten per SM and each has a step (16 x 16, N = 8, us with 1, 2, 4 and
+  // 8 warps: 80 block rows of 30 9.9, 7.0, 4.9, 3.9; 300 of 20 8.3, 5.4, 4.4, 4.8; 600 of 12 6.6, 4.8, 5.4, 6.1; 2,000 of 20 11.0,
+  // 11.4, 13.9, 17.5).  Blocks of 32 x 32 have four tiles of rows for four adding warps, up to 20 warps per SM, and four others that
+  // only load, up to 18 (1, 4 and 8 warps: 300 of 20, N = 8 12.2, 9.7, 7.9; 80 of 30, N = 48 19.8, 13.6, 11.1; 300 of 20, N = 48
+  // 18.0, 16.6, 18.9; 382 of 27, N = 29 31.3, 20.1, -; 1,000 of 20, N = 48 23.4, 40.7, 43.0).
   int split = 1;
-  while (split < MMA_WARPS && units * split * 2 <= (int64_t)sm_count * 10 && a.nnzb * BS * BS >= split * 16 * a.rows) split *= 2;
-  if (split > 1 && split < BS / 8) split = BS / 8;
+  for (int more = BS == 32 ? 4 : 2; more <= MMA_WARPS; more *= 2)
+    if (units * more <= (int64_t)sm_count * (BS != 32 ? 10 : more == 4 ? 20 : 18) && a.nnzb * BS * BS >= more * 8 * a.rows) split = more;
   unsigned grid = 0;
   if (!grid_dim(ceil_div(units * split, MMA_WARPS), &grid)) return cudaErrorInvalidConfiguration;
   const size_t smem = split > 1 ? MMA_WARPS * team_steps(BS, T) * step_words(BS, T) * 32 * 4 : 0;  // at most 48 KB
