@@ -86,8 +86,9 @@ typedef enum swb_spmm_mapping {
  * every cooperative mapping.
  *
  * All values are checked as the reference checks them.  A mapping fixes what
- * is summed in which way (thread-per-row, thread-per-output and BSR: in
- * position order, bit for bit the sequential loop; the others: in any order);
+ * is summed in which way (thread-per-row, thread-per-output and f32 BSR: in
+ * position order, bit for bit the sequential loop; bf16 BSR: see
+ * swb_bsr_spmm_bf16; the others: in any order);
  * the kernel behind it chooses its own launch shape where that is faster, and
  * then these values have no effect on the launch:
  *   - block_size with thread-per-row; spmm_block_size with thread-per-output
@@ -100,7 +101,8 @@ typedef enum swb_spmm_mapping {
  *   - block_size with wave-per-row and block-per-row where rows are dealt to
  *     groups of lanes or to one block per SM, and spmm_block_size and
  *     spmm_tile_size with wave-per-row-tile where the tiles of a row are one
- *     pass or blocks stage their rows.
+ *     pass, blocks stage their rows or, on up to 8192 rows, teams of warps
+ *     hold them.
  * swb_launch_shape_query reports both shapes. */
 typedef struct swb_options {
   int32_t mapping;                  /* swb_spmv_mapping, default thread-per-row  */
@@ -223,9 +225,18 @@ SWB_API int swb_bsr_spmm_f32(swb_context *ctx, const swb_options *opts,
 
 /* sparsewave.bsr_spmm on bf16 blocks with f32 accumulation and bf16 output
  * (the op requires one element type, SparseWaveOps.cpp:355-360).  Values are
- * raw bf16 bit patterns.  Blocks of 16 and 32 (and of 8 from 96 columns) on aligned
- * operands with n_rhs a multiple of 8 run on the tcgen05 tensor cores, the others
- * on the thread-per-output kernel. */
+ * raw bf16 bit patterns.  Blocks of 8, 16 and 32 run on tensor cores (tcgen05
+ * or warp-level MMAs, whichever is faster), the others on CUDA cores.  f32 sums
+ * over the blocks of a block row in storage order, rounded to bf16 once:
+ *   - other block sizes: bit for bit the sequential loop;
+ *   - blocks of 8, 16 and 32: 16 products at a time (two blocks of 8 x 8, half
+ *     the local columns of a block of 32 x 32) are a sum of the tensor core,
+ *     which is added to the f32 sum, rounded to nearest;
+ *   - the same with n_rhs a multiple of 8 from 64 on (8 x 8: 96) and 16-byte
+ *     aligned block_values and B: one chain of such steps inside the tensor
+ *     core, which cuts sums off where it would have to round them.
+ * A block row's results do not depend on the other block rows of the call, so
+ * that a shard has the bits of the whole matrix where both are aligned alike. */
 SWB_API int swb_bsr_spmm_bf16(swb_context *ctx, const swb_options *opts,
                               int64_t rows, int64_t cols, int64_t nnzb,
                               int64_t block_size, int64_t n_rhs,
@@ -244,7 +255,9 @@ SWB_API int swb_bsr_spmm_bf16(swb_context *ctx, const swb_options *opts,
  * locked cannot do that.  This entry point takes no context, calls no
  * cudaMalloc / cudaFree and keeps its status words in a fixed 128 KiB array
  * inside the library image (held by every GPU that loads the library until
- * the process exits), one word per (block row, 256-column tile) pair.
+ * the process exits), one word per (block row, 256-column tile) pair.  Its
+ * results have the bits of swb_bsr_spmm_bf16; small calls run on its kernel
+ * with warp-level MMAs, which never waits.
  *   - Limit: (rows / 16) * ceil(n_rhs / 256) <= 32768, else SWB_ERR_CAPACITY.
  *   - Needs nnzb > 0, n_rhs % 8 == 0 and 16-byte aligned block_values and B,
  *     else SWB_ERR_UNSUPPORTED (there is no second kernel behind it).
@@ -327,8 +340,8 @@ SWB_API int swb_spmm_resident_host(swb_context *ctx, const swb_options *opts,
 /* The same for a bf16 BSR matrix: swb_bsr_upload checks the block structure on
  * the host (offsets start at 0, are monotone and end at nnzb; block columns in
  * range) and copies it to the device once; swb_bsr_spmm_bf16_resident_host
- * copies B (cols x n_rhs bf16) in, runs the BSR SpMM (the tensor-core kernel
- * for 16 x 16 blocks), copies C (rows x n_rhs bf16) out and synchronises. */
+ * copies B (cols x n_rhs bf16) in, runs the BSR SpMM (swb_bsr_spmm_bf16),
+ * copies C (rows x n_rhs bf16) out and synchronises. */
 typedef struct swb_bsr_handle swb_bsr_handle;
 SWB_API int swb_bsr_upload(swb_context *ctx, int64_t rows, int64_t cols,
                            int64_t nnzb, int64_t block_size,

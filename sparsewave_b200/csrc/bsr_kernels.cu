@@ -6,10 +6,11 @@
 // A thread holds TR rows of one block row and V adjacent columns: a value of B serves TR outputs and a value of a block V
 // of them, where one thread per output reads both for every product.  Every output is still added up in the reference's
 // order, bit for bit.  Block values are the same for all threads of a block row (one L1 access per load), rows of B are
-// read V columns at a time.  With products and sums separate instructions the floor of 4 x 4 blocks is the FP32 pipe,
-// then the gather of slabs of B from L2.  4 x 4 f32 blocks, 16,384 block rows of 24, N = 32: 180 -> 43 us (11 us of FP32
-// pipe, 18 us of L2); 8 x 8, 8,192 block rows of 12, N = 64: 304 -> 70 us; 32 x 32 bf16, N = 64: 740 -> 245 us.  f32 blocks of 4 x 4
-// and 8 x 8 with enough outputs go on to groups of lanes (bsr_rows.cuh).
+// read V columns at a time.  With products and sums separate instructions the bound is the FP32 pipe (19 T products and sums a
+// second), then the gather of slabs of B from L2: f32, 32,768 block rows of 24 blocks of 2 x 2, N = 32 23.3 us (201 M products: 10.6
+// us of FP32 pipe); 4,096 of 20 of 16 x 16, N = 64 218 us (1.34 G: 71); bf16, 16,384 of 24 of 4 x 4, N = 32 43.5 us (180 with one
+// output per thread; f32 alike).  f32 blocks of 4 x 4 and 8 x 8 with enough outputs go on to groups of lanes (bsr_rows.cuh), bf16
+// blocks of 8, 16 and 32 to tensor cores.
 #include <cuda_bf16.h>
 
 #include "swb_chain.cuh"

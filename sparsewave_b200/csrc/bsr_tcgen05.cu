@@ -33,12 +33,13 @@
 // and lets tcgen05.commit arrive on `empty`.  There are two sets of accumulators: while warps 0 - 3 read one with tcgen05.ld,
 // round to bf16 and store C, the MMAs of the next unit fill the other.
 //
-// What bounds it is the path from L2 (13 TB/s of slabs and blocks), and below that the fixed cost of a step: a stage with one
-// MMA takes its thread some 500 clocks and its copies 300 (wait, arrive, issue, commit), whatever its size.  Hence groups,
-// several copying warps and persistence: with one block per stage, one copying thread and a CTA per unit, 3,419 block rows of
-// 8, N = 128 took 29.6 us (now 19.0), 847 of 16, N = 256 20.0 (15.2), 128 of 32, N = 512 21.3 (12.2), 1,024 of 51, N = 512
-// 63.4 (59.4).  Tried: a CTA per unit with these stages (65.8 on the last), 1 or 2 CTAs per SM with deeper rings (142, 77),
-// two chains of accumulators (no change).
+// What bounds it: no unit is at its limit on 1,024 block rows of 51, N = 512 (ncu, 64 us: 913 MB from L2 at 14.2 TB/s, which keeps
+// L2's ports to the crossbar busy 61 % of the time and the SMs' intake 41 %; shared memory read by the tensor cores 44 %, tensor
+// pipe 10 %, HBM 9 %).  The CTAs wait for their copies, and beside them pay the fixed cost of a step: a stage with one MMA takes its
+// thread some 500 clocks and its copies 300 (wait, arrive, issue, commit), whatever its size.  Hence groups, several copying
+// warps and persistence: with one block per stage, one copying thread and a CTA per unit, 3,419 block rows of 8, N = 128 took 29.6
+// us (now 19.0), 847 of 16, N = 256 20.0 (15.2), 128 of 32, N = 512 21.3 (12.2), 1,024 of 51, N = 512 65.6 (61.8).  Tried: a CTA per
+// unit with these stages (68 on the last), 1 or 2 CTAs per SM with deeper rings (142, 77), two chains of accumulators (no change).
 //
 // Every mbarrier wait is bounded: when one runs out the kernel raises the
 // status word, frees its TMEM columns and returns.

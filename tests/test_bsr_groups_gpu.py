@@ -5,6 +5,7 @@ import torch
 
 import oracle
 from sparsewave_b200 import workloads as W
+from tests.helpers import launched
 
 pytestmark = pytest.mark.gpu
 
@@ -31,3 +32,21 @@ def test_groups(ctx, bs, brows, n):
         Bd = torch.empty(B.numel() + off, device="cuda")[off:].view(B.shape).copy_(B)
         C = ctx.bsr_spmm("", brp.cuda(), bci.cuda(), v, Bd, bs).cpu().numpy().view(np.int32)
         assert np.array_equal(C, expected)
+
+
+@pytest.mark.parametrize("bs,n", [(4, 128), (8, 64)])
+def test_b_of_four_gib_and_more(ctx, bs, n):
+    """Whole numbers, so that every sum is exact: block columns on both sides of 4 GiB, aligned values and B."""
+    cols, brows = (1 << 30) // (bs * n) + 100, 2400
+    gen = torch.Generator("cuda").manual_seed(bs)
+    B = torch.empty((cols * bs, n), device="cuda").random_(-8, 9, generator=gen)
+    brp = torch.arange(0, 3 * brows + 1, 3, dtype=torch.int32, device="cuda")
+    bci = torch.randint(cols, (brows, 3), generator=gen, dtype=torch.int32, device="cuda")
+    bci[:, 2] = cols - 1 - torch.arange(brows, device="cuda", dtype=torch.int32) % 90
+    values = torch.randint(-8, 9, (brows, 3, bs, bs), generator=gen, device="cuda").float()
+    C, names = launched(lambda: ctx.bsr_spmm("", brp, bci.reshape(-1), values.reshape(-1), B, bs))
+    if names is not None:
+        assert len(names) == 1 and names[0].startswith(f"bsr_spmm_row_group_kernel<{bs}, ") and names[0].endswith("true, unsigned long>")
+    slabs = B.view(cols, bs, n)[bci.long()]
+    want = torch.einsum("bprk,bpkn->brn", values.double(), slabs.double()).float()
+    assert torch.equal(C.view(brows, bs, n), want)
