@@ -34,3 +34,26 @@ def test_few_rows(ctx, rows, mean, n, tiles, warps):
     C = torch.ones((rows, n), device="cuda")
     ctx.spmm(OPTIONS + " accumulate=1", *a, torch.from_numpy(B).cuda(), C)
     assert np.all(np.abs(C.cpu().numpy() - want - 1) <= 901 * 2**-23 * (bound + 1))
+
+
+@pytest.mark.parametrize("rows,mean,n,tiles,warps", [
+    (2500, 5, 19, 1, 2), (6001, 7, 9, 1, 1), (1025, 2, 511, 16, 1),  # one column per lane
+    (2500, 6, 50, 1, 2), (5000, 12, 50, 1, 2), (3000, 31, 130, 3, 2),  # two
+    (5000, 3, 12, 1, 1), (2500, 26, 100, 1, 4), (3500, 40, 12, 1, 2), (3001, 26, 36, 1, 4)])  # four, the last in small blocks
+def test_rows_far_longer_than_the_others(ctx, rows, mean, n, tiles, warps):
+    """A whole block takes them: alone and several in a share of 128 rows, in the first and the last one."""
+    rng = np.random.default_rng(rows + n)
+    lens = np.minimum(rng.geometric(1 / (mean + 1), rows) - 1, 10 * mean)
+    lens[[0, 3, 126, 400, rows - 1]] = 2500, 0, 3100, 5003, 2777
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = rng.integers(0, 1200, rp[-1]).astype(np.int32)
+    v = rng.uniform(-1, 1, rp[-1]).astype(np.float32)
+    B = rng.uniform(-1, 1, (1200, n)).astype(np.float32)
+    want, bound = oracle.csr_spmm(rp, ci, v, B, parallel=True), oracle.csr_abs_bound(rp, ci, v, B)
+    assert ctx.launch_shape(OPTIONS, rows, int(rp[-1]), n).physical_grid == -(-rows * tiles // (8 // warps))
+    a = [torch.from_numpy(t).cuda() for t in (rp, ci, v, B)]
+    C = ctx.spmm(OPTIONS, *a)
+    assert np.all(np.abs(C.cpu().numpy() - want) <= 5003 * 2**-23 * bound + 1e-30)  # either order of up to 5,003 terms
+    C = torch.ones((rows, n), device="cuda")
+    ctx.spmm(OPTIONS + " accumulate=1", *a, C)
+    assert np.all(np.abs(C.cpu().numpy() - want - 1) <= 5004 * 2**-23 * (bound + 1))
