@@ -28,9 +28,9 @@
 //     Both accumulators' MMAs read the same copy.
 //
 // Pipeline.  Persistent CTAs, three (256 columns) to five per SM, walk the units.  A stage holds a group of four 16 x 16
-// blocks (two of 32 x 32, one with 256 columns; eight of 8 x 8) with their slabs.  Lanes 0 of warps 4 - 7 copy: each takes its blocks of every
-// group, block columns held 32 at a time in the warp's lanes and requested ahead.  Lane 0 of warp 8 issues the group's MMAs
-// and lets tcgen05.commit arrive on `empty`.  There are two sets of accumulators: while warps 0 - 3 read one with tcgen05.ld,
+// blocks (two of 32 x 32, one with 256 columns; eight of 8 x 8) with their slabs.  Lanes 0 of warps 4 - 7 copy: each takes its
+// blocks of every group, block columns held 32 at a time in the warp's lanes and requested ahead.  Lane 0 of warp 8 issues the
+// group's MMAs and lets tcgen05.commit arrive on `empty`.  There are two sets of accumulators: while warps 0 - 3 read one with tcgen05.ld,
 // round to bf16 and store C, the MMAs of the next unit fill the other.
 //
 // What bounds it: no unit is at its limit on 1,024 block rows of 51, N = 512 (ncu, 64 us: 913 MB from L2 at 14.2 TB/s, which keeps
@@ -92,10 +92,11 @@ constexpr int most_stages() {
 }
 // CTAs per SM, and the stages of each: the shared memory of an SM shared out among the CTAs that run on it.  More CTAs gain
 // more than more stages each (1,024 x 1,024 16 x 16 blocks at 5 %, N = 512: one CTA of six stages 142 us, two of three 77,
-// three of two 59); their accumulators fit the 512 columns of TMEM.
+// three of two 59; 32 x 32, 700 block rows of 24, N = 192, two stages each: four CTAs 30.7, five 26.3); their accumulators fit the
+// 512 columns of TMEM, their registers the SM's.
 template <int BS, int HALVES>
 int ctas_per_sm(int64_t units, int sm_count, int *stages) {
-  constexpr int MOST = BS == 32 ? 4 : HALVES == 2 ? 3 : 5;
+  constexpr int MOST = HALVES == 1 ? 5 : BS == 32 ? 4 : 3;
   static_assert(MOST * Shape<BS, HALVES>::TMEM_COLS <= 512 && 222 * 1024 / MOST - 1024 >= 2 * Shape<BS, HALVES>::STAGE_BYTES, "");
   int64_t per_sm = (units + sm_count - 1) / sm_count;
   if (per_sm > MOST) per_sm = MOST;
@@ -166,7 +167,7 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
 
 // PER_UNIT_STATUS: raise status[unit] instead of status[0] when a wait gives up.
 template <bool PER_UNIT_STATUS, int BS, int HALVES>
-__global__ void __launch_bounds__(THREADS) bsr_spmm_tcgen05_kernel(
+__global__ void __launch_bounds__(THREADS, HALVES == 1 ? 5 : 3) bsr_spmm_tcgen05_kernel(
     const __grid_constant__ CUtensorMap map_slab, const __grid_constant__ CUtensorMap map_box,
     const __grid_constant__ CUtensorMap map_block, const __grid_constant__ CUtensorMap map_group, int64_t units, int64_t n_tiles,
     int64_t N, int cols, int value_rows, int stages, const int32_t *__restrict__ brp, const int32_t *__restrict__ bci,
@@ -363,33 +364,32 @@ __global__ void __launch_bounds__(THREADS) bsr_spmm_tcgen05_kernel(
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       }
-      // TMEM lane m of accumulator h = column n0 + 128 h + m of C; this warp reads lanes 32 warp .. +32
-      // (two accumulators of 32 columns after one another, for registers that leave room for three CTAs).
-      constexpr int ROWS = BS < 16 ? 16 : BS, AT_ONCE = BS == 32 ? 1 : HALVES;
+      // TMEM lane m of accumulator h = column n0 + 128 h + m of C; this warp reads lanes 32 warp .. +32 (16 rows of a 32 x 32 block
+      // at a time, for registers that leave room for five CTAs).
+      constexpr int AT_ONCE = BS == 32 ? 1 : HALVES, PARTS = BS == 32 ? 2 * HALVES : 1;
+#pragma unroll(HALVES == 1 ? 1 : PARTS)
+      for (int part = 0; part < PARTS; ++part) {
+        const int h0 = BS == 32 ? part / 2 : 0, r0 = BS == 32 ? part % 2 * 16 : 0;
+        uint32_t v[AT_ONCE][16];
 #pragma unroll
-      for (int h0 = 0; h0 < HALVES; h0 += AT_ONCE) {
-        uint32_t v[AT_ONCE][ROWS];
+        for (int h = 0; h < AT_ONCE; ++h) {
+          uint32_t *w = v[h];
+          if (empty || h0 + h >= halves) {
 #pragma unroll
-        for (int h = 0; h < AT_ONCE; ++h)
-#pragma unroll
-          for (int r0 = 0; r0 < ROWS; r0 += 16) {
-            uint32_t *w = &v[h][r0];
-            if (empty || h0 + h >= halves) {
-#pragma unroll
-              for (int r = 0; r < 16; ++r) w[r] = 0;
-            } else {
-              asm volatile(
-                  "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-                  "%15}, [%16];"
-                  : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]),
-                    "=r"(w[8]), "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
-                  : "r"(sums + (uint32_t)((h0 + h) * S::MMA_N + r0))
-                  : "memory");
-            }
+            for (int r = 0; r < 16; ++r) w[r] = 0;
+          } else {
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+                "%15}, [%16];"
+                : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]),
+                  "=r"(w[8]), "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
+                : "r"(sums + (uint32_t)((h0 + h) * S::MMA_N + r0))
+                : "memory");
           }
+        }
         if (!empty) {
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (h0 + AT_ONCE == HALVES) {
+          if (part == PARTS - 1) {
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             if (lane == 0)
               asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_stored[made & 1])) : "memory");
@@ -400,9 +400,9 @@ __global__ void __launch_bounds__(THREADS) bsr_spmm_tcgen05_kernel(
         for (int h = 0; h < AT_ONCE; ++h) {
           const int64_t col = (int64_t)n0 + (h0 + h) * HALF_N + warp * 32 + lane;
           if (col < N) {
-            __nv_bfloat16 *out = C + br * BS * N + col;
+            __nv_bfloat16 *out = C + (br * BS + r0) * N + col;
 #pragma unroll
-            for (int r = 0; r < BS; ++r) out[r * N] = __float2bfloat16_rn(__uint_as_float(v[h][r]));
+            for (int r = 0; r < (BS < 16 ? BS : 16); ++r) out[r * N] = __float2bfloat16_rn(__uint_as_float(v[h][r]));
           }
         }
       }
@@ -558,11 +558,13 @@ template <bool PER_UNIT_STATUS, int BS>
 cudaError_t launch_tcgen05(const BsrSpmmArgs &a, int *status, int sm_count, cudaStream_t s) {
   // Tiles of 256 columns fetch a block once for two accumulators; tiles of 128 where the second would be empty or nearly so,
   // and where 256 leave too few units (403 block rows of 9, N = 480: 13.2 us with 256, 12.4 with 128; 1,024 of 51, N = 512:
-  // 59 and 64).  32 x 32 has one block per stage with 256, which only many whole tiles make up for (us with 128 and 256: 2,000
-  // block rows of 30, N = 512 157, 134; 900 of 20 56.8, 50.5; 2,000 of 6, N = 192 26.0, 22.4; but 700 of 20, N = 512 41.9, 44.8;
-  // 2,000 of 30, N = 384 115, 123, N = 200 115, 120).  The status words of the static entry point are per 256 columns.
+  // 59 and 64).  32 x 32 has one block per stage with 256, which only many whole tiles of short block rows make up for (us with
+  // 128 and 256: 1,500 block rows of 4, N = 512 32.3, 28.2; 2,000 of 4, N = 192 23.1, 20.9; but 700 of 20, N = 512 40.0, 41.8;
+  // 2,000 of 20, N = 256 56.9, 59.6), or very many of any (3,000 of 20, N = 448 161, 146; but 1,200 of 20 60.9, 63.5).  The status
+  // words of the static entry point are per 256 columns.
   const int64_t n = a.n_rhs, pairs = a.rows / BS * ceil_div(n, 2 * HALF_N), tail = n % (2 * HALF_N);
-  const bool narrow = BS == 32 ? n % 64 != 0 || (tail > 0 && tail < 192) || pairs < 10 * (int64_t)sm_count
+  const int64_t many = a.nnzb < 8 * (a.rows / BS) ? 10 : 20;
+  const bool narrow = BS == 32 ? n % 64 != 0 || (tail > 0 && tail < 192) || pairs < many * sm_count
                                : n <= HALF_N || (tail > 0 && tail <= 64) || pairs < 6 * (int64_t)sm_count;
   if constexpr (!PER_UNIT_STATUS)
     if (narrow) return launch_halves<PER_UNIT_STATUS, BS, 1>(a, status, sm_count, s);
@@ -599,8 +601,8 @@ cudaError_t launch_bsr_spmm_tcgen05(const BsrSpmmArgs &a, int *status_flag, cons
 // which is part of the library image: every GPU that loads the library holds
 // its 128 KiB until the process exits, whether or not this entry point is used.
 //
-// One status word per CTA (block row x tile of 256 columns), hence the limit
-// of SWB_STATIC_MAX_CTAS CTAs per call.  All calls share the array and a call
+// One status word per unit (block row x tile of 256 columns), hence the limit
+// of SWB_STATIC_MAX_CTAS units per call.  All calls share the array and a call
 // begins by clearing the words it will use, so the array holds the outcome of
 // the most recent call only, and two calls that overlap on the GPU (different
 // streams) race on it.

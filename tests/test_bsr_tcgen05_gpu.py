@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 # block size, 128-column accumulators per tile, block rows, columns
 INSTANTIATIONS = [(8, 1, 310, 128), (8, 2, 930, 256), (16, 1, 310, 128), (16, 1, 170, 320), (16, 2, 930, 256), (16, 2, 640, 488),
-                  (32, 1, 310, 128), (32, 1, 90, 112), (32, 2, 1500, 256)]
+                  (32, 1, 310, 128), (32, 1, 90, 112), (32, 2, 1500, 512)]
 
 
 def _ran(names, kernel):
