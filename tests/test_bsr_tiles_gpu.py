@@ -1,4 +1,5 @@
-"""BSR thread-per-output kernel: tiles of rows and columns per thread, bit-exact in f32, the oracle's bits in bf16."""
+"""BSR thread-per-output kernel: tiles of rows and columns per thread, bit-exact in f32, the oracle's bits in bf16 (of which blocks
+of 8 and 16 run on warp-level MMAs)."""
 import numpy as np
 import pytest
 import torch
@@ -16,7 +17,7 @@ def test_row_tiles(ctx, bs, n):
     rows, cols = (40, 23) if n < 64 else (400, 23)  # few threads: narrow columns; many: the widest
     for dtype in (torch.float32, torch.bfloat16):
         if bs == 16 and n % 8 == 0 and dtype == torch.bfloat16:
-            continue  # the tensor-core kernel
+            continue  # aligned operands of the tensor-core kernels have tests of their own
         a = W.random_bsr(rows, cols, bs, 0.2, seed=bs * 100 + n, dtype=dtype)
         B = W.dense_normal((cols * bs, n), seed=n, dtype=dtype)
         h = (a.block_row_ptr.numpy(), a.block_col_idx.numpy())

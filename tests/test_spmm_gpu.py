@@ -165,13 +165,13 @@ def _bsr_bf16_case(ctx, grid_rows, grid_cols, bs, n, density, seed):
 @pytest.mark.parametrize("bs", [4, 8, 16, 32])
 def test_bsr_bf16(ctx, bs):
     _bsr_bf16_case(ctx, 24, 20, bs, 24, 0.25, seed=bs)
-    if bs != 16:  # (16 is the tensor-core kernel) rows shared by a warp
+    if bs != 16:  # more columns
         _bsr_bf16_case(ctx, 24, 20, bs, 64, 0.25, seed=bs + 1)
 
 
 @pytest.mark.parametrize("n", [8, 64, 128, 200, 512])
 def test_bsr16_bf16_shapes(ctx, n):
-    """16 x 16 blocks (the tensor-core path), with empty block rows and ragged N."""
+    """16 x 16 blocks on few block rows (warp-level MMAs), with empty ones and ragged N."""
     _bsr_bf16_case(ctx, 48, 40, 16, n, 0.08, seed=n)
 
 
