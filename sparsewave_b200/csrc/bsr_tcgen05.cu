@@ -493,11 +493,15 @@ bool bsr_tcgen05_supported(const BsrSpmmArgs &a) {
 //   less than a unit per SM too (80 of 24, N = 128 17.2, 11.8; of 6, N = 104 5.9, 6.5).
 //   16 x 16: whole groups of 64 columns from 128 on whatever the rows' length (300 of 6, N = 128 6.9, 5.9; 1,200 of 30, N = 256
 //   53.9, 26.9; but 80 of 6, N = 128 3.2, 4.4; 600 of 6, N = 192 8.5, 9.3); others from 8 blocks a row on (1,200 of 12, N = 160
-//   19.1, 16.7; of 5 10.9, 11.7), with rows of B that are no multiple of 32 bytes from 12 (150 of 40, N = 136 16.0, 11.1; 600 of 24
-//   16.7, 18.5; 1,200 of 30 32.0, 31.7); 64 columns from 12 a row and two units per SM on (300 of 24 10.5, 8.7; 150 of 12 4.5, 6.0).
+//   19.1, 16.7; of 5 10.9, 11.7), from 6 where the tiles are four fifths full (3,605 of 7, N = 416 83.4, 50.0; 540 of 7 14.8, 11.8;
+//   1,592 of 6, N = 224 17.4, 15.3; but of 5, N = 432 1.15 times), with rows of B that are no multiple of 32 bytes from 12 (150 of
+//   40, N = 136 16.0, 11.1; 600 of 24 16.7, 18.5; 1,200 of 30 32.0, 31.7); 64 columns from 12 a row and two units per SM on (300 of
+//   24 10.5, 8.7; 150 of 12 4.5, 6.0).
 //   8 x 8, half of whose MMA is padding: whole groups of 64 columns from 128 on and rows of 20 blocks (300 of 24, N = 256 11.1, 8.8,
-//   N = 192 8.2, 9.2; 1,200 of 30, N = 128 20.7, 12.6; but 2,500 of 20, N = 264 33.2, 43.3), or many units of whole tiles (5,000
-//   of 8, N = 512 78.1, 48.3; 1,200 of 12, N = 256 14.1, 11.9; 600 of 6 6.4, 8.3).
+//   N = 192 8.2, 9.2; 1,200 of 30, N = 128 20.7, 12.6; but 2,500 of 20, N = 264 33.2, 43.3), or many units: of whole tiles (5,000 of
+//   8, N = 512 78.1, 48.3; 1,200 of 12, N = 256 14.1, 11.9; 600 of 6 6.4, 8.3); of tiles four fifths full, from 12 a row with whole
+//   groups (2,904 of 15, N = 448 52.5, 39.4; but of 9, N = 384 1.08 times), from 27 with other multiples of 32 bytes (3,350 of 48,
+//   N = 240 91.5, 73.6; 2,002 of 54, N = 416 105, 90; 311 of 28, N = 496 16.7, 14.2; but of 18, N = 304 1.12 times).
 bool bsr_tcgen05_pays(const BsrSpmmArgs &a, int sm_count) {
   const int64_t n = a.n_rhs, brows = a.rows / a.block_size, units = brows * ceil_div(n, HALF_N);
   if (!bsr_chain_sums(a) || !bsr_tcgen05_supported(a) || brows == 0) return false;
@@ -506,8 +510,11 @@ bool bsr_tcgen05_pays(const BsrSpmmArgs &a, int sm_count) {
   if (units < sm_count) return false;
   const int64_t mean = a.nnzb / brows;
   const bool groups = n >= HALF_N && n % 64 == 0;
-  if (a.block_size == 8) return groups && (mean >= 20 || (mean >= 8 && n % (2 * HALF_N) == 0 && units >= 8 * (int64_t)sm_count));
-  if (groups) return true;
+  const bool full = 5 * n * brows >= 4 * HALF_N * units && n % 16 == 0;
+  if (a.block_size == 8)
+    return (groups && mean >= 20) ||
+           (units >= 8 * (int64_t)sm_count && full && mean >= (n % (2 * HALF_N) == 0 ? 8 : groups ? 12 : 27));
+  if (groups || (full && n > HALF_N && mean >= 6)) return true;
   if (n < 72) return mean >= 12 && units >= 2 * (int64_t)sm_count;
   return mean >= (n > HALF_N && n % 16 != 0 ? 12 : 8);
 }

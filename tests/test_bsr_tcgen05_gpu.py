@@ -135,7 +135,10 @@ def test_static_entry_point(ctx, sizes):
                                                   (16, 2, 12, 64, True), (16, 1.99, 12, 64, False), (16, 2, 11, 64, False),
                                                   (16, 1, 12, 136, True), (16, 1, 11, 136, False), (16, 1, 8, 144, True),
                                                   (16, 3, 30, 56, False), (8, 1, 20, 128, True), (8, 1, 19, 128, False),
-                                                  (8, 4, 8, 256, True), (8, 3.99, 8, 256, False), (8, 9, 8, 384, False), (8, 1, 20, 136, False)])
+                                                  (8, 4, 8, 256, True), (8, 3.99, 8, 256, False), (8, 9, 8, 384, False), (8, 1, 20, 136, False),
+                                                  (16, 1, 6, 208, True), (16, 1, 5, 208, False), (16, 1, 6, 192 + 8, False),
+                                                  (8, 2, 12, 448, True), (8, 2, 11, 448, False), (8, 1.99, 12, 448, False),
+                                                  (8, 4, 27, 208, True), (8, 4, 26, 208, False), (8, 3.99, 27, 208, False)])
 def test_line_between_the_kernels(ctx, bs, per_sm, per, n, here):
     """Both sides of each limit: block rows per SM, blocks per block row and columns."""
     brows = int(per_sm * torch.cuda.get_device_properties(0).multi_processor_count)
