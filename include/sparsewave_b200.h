@@ -229,12 +229,13 @@ SWB_API int swb_bsr_spmm_f32(swb_context *ctx, const swb_options *opts,
  * or warp-level MMAs, whichever is faster), the others on CUDA cores.  f32 sums
  * over the blocks of a block row in storage order, rounded to bf16 once:
  *   - other block sizes: bit for bit the sequential loop;
- *   - blocks of 8, 16 and 32: 16 products at a time (two blocks of 8 x 8, half
- *     the local columns of a block of 32 x 32) are a sum of the tensor core,
- *     which is added to the f32 sum, rounded to nearest;
+ *   - blocks of 8, 16 and 32: 16 products at a time (two blocks of 8 x 8, a
+ *     block of 16 x 16), or two, four or eight blocks of 32 x 32 (of a block row
+ *     of up to 16, 64 or more), are a sum of the tensor core, which is added to
+ *     the f32 sum, rounded to nearest;
  *   - the same with n_rhs a multiple of 8 from 64 on (8 x 8: 96) and 16-byte
- *     aligned block_values and B: one chain of such steps inside the tensor
- *     core, which cuts sums off where it would have to round them.
+ *     aligned block_values and B: one chain inside the tensor core, which cuts
+ *     sums off where it would have to round them.
  * A block row's results do not depend on the other block rows of the call, so
  * that a shard has the bits of the whole matrix where both are aligned alike. */
 SWB_API int swb_bsr_spmm_bf16(swb_context *ctx, const swb_options *opts,

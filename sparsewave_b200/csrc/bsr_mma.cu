@@ -9,19 +9,23 @@
 // load of up to 16 bytes, and its results are adjacent columns of C.  Pairs of rows of B are interleaved by byte permutes.
 // The next steps' loads are in flight during this step's MMAs, block columns are held 32 at a time by the warp's lanes.
 //
-// Every output is added up over its block row's steps in storage order, as one chain of MMAs or (bsr_chain_sums) as f32 sums of
-// steps, so that a part of a matrix has the bits of the whole, whichever kernel takes either.  Where block rows are few, a team
-// of up to eight warps shares one all the same: its members load the steps in turn and hand them over in shared memory, and each
-// of the first members adds up its share of the block row's rows.
+// Every output is added up over its block row's steps in storage order, so that a part of a matrix has the bits of the whole,
+// whichever kernel takes either: as one chain of MMAs or (bsr_chain_sums) as f32 sums of steps or, 32 x 32 blocks, of segments of
+// two, four or eight blocks by the block row's length, each of which is a chain of its own.  Where block rows are few, a team of up to
+// eight warps shares one all the same.  Its members take segments in turn and add up each other's sums, in order, for their tiles of
+// 8 rows; or they load the steps in turn and hand them over in shared memory, and each of the first members adds up its share of
+// the block row's rows.
 //
 // What bounds it: launch and latency on small calls, L1 on large ones (eight lanes of a load touch four lines, some 64 lookups
 // for 2 KB of B; ncu: L1 data pipe 67 %, tensor pipe 18 % on 1,024 block rows of 51, N = 512), which bsr_tcgen05.cu then takes.
 // Tried: the same loads through a ring in shared memory (178 us against 134 on that size).  Before, on the CUDA cores or with
-// tcgen05 at any size: 123 block rows of 61 blocks of 32 x 32, N = 2 132 -> 12.0 us; 382 of 27, N = 29 105 -> 19.9; 1,438 of 15
-// blocks of 8 x 8, N = 80 30.0 -> 10.0; 90 of 36 blocks of 16 x 16, N = 88 17.5 -> 7.9.  Sums in storage order have
-// their price where few warps have much to add up: a block row in parts with sums of their own, added up at the end, took 5.8,
-// 12.1, 10.4 and 5.8 us.  Tried for teams: two rounds' loads in flight (spills; 1.09 times the time over 170 sizes), a barrier per
-// step (1.13), sums of steps handed over in place of operands (1.00 to 1.2).
+// tcgen05 at any size: 123 block rows of 61 blocks of 32 x 32, N = 2 138 -> 7.6 us; 382 of 27, N = 29 109 -> 15.9; 1,438 of 15
+// blocks of 8 x 8, N = 80 30.0 -> 10.0; 90 of 36 blocks of 16 x 16, N = 88 17.5 -> 7.9.  A fixed order of sums has its price
+// where few warps have much to add up: a block row in as many parts as there are warps, added up at the end, took 5.8, 12.8, 10.4
+// and 5.8 us.  With operands handed over the two sizes of 32 x 32 took 11.7 and 20.4, and 107 of 1 to 63 and odd numbers of columns
+// 1.19 times the time of segments.  Segments for the smaller blocks too: 1.06 and 1.04 times the time (8 x 8, 16 x 16; where a
+// warp has whole block rows 1.09 and 1.14).  Tried for teams that hand over operands: two rounds' loads in flight (spills; 1.09
+// times the time over 170 sizes), a barrier per step (1.13), sums of steps in place of operands (1.00 to 1.2).
 #include <cuda_bf16.h>
 
 #include "swb_chain.cuh"
@@ -136,20 +140,18 @@ __device__ __forceinline__ void add_step(float (&sum)[4], const uint32_t (&a)[4]
 }
 
 // V: elements per load of a row of B, or 0: N is odd and B starts at a word, so that rows in turn start at a word and in the
-// middle of one.  WIDE: block values are aligned for loads of a lane's four.  TEAM: several warps share a unit, 2, 4 or 8 but
+// middle of one.  WIDE: block values are aligned for loads of a lane's share of a row.  TEAM: several warps share a unit, 2, 4 or 8 but
 // no fewer than there are tiles of 8 rows in a block.
 template <int BS, int T, int V, bool WIDE, bool TEAM, bool CHAIN>
-__global__ void __launch_bounds__(32 * MMA_WARPS, TEAM ? 2 : mma_ctas(BS, T, V))
-    bsr_spmm_mma_kernel(int64_t units, int tiles, int team_warps, int64_t N, const int32_t *__restrict__ brp,
-                        const int32_t *__restrict__ bci, const __nv_bfloat16 *__restrict__ bv,
-                        const __nv_bfloat16 *__restrict__ B, __nv_bfloat16 *__restrict__ C) {
+__device__ __forceinline__ void add_in_order(int64_t units, int tiles, int team_warps, int64_t N, const int32_t *__restrict__ brp,
+                                             const int32_t *__restrict__ bci, const __nv_bfloat16 *__restrict__ bv,
+                                             const __nv_bfloat16 *__restrict__ B, __nv_bfloat16 *__restrict__ C) {
   constexpr int H = BS == 32 && !TEAM ? 2 : 1;
   using F = Fragments<BS, T, V, H>;
   // Steps of this kernel per two blocks, and those whose block columns the warp holds.
   constexpr int PER_TWO = BS == 8 ? 1 : BS == 16 || H == 2 ? 2 : 4, BATCH = 16 * PER_TWO;
   constexpr int DEPTH = TEAM ? team_steps(BS, T) : mma_depth(BS, T);
   constexpr int WORDS = step_words(BS, T);
-  after_previous_kernel();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
   const int split = TEAM ? team_warps : 1, team = warp / split, member = warp % split;
   const int64_t unit = (int64_t)blockIdx.x * (MMA_WARPS / split) + team;
@@ -298,20 +300,221 @@ __global__ void __launch_bounds__(32 * MMA_WARPS, TEAM ? 2 : mma_ctas(BS, T, V))
   }
 }
 
+// 32 x 32 blocks as sums of segments.  A step is a block, of which lane (g, q) takes local columns 8 q .. 8 q + 7.
+template <int T, int V>
+struct SegmentFragments {
+  uint32_t slab[8][T + (V == 0)];  // eight rows of B, 2 T adjacent columns each (V = 0: the words that hold them)
+  uint32_t block[4][4];            // block row 8 u + g, eight local columns
+};
+// Blocks of a segment: by the block row's length alone.  A chain of L MMAs is off by some 1.5e-8 L of its size, sums rounded one by
+// one by 8e-9 times the root of their number, hence longer segments on longer rows only.
+__device__ __forceinline__ int segment_log2_length(int blocks) { return blocks <= 16 ? 1 : blocks <= 64 ? 2 : 3; }
+// Tiles of 8 rows whose sums a warp adds up, and whether it does so in registers.
+constexpr int share_of_sums(bool team) { return team ? 2 : 4; }
+constexpr bool sums_in_registers(int T) { return T == 1; }
+// Segments that a member of a team sums before they are handed over, and shared memory, of which the default 48 KB are the limit.
+constexpr int segments_at_once(int T) { return T == 1 ? 3 : 1; }
+constexpr int segment_smem(int T, bool team) {
+  return MMA_WARPS * T * 512 * ((sums_in_registers(T) ? 0 : share_of_sums(team)) + (team ? 4 * segments_at_once(T) : 0));
+}
+__device__ __forceinline__ void add4(float4 &a, const float4 &b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+
+template <int T, int V, bool WIDE, bool TEAM>
+__device__ __forceinline__ void add_in_segments(int64_t units, int tiles, int team_warps, int64_t N,
+                                                const int32_t *__restrict__ brp, const int32_t *__restrict__ bci,
+                                                const __nv_bfloat16 *__restrict__ bv, const __nv_bfloat16 *__restrict__ B,
+                                                __nv_bfloat16 *__restrict__ C) {
+  using F = SegmentFragments<T, V>;
+  constexpr int BS = 32, TILES = BS / 8;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+  const int split = TEAM ? team_warps : 1, team = warp / split, member = warp % split;
+  const int64_t unit = (int64_t)blockIdx.x * (MMA_WARPS / split) + team;
+  const bool active = unit < units;
+  const int64_t brow = active ? unit / tiles : 0;
+  const int64_t col0 = (active ? unit - brow * tiles : 0) * (16 * T) + g * (2 * T);
+  const int valid = N - col0 >= 2 * T ? 2 * T : N > col0 ? (int)(N - col0) : 0;
+  int start = 0, end = 0;
+  if (active) {
+    start = brp[brow];
+    end = brp[brow + 1];
+  }
+  const int steps = end - start;
+  const int log2_length = segment_log2_length(steps), length = 1 << log2_length;
+  const int segments = (steps + length - 1) >> log2_length;
+  auto own = [&](int j) { return ((((j >> log2_length) * split) + member) << log2_length) | (j & (length - 1)); };  // the j-th step
+
+  float acc[TILES][T][4];  // the segment's sums
+#pragma unroll
+  for (int u = 0; u < TILES; ++u)
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[u][t][i] = 0.0f;
+  // The block row's: all of its rows, or a team member's share of the tiles of 8 rows.  In registers, where there are any left.
+  constexpr int SUMS = share_of_sums(TEAM);
+  constexpr bool KEPT = sums_in_registers(T);
+  extern __shared__ __align__(16) uint4 handed[];
+  float4 *shared_sums = reinterpret_cast<float4 *>(handed) + warp * (SUMS * T * 32) + lane;
+  float4 sum[KEPT ? SUMS : 1][KEPT ? T : 1];
+#pragma unroll
+  for (int u = 0; u < SUMS; ++u)
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      if constexpr (KEPT) sum[u][t] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      else shared_sums[(u * T + t) * 32] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+  auto of_sums = [&](int u, int t) -> float4 & {
+    if constexpr (KEPT) return sum[u][t];
+    else return shared_sums[(u * T + t) * 32];
+  };
+
+  const __nv_bfloat16 *Bt = B + col0 + (int64_t)(8 * q) * N;
+  auto column = [&](int k) {  // block columns of the steps from k on
+    const int p = start + k + lane;
+    return p < end ? __ldg(bci + p) : 0;
+  };
+  // Held: 32 of them, or (a member of a team on a longer row) a segment's, and those behind them.
+  const bool whole = steps <= 32;
+  int held = TEAM && !whole ? own(0) : 0;
+  int here = column(held), ahead = whole ? 0 : column(held + (TEAM ? split << log2_length : 32));
+  auto load = [&](F &f, int k) {
+    if (!whole && k != held && (k & (TEAM ? length - 1 : 31)) == 0) {
+      held = k;
+      here = ahead;
+      ahead = column(k + (TEAM ? split << log2_length : 32));
+    }
+    const int bc = __shfl_sync(FULL, here, k - held);
+    const __nv_bfloat16 *b = Bt + (int64_t)bc * BS * N;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      if constexpr (V == 0) load_words<T>(f.slab[r], b + r * N, r & 1, valid);
+      else load_row<T, V>(f.slab[r], b + r * N, valid);
+    }
+    const __nv_bfloat16 *a = bv + (int64_t)(start + k) * (BS * BS) + g * BS + 8 * q;
+#pragma unroll
+    for (int u = 0; u < TILES; ++u) load_row<4, WIDE ? 8 : 1>(f.block[u], a + u * 8 * BS, 8);
+  };
+  auto compute = [&](const F &f) {
+#pragma unroll
+    for (int r = 0; r < 8; r += 4)
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        uint32_t x[4];  // columns 2 t and 2 t + 1 of four rows
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if constexpr (V == 0) x[i] = i & 1 ? __byte_perm(f.slab[r + i][t], f.slab[r + i][t + 1], 0x5432) : f.slab[r + i][t];
+          else x[i] = f.slab[r + i][t];
+        }
+        const uint32_t a0 = __byte_perm(x[0], x[1], 0x5410), a1 = __byte_perm(x[0], x[1], 0x7632);
+        const uint32_t a2 = __byte_perm(x[2], x[3], 0x5410), a3 = __byte_perm(x[2], x[3], 0x7632);
+#pragma unroll
+        for (int u = 0; u < TILES; ++u) mma(acc[u][t], a0, a1, a2, a3, f.block[u][r / 2], f.block[u][r / 2 + 1]);
+      }
+  };
+  // The end of a segment: its sums are added to the block row's.  The members of a team put theirs into shared memory and add up
+  // an exchange's, in order, for their tiles of 8 rows.
+  constexpr int SLOT = TILES * T * 32, AT_ONCE = segments_at_once(T);
+  float4 *slots = reinterpret_cast<float4 *>(handed) + (KEPT ? 0 : MMA_WARPS * SUMS * T * 32) + (warp - member) * (AT_ONCE * SLOT) +
+                  lane;
+  int first = 0;  // segment of the exchange
+  auto meet = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(32 * split) : "memory"); };
+  auto exchange = [&] {
+    meet();
+    const int n = segments - first < AT_ONCE * split ? segments - first : AT_ONCE * split;
+#pragma unroll
+    for (int i = 0; i < SUMS; ++i) {
+      const int u = member + i * split;
+      if (u < TILES) {
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+          float4 w = of_sums(i, t);
+#pragma unroll 4
+          for (int m = 0; m < n; ++m) add4(w, slots[m * SLOT + (u * T + t) * 32]);
+          of_sums(i, t) = w;
+        }
+      }
+    }
+    first += AT_ONCE * split;
+    if (first < segments) meet();
+  };
+  auto end_segment = [&](int segment) {
+#pragma unroll
+    for (int u = 0; u < TILES; ++u)
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        const float4 w = make_float4(acc[u][t][0], acc[u][t][1], acc[u][t][2], acc[u][t][3]);
+        if constexpr (TEAM) slots[(segment - first) * SLOT + (u * T + t) * 32] = w;
+        else add4(of_sums(u, t), w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[u][t][i] = 0.0f;
+      }
+    if (TEAM && segment - first >= (AT_ONCE - 1) * split) exchange();
+  };
+  F f[2];
+  int last = -1;  // segment
+  if (own(0) < steps) load(f[0], own(0));
+  // Segments have an even number of blocks, but for the block row's last one, which ends behind the loop.
+  for (int j = 0; own(j) < steps;) {
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+      if (own(j + 1) < steps) load(f[1 - d], own(j + 1));
+      compute(f[d]);
+      last = own(j) >> log2_length;
+      if (own(++j) >= steps) break;
+      if (d == 1 && (j & (length - 1)) == 0) end_segment(last);
+    }
+  }
+  if (last >= 0) end_segment(last);
+  if constexpr (TEAM)
+    while (first < segments) exchange();
+  if (!active) return;
+#pragma unroll
+  for (int i = 0; i < SUMS; ++i) {
+    const int u = TEAM ? member + i * split : i;
+    if (u >= TILES) break;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      uint32_t w[T];
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        const float4 v = of_sums(i, t);
+        const __nv_bfloat162 h = r == 0 ? __floats2bfloat162_rn(v.x, v.z) : __floats2bfloat162_rn(v.y, v.w);
+        w[t] = *reinterpret_cast<const uint32_t *>(&h);
+      }
+      store_row<T, V ? V : 1>(C + (brow * BS + 8 * u + 2 * q + r) * N + col0, w, valid);
+    }
+  }
+}
+
+template <int BS, int T, int V, bool WIDE, bool TEAM, bool CHAIN>
+__global__ void __launch_bounds__(32 * MMA_WARPS, TEAM ? 2 : mma_ctas(BS, T, V))
+    bsr_spmm_mma_kernel(int64_t units, int tiles, int team_warps, int64_t N, const int32_t *__restrict__ brp,
+                        const int32_t *__restrict__ bci, const __nv_bfloat16 *__restrict__ bv,
+                        const __nv_bfloat16 *__restrict__ B, __nv_bfloat16 *__restrict__ C) {
+  after_previous_kernel();
+  if constexpr (BS == 32 && !CHAIN) add_in_segments<T, V, WIDE, TEAM>(units, tiles, team_warps, N, brp, bci, bv, B, C);
+  else add_in_order<BS, T, V, WIDE, TEAM, CHAIN>(units, tiles, team_warps, N, brp, bci, bv, B, C);
+}
+
 template <int BS, int T, int V, bool WIDE, bool CHAIN = false>
 cudaError_t launch_mma(const BsrSpmmArgs &a, int sm_count, cudaStream_t s) {
   const int64_t tiles = ceil_div(a.n_rhs, 16 * T), units = a.rows / BS * tiles;
   // Warps of a block row: more while the GPU has no more than ten per SM and each has a step (16 x 16, N = 8, us with 1, 2, 4 and
   // 8 warps: 80 block rows of 30 9.9, 7.0, 4.9, 3.9; 300 of 20 8.3, 5.4, 4.4, 4.8; 600 of 12 6.6, 4.8, 5.4, 6.1; 2,000 of 20 11.0,
   // 11.4, 13.9, 17.5).  Blocks of 32 x 32 have four tiles of rows for four adding warps, up to 20 warps per SM, and four others that
-  // only load, up to 18 (1, 4 and 8 warps: 300 of 20, N = 8 12.2, 9.7, 7.9; 80 of 30, N = 48 19.8, 13.6, 11.1; 300 of 20, N = 48
+  // only load, up to 18 (on narrow B before segments, 1, 4 and 8 warps: 300 of 20, N = 8 12.2, 9.7, 7.9; 80 of 30, N = 48 19.8, 13.6, 11.1; 300 of 20, N = 48
   // 18.0, 16.6, 18.9; 382 of 27, N = 29 31.3, 20.1, -; 1,000 of 20, N = 48 23.4, 40.7, 43.0).
   int split = 1;
-  for (int more = BS == 32 ? 4 : 2; more <= MMA_WARPS; more *= 2)
+  // Segments of 32 x 32: more while all are ten per SM and each has two blocks (with up to 16 per SM 1.02 times the time).
+  if (BS == 32 && !CHAIN) {
+    while (split < MMA_WARPS && units * split < 10 * (int64_t)sm_count && a.nnzb * BS >= split * 2 * a.rows) split *= 2;
+  }
+  for (int more = BS == 32 ? 4 : 2; more <= MMA_WARPS && (BS != 32 || CHAIN); more *= 2)
     if (units * more <= (int64_t)sm_count * (BS != 32 ? 10 : more == 4 ? 20 : 18) && a.nnzb * BS * BS >= more * 8 * a.rows) split = more;
   unsigned grid = 0;
   if (!grid_dim(ceil_div(units * split, MMA_WARPS), &grid)) return cudaErrorInvalidConfiguration;
-  const size_t smem = split > 1 ? MMA_WARPS * team_steps(BS, T) * step_words(BS, T) * 32 * 4 : 0;  // at most 48 KB
+  const size_t smem = BS == 32 && !CHAIN ? segment_smem(T, split > 1)  // at most 48 KB
+                      : split > 1 ? MMA_WARPS * team_steps(BS, T) * step_words(BS, T) * 32 * 4 : 0;
   launch_chained(split > 1 ? bsr_spmm_mma_kernel<BS, T, V, WIDE, true, CHAIN> : bsr_spmm_mma_kernel<BS, T, V, WIDE, false, CHAIN>,
                  grid, 32 * MMA_WARPS, smem, s, units, (int)tiles, split, a.n_rhs, a.block_row_ptr, a.block_col_idx,
                  static_cast<const __nv_bfloat16 *>(a.block_values), static_cast<const __nv_bfloat16 *>(a.B),
@@ -321,7 +524,7 @@ cudaError_t launch_mma(const BsrSpmmArgs &a, int sm_count, cudaStream_t s) {
 
 template <int BS, int T, int V>
 cudaError_t launch_wide(const BsrSpmmArgs &a, int sm_count, cudaStream_t s) {
-  const bool wide = reinterpret_cast<uintptr_t>(a.block_values) % 8 == 0;
+  const bool wide = reinterpret_cast<uintptr_t>(a.block_values) % (BS == 32 ? 16 : 8) == 0;
   return wide ? launch_mma<BS, T, V, true>(a, sm_count, s) : launch_mma<BS, T, V, false>(a, sm_count, s);
 }
 
