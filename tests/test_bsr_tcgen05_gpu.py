@@ -152,3 +152,17 @@ def test_line_between_the_kernels(ctx, bs, per_sm, per, n, here):
         assert len(names) == 1 and names[0].startswith("bsr_spmm_tcgen05_kernel" if here else "bsr_spmm_mma_kernel")
     assert ctx.device_status() == 0
     assert_bf16_close(C, brp.numpy(), bci.numpy(), values.view(torch.uint16).numpy(), B.view(torch.uint16).numpy(), bs)
+
+
+@pytest.mark.parametrize("bs,cols,per,here", [(16, 2605, 4, True), (16, 2604, 4, False), (8, 6741, 8, True), (8, 6740, 8, False),
+                                              (8, 5515, 9, True), (8, 5514, 9, False)])
+def test_line_by_the_size_of_b(ctx, bs, cols, per, here):
+    brows, n = 160, 408
+    gen = torch.Generator().manual_seed(cols)
+    brp = torch.arange(0, per * brows + 1, per, dtype=torch.int32)
+    bci = torch.randint(cols, (per * brows,), generator=gen, dtype=torch.int32)
+    values, B = W.dense_normal((per * brows * bs, bs), seed=bs).view(-1), W.dense_normal((cols * bs, n), seed=n)
+    C, names = launched(lambda: ctx.bsr_spmm("", brp.cuda(), bci.cuda(), values.cuda(), B.cuda(), bs))
+    if names is not None:
+        assert len(names) == 1 and names[0].startswith("bsr_spmm_tcgen05_kernel" if here else "bsr_spmm_mma_kernel")
+    assert_bf16_close(C, brp.numpy(), bci.numpy(), values.view(torch.uint16).numpy(), B.view(torch.uint16).numpy(), bs)
