@@ -11,8 +11,8 @@
 //
 // Every output is added up over its block row's steps in storage order, so that a part of a matrix has the bits of the whole,
 // whichever kernel takes either: as one chain of MMAs or (bsr_chain_sums) as f32 sums of steps or, 32 x 32 blocks, of segments of
-// two, four or eight blocks by the block row's length, each of which is a chain of its own.  Where block rows are few, a team of up to
-// eight warps shares one all the same.  Its members take segments in turn and add up each other's sums, in order, for their tiles of
+// two, four or eight blocks by the block row's length, each of which is a chain of its own.  Where block rows are few, a team of
+// up to eight warps shares one all the same.  Its members take segments in turn and add up each other's sums, in order, for their tiles of
 // 8 rows; or they load the steps in turn and hand them over in shared memory, and each of the first members adds up its share of
 // the block row's rows.
 //
@@ -501,11 +501,11 @@ cudaError_t launch_mma(const BsrSpmmArgs &a, int sm_count, cudaStream_t s) {
   const int64_t tiles = ceil_div(a.n_rhs, 16 * T), units = a.rows / BS * tiles;
   // Warps of a block row: more while the GPU has no more than ten per SM and each has a step (16 x 16, N = 8, us with 1, 2, 4 and
   // 8 warps: 80 block rows of 30 9.9, 7.0, 4.9, 3.9; 300 of 20 8.3, 5.4, 4.4, 4.8; 600 of 12 6.6, 4.8, 5.4, 6.1; 2,000 of 20 11.0,
-  // 11.4, 13.9, 17.5).  Blocks of 32 x 32 have four tiles of rows for four adding warps, up to 20 warps per SM, and four others that
-  // only load, up to 18 (on narrow B before segments, 1, 4 and 8 warps: 300 of 20, N = 8 12.2, 9.7, 7.9; 80 of 30, N = 48 19.8, 13.6, 11.1; 300 of 20, N = 48
-  // 18.0, 16.6, 18.9; 382 of 27, N = 29 31.3, 20.1, -; 1,000 of 20, N = 48 23.4, 40.7, 43.0).
+  // 11.4, 13.9, 17.5).  Blocks of 32 x 32 have four tiles of rows for four adding warps, up to 20 warps per SM, and four others
+  // that only load, up to 18 (measured on narrow B, which has segments since, 1, 4 and 8 warps: 300 of 20, N = 8 12.2, 9.7, 7.9; 80 of
+  // 30, N = 48 19.8, 13.6, 11.1; 300 of 20, N = 48 18.0, 16.6, 18.9; 382 of 27, N = 29 31.3, 20.1, -; 1,000 of 20, N = 48 23.4, 40.7,
+  // 43.0).  With segments twice as many while there are fewer than ten per SM and each has two blocks (16 per SM: 1.02 times the time).
   int split = 1;
-  // Segments of 32 x 32: more while all are ten per SM and each has two blocks (with up to 16 per SM 1.02 times the time).
   if (BS == 32 && !CHAIN) {
     while (split < MMA_WARPS && units * split < 10 * (int64_t)sm_count && a.nnzb * BS >= split * 2 * a.rows) split *= 2;
   }

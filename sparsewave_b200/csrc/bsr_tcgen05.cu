@@ -502,8 +502,8 @@ bool bsr_tcgen05_supported(const BsrSpmmArgs &a) {
 //   8, N = 512 78.1, 48.3; 1,200 of 12, N = 256 14.1, 11.9; 600 of 6 6.4, 8.3); of tiles four fifths full, from 12 a row with whole
 //   groups (2,904 of 15, N = 448 52.5, 39.4; but of 9, N = 384 1.08 times), from 27 with other multiples of 32 bytes (3,350 of 48,
 //   N = 240 91.5, 73.6; 2,002 of 54, N = 416 105, 90; 311 of 28, N = 496 16.7, 14.2; but of 18, N = 304 1.12 times).
-//   16 x 16 and 8 x 8 on tiles three quarters full, where B outgrows the part of L2 that is near an SM, which the copies hide and the
-//   loads do not: from 34 MB (16 x 16, blocks of 4 and 16 a row: N = 408 30 MB 1.07 and 0.82 times the time, 43 MB 0.78 and 0.75;
+//   16 x 16 and 8 x 8 on tiles three quarters full, where B is large (with C it then outgrows the half of L2 on an SM's die, whose
+//   longer way the copies would hide and the loads not; the counters were not read): from 34 MB (16 x 16, blocks of 4 and 16 a row: N = 408 30 MB 1.07 and 0.82 times the time, 43 MB 0.78 and 0.75;
 //   N = 344 34 MB 1.03 and 0.86; N = 504 53 MB 56.9 -> 42.2 us and 150 -> 106) and 44 MB, from nine blocks a row 36 MB (8 x 8:
 //   N = 408 30 MB 1.40 and 1.10, 45 MB 1.02 and 0.89; N = 504 38 MB 1.05 and 0.86, 56 MB 0.88 and 0.79).
 bool bsr_tcgen05_pays(const BsrSpmmArgs &a, int sm_count) {
